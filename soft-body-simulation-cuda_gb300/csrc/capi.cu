@@ -59,10 +59,10 @@ struct pdgb_engine {
     // Cholesky factor
     CholFactor chol;
     int chol_ordering = -1;
+    double chol_level_entries = -1.0;
     float chol_dt = 0.f, chol_pw = -1.f;
-    DBuf<int> ch_fwd, ch_bwd, ch_rows, ch_body_level, ch_body_order, ch_fwdb, ch_bwdb, ch_fwds, ch_bwds, ch_tiny,
-        ch_zstage;
-    DBuf<float4> ch_zbuf;
+    DBuf<int> ch_fwd, ch_bwd, ch_rows, ch_body_level, ch_body_order, ch_blocks, ch_small, ch_tiny;
+    DBuf<float4> y2;  // second y buffer: solves alternate, each clears the other one's
     DBuf<int4> ch_levels;
     DBuf<SolveLevel> ch_step_lv;  // per-level item ranges on the device (persistent solve)
     // distributed-shared-memory solve of a single body (when it fits)
@@ -298,8 +298,7 @@ void record_chol_step(pdgb_engine* e) {
     launch_begin(ba, s);
     const LocalArgs la = local_args(e, &st->done);
     CholArgs ca{e->ch_fwd.p, e->ch_bwd.p, e->ch_rows.p, e->ch_mval.p, e->ch_levels.p, e->ch_body_level.p,
-                e->ch_body_order.p, e->b.p, e->y.p, e->sn.p, &st->done, e->ch_fwdb.p, e->ch_bwdb.p,
-                e->ch_fwds.p, e->ch_bwds.p, e->ch_tiny.p, e->ch_zstage.p, e->ch_zbuf.p};
+                e->ch_body_order.p, e->b.p, e->y.p, e->sn.p, &st->done, e->ch_blocks.p, e->ch_small.p, e->ch_tiny.p};
     CholVertexArgs cv{};
     cv.nv = e->nv;
     cv.tol = use_tol ? e->prm.tol : 0.f;
@@ -317,34 +316,51 @@ void record_chol_step(pdgb_engine* e) {
     cv.sc = scene_args(e);
     const bool drag_rhs = cv.sc.drag_w && cv.sc.drag_rhs;
     const int refine = e->nbodies == 1 ? e->prm.refine_steps : 0;
-    CholArgs cd = ca;  // refinement solves write the correction into dx
-    cd.x = e->dx.p;
     RefineArgs ra{e->nv, e->k_rowptr.p, e->k_colind.p, e->k_val.p, e->bsave.p, e->sn.p, e->b.p, e->y.p,
                   e->dx.p, e->sn.p, &st->done};
-    auto solve = [&](const CholArgs& args) {
+    // Per-level launches without the convergence test: each solve's backward
+    // pass clears the y buffer of the next solve (two alternate) and the last
+    // solve of an iteration resets b, so that no vertex kernel runs between
+    // iterations.  The other schedules, and the test (which needs every
+    // vertex's change), keep the kernel and one y.
+    const bool fused = e->solve_mode == PDGB_SOLVE_LEVELS && !use_tol;
+    float4* ybuf[2] = {e->y.p, fused ? e->y2.p : e->y.p};
+    int parity = 0;  // y buffer of the next solve; zero when the step begins
+    auto solve = [&](float4* x, bool last) {
+        CholArgs args = ca;
+        args.x = x;
+        args.y = ybuf[parity];
         if (e->solve_mode == PDGB_SOLVE_CTA) launch_chol_solve_cta(args, e->nbodies, s);
         else if (e->solve_mode == PDGB_SOLVE_CLUSTER) launch_chol_solve_cluster(args, e->nbodies, s);
         else if (e->solve_mode == PDGB_SOLVE_DSM) launch_chol_solve_dsm(args, dsm_args(e), e->dsm.smem_bytes, s);
         else if (e->solve_mode == PDGB_SOLVE_PERSISTENT)
             launch_chol_solve_persistent(args, e->ch_step_lv.p, (int)e->chol.step_levels.size(), &st->bar,
                                          kPersistSpinLimit, s);
-        else launch_chol_solve_levels(args, e->chol.step_levels, s);
+        else {
+            ResetArgs reset{};
+            if (fused)
+                reset = ResetArgs{e->nv, ybuf[parity ^ 1], last ? e->b.p : nullptr, e->base.p, e->coef.p, e->pin_rhs.p};
+            launch_chol_solve_levels(args, e->chol.step_levels, s, reset);
+            if (fused) parity ^= 1;
+        }
     };
     for (int i = 0; i < n; ++i) {
         record_local(e, la, false, i);
         if (drag_rhs) launch_drag_rhs(e->nv, cv.sc, e->base.p, e->b.p, &st->done, s);
         if (refine > 0) launch_copy_rhs(e->nv, e->b.p, e->bsave.p, &st->done, s);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i], s, cudaEventRecordExternal));
-        solve(ca);
+        solve(e->sn.p, refine == 0);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i + 1], s, cudaEventRecordExternal));
         for (int r = 0; r < refine; ++r) {
+            ra.y = ybuf[parity];
             launch_refine_residual(ra, s);
-            solve(cd);
+            solve(e->dx.p, r + 1 == refine);  // the correction
             launch_refine_update(ra, s);
         }
         cv.iteration = i;
-        launch_chol_vertex(cv, s);
+        if (!fused) launch_chol_vertex(cv, s);
     }
+    cv.y = ybuf[fused ? parity ^ 1 : 0];  // the last solve's: both are zero for the next step
     launch_chol_finish(cv, s);
 }
 
@@ -425,7 +441,10 @@ int choose_solve_mode(const pdgb_engine* e) {
 void prepare_cholesky(pdgb_engine* e) {
     // the distributed-shared-memory solve stages the factor from host memory
     const int dev = e->solve_req == PDGB_SOLVE_DSM ? PDGB_FACTOR_HOST : e->factor_req;
-    if (e->chol_ordering == e->ordering && e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight &&
+    // ... and its vectors and blocks share a cluster's shared memory: there
+    // every stored entry counts and a level is only a cluster barrier
+    const double level_entries = e->solve_req == PDGB_SOLVE_DSM ? kDsmLevelEntries : kLevelEntries;
+    if (level_entries == e->chol_level_entries && e->chol_ordering == e->ordering && e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight &&
         e->chol.n == e->nv && e->factor_dev == dev) {
         e->solve_mode = choose_solve_mode(e);
         return;  // the system matrix depends only on the mesh, dt and the pin weight
@@ -447,7 +466,7 @@ void prepare_cholesky(pdgb_engine* e) {
                                e->L.dminv_d.data(), e->L.coef_d.data(), mdt2, e->ordering, xyz.data(), e->chol,
                                gpu);
     } else {
-        cholesky_factor(K, e->ordering, xyz.data(), e->chol, kBwdChunkRows, gpu);
+        cholesky_factor(K, e->ordering, xyz.data(), e->chol, gpu, true, level_entries);
     }
     cudaStream_t s = e->stream;
     const CholFactor& f = e->chol;
@@ -466,13 +485,11 @@ void prepare_cholesky(pdgb_engine* e) {
     e->factor_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     e->ch_fwd.upload(f.fwd_items, s);
     e->ch_bwd.upload(f.bwd_items, s);
-    e->ch_fwdb.upload(f.fwd_blocks, s);
-    e->ch_bwdb.upload(f.bwd_blocks, s);
-    e->ch_fwds.upload(f.fwd_small, s);
-    e->ch_bwds.upload(f.bwd_small, s);
+    e->ch_blocks.upload(f.blocks, s);
+    e->ch_small.upload(f.small, s);
     e->ch_tiny.upload(f.tiny, s);
-    e->ch_zstage.upload(f.zstage, s);
-    e->ch_zbuf.alloc((size_t)std::max<int64_t>(f.zrows, 1));
+    e->y2.alloc(e->nv);
+    PDGB_CUDA_TRY(cudaMemsetAsync(e->y2.p, 0, (size_t)e->nv * sizeof(float4), s));
     e->ch_rows.upload(f.rows, s);
     std::vector<int4> lv(f.levels.size());
     for (size_t i = 0; i < lv.size(); ++i)
@@ -505,6 +522,7 @@ void prepare_cholesky(pdgb_engine* e) {
         }
     }
     e->solve_mode = choose_solve_mode(e);
+    e->chol_level_entries = level_entries;
     e->chol_ordering = e->ordering;
     e->chol_dt = e->prm.dt;
     e->chol_pw = e->prm.positional_weight;
@@ -517,6 +535,7 @@ void prepare(pdgb_engine* e) {
     e->pin_rhs.upload(e->L.pin_rhs, e->stream);
     if (e->prm.solver == PDGB_SOLVER_CHOLESKY) prepare_cholesky(e);
     PDGB_CUDA_TRY(cudaMemsetAsync(e->y.p, 0, (size_t)e->nv * sizeof(float4), e->stream));
+    if (e->y2.p) PDGB_CUDA_TRY(cudaMemsetAsync(e->y2.p, 0, (size_t)e->nv * sizeof(float4), e->stream));
     // resident CTAs of the pipelined local step for the current tile cut
     // (queried here, not while the step graph is being captured)
     e->pipe_grid = e->local_kernel == PDGB_LOCAL_PIPELINED ? local_pipe_grid(e->L.ntiles, e->L.max_patch) : 0;
@@ -1537,13 +1556,8 @@ namespace {
 int solve_launches(const pdgb_engine* e) {
     if (e->solve_mode != PDGB_SOLVE_LEVELS) return 1;  // PERSISTENT: one launch (and a barrier reset)
     int n = 0;
-    for (const SolveLevel& v : e->chol.step_levels) {
-        const int fb = v.fwdb_end - v.fwdb_begin, fw = v.fwdw_end - v.fwdw_begin;
-        const int bb = v.bwdb_end - v.bwdb_begin, bw = v.bwdw_end - v.bwdw_begin;
-        n += mix_level(fb, fw) ? 1 : (fb > 0) + (fw > 0);
-        n += mix_level(bb, bw) ? 1 : (bb > 0) + (bw > 0);
-        n += 2 * (v.tiny_end > v.tiny_begin) + (v.zst_end > v.zst_begin);
-    }
+    for (const SolveLevel& v : e->chol.step_levels)
+        n += 2 * (v.blk_end > v.blk_begin || v.sml_end > v.sml_begin || v.tiny_end > v.tiny_begin);
     return n;
 }
 }  // namespace

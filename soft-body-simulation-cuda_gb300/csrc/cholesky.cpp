@@ -385,6 +385,78 @@ std::vector<int> postorder(const std::vector<int>& parent) {
     return post;
 }
 
+// Supernode amalgamation.  fk, fm, fpar: pivots, rows and parent of each
+// fundamental supernode, children before parents.  Returns the root of the
+// merged supernode that each one joins (itself for a root).
+//
+// The solve pays for every level of the supernodal tree (a chain of
+// dependent launches, however little they do) and for every stored entry of
+// the blocks M_s.  Supernodes are merged by the size of their subtrees:
+// those whose subtree's columns fall between the same two thresholds t,
+// t r, t r^2, ... are one supernode with their parent where the parent's do
+// too, siblings included.  A merged supernode has its root's off-diagonal
+// rows, so k columns and `off` rows below them store k (k + 1) / 2 + k off
+// entries.  Bisection-like trees lose most of their levels for few explicit
+// zeros that way, because a level of the merged tree spans a factor r of
+// subtree sizes: the 40^3 grid has 13 levels and 31.2 M entries when each
+// supernode is only merged with the last child before it (at most 2,048 or a
+// quarter added zeros), and 8 levels and 31.4 M, or 5 and 38.9 M, this way.
+// Of the grid of (t, r) the cheapest is taken, a level costing level_entries
+// entries and the one-time factorisation kEntriesPerFlop entries per
+// multiply-add (spread over the solves of about a hundred steps).
+std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& fm, const std::vector<int>& fpar,
+                            double level_entries) {
+    constexpr double kEntriesPerFlop = 1e-3;
+    const int nf = (int)fk.size();
+    std::vector<int> sub(fk);  // columns of the subtree
+    int n = 0;
+    for (int s = 0; s < nf; ++s) {
+        if (fpar[s] >= 0) sub[fpar[s]] += sub[s];
+        n += fk[s];
+    }
+    std::vector<int> root(nf), best_root(nf), band(n + 1), height(nf);
+    std::vector<int64_t> cols(nf);
+    double best = -1.0;
+    for (int t : {8, 16, 24, 32, 48, 96, 192})
+        for (double r : {2.0, 3.0, 4.0, 6.0, 10.0, 16.0, 32.0}) {
+            double top = t;
+            for (int c = 0, q = 0; c <= n; ++c) {
+                while ((double)c > top) {
+                    top *= r;
+                    ++q;
+                }
+                band[c] = q;
+            }
+            std::fill(cols.begin(), cols.end(), 0);
+            std::fill(height.begin(), height.end(), 0);
+            for (int s = nf - 1; s >= 0; --s) {
+                const int p = fpar[s];
+                root[s] = p >= 0 && band[sub[s]] == band[sub[p]] ? root[p] : s;
+                cols[root[s]] += fk[s];
+            }
+            int levels = 0;
+            double entries = 0.0, flops = 0.0;
+            for (int s = 0; s < nf; ++s) {  // every descendant comes first
+                if (root[s] != s) continue;
+                const double k = (double)cols[s], off = (double)(fm[s] - fk[s]);
+                entries += k * (0.5 * (k + 1.0) + off);
+                flops += k * (k + off) * (k + off);
+                levels = std::max(levels, height[s] + 1);
+                if (fpar[s] >= 0) {
+                    int& h = height[root[fpar[s]]];
+                    h = std::max(h, height[s] + 1);
+                }
+            }
+            const double cost = level_entries * levels + entries + kEntriesPerFlop * flops;
+            if (best < 0.0 || cost < best) {
+                best = cost;
+                best_root.swap(root);
+            }
+            if (top > n && t >= n) break;  // one band: every r merges the whole tree
+        }
+    return best_root;
+}
+
 // Dense lower-triangular m x m front (column major, leading dimension m):
 // factor the first k columns in place (right-looking, blocked).
 bool partial_cholesky(double* F, int m, int k) {
@@ -425,8 +497,8 @@ bool partial_cholesky(double* F, int m, int k) {
 
 }  // namespace
 
-void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFactor& out, int bwd_chunk_rows,
-                     bool gpu_numeric, bool finish_plan, int amalgamation) {
+void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFactor& out,
+                     bool gpu_numeric, bool finish_plan, double level_entries) {
     const int n = K.n;
     out = CholFactor();
     out.n = n;
@@ -443,13 +515,12 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
         perm0.swap(perm);
         for (int k = 0; k < n; ++k) iperm[perm0[k]] = k;
     }
-    const std::vector<int>& perm = perm0;
-    std::vector<int> parent = etree(K, perm, iperm);
+    std::vector<int> parent = etree(K, perm0, iperm);
     // ---- column counts via row subtrees (ereach)
-    std::vector<int> colcount(n, 1), wmark(n, -1), stk(n);
+    std::vector<int> colcount(n, 1), wmark(n, -1);
     for (int k = 0; k < n; ++k) {
         wmark[k] = k;
-        const int v = perm[k];
+        const int v = perm0[k];
         for (int64_t e = K.p[v]; e < K.p[v + 1]; ++e) {
             int i = iperm[K.i[e]];
             if (i >= k) continue;
@@ -471,58 +542,45 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
         const bool cont = j > 0 && parent[j - 1] == j && colcount[j - 1] == colcount[j] + 1 && nchild[j] == 1;
         if (!cont) sfirst.push_back(j);
     }
-    // ---- relaxed amalgamation: merge a supernode into its parent when its
-    // columns immediately precede the parent's (it is the parent's last child
-    // in postorder) and the explicit zeros stay small.  The merged block has
-    // the parent's off-diagonal rows, so k = k_s + k_p and m = k_s + m_p.
-    // This removes the 1-3 column supernodes that break chains at the top of
-    // AMD trees (each one a level of the solve) and most leaf singletons.
-    // kAmalgChain: at most 2,048 more zeros, or at most a quarter of the
-    // merged block.  The engine's solve is bound by its chain of levels more
-    // than by the factor's bytes: against kAmalgBytes (256 zeros or an
-    // eighth) this stores 18 % more entries on the 512-body batch and 21 %
-    // more on the 40^3 cube, and solves 12 % and 4 % faster (11 levels
-    // instead of 14, 14 instead of 16).  kAmalgBytes serves the serving
-    // step, whose many requests' solves together are bound by bytes.
-    {
+    // ---- amalgamation, then the columns of every merged supernode made
+    // contiguous: supernodes in the order of their roots, columns in
+    // postorder within one.  That is another topological order of the same
+    // elimination tree, so the fill (and every column count) stays.
+    std::vector<int> permv(perm0);
+    if (ordering != 2) {
         const int nf = (int)sfirst.size();
         sfirst.push_back(n);
-        std::vector<long long> bk(nf), bm(nf), btrue(nf);
-        for (int s = 0; s < nf; ++s) {
-            bk[s] = sfirst[s + 1] - sfirst[s];
-            bm[s] = colcount[sfirst[s]];
-            long long t = 0;
-            for (int j = sfirst[s]; j < sfirst[s + 1]; ++j) t += colcount[j];
-            btrue[s] = t;
-        }
-        std::vector<int> col2f(n);
+        std::vector<int> col2f(n), fk(nf), fm(nf), fpar(nf, -1);
         for (int s = 0; s < nf; ++s)
             for (int j = sfirst[s]; j < sfirst[s + 1]; ++j) col2f[j] = s;
-        // merged[s] = true if block s was merged into the following block
-        std::vector<char> merged(nf, 0);
-        auto stored = [](long long k, long long m) { return k * m - k * (k - 1) / 2; };
-        for (int s = 0; s + 1 < nf; ++s) {
-            const int last = sfirst[s + 1] - 1;
-            if (parent[last] != sfirst[s + 1]) continue;  // parent block must start right after
-            const int p = s + 1;
-            const long long k = bk[s] + bk[p], m = bk[s] + bm[p];
-            const long long tr = btrue[s] + btrue[p];
-            const long long zeros = stored(k, m) - tr;
-            const long long added = zeros - (stored(bk[s], bm[s]) - btrue[s]) - (stored(bk[p], bm[p]) - btrue[p]);
-            const bool take = amalgamation == kAmalgChain ? (added <= 2048 || zeros * 4 <= stored(k, m))
-                                                          : (added <= 256 || zeros * 8 <= stored(k, m));
-            if (take) {
-                merged[s] = 1;
-                bk[p] = k;
-                bm[p] = m;
-                btrue[p] = tr;
-            }
+        for (int s = 0; s < nf; ++s) {
+            fk[s] = sfirst[s + 1] - sfirst[s];
+            fm[s] = colcount[sfirst[s]];
+            const int up = parent[sfirst[s + 1] - 1];
+            if (up >= 0) fpar[s] = col2f[up];
         }
+        const std::vector<int> root = amalgamate(fk, fm, fpar, level_entries);
+        std::vector<int> start(nf + 1, 0);  // first column of the supernode rooted at s (0 columns elsewhere)
+        for (int s = 0; s < nf; ++s) start[root[s] + 1] += fk[s];
         std::vector<int> sf;
+        for (int s = 0; s < nf; ++s) {
+            if (root[s] == s) sf.push_back(start[s]);
+            start[s + 1] += start[s];
+        }
+        std::vector<int> newpos(n), par2(n), cc2(n);
         for (int s = 0; s < nf; ++s)
-            if (s == 0 || !merged[s - 1]) sf.push_back(sfirst[s]);
+            for (int j = sfirst[s]; j < sfirst[s + 1]; ++j) newpos[j] = start[root[s]]++;
+        for (int j = 0; j < n; ++j) {
+            permv[newpos[j]] = perm0[j];
+            par2[newpos[j]] = parent[j] >= 0 ? newpos[parent[j]] : -1;
+            cc2[newpos[j]] = colcount[j];
+        }
+        for (int k = 0; k < n; ++k) iperm[permv[k]] = k;
+        parent.swap(par2);
+        colcount.swap(cc2);
         sfirst.swap(sf);
     }
+    const std::vector<int>& perm = permv;
     if (ordering == 2) sfirst.assign(1, 0);  // one dense supernode: every pivot, every row
     const int ns = (int)sfirst.size();
     sfirst.push_back(n);
@@ -717,12 +775,9 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
         SolveLevel lv;
         lv.fwd_begin = (int)(out.fwd_items.size() / kItemInts);
         lv.bwd_begin = (int)(out.bwd_items.size() / kItemInts);
-        lv.fwdb_begin = (int)(out.fwd_blocks.size() / kItemInts);
-        lv.bwdb_begin = (int)(out.bwd_blocks.size() / kItemInts);
-        lv.fwdw_begin = (int)(out.fwd_small.size() / kItemInts);
-        lv.bwdw_begin = (int)(out.bwd_small.size() / kItemInts);
+        lv.blk_begin = (int)(out.blocks.size() / kItemInts);
+        lv.sml_begin = (int)(out.small.size() / kItemInts);
         lv.tiny_begin = (int)(out.tiny.size() / kItemInts);
-        lv.zst_begin = (int)(out.zstage.size() / kItemInts);
         for (int s : bylevel[L]) {
             const int k = out.sk[s], m = out.sm[s];
             const int64_t mo = out.moff[s];
@@ -735,47 +790,24 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
                                          {lo, hi, out.roff[s], m, k, r0, c0, std::min(cmax, c0 + kFwdItemCols)});
             }
             for (int c = 0; c < k; ++c) out.bwd_items.insert(out.bwd_items.end(), {lo, hi, out.roff[s], m, k, c, 0, 0});
-            if (k <= kTinyCols && m <= kTinyRows) {  // tiny: one thread per supernode (per-level launches)
+            if (k == 1 && m <= kTinyRows) {
                 out.tiny.insert(out.tiny.end(), {lo, hi, out.roff[s], m, k, 0, 0, 0});
-                continue;
-            }
-            if (m < kBlockMinRows) {  // small: the warp items, again, for the per-level launches
-                for (int r0 = 0; r0 < m; r0 += kFwdItemRows) {
-                    const int cmax = std::min(k, r0 + kFwdItemRows);
-                    for (int c0 = 0; c0 < cmax; c0 += kFwdItemCols)
-                        out.fwd_small.insert(out.fwd_small.end(),
-                                             {lo, hi, out.roff[s], m, k, r0, c0, std::min(cmax, c0 + kFwdItemCols)});
+            } else if (m < kBlockMinRows && k <= kSmallCols) {
+                out.small.insert(out.small.end(), {lo, hi, out.roff[s], m, k, 0, 0, 0});
+            } else {
+                for (int r0 = 0; r0 < m; r0 += kTileRows) {
+                    const int cmax = std::min(k, r0 + kTileRows);  // rows >= c only
+                    for (int c0 = 0; c0 < cmax; c0 += kTileCols)
+                        out.blocks.insert(out.blocks.end(),
+                                          {lo, hi, out.roff[s], m, k, r0, c0, std::min(cmax, c0 + kTileCols)});
                 }
-                for (int c = 0; c < k; ++c) out.bwd_small.insert(out.bwd_small.end(), {lo, hi, out.roff[s], m, k, c, 0, 0});
-                continue;
-            }
-            for (int r0 = 0; r0 < m; r0 += kFwdBlockRows) {
-                const int cmax = std::min(k, r0 + kFwdBlockRows);
-                for (int c0 = 0; c0 < cmax; c0 += kFwdBlockCols)
-                    out.fwd_blocks.insert(out.fwd_blocks.end(),
-                                          {lo, hi, out.roff[s], m, k, r0, c0, std::min(cmax, c0 + kFwdBlockCols)});
-            }
-            const int zoff = (int)out.zrows;
-            out.zrows += m;
-            const int chunk = bwd_chunk_rows > 0 ? bwd_chunk_rows : m;
-            const int split = chunk < m ? 1 : 0;  // columns split into row chunks: x is accumulated
-            for (int r0 = 0; r0 < m; r0 += kStageRows)
-                out.zstage.insert(out.zstage.end(), {lo, hi, out.roff[s], m, k, r0, split, zoff});
-            for (int c0 = 0; c0 < k; c0 += kBwdBlockCols) {
-                const int cpack = (int)((unsigned)c0 | ((unsigned)(std::min(k, c0 + kBwdBlockCols) - c0) << kBwdColShift));
-                for (int r0 = c0 - c0 % chunk; r0 < m; r0 += chunk)  // rows >= c0 only
-                    out.bwd_blocks.insert(out.bwd_blocks.end(),
-                                          {lo, hi, out.roff[s], m, r0, cpack, std::min(m, r0 + chunk), zoff});
             }
         }
         lv.fwd_end = (int)(out.fwd_items.size() / kItemInts);
         lv.bwd_end = (int)(out.bwd_items.size() / kItemInts);
-        lv.fwdb_end = (int)(out.fwd_blocks.size() / kItemInts);
-        lv.bwdb_end = (int)(out.bwd_blocks.size() / kItemInts);
-        lv.fwdw_end = (int)(out.fwd_small.size() / kItemInts);
-        lv.bwdw_end = (int)(out.bwd_small.size() / kItemInts);
+        lv.blk_end = (int)(out.blocks.size() / kItemInts);
+        lv.sml_end = (int)(out.small.size() / kItemInts);
         lv.tiny_end = (int)(out.tiny.size() / kItemInts);
-        lv.zst_end = (int)(out.zstage.size() / kItemInts);
         out.levels[L] = lv;
     }
     out.body_level = {0, nl};
@@ -898,6 +930,11 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
         return tstart[a + 1] - tstart[a] > tstart[b + 1] - tstart[b];
     });
     std::vector<int> failed(nbodies, 0);
+    // a level is one chain of launches for all bodies: each pays a share of
+    // it, by its expected factor size
+    double weight = 0.0;
+    auto factor_size = [](int nv) { return std::pow((double)nv, 1.58); };
+    for (int b = 0; b < nbodies; ++b) weight += factor_size(vstart[b + 1] - vstart[b]);
 #pragma omp parallel for schedule(dynamic, 1)
     for (int q = 0; q < nbodies; ++q) {
         const int b = order[q];
@@ -907,7 +944,8 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
             for (size_t i = 0; i < lt.size(); ++i) lt[i] = tets4[4 * (size_t)t0 + i] - (uint32_t)v0;
             std::vector<double> md(mdt2.begin() + v0, mdt2.begin() + v0 + nvb);
             SparseSym Kb = assemble_system(nvb, ntb, lt.data(), dminv + 9 * (size_t)t0, coef + t0, md);
-            cholesky_factor(Kb, ordering, xyz ? xyz + 3 * (size_t)v0 : nullptr, fs[b], 0, gpu_numeric, false);
+            cholesky_factor(Kb, ordering, xyz ? xyz + 3 * (size_t)v0 : nullptr, fs[b], gpu_numeric, false,
+                            kLevelEntries * factor_size(nvb) / weight);
         } catch (const Error& e) {
             failed[b] = e.status;
         } catch (...) {
@@ -920,11 +958,11 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
                                        (failed[b] == PDGB_ERR_NOT_SPD ? "not positive definite" : "error") + ")"};
     out = CholFactor();
     out.n = vstart[nbodies];
-    int64_t mbase = 0, rbase = 0, zbase = 0;
+    int64_t mbase = 0, rbase = 0;
     int sbase = 0;
     out.body_level.assign(1, 0);
-    // per-level buckets of the block / small items of all bodies
-    std::vector<std::vector<int>> bfb, bfw, bbb, bbw, btn, bzs;
+    // per-level buckets of the items of all bodies
+    std::vector<std::vector<int>> bbl, bsm, btn;
     for (int b = 0; b < nbodies; ++b) {
         CholFactor& f = fs[b];
         const int v0 = vstart[b];
@@ -959,15 +997,14 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
             P.rel.insert(P.rel.end(), Q.rel.begin(), Q.rel.end());
         }
         for (int r : f.rows) out.rows.push_back(r + v0);
-        auto shift = [&](std::vector<int>& dst, const std::vector<int>& src, bool zfield = false) {
+        auto shift = [&](std::vector<int>& dst, const std::vector<int>& src) {
             const int base_item = (int)(dst.size() / kItemInts);
             for (size_t i = 0; i < src.size(); i += kItemInts) {
                 const int64_t mo = ((int64_t)(uint32_t)src[i] | ((int64_t)src[i + 1] << 32)) + mbase;
                 dst.push_back((int)(mo & 0xffffffff));
                 dst.push_back((int)(mo >> 32));
                 dst.push_back(src[i + 2] + (int)rbase);
-                for (int j = 3; j < kItemInts - 1; ++j) dst.push_back(src[i + j]);
-                dst.push_back(src[i + kItemInts - 1] + (zfield ? (int)zbase : 0));
+                for (int j = 3; j < kItemInts; ++j) dst.push_back(src[i + j]);
             }
             return base_item;
         };
@@ -976,27 +1013,21 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
         auto slice = [](const std::vector<int>& v, int b0, int b1) {
             return std::vector<int>(v.begin() + (size_t)kItemInts * b0, v.begin() + (size_t)kItemInts * b1);
         };
-        if ((int)bfb.size() < f.nlevels) {
-            bfb.resize(f.nlevels); bfw.resize(f.nlevels); bbb.resize(f.nlevels); bbw.resize(f.nlevels);
+        if ((int)bbl.size() < f.nlevels) {
+            bbl.resize(f.nlevels);
+            bsm.resize(f.nlevels);
             btn.resize(f.nlevels);
-            bzs.resize(f.nlevels);
         }
         for (int L = 0; L < (int)f.levels.size(); ++L) {
             const SolveLevel& lv = f.levels[L];
-            out.levels.push_back({lv.fwd_begin + fb, lv.fwd_end + fb, lv.bwd_begin + bb, lv.bwd_end + bb,
-                                  0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+            out.levels.push_back({lv.fwd_begin + fb, lv.fwd_end + fb, lv.bwd_begin + bb, lv.bwd_end + bb, 0, 0, 0, 0, 0, 0});
+            shift(bbl[L], slice(f.blocks, lv.blk_begin, lv.blk_end));
+            shift(bsm[L], slice(f.small, lv.sml_begin, lv.sml_end));
             shift(btn[L], slice(f.tiny, lv.tiny_begin, lv.tiny_end));
-            shift(bzs[L], slice(f.zstage, lv.zst_begin, lv.zst_end), true);
-            shift(bfb[L], slice(f.fwd_blocks, lv.fwdb_begin, lv.fwdb_end));
-            shift(bfw[L], slice(f.fwd_small, lv.fwdw_begin, lv.fwdw_end));
-            shift(bbb[L], slice(f.bwd_blocks, lv.bwdb_begin, lv.bwdb_end), true);
-            shift(bbw[L], slice(f.bwd_small, lv.bwdw_begin, lv.bwdw_end));
         }
         out.body_level.push_back((int)out.levels.size());
         mbase += f.mval_size;
         rbase += (int64_t)f.rows.size();
-        zbase += f.zrows;
-        out.zrows += f.zrows;
         sbase += f.nsuper;
         out.K.n = 0;  // per-body systems are not kept
         f = CholFactor();  // release the per-body copy
@@ -1006,20 +1037,17 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
         out.fp.on = true;
         finish_front_plan(out);
     }
-    for (size_t L = 0; L < bfb.size(); ++L) {
-        SolveLevel lv{0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (size_t L = 0; L < bbl.size(); ++L) {
+        SolveLevel lv{};
         auto put = [&](std::vector<int>& dst, std::vector<int>& src, int& b0, int& b1) {
             b0 = (int)(dst.size() / kItemInts);
             dst.insert(dst.end(), src.begin(), src.end());
             b1 = (int)(dst.size() / kItemInts);
             std::vector<int>().swap(src);
         };
-        put(out.fwd_blocks, bfb[L], lv.fwdb_begin, lv.fwdb_end);
-        put(out.fwd_small, bfw[L], lv.fwdw_begin, lv.fwdw_end);
-        put(out.bwd_blocks, bbb[L], lv.bwdb_begin, lv.bwdb_end);
-        put(out.bwd_small, bbw[L], lv.bwdw_begin, lv.bwdw_end);
+        put(out.blocks, bbl[L], lv.blk_begin, lv.blk_end);
+        put(out.small, bsm[L], lv.sml_begin, lv.sml_end);
         put(out.tiny, btn[L], lv.tiny_begin, lv.tiny_end);
-        put(out.zstage, bzs[L], lv.zst_begin, lv.zst_end);
         out.step_levels.push_back(lv);
     }
     std::vector<std::pair<int64_t, int>> sz(nbodies);

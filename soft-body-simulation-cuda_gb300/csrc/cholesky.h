@@ -43,12 +43,9 @@ std::vector<int> nd_order(const SparseSym& A, const float* xyz);
 struct SolveLevel {
     int fwd_begin, fwd_end;  // warp work items of the forward pass for this level
     int bwd_begin, bwd_end;  // warp work items of the backward pass
-    int fwdb_begin, fwdb_end;  // per-level launches: CTA block items (large supernodes)
-    int bwdb_begin, bwdb_end;
-    int fwdw_begin, fwdw_end;  // per-level launches: warp items of the small supernodes
-    int bwdw_begin, bwdw_end;
-    int tiny_begin, tiny_end;  // per-level launches: tiny supernodes, one thread each
-    int zst_begin, zst_end;    // per-level launches: backward z staging of the block supernodes
+    int blk_begin, blk_end;    // per-level launches: block items (both directions)
+    int sml_begin, sml_end;    // per-level launches: small supernodes, one warp each
+    int tiny_begin, tiny_end;  // per-level launches: tiny supernodes, a few lanes each
 };
 
 // Warp work items, 8 ints each (two int4 loads, no dependent metadata loads):
@@ -59,61 +56,21 @@ struct SolveLevel {
 constexpr int kItemInts = 8;
 constexpr int kFwdItemRows = 32;
 constexpr int kFwdItemCols = 64;
-// CTA block items (same 8-int layout) of the per-level launches:
-//   forward : {moff_lo, moff_hi, roff, m, k, r0, c0, c1}: rows r0 .. r0+128,
-//             pivot columns c0 .. c1 (at most 256, staged in shared memory)
-//   backward: {moff_lo, moff_hi, roff, m, r0, c0 | (c1 - c0) << 27, r1,
-//             zoff}: pivot columns c0 .. c1 against rows r0 .. r1 of
-//             z = [y_pivots ; -x_offdiag] of the supernode, staged once per
-//             level at zbuf[zoff ..] by z-staging items
-//             {moff_lo, moff_hi, roff, m, k, r0, split, zoff} of kStageRows
-//             rows; when split != 0 the columns are split into row chunks
-//             that add their partial sums into x, and staging clears x at
-//             the pivot rows first
-// Supernodes with at least kBlockMinRows rows use block items in the
-// per-level launches; smaller ones keep warp items (packed 4 per CTA).
-// Columns per forward block item and per warp of a backward block item.
-// With the amalgamated supernodes, 32 forward columns (against 16) solve the
-// 512-body batch in 677 instead of 703 us and the 40^3 cube in 182 instead
-// of 188 us (same box).
-#ifndef PDGB_FWDB_COLS
-#define PDGB_FWDB_COLS 32
-#endif
-#ifndef PDGB_BWD_WARP_COLS
-#define PDGB_BWD_WARP_COLS 2
-#endif
-// Rows of one backward block item of a single-body factor: a column's rows
-// are split into chunks so that no warp walks a long column alone.  (A
-// batch's levels hold many bodies' supernodes, enough parallelism without
-// the split, which would only add items and atomics: there a column is one
-// item.)
-#ifndef PDGB_BWD_CHUNK_ROWS
-#define PDGB_BWD_CHUNK_ROWS 256
-#endif
-constexpr int kBwdColShift = 27;  // backward block: c1 - c0 above c0 in one int
-#ifndef PDGB_BLOCK_MIN_ROWS
-#define PDGB_BLOCK_MIN_ROWS 64
-#endif
-// Tiny supernodes (at most kTinyCols pivots and kTinyRows rows -- most of
-// them are leaves with one pivot) are solved one per thread in the per-level
-// launches: descriptor {moff_lo, moff_hi, roff, m, k, 0, 0, 0}.
-#ifndef PDGB_TINY_COLS
-#define PDGB_TINY_COLS 1
-#endif
-#ifndef PDGB_TINY_ROWS
-#define PDGB_TINY_ROWS 32
-#endif
-constexpr int kTinyCols = PDGB_TINY_COLS;
-constexpr int kTinyRows = PDGB_TINY_ROWS;
-constexpr int kFwdBlockRows = 128;
-constexpr int kFwdBlockCols = PDGB_FWDB_COLS;
-constexpr int kBwdWarpCols = PDGB_BWD_WARP_COLS;   // backward block: columns per warp (4 warps)
-constexpr int kBwdBlockCols = 4 * kBwdWarpCols;
-static_assert(kBwdBlockCols < (1 << (32 - kBwdColShift)), "backward block: column count field");
-static_assert(kFwdBlockCols <= 128, "forward block: pivot right-hand sides staged by the first threads");
-constexpr int kStageRows = 128;
-constexpr int kBwdChunkRows = PDGB_BWD_CHUNK_ROWS;
-constexpr int kBlockMinRows = PDGB_BLOCK_MIN_ROWS;
+// Items of the per-level launches (same 8-int layout):
+//   block: {moff_lo, moff_hi, roff, m, k, r0, c0, c1}: the tile of M_s with
+//          rows r0 .. r0 + kTileRows and pivot columns c0 .. c1 (at most
+//          kTileCols), for one CTA and both directions
+//   small: {moff_lo, moff_hi, roff, m, k, 0, 0, 0}: a whole supernode of fewer
+//          than kBlockMinRows rows and at most kSmallCols pivots, for a warp
+//   tiny : the same for a supernode of one pivot and at most kTinyRows rows
+// A tile has one thread a row (forward) and 8 columns a warp (backward), 32
+// entries a thread: enough loads in flight with 8 CTAs on an SM, and few
+// enough registers for them.
+constexpr int kTileRows = 128;
+constexpr int kTileCols = 32;
+constexpr int kBlockMinRows = 64;
+constexpr int kSmallCols = 32;
+constexpr int kTinyRows = 32;
 
 // Numeric factorisation on the GPU (factor.cu): everything the device needs
 // beyond the symbolic structure of CholFactor.  Each supernode s has a dense
@@ -154,13 +111,9 @@ struct CholFactor {
     // GPU warp work items grouped by level (see kItemInts).
     std::vector<int> fwd_items;
     std::vector<int> bwd_items;
-    std::vector<int> fwd_blocks;     // CTA block items (see kFwdBlockRows)
-    std::vector<int> bwd_blocks;
-    std::vector<int> fwd_small;      // warp items of the small supernodes (per-level launches)
-    std::vector<int> bwd_small;
-    std::vector<int> tiny;           // tiny supernode descriptors (per-level launches)
-    std::vector<int> zstage;         // backward z-staging items of the block supernodes
-    int64_t zrows = 0;               // rows of the z staging buffer
+    std::vector<int> blocks;         // items of the per-level launches (see kTileRows)
+    std::vector<int> small;
+    std::vector<int> tiny;
     std::vector<SolveLevel> levels;  // body-major: body b owns levels[body_level[b] .. body_level[b+1])
     // Per-level launches (block and small items): level L of every body in
     // one launch, levels counted from the leaves.  Equal to `levels` for a
@@ -205,20 +158,22 @@ void build_dsm_plan(const CholFactor& f, int ctas, int warps_per_cta, size_t max
 
 // Factors K (vertex-indexed, n x n SPD).  ordering: 0 = AMD, 1 = nested
 // dissection (xyz required), 2 = AMD order stored as one dense supernode.  Throws Error(PDGB_ERR_NOT_SPD) if a pivot is
-// not positive.  bwd_chunk_rows: rows per backward block item (0: whole
-// columns).
+// not positive.
 // gpu_numeric: stop after the symbolic analysis and fill out.fp for the
 // GPU factorisation (factor.cu) instead of computing mval on the host;
 // finish_plan: complete it (finish_front_plan) -- a batch completes the
 // combined plan of its bodies instead.
-// amalgamation: how many explicit zeros a supernode may take on when it is
-// merged into its parent (kAmalgChain for the engine's solves, bound by
-// their chain of levels; kAmalgBytes for the serving step, bound by the
-// factor's bytes).
-enum : int { kAmalgChain = 0, kAmalgBytes = 1 };
+// level_entries: what a level of the solve costs, in stored entries, when
+// supernodes are amalgamated.  kLevelEntries is a single body's: about 6 us
+// of dependent launches a level, forward and backward, against 8 bytes an
+// entry at some 5 TB/s.  Bodies that share their launches pay a share:
+// batches by size, requests of a server 1 / kServerBodies.
+constexpr double kLevelEntries = 3.75e6;
+constexpr double kServerBodies = 16.0;
+constexpr double kDsmLevelEntries = 1e3;
 void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFactor& out,
-                     int bwd_chunk_rows = kBwdChunkRows, bool gpu_numeric = false, bool finish_plan = true,
-                     int amalgamation = kAmalgChain);
+                     bool gpu_numeric = false, bool finish_plan = true,
+                     double level_entries = kLevelEntries);
 
 // Factors the block-diagonal system of independent bodies, one block per
 // body (vertex range vstart[b]..vstart[b+1], tets tstart[b]..tstart[b+1] in

@@ -90,7 +90,7 @@ template <class T> struct Pinned {
     }
 };
 
-constexpr int kItemKinds = 6;  // fwd blocks, bwd blocks, fwd small, bwd small, tiny, z staging
+constexpr int kItemKinds = 3;  // blocks, small, tiny (items of the per-level launches)
 
 // What the workers prepare for a mesh, shared by the requests that submit
 // the same mesh (cache by content).  The images are built by the tick
@@ -102,7 +102,7 @@ struct MeshEntry {
     size_t layout_bytes = 0;        // tile layout part of a request's block
     Pinned<unsigned char> layout;   // that part, as laid out in the block
     Pinned<int> rows;               // row lists (mesh vertex ids)
-    Pinned<int> items;              // work items of the 6 kinds, back to back (mesh offsets)
+    Pinned<int> items;              // work items by kind, back to back (mesh offsets)
     int64_t kbase[kItemKinds + 1] = {0};  // ints: start of each kind in items
     Pinned<float> mval;             // numeric factor once computed
     bool numeric = false;
@@ -206,7 +206,7 @@ struct Request {
     int flag_host = 0;
     int64_t hin = -1, hout = -1;          // page-locked staging ranges (input state, results)
     // arena ranges of a Cholesky request
-    int64_t v0 = 0, m0 = 0, r0 = 0, z0 = 0, io = 0;
+    int64_t v0 = 0, m0 = 0, r0 = 0, io = 0;
     float4 *x = nullptr, *v = nullptr, *prev = nullptr, *base = nullptr;
     const float4 *coef = nullptr, *pin = nullptr;
     std::vector<float> X_out, V_out;
@@ -216,21 +216,20 @@ struct Request {
 template <class T> size_t bytes_of(const std::vector<T>& v) { return align256(v.size() * sizeof(T)); }
 
 int64_t item_ints(const CholFactor& f) {
-    return (int64_t)(f.fwd_blocks.size() + f.bwd_blocks.size() + f.fwd_small.size() + f.bwd_small.size() +
-                     f.tiny.size() + f.zstage.size());
+    return (int64_t)(f.blocks.size() + f.small.size() + f.tiny.size());
 }
 
-// Arena bytes of a Cholesky request: 3 solve vectors, rows, M_s, backward
-// staging and work items.
+// Arena bytes of a Cholesky request: 3 solve vectors, rows, M_s and work
+// items.
 size_t arena_bytes(const Request& r) {
     const CholFactor& f = *r.me->f;
     return 3 * (size_t)r.nv * sizeof(float4) + f.rows.size() * sizeof(int) + (size_t)f.mval_size * sizeof(float) +
-           (size_t)f.zrows * sizeof(float4) + (size_t)item_ints(f) * sizeof(int);
+           (size_t)item_ints(f) * sizeof(int);
 }
 
 // Device bytes of a prepared request: its block (layout arrays, the state
 // vectors it owns, staging for the state transfers, the status word) and,
-// on the Cholesky path, its arena ranges (3 vectors, rows, M_s, staging).
+// on the Cholesky path, its arena ranges (3 vectors, rows, M_s, items).
 size_t request_bytes(const Request& r, bool chol) {
     const HostLayout& L = *r.L;
     size_t b = bytes_of(L.inc_ent) + bytes_of(L.inc_end) + bytes_of(L.geo) + bytes_of(L.tile_tet_ptr) +
@@ -270,27 +269,16 @@ __global__ void k_add_offset(int* a, int64_t n, int off) {
     if (i < n) a[i] += off;
 }
 
-// A request's work items (kinds back to back, kb[k] = first item of kind k)
-// moved to its arena ranges: factor offset m0 into the 64-bit field of
-// ints 0-1, row-list offset r0 into int 2, backward staging offset z0 into
-// int 7 of the backward blocks (kind 1) and staging items (kind 5).
-struct ItemShift {
-    long long m0;
-    int r0, z0;
-    long long kb[kItemKinds + 1];
-};
-
-__global__ void k_shift_items(int* items, ItemShift sh) {
+// A request's work items moved to its arena ranges: factor offset m0 into
+// the 64-bit field of ints 0-1, row-list offset r0 into int 2.
+__global__ void k_shift_items(int* items, long long n, long long m0, int r0) {
     const long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= sh.kb[kItemKinds]) return;
-    int kind = 0;
-    while (kind + 1 < kItemKinds && it >= sh.kb[kind + 1]) ++kind;
+    if (it >= n) return;
     int* w = items + it * kItemInts;
-    const long long mo = ((long long)(uint32_t)w[0] | ((long long)w[1] << 32)) + sh.m0;
+    const long long mo = ((long long)(uint32_t)w[0] | ((long long)w[1] << 32)) + m0;
     w[0] = (int)(mo & 0xffffffff);
     w[1] = (int)(mo >> 32);
-    w[2] += sh.r0;
-    if (kind == 1 || kind == 5) w[7] += sh.z0;
+    w[2] += r0;
 }
 
 }  // namespace
@@ -332,7 +320,6 @@ struct pdgb_server {
     Arena<float4> va_sn, va_b, va_y;  // one vertex range per request, same offset in all three
     Arena<float> ar_mval;
     Arena<int> ar_rows;
-    Arena<float4> ar_zbuf;
     Arena<int> ar_items;               // every request's work items, its offsets applied
     DBuf<int> d_comb[kItemKinds];       // the step's combined per-level lists, by kind
     Pinned<ItemSeg> h_seg;              // segments gathered into them
@@ -483,7 +470,8 @@ void worker_loop(pdgb_server* S) {
                     // columns per backward item, as the bodies of a batch.
                     auto f = std::make_shared<CholFactor>();
                     const std::vector<float> xyz = layout_xyz(*L);
-                    cholesky_factor(layout_system(*L), PDGB_ORDER_AMD, xyz.data(), *f, 0, true, true, kAmalgBytes);
+                    cholesky_factor(layout_system(*L), PDGB_ORDER_AMD, xyz.data(), *f, true, true,
+                                    kLevelEntries / kServerBodies);
                     f->K = SparseSym();  // no refinement residuals in the server
                     me->f = f;
                 }
@@ -633,8 +621,7 @@ void build_images(pdgb_server* S, MeshEntry& me) {
         const CholFactor& f = *me.f;
         me.rows.reserve(f.rows.size());
         if (!f.rows.empty()) std::memcpy(me.rows.p, f.rows.data(), f.rows.size() * sizeof(int));
-        const std::vector<int>* kinds[kItemKinds] = {&f.fwd_blocks, &f.bwd_blocks, &f.fwd_small,
-                                                     &f.bwd_small,  &f.tiny,       &f.zstage};
+        const std::vector<int>* kinds[kItemKinds] = {&f.blocks, &f.small, &f.tiny};
         me.kbase[0] = 0;
         for (int k = 0; k < kItemKinds; ++k) me.kbase[k + 1] = me.kbase[k] + (int64_t)kinds[k]->size();
         me.items.reserve((size_t)me.kbase[kItemKinds]);
@@ -698,20 +685,18 @@ void admit(pdgb_server* S, Request* r) {
     r->la = LocalArgs{sn, b, inc_ent, inc_end, geo, ttp, tvp, tv, L.nt_pad, nullptr};
     if (chol) {
         const CholFactor& f = *me.f;
-        int64_t v0, m0, r0, z0, io, tmp;
+        int64_t v0, m0, r0, io, tmp;
         const int64_t nitems = me.kbase[kItemKinds];
         bool moved = S->va_sn.take(nv, v0, s);
         moved |= S->va_b.take(nv, tmp, s);
         moved |= S->va_y.take(nv, tmp, s);
         moved |= S->ar_mval.take(f.mval_size, m0, s);
         moved |= S->ar_rows.take((int64_t)f.rows.size(), r0, s);
-        moved |= S->ar_zbuf.take(f.zrows, z0, s);
         moved |= S->ar_items.take(nitems, io, s);
         if (moved) S->lists_dirty = true;  // every request's arena pointers change
         r->v0 = v0;
         r->m0 = m0;
         r->r0 = r0;
-        r->z0 = z0;
         r->io = io;
         const int64_t nrows = (int64_t)f.rows.size();
         if (nrows) {
@@ -722,13 +707,8 @@ void admit(pdgb_server* S, Request* r) {
         if (nitems) {
             PDGB_CUDA_TRY(cudaMemcpyAsync(S->ar_items.p + io, me.items.p, (size_t)nitems * sizeof(int),
                                           cudaMemcpyHostToDevice, s));
-            ItemShift sh{};
-            sh.m0 = m0;
-            sh.r0 = (int)r0;
-            sh.z0 = (int)z0;
-            for (int k = 0; k <= kItemKinds; ++k) sh.kb[k] = me.kbase[k] / kItemInts;
-            const long long n = sh.kb[kItemKinds];
-            if (n) k_shift_items<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(S->ar_items.p + io, sh);
+            const long long n = nitems / kItemInts;
+            k_shift_items<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(S->ar_items.p + io, n, m0, (int)r0);
         }
         PDGB_CUDA_TRY(cudaMemsetAsync(S->va_y.p + v0, 0, (size_t)nv * sizeof(float4), s));
         // the numeric factor: computed on the GPU the first time the mesh is
@@ -768,7 +748,6 @@ void release_arenas(pdgb_server* S, Request* r) {
     S->va_y.give(r->v0, r->nv);
     S->ar_mval.give(r->m0, f.mval_size);
     S->ar_rows.give(r->r0, (int64_t)f.rows.size());
-    S->ar_zbuf.give(r->z0, f.zrows);
     S->ar_items.give(r->io, r->me->kbase[kItemKinds]);
 }
 
@@ -863,13 +842,9 @@ void launch_step(pdgb_server* S) {
     ca.y = S->va_y.p;
     ca.x = S->va_sn.p;
     ca.done = nullptr;
-    ca.fwd_blocks = S->d_comb[0].p;
-    ca.bwd_blocks = S->d_comb[1].p;
-    ca.fwd_small = S->d_comb[2].p;
-    ca.bwd_small = S->d_comb[3].p;
-    ca.tiny = S->d_comb[4].p;
-    ca.zstage = S->d_comb[5].p;
-    ca.zbuf = S->ar_zbuf.p;
+    ca.blocks = S->d_comb[0].p;
+    ca.small = S->d_comb[1].p;
+    ca.tiny = S->d_comb[2].p;
     launch_begin_multi(S->d_ba, S->d_chunks, S->d_counts + 1, S->cap_chunks, s);
     for (int i = 0; i < n; ++i) {
         launch_local_multi(S->d_la, S->d_tiles, S->d_counts, S->cap_tiles, s, false);
@@ -888,18 +863,15 @@ void launch_step(pdgb_server* S) {
 void build_solve_lists(pdgb_server* S) {
     int nl = 0;
     for (Request* r : S->active) nl = std::max(nl, (int)r->me->f->step_levels.size());
-    S->step_levels.assign(nl, SolveLevel{0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0});
+    S->step_levels.assign(nl, SolveLevel{});
     std::vector<ItemSeg> seg;
     seg.reserve((size_t)nl * S->active.size() * 2);
     int64_t tot[kItemKinds] = {0};
     auto range = [](const SolveLevel& q, int k, int& b, int& e) {
         switch (k) {
-            case 0: b = q.fwdb_begin; e = q.fwdb_end; break;
-            case 1: b = q.bwdb_begin; e = q.bwdb_end; break;
-            case 2: b = q.fwdw_begin; e = q.fwdw_end; break;
-            case 3: b = q.bwdw_begin; e = q.bwdw_end; break;
-            case 4: b = q.tiny_begin; e = q.tiny_end; break;
-            default: b = q.zst_begin; e = q.zst_end; break;
+            case 0: b = q.blk_begin; e = q.blk_end; break;
+            case 1: b = q.sml_begin; e = q.sml_end; break;
+            default: b = q.tiny_begin; e = q.tiny_end; break;
         }
     };
     for (int L = 0; L < nl; ++L) {
@@ -922,12 +894,9 @@ void build_solve_lists(pdgb_server* S) {
         SolveLevel& lv = S->step_levels[L];
         int end[kItemKinds];
         for (int k = 0; k < kItemKinds; ++k) end[k] = (int)(tot[k] / kItemInts);
-        lv.fwdb_begin = begin[0]; lv.fwdb_end = end[0];
-        lv.bwdb_begin = begin[1]; lv.bwdb_end = end[1];
-        lv.fwdw_begin = begin[2]; lv.fwdw_end = end[2];
-        lv.bwdw_begin = begin[3]; lv.bwdw_end = end[3];
-        lv.tiny_begin = begin[4]; lv.tiny_end = end[4];
-        lv.zst_begin = begin[5]; lv.zst_end = end[5];
+        lv.blk_begin = begin[0]; lv.blk_end = end[0];
+        lv.sml_begin = begin[1]; lv.sml_end = end[1];
+        lv.tiny_begin = begin[2]; lv.tiny_end = end[2];
     }
     cudaStream_t s = S->stream;
     bool grow = seg.size() > S->h_seg.n || seg.size() > S->d_seg.n;

@@ -67,20 +67,6 @@ __device__ __forceinline__ void fwd_warp_item(const CholArgs& a, const int* w, f
     else atomicAdd(&a.r[vid], make_float4(-ax, -ay, -az, 0.f));
 }
 
-// L2 prefetch of a forward warp item's static data (row ids and up to 16
-// columns of the lane's row of M_s), issued before the grid dependency wait.
-__device__ __forceinline__ void fwd_warp_prefetch(const CholArgs& a, const int* w, int lane) {
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(w));
-    const int4 h1 = __ldg(reinterpret_cast<const int4*>(w) + 1);
-    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    const int m = h0.w, k = h1.x, row = h1.y + lane, c0 = h1.z, c1 = h1.w;
-    if (row >= m) return;
-    const int cend = min(row < k ? min(c1, row + 1) : c1, c0 + 16);
-    const float* Mr = a.mval + moff + row;
-    for (int c = c0; c < cend; ++c) prefetch_l2(Mr + (size_t)c * m);
-    if (lane == 0) prefetch_l2(a.rows + h0.z + h1.y);
-}
-
 // Backward warp item {moff, roff, m, k, c}: x[pivot c] = sum_{i >= c}
 // M_s[i, c] z_i with z = [y_pivots ; -x_offdiag]; lanes stride over rows
 // (a coalesced column of M_s, 4 independent loads in flight per lane),
@@ -118,482 +104,469 @@ __device__ __forceinline__ void bwd_warp_item(const CholArgs& a, const int* w, f
     if (lane == 0) a.x[__ldg(&rows[c])] = make_float4(ax, ay, az, 0.f);
 }
 
-// Backward warp item with its first 64 rows of M_s and row ids loaded
-// into registers before the grid dependency wait (the small supernodes of
-// the per-level kernels have fewer rows than that); same sums, same order
-// as bwd_warp_item.
-__device__ __forceinline__ void bwd_warp_item_pre(const CholArgs& a, const int* w, int lane, bool item) {
-    int m = 0, k = 0, c = 0;
-    const int* rows = a.rows;
-    const float* Mc = a.mval;
-    float mv[2] = {0.f, 0.f};
-    int vid[2] = {0, 0};
-    if (item) {
-        const int4 h0 = __ldg(reinterpret_cast<const int4*>(w));
-        const int4 h1 = __ldg(reinterpret_cast<const int4*>(w) + 1);
-        const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-        m = h0.w;
-        k = h1.x;
-        c = h1.y;
-        rows = a.rows + h0.z;
-        Mc = a.mval + moff + (size_t)c * m;
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int i = c + lane + 32 * t;
-            if (i < m) {
-                mv[t] = __ldg(Mc + i);
-                vid[t] = __ldg(&rows[i]);
-            }
-        }
-    }
-    pdl_wait();
-    if ((a.done && *a.done) || !item) return;
-    float ax = 0.f, ay = 0.f, az = 0.f;
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int i = c + lane + 32 * t;
-        if (i < m) {
-            float4 z;
-            if (i < k) z = a.y[vid[t]];
-            else {
-                const float4 xv = a.x[vid[t]];
-                z = make_float4(-xv.x, -xv.y, -xv.z, 0.f);
-            }
-            ax = fmaf(mv[t], z.x, ax);
-            ay = fmaf(mv[t], z.y, ay);
-            az = fmaf(mv[t], z.z, az);
-        }
-    }
-    for (int i = c + lane + 64; i < m; i += 32) {
-        const int v = __ldg(&rows[i]);
-        const float mvi = __ldg(Mc + i);
-        float4 z;
-        if (i < k) z = a.y[v];
-        else {
-            const float4 xv = a.x[v];
-            z = make_float4(-xv.x, -xv.y, -xv.z, 0.f);
-        }
-        ax = fmaf(mvi, z.x, ax);
-        ay = fmaf(mvi, z.y, ay);
-        az = fmaf(mvi, z.z, az);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, off);
-        ay += __shfl_xor_sync(0xffffffffu, ay, off);
-        az += __shfl_xor_sync(0xffffffffu, az, off);
-    }
-    if (lane == 0) a.x[__ldg(&rows[c])] = make_float4(ax, ay, az, 0.f);
+// ---- per-level launches: one per level and direction.  A launch's CTAs
+// (kLevelThreads threads) take, by index, first the level's block items, then
+// its small supernodes (one warp each), then its tiny ones (kTinyLanes lanes
+// each), then -- in the solve's first backward launch, when asked -- the
+// resets of the next iteration's vectors.  Each CTA reads its descriptors,
+// row ids and factor entries into registers before the grid dependency wait,
+// so that a level's factor bytes are under way while the level before drains;
+// after the wait come one gather from L2, the products, one reduction and the
+// stores.  What bounds a narrow level is that chain of latencies, about 3 us
+// with the launch, so a level is one launch and nothing is staged by another.
+
+// Block item {moff, roff, m, k, r0, c0, c1}: the tile rows r0 .. r0 + 128,
+// pivot columns c0 .. c1 (at most 32) of M_s; both directions use the same
+// items.
+struct BlockItem {
+    const float* M;   // M_s, column major
+    const int* rows;
+    int m, k, r0, c0, c1;
+};
+
+__device__ __forceinline__ BlockItem block_item(const CholArgs& a, const int* list, int item) {
+    const int4* w = reinterpret_cast<const int4*>(list + (size_t)kItemInts * item);
+    const int4 h0 = __ldg(w), h1 = __ldg(w + 1);
+    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
+    return BlockItem{a.mval + moff, a.rows + h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 }
 
-// ---- per-level launches with CTA block items.
-// Forward block {moff, roff, m, k, r0, c0, c1}: the pivot right-hand sides
-// r[c0 .. c1) are staged in shared memory once; thread t owns row r0 + t and
-// streams its row of M_s (column-major, so a warp's loads of one column are
-// contiguous), 8 independent loads in flight.  Pivot rows add into y,
-// off-diagonal rows subtract from r (ancestor pivots, read at a later level).
-// Static part of a forward block item (no vector reads): the thread's row of
-// M_s (at most kFwdBlockCols columns, zero past cend), its vertex id and
-// the staging index.
+// Forward block, static part: thread t owns row r0 + t, its (at most 32)
+// entries of the tile in registers.  A warp's loads of one column are
+// contiguous.
 struct FwdBlockPre {
-    float mv[kFwdBlockCols];
-    int vid, sv, ncols, row, k;
-    bool active;
+    float mv[kTileCols];
+    int vid, sv, ncols, row, k, m;
+    bool first;   // the tile holds the first pivot columns
 };
 
 __device__ __forceinline__ void fwd_block_load(const CholArgs& a, int item, FwdBlockPre& p) {
-    const int* w = a.fwd_blocks + (size_t)kItemInts * item;
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(w));
-    const int4 h1 = __ldg(reinterpret_cast<const int4*>(w) + 1);
-    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    const int roff = h0.z, m = h0.w, k = h1.x, r0 = h1.y, c0 = h1.z, c1 = h1.w;
-    const int* rows = a.rows + roff;
-    const int row = r0 + threadIdx.x;
-    const bool active = row < m && row < r0 + kFwdBlockRows;
-    const int cend = !active ? c0 : (row < k ? min(c1, row + 1) : c1);
-    const float* Mr = a.mval + moff + row;
+    const BlockItem b = block_item(a, a.blocks, item);
+    const int row = b.r0 + threadIdx.x;
+    const bool active = row < b.m && row >= b.c0;  // rows above the tile's columns have nothing in it
+    const int cend = !active ? b.c0 : (row < b.k ? min(b.c1, row + 1) : b.c1);
+    const float* Mr = b.M + row;
 #pragma unroll
-    for (int q = 0; q < kFwdBlockCols; ++q) p.mv[q] = (c0 + q < cend) ? __ldg(Mr + (size_t)(c0 + q) * m) : 0.f;
-    p.vid = active ? __ldg(&rows[row]) : 0;
-    p.ncols = c1 - c0;
-    p.sv = (int)threadIdx.x < p.ncols ? __ldg(&rows[c0 + threadIdx.x]) : 0;
+    for (int q = 0; q < kTileCols; ++q) p.mv[q] = (b.c0 + q < cend) ? __ldg(Mr + (size_t)(b.c0 + q) * b.m) : 0.f;
+    p.vid = active ? __ldg(&b.rows[row]) : -1;
+    p.ncols = b.c1 - b.c0;
+    p.sv = (int)threadIdx.x < p.ncols ? __ldg(&b.rows[b.c0 + threadIdx.x]) : 0;
     p.row = row;
-    p.k = k;
-    p.active = active;
+    p.k = b.k;
+    p.m = b.m;
+    p.first = b.c0 == 0;
 }
 
-// Vector part: stage the pivot right-hand sides (one barrier of the whole
-// CTA), then the thread's row sum into y (pivot rows) or r (ancestor rows).
+// Vector part: the pivot right-hand sides staged in shared memory, then the
+// row's sum into y (pivot rows; stored where no other tile adds to it) or out
+// of r (ancestor rows, pivots of later levels).  The backward pass adds the
+// partial sums of a supernode with more rows than a tile into x, which is
+// cleared here.
 __device__ __forceinline__ void fwd_block_run(const CholArgs& a, const FwdBlockPre& p, float4* rs) {
-    if (threadIdx.x < kFwdBlockCols)
-        rs[threadIdx.x] = (int)threadIdx.x < p.ncols ? a.r[p.sv] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (threadIdx.x < kTileCols)
+        rs[threadIdx.x] = (int)threadIdx.x < p.ncols ? __ldcg(&a.r[p.sv]) : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    if (!p.active) return;
+    if (p.vid < 0) return;
     float ax = 0.f, ay = 0.f, az = 0.f;
 #pragma unroll
-    for (int q = 0; q < kFwdBlockCols; ++q) {
+    for (int q = 0; q < kTileCols; ++q) {
         const float4 v = rs[q];
         ax = fmaf(p.mv[q], v.x, ax);
         ay = fmaf(p.mv[q], v.y, ay);
         az = fmaf(p.mv[q], v.z, az);
     }
-    if (p.row < p.k) atomicAdd(&a.y[p.vid], make_float4(ax, ay, az, 0.f));
-    else atomicAdd(&a.r[p.vid], make_float4(-ax, -ay, -az, 0.f));
-}
-
-__global__ void __launch_bounds__(kBlockThreads) k_chol_fwd_block(CholArgs a, int item0) {
-    __shared__ float4 rs[kFwdBlockCols];
-    pdl_trigger();
-    FwdBlockPre p;
-    fwd_block_load(a, item0 + blockIdx.x, p);  // static data before the wait
-    pdl_wait();
-    if (a.done && *a.done) return;
-    fwd_block_run(a, p, rs);
-}
-
-// Backward z staging {roff, m, k, r0, zoff}: z = [y_pivots ; -x_offdiag]
-// over rows r0 .. r0 + kStageRows of the supernode, gathered once per level
-// into zbuf[zoff ..] so that the backward blocks of all its column groups
-// read it contiguously.  For a supernode whose columns are split into row
-// chunks, x at the pivot rows is cleared here: the backward blocks of the
-// level add their chunk sums into it.
-__device__ __forceinline__ void zstage_item(const CholArgs& a, int item, bool pdl) {
-    const int* w = a.zstage + (size_t)kItemInts * item;
-    const int roff = __ldg(w + 2), m = __ldg(w + 3), k = __ldg(w + 4), r0 = __ldg(w + 5), split = __ldg(w + 6),
-              zoff = __ldg(w + 7);
-    const int* rows = a.rows + roff;
-    const int r1 = min(m, r0 + kStageRows);
-    const int i0 = r0 + threadIdx.x;
-    const int vid0 = i0 < r1 ? __ldg(&rows[i0]) : 0;
-    if (pdl) {
-        pdl_wait();
-        if (a.done && *a.done) return;
+    if (p.row >= p.k) {
+        atomicAdd(&a.r[p.vid], make_float4(-ax, -ay, -az, 0.f));
+        return;
     }
-    for (int i = i0; i < r1; i += kStageThreads) {
-        const int vid = i == i0 ? vid0 : __ldg(&rows[i]);
-        float4 z;
-        if (i < k) {
-            z = a.y[vid];
-            if (split) a.x[vid] = make_float4(0.f, 0.f, 0.f, 0.f);
-        } else {
-            const float4 xv = a.x[vid];
-            z = make_float4(-xv.x, -xv.y, -xv.z, 0.f);
+    if (p.row < kTileCols) a.y[p.vid] = make_float4(ax, ay, az, 0.f);
+    else atomicAdd(&a.y[p.vid], make_float4(ax, ay, az, 0.f));
+    if (p.first && p.m > kTileRows) a.x[p.vid] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// z of a row: y at a pivot, -x at an ancestor.
+__device__ __forceinline__ float4 z_of(const CholArgs& a, bool pivot, int vid) {
+    if (pivot) return __ldcg(&a.y[vid]);
+    const float4 v = __ldcg(&a.x[vid]);
+    return make_float4(-v.x, -v.y, -v.z, 0.f);
+}
+
+// Sums of 8 columns x 3 coordinates over the 32 lanes of a warp: three
+// exchanges that halve the columns a lane holds, then two plain ones.  Lane l
+// ends with the sums of column (l >> 2).
+__device__ __forceinline__ float3 reduce_cols8(float (&v)[8][3], int lane) {
+    float w[4][3], u[2][3], t[3];
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float keep = b4 ? v[j + 4][d] : v[j][d], give = b4 ? v[j][d] : v[j + 4][d];
+            w[j][d] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
         }
-        a.zbuf[zoff + i] = z;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float keep = b3 ? w[j + 2][d] : w[j][d], give = b3 ? w[j][d] : w[j + 2][d];
+            u[j][d] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+        }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float keep = b2 ? u[1][d] : u[0][d], give = b2 ? u[0][d] : u[1][d];
+        t[d] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+        t[d] += __shfl_xor_sync(0xffffffffu, t[d], 2);
+        t[d] += __shfl_xor_sync(0xffffffffu, t[d], 1);
     }
+    return make_float3(t[0], t[1], t[2]);
 }
 
-__global__ void __launch_bounds__(kStageThreads) k_chol_bwd_zstage(CholArgs a, int item0) {
-    pdl_trigger();
-    zstage_item(a, item0 + blockIdx.x, true);
-}
-
-// Static part of a backward block item: the warp's first 256 rows of each
-// of its columns in registers (a whole 256-row chunk).
-constexpr int kBwdPre = 8;
+// Backward block, static part: warp w owns the tile's columns c0 + 8 w ..,
+// lane l its rows r0 + l, + 32, ..: 4 x 8 entries in registers.
+constexpr int kBwdWarpCols = kTileCols / (kLevelThreads / 32);
+constexpr int kBwdRows = kTileRows / 32;
+static_assert(kBwdWarpCols == 8, "reduce_cols8");
 struct BwdBlockPre {
-    float mpre[kBwdPre][kBwdWarpCols];
-    const float* Mc;
-    const int* rows;
-    const float4* z;
-    int m, r0, rend, cw, nc, ib;
-    bool live;
+    float mv[kBwdRows][kBwdWarpCols];
+    int vid;      // of row r0 + thread, -1 past the last
+    int cv;       // vertex of this lane's result column, -1: none
+    bool pivot, split;
 };
 
 __device__ __forceinline__ void bwd_block_load(const CholArgs& a, int item, BwdBlockPre& p) {
-    const int* w = a.bwd_blocks + (size_t)kItemInts * item;
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(w));
-    const int4 h1 = __ldg(reinterpret_cast<const int4*>(w) + 1);
-    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    const int roff = h0.z, m = h0.w, r0 = h1.x, c0 = h1.y & ((1 << kBwdColShift) - 1),
-              c1 = c0 + (int)((unsigned)h1.y >> kBwdColShift), rend = h1.z, zoff = h1.w;
+    const BlockItem b = block_item(a, a.blocks, item);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cw = c0 + kBwdWarpCols * warp;  // first column of this warp
-    p.nc = min(kBwdWarpCols, c1 - cw);
-    p.Mc = a.mval + moff + (size_t)cw * m;
-    p.rows = a.rows + roff;
-    p.z = a.zbuf + zoff;
-    p.m = m;
-    p.r0 = r0;
-    p.rend = rend;
-    p.cw = cw;
-    p.live = cw < c1 && cw < rend;
-    p.ib = max(cw, r0) + lane;
+    const int cw = b.c0 + kBwdWarpCols * warp;
+    const float* Mc = b.M + (size_t)cw * b.m;
 #pragma unroll
-    for (int t = 0; t < kBwdPre; ++t) {
-        const int i = p.ib + 32 * t;
+    for (int t = 0; t < kBwdRows; ++t) {
+        const int i = b.r0 + lane + 32 * t;
 #pragma unroll
         for (int j = 0; j < kBwdWarpCols; ++j)
-            p.mpre[t][j] =
-                (p.live && j < p.nc && i < rend && i >= cw + j) ? __ldg(p.Mc + (size_t)j * m + i) : 0.f;
+            p.mv[t][j] = (i < b.m && cw + j < b.c1 && i >= cw + j) ? __ldg(Mc + (size_t)j * b.m + i) : 0.f;
     }
+    const int row = b.r0 + threadIdx.x;
+    p.vid = row < b.m ? __ldg(&b.rows[row]) : -1;
+    p.pivot = row < b.k;
+    const int c = cw + (lane >> 2);
+    p.cv = ((lane & 3) == 0 && c < b.c1) ? __ldg(&b.rows[c]) : -1;
+    p.split = b.m > kTileRows;
 }
 
-// Vector part: the staged z against the warp's columns, warp reductions,
-// sums stored (whole column) or added (row chunk) into x.  Warp-level only.
-__device__ __forceinline__ void bwd_block_run(const CholArgs& a, const BwdBlockPre& p) {
-    if (!p.live) return;
+// Vector part: z of the tile's rows staged in shared memory, the products,
+// the warp's reduction; sums stored, or added where the supernode's rows take
+// several tiles.
+__device__ __forceinline__ void bwd_block_run(const CholArgs& a, const BwdBlockPre& p, float4* zs) {
+    zs[threadIdx.x] = p.vid >= 0 ? z_of(a, p.pivot, p.vid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     float acc[kBwdWarpCols][3];
 #pragma unroll
     for (int j = 0; j < kBwdWarpCols; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.f;
 #pragma unroll
-    for (int t = 0; t < kBwdPre; ++t) {
-        const int i = p.ib + 32 * t;
-        if (i < p.rend) {
-            const float4 zz = p.z[i];
-#pragma unroll
-            for (int j = 0; j < kBwdWarpCols; ++j) {
-                if (j < p.nc && i >= p.cw + j) {
-                    acc[j][0] = fmaf(p.mpre[t][j], zz.x, acc[j][0]);
-                    acc[j][1] = fmaf(p.mpre[t][j], zz.y, acc[j][1]);
-                    acc[j][2] = fmaf(p.mpre[t][j], zz.z, acc[j][2]);
-                }
-            }
-        }
-    }
-#pragma unroll 2
-    for (int i = p.ib + 32 * kBwdPre; i < p.rend; i += 32) {
-        const float4 zz = p.z[i];
+    for (int t = 0; t < kBwdRows; ++t) {
+        const float4 z = zs[lane + 32 * t];
 #pragma unroll
         for (int j = 0; j < kBwdWarpCols; ++j) {
-            if (j < p.nc && i >= p.cw + j) {
-                const float mv = __ldg(p.Mc + (size_t)j * p.m + i);
-                acc[j][0] = fmaf(mv, zz.x, acc[j][0]);
-                acc[j][1] = fmaf(mv, zz.y, acc[j][1]);
-                acc[j][2] = fmaf(mv, zz.z, acc[j][2]);
+            acc[j][0] = fmaf(p.mv[t][j], z.x, acc[j][0]);
+            acc[j][1] = fmaf(p.mv[t][j], z.y, acc[j][1]);
+            acc[j][2] = fmaf(p.mv[t][j], z.z, acc[j][2]);
+        }
+    }
+    const float3 s = reduce_cols8(acc, lane);
+    if (p.cv < 0) return;
+    if (p.split) atomicAdd(&a.x[p.cv], make_float4(s.x, s.y, s.z, 0.f));
+    else a.x[p.cv] = make_float4(s.x, s.y, s.z, 0.f);
+}
+
+// Small supernodes {moff, roff, m, k} (m < kBlockMinRows = 64 rows, at most
+// kSmallCols pivots): one warp, lane l owns rows l and l + 32.  Forward: the
+// first kSmallPre columns before the wait, the rest after it.
+constexpr int kSmallPre = 16;
+struct SmallPre {
+    float mv[2][kSmallPre];
+    const float* M;
+    int m, k, vid[2];
+};
+
+__device__ __forceinline__ void small_load(const CholArgs& a, int item, bool live, int lane, SmallPre& p) {
+    p.m = p.k = 0;
+    p.M = a.mval;
+    p.vid[0] = p.vid[1] = -1;
+    if (live) {
+        const BlockItem b = block_item(a, a.small, item);
+        p.M = b.M;
+        p.m = b.m;
+        p.k = b.k;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (lane + 32 * h < p.m) p.vid[h] = __ldg(&b.rows[lane + 32 * h]);
+    }
+#pragma unroll
+    for (int c = 0; c < kSmallPre; ++c)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = lane + 32 * h;
+            p.mv[h][c] = (c < p.k && row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
+        }
+}
+
+__device__ __forceinline__ void fwd_small_run(const CholArgs& a, const SmallPre& p, int lane, float4* stage) {
+    stage[lane] = lane < p.k ? __ldcg(&a.r[p.vid[0]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    float s[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int c = 0; c < kSmallPre; ++c) {
+        const float4 v = stage[c];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            s[h][0] = fmaf(p.mv[h][c], v.x, s[h][0]);
+            s[h][1] = fmaf(p.mv[h][c], v.y, s[h][1]);
+            s[h][2] = fmaf(p.mv[h][c], v.z, s[h][2]);
+        }
+    }
+#pragma unroll 4
+    for (int c = kSmallPre; c < p.k; ++c) {
+        const float4 v = stage[c];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = lane + 32 * h;
+            const float mv = (row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
+            s[h][0] = fmaf(mv, v.x, s[h][0]);
+            s[h][1] = fmaf(mv, v.y, s[h][1]);
+            s[h][2] = fmaf(mv, v.z, s[h][2]);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (p.vid[h] < 0) continue;
+        if (lane + 32 * h < p.k) a.y[p.vid[h]] = make_float4(s[h][0], s[h][1], s[h][2], 0.f);
+        else atomicAdd(&a.r[p.vid[h]], make_float4(-s[h][0], -s[h][1], -s[h][2], 0.f));
+    }
+}
+
+// Backward: z of the warp's rows in registers, 8 columns at a time.
+__device__ __forceinline__ void bwd_small_run(const CholArgs& a, const SmallPre& p, int lane) {
+    float4 z[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        z[h] = p.vid[h] >= 0 ? z_of(a, lane + 32 * h < p.k, p.vid[h]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    auto columns = [&](int c0, const float (&mv)[2][8]) {
+        float acc[8][3];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j][0] = fmaf(mv[0][j], z[0].x, mv[1][j] * z[1].x);
+            acc[j][1] = fmaf(mv[0][j], z[0].y, mv[1][j] * z[1].y);
+            acc[j][2] = fmaf(mv[0][j], z[0].z, mv[1][j] * z[1].z);
+        }
+        const float3 s = reduce_cols8(acc, lane);
+        const int c = c0 + (lane >> 2);  // pivots are the first rows: vertex in lane c
+        const int vid = __shfl_sync(0xffffffffu, p.vid[0], c & 31);
+        if ((lane & 3) == 0 && c < p.k) a.x[vid] = make_float4(s.x, s.y, s.z, 0.f);
+    };
+    static_assert(kSmallPre % 8 == 0 && kSmallCols <= 32, "column groups");
+#pragma unroll
+    for (int g = 0; g < kSmallPre / 8; ++g) {
+        if (8 * g >= p.k) break;
+        float mv[2][8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            mv[0][j] = p.mv[0][8 * g + j];
+            mv[1][j] = p.mv[1][8 * g + j];
+        }
+        columns(8 * g, mv);
+    }
+    for (int c0 = kSmallPre; c0 < p.k; c0 += 8) {
+        float mv[2][8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = lane + 32 * h, c = c0 + j;
+                mv[h][j] = (c < p.k && row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
             }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kBwdWarpCols; ++j) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            acc[j][0] += __shfl_xor_sync(0xffffffffu, acc[j][0], off);
-            acc[j][1] += __shfl_xor_sync(0xffffffffu, acc[j][1], off);
-            acc[j][2] += __shfl_xor_sync(0xffffffffu, acc[j][2], off);
-        }
-        if (lane == 0 && j < p.nc) {
-            float4* xc = &a.x[__ldg(&p.rows[p.cw + j])];
-            const float4 sum = make_float4(acc[j][0], acc[j][1], acc[j][2], 0.f);
-            if (p.r0 == 0 && p.rend == p.m) *xc = sum;  // the whole column in one item
-            else atomicAdd(xc, sum);
-        }
+        columns(c0, mv);
     }
 }
 
-// Backward block {moff, roff, m, r0, c0 | ncols, r1, zoff}: warp w owns the
-// kBwdWarpCols consecutive columns c0 + kBwdWarpCols w .. over the rows
-// r0 .. r1; lanes stride the rows, each z (staged, contiguous) is loaded
-// once and used for all of the warp's columns (contiguous loads of M_s, one
-// per column), then a warp reduction per column whose sum is added into x.
-// Column c uses rows i >= c only.  The warp's first 256 rows of each column
-// are loaded into registers before the wait; longer columns of whole-column
-// items stream the rest afterwards.
-__global__ void __launch_bounds__(kBlockThreads) k_chol_bwd_block(CholArgs a, int item0) {
-    pdl_trigger();
-    BwdBlockPre p;
-    bwd_block_load(a, item0 + blockIdx.x, p);
-    pdl_wait();
-    if (a.done && *a.done) return;
-    bwd_block_run(a, p);
+// Tiny supernodes {moff, roff, m, 1} (one pivot, at most kTinyRows rows --
+// half the vertices of a grid are eliminated that way): kTinyLanes lanes,
+// lane j its rows j, j + kTinyLanes, ..; the first one before the wait.
+struct TinyPre {
+    const float* M;
+    const int* rows;
+    int m, vid;
+    float mv;
+};
+
+__device__ __forceinline__ void tiny_load(const CholArgs& a, int item, bool live, int j, TinyPre& p) {
+    p.m = 0;
+    p.vid = 0;
+    p.mv = 0.f;
+    p.M = a.mval;
+    p.rows = a.rows;
+    if (!live) return;
+    const int4 h0 = __ldg(reinterpret_cast<const int4*>(a.tiny + (size_t)kItemInts * item));
+    p.M = a.mval + ((int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32));
+    p.rows = a.rows + h0.z;
+    p.m = h0.w;
+    if (j < p.m) {
+        p.vid = __ldg(p.rows + j);
+        p.mv = __ldg(p.M + j);
+    }
 }
 
-// Small supernodes of a level (per-level launches): one warp item per warp,
-// in kernels of their own so that the many warps of the leaf levels are not
-// limited by the block kernels' registers and shared memory.
-__global__ void __launch_bounds__(kSmallThreads) k_chol_fwd_small(CholArgs a, int item0, int nitems) {
-    __shared__ float4 stage[kSmallThreads / 32][32];
+__device__ __forceinline__ void fwd_tiny_run(const CholArgs& a, const TinyPre& p, int j) {
+    const int piv = __shfl_sync(0xffffffffu, p.vid, 0, kTinyLanes);
+    if (p.m == 0) return;
+    const float4 r = __ldcg(&a.r[piv]);
+    if (j == 0) a.y[piv] = make_float4(p.mv * r.x, p.mv * r.y, p.mv * r.z, 0.f);
+    else if (j < p.m) atomicAdd(&a.r[p.vid], make_float4(-p.mv * r.x, -p.mv * r.y, -p.mv * r.z, 0.f));
+    for (int i = j + kTinyLanes; i < p.m; i += kTinyLanes) {
+        const float mv = __ldg(p.M + i);
+        atomicAdd(&a.r[__ldg(p.rows + i)], make_float4(-mv * r.x, -mv * r.y, -mv * r.z, 0.f));
+    }
+}
+
+__device__ __forceinline__ void bwd_tiny_run(const CholArgs& a, const TinyPre& p, int j) {
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    if (j < p.m) {
+        const float4 z = z_of(a, j == 0, p.vid);
+        sx = p.mv * z.x;
+        sy = p.mv * z.y;
+        sz = p.mv * z.z;
+    }
+    for (int i = j + kTinyLanes; i < p.m; i += kTinyLanes) {
+        const float4 z = z_of(a, false, __ldg(p.rows + i));
+        const float mv = __ldg(p.M + i);
+        sx = fmaf(mv, z.x, sx);
+        sy = fmaf(mv, z.y, sy);
+        sz = fmaf(mv, z.z, sz);
+    }
+#pragma unroll
+    for (int off = kTinyLanes / 2; off > 0; off >>= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, off);
+        sy += __shfl_xor_sync(0xffffffffu, sy, off);
+        sz += __shfl_xor_sync(0xffffffffu, sz, off);
+    }
+    if (j == 0 && p.m > 0) a.x[p.vid] = make_float4(sx, sy, sz, 0.f);
+}
+
+// Item ranges of one launch: first item and count of each kind; CTAs past
+// them reset vertices (ResetArgs).
+struct LevelRange {
+    int b0, nb, s0, ns, t0, nt;
+};
+constexpr int kLevelWarps = kLevelThreads / 32;
+constexpr int kTinyPerCta = kLevelThreads / kTinyLanes;
+__host__ __device__ inline int small_ctas(int n) { return (n + kLevelWarps - 1) / kLevelWarps; }
+__host__ __device__ inline int tiny_ctas(int n) { return (n + kTinyPerCta - 1) / kTinyPerCta; }
+
+__global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_fwd_level(CholArgs a, LevelRange v) {
+    __shared__ float4 rs[kLevelThreads];
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int it = blockIdx.x * (kSmallThreads / 32) + warp;
-    if (it < nitems) fwd_warp_prefetch(a, a.fwd_small + (size_t)kItemInts * (item0 + it), lane);
-    pdl_wait();
-    if (a.done && *a.done) return;
-    if (it < nitems) fwd_warp_item(a, a.fwd_small + (size_t)kItemInts * (item0 + it), stage[warp], lane);
-}
-
-__global__ void __launch_bounds__(kSmallThreads) k_chol_bwd_small(CholArgs a, int item0, int nitems) {
-    pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int it = blockIdx.x * (kSmallThreads / 32) + warp;
-    bwd_warp_item_pre(a, a.bwd_small + (size_t)kItemInts * (item0 + min(it, nitems - 1)), lane, it < nitems);
-}
-
-// L2 prefetch of a tiny supernode's columns of M_s and row ids.
-__device__ __forceinline__ void tiny_prefetch(const CholArgs& a, int item) {
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(a.tiny + (size_t)kItemInts * item));
-    const float* M = a.mval + ((int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32));
-    const int m = h0.w, k = __ldg(a.tiny + (size_t)kItemInts * item + 4);
-    for (int i = 0; i < k * m; i += 32) prefetch_l2(M + i);
-    prefetch_l2(a.rows + h0.z);
-}
-
-// Tiny supernodes (at most kTinyCols pivots, kTinyRows rows): one thread
-// solves a whole supernode, so the many leaves of a level cost one thread
-// each instead of one warp per item.  Forward: pivot rows store y (only this
-// supernode writes them), off-diagonal rows subtract from r.  Backward:
-// x_c = sum_{i >= c} M[i, c] z_i over the supernode's rows.
-__device__ __forceinline__ void fwd_tiny_item(const CholArgs& a, int item) {
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(a.tiny + (size_t)kItemInts * item));
-    const int k = __ldg(a.tiny + (size_t)kItemInts * item + 4);
-    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    const int m = h0.w;
-    const int* rows = a.rows + h0.z;
-    const float* M = a.mval + moff;
-    float4 rc[kTinyCols];
-#pragma unroll
-    for (int c = 0; c < kTinyCols; ++c) rc[c] = c < k ? a.r[__ldg(&rows[c])] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int i = 0; i < m; ++i) {
-        float ax = 0.f, ay = 0.f, az = 0.f;
-#pragma unroll
-        for (int c = 0; c < kTinyCols; ++c) {
-            if (c < k && c <= i) {
-                const float mv = __ldg(M + (size_t)c * m + i);
-                ax = fmaf(mv, rc[c].x, ax);
-                ay = fmaf(mv, rc[c].y, ay);
-                az = fmaf(mv, rc[c].z, az);
-            }
-        }
-        const int vid = __ldg(&rows[i]);
-        if (i < k) a.y[vid] = make_float4(ax, ay, az, 0.f);
-        else atomicAdd(&a.r[vid], make_float4(-ax, -ay, -az, 0.f));
-    }
-}
-
-__device__ __forceinline__ void bwd_tiny_item(const CholArgs& a, int item) {
-    const int4 h0 = __ldg(reinterpret_cast<const int4*>(a.tiny + (size_t)kItemInts * item));
-    const int k = __ldg(a.tiny + (size_t)kItemInts * item + 4);
-    const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    const int m = h0.w;
-    const int* rows = a.rows + h0.z;
-    const float* M = a.mval + moff;
-    float acc[kTinyCols][3];
-#pragma unroll
-    for (int c = 0; c < kTinyCols; ++c) acc[c][0] = acc[c][1] = acc[c][2] = 0.f;
-#pragma unroll 4
-    for (int i = 0; i < m; ++i) {
-        const int vid = __ldg(&rows[i]);
-        float4 z;
-        if (i < k) z = a.y[vid];
-        else {
-            const float4 xv = a.x[vid];
-            z = make_float4(-xv.x, -xv.y, -xv.z, 0.f);
-        }
-#pragma unroll
-        for (int c = 0; c < kTinyCols; ++c) {
-            if (c < k && c <= i) {
-                const float mv = __ldg(M + (size_t)c * m + i);
-                acc[c][0] = fmaf(mv, z.x, acc[c][0]);
-                acc[c][1] = fmaf(mv, z.y, acc[c][1]);
-                acc[c][2] = fmaf(mv, z.z, acc[c][2]);
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < kTinyCols; ++c)
-        if (c < k) a.x[__ldg(&rows[c])] = make_float4(acc[c][0], acc[c][1], acc[c][2], 0.f);
-}
-
-__global__ void __launch_bounds__(kSmallThreads) k_chol_fwd_tiny(CholArgs a, int t0, int n) {
-    pdl_trigger();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) tiny_prefetch(a, t0 + t);
-    pdl_wait();
-    if (a.done && *a.done) return;
-    if (t < n) fwd_tiny_item(a, t0 + t);
-}
-
-__global__ void __launch_bounds__(kSmallThreads) k_chol_bwd_tiny(CholArgs a, int t0, int n) {
-    pdl_trigger();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) tiny_prefetch(a, t0 + t);
-    pdl_wait();
-    if (a.done && *a.done) return;
-    if (t < n) bwd_tiny_item(a, t0 + t);
-}
-
-// A level's block items and a few warp items in one launch (128-thread
-// CTAs: CTAs 0 .. nb-1 take the block items, the others four warp items
-// each).  Items of one level are independent, so where the warp items are
-// few (the upper levels of a batch, where only some bodies still have small
-// supernodes) they run beside the block items instead of in a launch of a
-// handful of CTAs that the next level's launch would wait for.
-__global__ void __launch_bounds__(kBlockThreads) k_chol_fwd_mixed(CholArgs a, int b0, int nb, int w0, int nw) {
-    __shared__ float4 rs[kFwdBlockCols];
-    __shared__ float4 stage[kBlockThreads / 32][32];
-    pdl_trigger();
-    if ((int)blockIdx.x < nb) {
+    int u = blockIdx.x;
+    if (u < v.nb) {
         FwdBlockPre p;
-        fwd_block_load(a, b0 + blockIdx.x, p);  // static data before the wait
+        fwd_block_load(a, v.b0 + u, p);
         pdl_wait();
         if (a.done && *a.done) return;
         fwd_block_run(a, p, rs);
-    } else {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int it = ((int)blockIdx.x - nb) * (kBlockThreads / 32) + warp;
-        if (it < nw) fwd_warp_prefetch(a, a.fwd_small + (size_t)kItemInts * (w0 + it), lane);
+        return;
+    }
+    u -= v.nb;
+    if (u < small_ctas(v.ns)) {
+        const int it = u * kLevelWarps + warp;
+        SmallPre p;
+        small_load(a, v.s0 + it, it < v.ns, lane, p);
         pdl_wait();
         if (a.done && *a.done) return;
-        if (it < nw) fwd_warp_item(a, a.fwd_small + (size_t)kItemInts * (w0 + it), stage[warp], lane);
+        if (it < v.ns) fwd_small_run(a, p, lane, rs + 32 * warp);
+        return;
     }
+    u -= small_ctas(v.ns);
+    const int it = u * kTinyPerCta + (int)threadIdx.x / kTinyLanes, j = threadIdx.x % kTinyLanes;
+    TinyPre p;
+    tiny_load(a, v.t0 + it, it < v.nt, j, p);
+    pdl_wait();
+    if (a.done && *a.done) return;
+    fwd_tiny_run(a, p, j);
 }
 
-__global__ void __launch_bounds__(kBlockThreads) k_chol_bwd_mixed(CholArgs a, int b0, int nb, int w0, int nw) {
+__global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_bwd_level(CholArgs a, LevelRange v, ResetArgs q) {
+    __shared__ float4 zs[kLevelThreads];
     pdl_trigger();
-    if ((int)blockIdx.x < nb) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int u = blockIdx.x;
+    if (u < v.nb) {
         BwdBlockPre p;
-        bwd_block_load(a, b0 + blockIdx.x, p);
+        bwd_block_load(a, v.b0 + u, p);
         pdl_wait();
         if (a.done && *a.done) return;
-        bwd_block_run(a, p);
-    } else {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int it = ((int)blockIdx.x - nb) * (kBlockThreads / 32) + warp;
-        bwd_warp_item_pre(a, a.bwd_small + (size_t)kItemInts * (w0 + min(it, nw - 1)), lane, it < nw);
+        bwd_block_run(a, p, zs);
+        return;
     }
+    u -= v.nb;
+    if (u < small_ctas(v.ns)) {
+        const int it = u * kLevelWarps + warp;
+        SmallPre p;
+        small_load(a, v.s0 + it, it < v.ns, lane, p);
+        pdl_wait();
+        if (a.done && *a.done) return;
+        if (it < v.ns) bwd_small_run(a, p, lane);
+        return;
+    }
+    u -= small_ctas(v.ns);
+    if (u < tiny_ctas(v.nt)) {
+        const int it = u * kTinyPerCta + (int)threadIdx.x / kTinyLanes, j = threadIdx.x % kTinyLanes;
+        TinyPre p;
+        tiny_load(a, v.t0 + it, it < v.nt, j, p);
+        pdl_wait();
+        if (a.done && *a.done) return;
+        bwd_tiny_run(a, p, j);
+        return;
+    }
+    // resets for the next solve: the right-hand side is dead once the forward
+    // pass is done, and y_next is the buffer this solve does not use
+    u -= tiny_ctas(v.nt);
+    const int i = u * kLevelThreads + threadIdx.x;
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < q.nv && q.b) b = __ldg(&q.coef[i]).z != 0.f ? __ldg(&q.pin_rhs[i]) : __ldg(&q.base[i]);
+    pdl_wait();
+    if ((a.done && *a.done) || i >= q.nv) return;
+    q.y_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q.b) q.b[i] = b;
 }
 
-void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s) {
-    constexpr int kWarps = kSmallThreads / 32;
-    for (size_t L = 0; L < levels.size(); ++L) {
+void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s,
+                              const ResetArgs& reset) {
+    const int nl = (int)levels.size();
+    auto range = [&](int L) {
         const SolveLevel& v = levels[L];
-        const int nb = v.fwdb_end - v.fwdb_begin, nw = v.fwdw_end - v.fwdw_begin, nt = v.tiny_end - v.tiny_begin;
-        if (nt > 0) launch_pdl(k_chol_fwd_tiny, (nt + kSmallThreads - 1) / kSmallThreads, kSmallThreads, 0, s, a, v.tiny_begin, nt);
-        if (mix_level(nb, nw)) {
-            constexpr int kMixWarps = kBlockThreads / 32;
-            launch_pdl(k_chol_fwd_mixed, nb + (nw + kMixWarps - 1) / kMixWarps, kBlockThreads, 0, s, a, v.fwdb_begin, nb,
-                       v.fwdw_begin, nw);
-            continue;
-        }
-        if (nw > 0) launch_pdl(k_chol_fwd_small, (nw + kWarps - 1) / kWarps, kSmallThreads, 0, s, a, v.fwdw_begin, nw);
-        if (nb > 0) launch_pdl(k_chol_fwd_block, nb, kBlockThreads, 0, s, a, v.fwdb_begin);
+        return LevelRange{v.blk_begin, v.blk_end - v.blk_begin, v.sml_begin, v.sml_end - v.sml_begin, v.tiny_begin,
+                          v.tiny_end - v.tiny_begin};
+    };
+    for (int L = 0; L < nl; ++L) {
+        const LevelRange r = range(L);
+        const int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
+        if (grid > 0) launch_pdl(k_chol_fwd_level, grid, kLevelThreads, 0, s, a, r);
     }
-    for (size_t L = levels.size(); L-- > 0;) {
-        const SolveLevel& v = levels[L];
-        const int nb = v.bwdb_end - v.bwdb_begin, nw = v.bwdw_end - v.bwdw_begin, nt = v.tiny_end - v.tiny_begin;
-        const int nz = v.zst_end - v.zst_begin;
-        if (nz > 0) launch_pdl(k_chol_bwd_zstage, nz, kStageThreads, 0, s, a, v.zst_begin);
-        if (mix_level(nb, nw)) {
-            constexpr int kMixWarps = kBlockThreads / 32;
-            launch_pdl(k_chol_bwd_mixed, nb + (nw + kMixWarps - 1) / kMixWarps, kBlockThreads, 0, s, a, v.bwdb_begin, nb,
-                       v.bwdw_begin, nw);
-        } else {
-            if (nb > 0) launch_pdl(k_chol_bwd_block, nb, kBlockThreads, 0, s, a, v.bwdb_begin);
-            if (nw > 0)
-                launch_pdl(k_chol_bwd_small, (nw + kWarps - 1) / kWarps, kSmallThreads, 0, s, a, v.bwdw_begin, nw);
-        }
-        if (nt > 0) launch_pdl(k_chol_bwd_tiny, (nt + kSmallThreads - 1) / kSmallThreads, kSmallThreads, 0, s, a, v.tiny_begin, nt);
+    bool first = reset.y_next != nullptr;
+    for (int L = nl - 1; L >= 0; --L) {
+        const LevelRange r = range(L);
+        int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
+        if (first) grid += (reset.nv + kLevelThreads - 1) / kLevelThreads;
+        if (grid > 0) launch_pdl(k_chol_bwd_level, grid, kLevelThreads, 0, s, a, r, first ? reset : ResetArgs{});
+        first = false;
     }
 }
 
 // ---- the whole solve in one persistent launch over the GPU.
-// All CTAs are resident (cooperative launch), 128 threads each.  Per
-// forward level the CTAs stride over the level's units -- one block item,
-// four warp items or 128 tiny supernodes per unit -- and meet at a
-// grid-wide barrier; per backward level the z staging (when the level has
-// block items) and the backward items are separated by barriers as well.
+// All CTAs are resident (cooperative launch), 128 threads each.  Per level
+// and direction the CTAs stride over the level's units -- one block item,
+// four small supernodes or sixteen tiny ones -- and meet at a grid-wide
+// barrier.
 // The barrier spins for a bounded time: past the limit it sets a sticky
 // timeout word and every CTA returns at its next barrier (the step's result
 // is then invalid and the engine reports PDGB_ERR_TIMEOUT).
@@ -633,58 +606,48 @@ __device__ __forceinline__ bool grid_sync(GridSync* g, unsigned& gen, unsigned e
     return ok;
 }
 
-__global__ void __launch_bounds__(kBlockThreads) k_chol_solve_persistent(CholArgs a, const SolveLevel* __restrict__ lv,
+__global__ void __launch_bounds__(kLevelThreads) k_chol_solve_persistent(CholArgs a, const SolveLevel* __restrict__ lv,
                                                                          int nl, GridSync* bar, long long spin) {
-    __shared__ float4 rs[kFwdBlockCols];
-    __shared__ float4 stage[kBlockThreads / 32][32];
+    __shared__ float4 rs[kLevelThreads];
     if (a.done && *a.done) return;  // set before this launch: the same for every CTA
-    constexpr int kWarps = kBlockThreads / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned expect = gridDim.x;
     unsigned gen = 0;
-    for (int L = 0; L < nl; ++L) {
-        const SolveLevel v = lv[L];
-        const int nb = v.fwdb_end - v.fwdb_begin, nw = v.fwdw_end - v.fwdw_begin, nt = v.tiny_end - v.tiny_begin;
-        const int nwu = (nw + kWarps - 1) / kWarps, ntu = (nt + kBlockThreads - 1) / kBlockThreads;
-        for (int u = blockIdx.x; u < nb + nwu + ntu; u += gridDim.x) {
+    for (int pass = 0; pass < 2 * nl; ++pass) {
+        const bool fwd = pass < nl;
+        const SolveLevel v = lv[fwd ? pass : 2 * nl - 1 - pass];
+        const int nb = v.blk_end - v.blk_begin, ns = v.sml_end - v.sml_begin, nt = v.tiny_end - v.tiny_begin;
+        const int nsu = small_ctas(ns), ntu = tiny_ctas(nt);
+        for (int u = blockIdx.x; u < nb + nsu + ntu; u += gridDim.x) {
+            __syncthreads();  // rs of the previous unit is read
             if (u < nb) {
-                __syncthreads();  // rs of the previous block item is read
-                FwdBlockPre p;
-                fwd_block_load(a, v.fwdb_begin + u, p);
-                fwd_block_run(a, p, rs);
-            } else if (u < nb + nwu) {
-                const int it = (u - nb) * kWarps + warp;
-                if (it < nw) fwd_warp_item(a, a.fwd_small + (size_t)kItemInts * (v.fwdw_begin + it), stage[warp], lane);
+                if (fwd) {
+                    FwdBlockPre p;
+                    fwd_block_load(a, v.blk_begin + u, p);
+                    fwd_block_run(a, p, rs);
+                } else {
+                    BwdBlockPre p;
+                    bwd_block_load(a, v.blk_begin + u, p);
+                    bwd_block_run(a, p, rs);
+                }
+            } else if (u < nb + nsu) {
+                const int it = (u - nb) * kLevelWarps + warp;
+                SmallPre p;
+                small_load(a, v.sml_begin + it, it < ns, lane, p);
+                if (it < ns) {
+                    if (fwd) fwd_small_run(a, p, lane, rs + 32 * warp);
+                    else bwd_small_run(a, p, lane);
+                }
             } else {
-                const int t = (u - nb - nwu) * kBlockThreads + threadIdx.x;
-                if (t < nt) fwd_tiny_item(a, v.tiny_begin + t);
+                const int it = (u - nb - nsu) * kTinyPerCta + (int)threadIdx.x / kTinyLanes,
+                          j = threadIdx.x % kTinyLanes;
+                TinyPre p;
+                tiny_load(a, v.tiny_begin + it, it < nt, j, p);
+                if (fwd) fwd_tiny_run(a, p, j);
+                else bwd_tiny_run(a, p, j);
             }
         }
-        if (!grid_sync(bar, gen, expect, spin)) return;
-    }
-    for (int L = nl - 1; L >= 0; --L) {
-        const SolveLevel v = lv[L];
-        const int nz = v.zst_end - v.zst_begin;
-        if (nz > 0) {
-            for (int u = blockIdx.x; u < nz; u += gridDim.x) zstage_item(a, v.zst_begin + u, false);
-            if (!grid_sync(bar, gen, expect, spin)) return;
-        }
-        const int nb = v.bwdb_end - v.bwdb_begin, nw = v.bwdw_end - v.bwdw_begin, nt = v.tiny_end - v.tiny_begin;
-        const int nwu = (nw + kWarps - 1) / kWarps, ntu = (nt + kBlockThreads - 1) / kBlockThreads;
-        for (int u = blockIdx.x; u < nb + nwu + ntu; u += gridDim.x) {
-            if (u < nb) {
-                BwdBlockPre p;
-                bwd_block_load(a, v.bwdb_begin + u, p);
-                bwd_block_run(a, p);
-            } else if (u < nb + nwu) {
-                const int it = (u - nb) * kWarps + warp;
-                if (it < nw) bwd_warp_item(a, a.bwd_small + (size_t)kItemInts * (v.bwdw_begin + it), stage[warp], lane);
-            } else {
-                const int t = (u - nb - nwu) * kBlockThreads + threadIdx.x;
-                if (t < nt) bwd_tiny_item(a, v.tiny_begin + t);
-            }
-        }
-        if (L > 0 && !grid_sync(bar, gen, expect, spin)) return;
+        if (pass + 1 < 2 * nl && !grid_sync(bar, gen, expect, spin)) return;
     }
 }
 
@@ -698,7 +661,7 @@ int persistent_grid() {
     if (!grid[dev]) {
         int sms = 0, per = 0;
         PDGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PDGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_chol_solve_persistent, kBlockThreads, 0));
+        PDGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_chol_solve_persistent, kLevelThreads, 0));
         int cap = 8;
         if (const char* e = std::getenv("PDGB_PERSIST_CTAS_PER_SM")) cap = std::max(1, std::atoi(e));
         grid[dev] = sms * std::max(1, std::min(per, cap));
@@ -712,7 +675,7 @@ void launch_chol_solve_persistent(const CholArgs& a, const SolveLevel* levels, i
     PDGB_CUDA_TRY(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s));  // arrival count and generation
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(persistent_grid());
-    cfg.blockDim = dim3(kBlockThreads);
+    cfg.blockDim = dim3(kLevelThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -736,7 +699,7 @@ void launch_grid_sync_check(GridSync* bar, int ctas, int rounds, int missing, lo
     PDGB_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(GridSync), s));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kBlockThreads);
+    cfg.blockDim = dim3(kLevelThreads);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

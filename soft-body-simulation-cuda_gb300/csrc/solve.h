@@ -27,18 +27,28 @@ struct CholArgs {
     float4* y;  // forward result (must be zero on entry)
     float4* x;  // solution out
     const int* done;  // early-exit flag of the step (tol rule), may be null
-    const int* fwd_blocks;  // CTA block items (per-level launches)
-    const int* bwd_blocks;
-    const int* fwd_small;   // warp items of small supernodes (per-level launches)
-    const int* bwd_small;
-    const int* tiny;        // tiny supernode descriptors (per-level launches)
-    const int* zstage;      // backward z-staging items (per-level launches)
-    float4* zbuf;           // staged z of the block supernodes
+    const int* blocks;      // block items (per-level launches, both directions)
+    const int* small;       // small supernodes (per-level launches)
+    const int* tiny;        // tiny supernodes (per-level launches)
 };
 
-constexpr int kBlockThreads = 128;      // block-item kernels: 4 warps
-constexpr int kSmallThreads = 256;      // small-supernode kernels: one warp item per warp
-constexpr int kStageThreads = 128;      // backward z staging: one CTA per 128-row chunk (kStageRows)
+// What the first backward launch of a solve resets beside its own items, so
+// that no vertex kernel is needed between iterations: y_next, the y buffer of
+// the next solve, to zero, and (b not null) the right-hand side of the next
+// iteration to base, or to the pin term at pinned vertices.
+struct ResetArgs {
+    int nv;
+    float4* y_next;         // null: nothing is reset
+    float4* b;
+    const float4* base;
+    const float4* coef;
+    const float4* pin_rhs;
+};
+
+constexpr int kLevelThreads = kTileRows;  // per-level kernels: one thread a tile row
+// Resident CTAs per SM the per-level kernels' registers are allocated for.
+constexpr int kLevelMinBlocks = 8;
+constexpr int kTinyLanes = 8;             // lanes of a tiny supernode: most have 7 rows
 
 // Grid-wide barrier of the persistent solve (device memory): arrivals and
 // generation are cleared before each launch; timeout is set when a wait
@@ -80,15 +90,8 @@ struct CholVertexArgs {
 };
 
 // One launch per level and direction (large systems).
-void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s);
-// Whether a level's warp items go into its block launch: when there are
-// block items and at most kMixWarpsPerBlock warp items per block item.  The
-// leaf levels of a batch, with many warp items and few blocks, keep their
-// own launch of 256-thread CTAs (merging every level measured 2 % faster on
-// the 40^3 cube and 2 % slower on the 512-body batch; 8 or 32 per block:
-// the same on the batch, 32 better on the cube).
-constexpr int kMixWarpsPerBlock = 32;
-inline bool mix_level(int nb, int nw) { return nb > 0 && nw > 0 && nw <= kMixWarpsPerBlock * nb; }
+void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s,
+                              const ResetArgs& reset = ResetArgs{});
 // The whole solve in one persistent cooperative launch over the GPU (all
 // bodies of a batch), levels separated by a bounded grid barrier; levels is
 // the device copy of the per-level item ranges.
