@@ -296,9 +296,12 @@ void record_chol_step(pdgb_engine* e) {
     ba.iterations = &st->iterations;
     ba.prev = use_tol ? e->prev.p : nullptr;
     launch_begin(ba, s);
-    const LocalArgs la = local_args(e, &st->done);
+    // without the convergence test nothing sets the flag: the step's kernels do
+    // not wait for a read of it
+    const int* done = use_tol ? &st->done : nullptr;
+    const LocalArgs la = local_args(e, done);
     CholArgs ca{e->ch_fwd.p, e->ch_bwd.p, e->ch_rows.p, e->ch_mval.p, e->ch_levels.p, e->ch_body_level.p,
-                e->ch_body_order.p, e->b.p, e->y.p, e->sn.p, &st->done, e->ch_blocks.p, e->ch_small.p, e->ch_tiny.p};
+                e->ch_body_order.p, e->b.p, e->y.p, e->sn.p, done, e->ch_blocks.p, e->ch_small.p, e->ch_tiny.p};
     CholVertexArgs cv{};
     cv.nv = e->nv;
     cv.tol = use_tol ? e->prm.tol : 0.f;
@@ -317,7 +320,7 @@ void record_chol_step(pdgb_engine* e) {
     const bool drag_rhs = cv.sc.drag_w && cv.sc.drag_rhs;
     const int refine = e->nbodies == 1 ? e->prm.refine_steps : 0;
     RefineArgs ra{e->nv, e->k_rowptr.p, e->k_colind.p, e->k_val.p, e->bsave.p, e->sn.p, e->b.p, e->y.p,
-                  e->dx.p, e->sn.p, &st->done};
+                  e->dx.p, e->sn.p, done};
     // Per-level launches without the convergence test: each solve's backward
     // pass clears the y buffer of the next solve (two alternate) and the last
     // solve of an iteration resets b, so that no vertex kernel runs between
@@ -346,8 +349,8 @@ void record_chol_step(pdgb_engine* e) {
     };
     for (int i = 0; i < n; ++i) {
         record_local(e, la, false, i);
-        if (drag_rhs) launch_drag_rhs(e->nv, cv.sc, e->base.p, e->b.p, &st->done, s);
-        if (refine > 0) launch_copy_rhs(e->nv, e->b.p, e->bsave.p, &st->done, s);
+        if (drag_rhs) launch_drag_rhs(e->nv, cv.sc, e->base.p, e->b.p, done, s);
+        if (refine > 0) launch_copy_rhs(e->nv, e->b.p, e->bsave.p, done, s);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i], s, cudaEventRecordExternal));
         solve(e->sn.p, refine == 0);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i + 1], s, cudaEventRecordExternal));
@@ -1552,6 +1555,13 @@ int pdgb_inspect_layout(const pdgb_mesh_desc* mesh, pdgb_layout_info* info, int*
 }
 
 namespace {
+// Entries of the M_s blocks, without the padding of their columns.
+long long m_entries(const CholFactor& f) {
+    long long n = 0;
+    for (int q = 0; q < f.nsuper; ++q) n += (long long)f.sk[q] * f.sm[q];
+    return n;
+}
+
 // Kernel launches of one solve in the schedule in use.
 int solve_launches(const pdgb_engine* e) {
     if (e->solve_mode != PDGB_SOLVE_LEVELS) return 1;  // PERSISTENT: one launch (and a barrier reset)
@@ -1568,7 +1578,7 @@ int pdgb_get_factor_info(pdgb_engine* e, pdgb_factor_info* info) {
     if (e->prm.solver != PDGB_SOLVER_CHOLESKY || e->chol.n != e->nv) return PDGB_OK;
     const CholFactor& f = e->chol;
     info->nnz_L = f.nnz_L;
-    info->m_entries = (long long)f.mval_size;
+    info->m_entries = m_entries(f);
     info->num_supernodes = f.nsuper;
     info->num_levels = f.nlevels;
     info->fwd_items = (int)(f.fwd_items.size() / kItemInts);
@@ -1599,10 +1609,15 @@ int pdgb_get_factor_blocks(pdgb_engine* e, float* out, long long capacity) {
     return guarded([&] {
         if (e->prm.solver != PDGB_SOLVER_CHOLESKY || e->chol.n != e->nv || !e->ch_mval.p)
             throw Error{PDGB_ERR_INVALID_ARGUMENT, "no prepared Cholesky factor"};
-        const long long n = (long long)e->chol.mval_size;
-        if (capacity < n) throw Error{PDGB_ERR_INVALID_ARGUMENT, "capacity below the factor's m_entries"};
-        PDGB_CUDA_TRY(cudaMemcpyAsync(out, e->ch_mval.p, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+        const CholFactor& f = e->chol;
+        if (capacity < m_entries(f)) throw Error{PDGB_ERR_INVALID_ARGUMENT, "capacity below the factor's m_entries"};
+        std::vector<float> padded((size_t)std::max<int64_t>(f.mval_size, 1));
+        PDGB_CUDA_TRY(cudaMemcpyAsync(padded.data(), e->ch_mval.p, (size_t)f.mval_size * sizeof(float),
+                                      cudaMemcpyDeviceToHost, e->stream));
         PDGB_CUDA_TRY(cudaStreamSynchronize(e->stream));
+        for (int q = 0; q < f.nsuper; ++q)  // the caller's blocks are not padded
+            for (int c = 0; c < f.sk[q]; ++c, out += f.sm[q])
+                std::memcpy(out, &padded[f.moff[q] + (int64_t)c * m_stride(f.sm[q], f.sk[q])], f.sm[q] * sizeof(float));
     });
 }
 
@@ -1630,7 +1645,7 @@ int pdgb_host_factor_check(const pdgb_mesh_desc* mesh, const pdgb_params* params
         const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (info) {
             info->nnz_L = f.nnz_L;
-            info->m_entries = (long long)f.mval_size;
+            info->m_entries = m_entries(f);
             info->num_supernodes = f.nsuper;
             info->num_levels = f.nlevels;
             info->fwd_items = (int)(f.fwd_items.size() / kItemInts);

@@ -406,7 +406,7 @@ std::vector<int> postorder(const std::vector<int>& parent) {
 // multiply-add (spread over the solves of about a hundred steps).
 std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& fm, const std::vector<int>& fpar,
                             double level_entries) {
-    constexpr double kEntriesPerFlop = 1e-3;
+    constexpr double kEntriesPerFlop = 3e-4;
     const int nf = (int)fk.size();
     std::vector<int> sub(fk);  // columns of the subtree
     int n = 0;
@@ -638,7 +638,7 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
         out.sm[s] = (int)sstruct[s].size();
         out.moff[s] = mtot;
         out.roff[s] = (int)rtot;
-        mtot += (int64_t)out.sk[s] * out.sm[s];
+        mtot += (int64_t)out.sk[s] * m_stride(out.sm[s], out.sk[s]);
         rtot += out.sm[s];
     }
     out.moff[ns] = mtot;
@@ -740,7 +740,7 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
                 if (xq != 0.0)
                     for (int j = q + 1; j < k; ++j) x[j] -= Lq[j] * xq;
             }
-            float* Mc = M + (size_t)c * m;
+            float* Mc = M + (size_t)c * m_stride(m, k);
             for (int r = 0; r < k; ++r) Mc[r] = (float)x[r];
             if (m > k) {
                 std::vector<double> acc(m - k, 0.0);
@@ -792,7 +792,7 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
             for (int c = 0; c < k; ++c) out.bwd_items.insert(out.bwd_items.end(), {lo, hi, out.roff[s], m, k, c, 0, 0});
             if (k == 1 && m <= kTinyRows) {
                 out.tiny.insert(out.tiny.end(), {lo, hi, out.roff[s], m, k, 0, 0, 0});
-            } else if (m < kBlockMinRows && k <= kSmallCols) {
+            } else if (is_small(m, k)) {
                 out.small.insert(out.small.end(), {lo, hi, out.roff[s], m, k, 0, 0, 0});
             } else {
                 for (int r0 = 0; r0 < m; r0 += kTileRows) {
@@ -1071,12 +1071,13 @@ void cholesky_solve_host(const CholFactor& f, const double* b3, double* x3) {
             const int* w = &f.fwd_items[kItemInts * (size_t)it];
             const int roff = w[2], m = w[3], k = w[4], r0 = w[5], c0 = w[6], c1 = w[7];
             const float* M = &f.mval[moff_of(w)];
+            const size_t ld = m_stride(m, k);
             const int* rows = &f.rows[roff];
             for (int row = r0; row < std::min(m, r0 + kFwdItemRows); ++row) {
                 double acc[3] = {0, 0, 0};
                 const int cend = row < k ? std::min(c1, row + 1) : c1;
                 for (int c = c0; c < cend; ++c)
-                    for (int d = 0; d < 3; ++d) acc[d] += (double)M[(size_t)c * m + row] * r[3 * (size_t)rows[c] + d];
+                    for (int d = 0; d < 3; ++d) acc[d] += (double)M[c * ld + row] * r[3 * (size_t)rows[c] + d];
                 const size_t o = 3 * (size_t)rows[row];
                 for (int d = 0; d < 3; ++d) {
                     if (row < k) y[o + d] += acc[d];
@@ -1095,7 +1096,7 @@ void cholesky_solve_host(const CholFactor& f, const double* b3, double* x3) {
             double acc[3] = {0, 0, 0};
             for (int i = c; i < m; ++i) {
                 const size_t o = 3 * (size_t)rows[i];
-                const double mv = M[(size_t)c * m + i];
+                const double mv = M[(size_t)c * m_stride(m, k) + i];
                 for (int d = 0; d < 3; ++d) acc[d] += mv * (i < k ? y[o + d] : -x3[o + d]);
             }
             for (int d = 0; d < 3; ++d) x3[3 * (size_t)rows[c] + d] = acc[d];
@@ -1138,7 +1139,10 @@ void build_dsm_plan(const CholFactor& f, int ctas, int warps_per_cta, size_t max
         for (int s : mine[c]) {
             moff_smem[s] = mo;
             const int64_t cnt = (int64_t)f.sm[s] * f.sk[s];
-            plan.mcopy.insert(plan.mcopy.end(), f.mval.begin() + f.moff[s], f.mval.begin() + f.moff[s] + cnt);
+            for (int j = 0; j < f.sk[s]; ++j) {  // back to back there: columns m apart
+                const auto col = f.mval.begin() + f.moff[s] + (int64_t)j * m_stride(f.sm[s], f.sk[s]);
+                plan.mcopy.insert(plan.mcopy.end(), col, col + f.sm[s]);
+            }
             mo += (int)cnt;
             roff_smem[s] = ro;
             plan.rcopy.insert(plan.rcopy.end(), f.rows.begin() + f.roff[s], f.rows.begin() + f.roff[s] + f.sm[s]);

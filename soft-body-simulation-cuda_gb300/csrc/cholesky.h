@@ -10,7 +10,8 @@
 // Solve representation.  For every supernode s with pivot columns C_s
 // (k_s of them) and off-diagonal rows O_s (m_s - k_s), the GPU stores the
 // m_s x k_s matrix
-//     M_s = [ L_ss^-1 ; L_os L_ss^-1 ]       (column major, FP32)
+//     M_s = [ L_ss^-1 ; L_os L_ss^-1 ]       (column major, FP32, columns
+//                                              m_stride floats apart)
 // so that the forward step of s is y_s = L_ss^-1 r_s plus the update
 // r_O -= (L_os L_ss^-1) r_s, and the backward step is
 // x_s = (L_ss^-1)^T y_s - (L_os L_ss^-1)^T x_O: both are dense
@@ -61,16 +62,35 @@ constexpr int kFwdItemCols = 64;
 //          rows r0 .. r0 + kTileRows and pivot columns c0 .. c1 (at most
 //          kTileCols), for one CTA and both directions
 //   small: {moff_lo, moff_hi, roff, m, k, 0, 0, 0}: a whole supernode of fewer
-//          than kBlockMinRows rows and at most kSmallCols pivots, for a warp
+//          than kSmallRows rows and at most kSmallCols pivots, for a warp
 //   tiny : the same for a supernode of one pivot and at most kTinyRows rows
-// A tile has one thread a row (forward) and 8 columns a warp (backward), 32
-// entries a thread: enough loads in flight with 8 CTAs on an SM, and few
-// enough registers for them.
 constexpr int kTileRows = 128;
 constexpr int kTileCols = 32;
-constexpr int kBlockMinRows = 64;
+constexpr int kSmallRows = 64;
 constexpr int kSmallCols = 32;
 constexpr int kTinyRows = 32;
+// Shared memory of a warp that takes a small supernode: its block, then z of
+// its rows, in floats.
+constexpr int kSmallFloats = 896;
+constexpr int kWarpFloats = kSmallFloats + 4 * kSmallRows;
+static_assert(4 * kWarpFloats >= kTileRows * kTileCols, "a tile fits the same shared memory");
+
+#ifdef __CUDACC__
+#define PDGB_HD __host__ __device__
+#else
+#define PDGB_HD
+#endif
+// Floats between the columns of M_s: a multiple of 4, so that its rows can be
+// loaded 16 bytes at a time; of a supernode that a warp copies whole, an odd
+// multiple, so that the 8 lanes of a quarter-warp that read 4 rows of 8
+// neighbouring columns in shared memory hit 8 groups of banks.
+PDGB_HD inline int m_stride(int m, int k) {
+    const int q = (m + 3) / 4;
+    return 4 * (k > 1 && k <= kSmallCols && m < kSmallRows ? (q | 1) : q);
+}
+PDGB_HD inline bool is_small(int m, int k) {
+    return m < kSmallRows && k <= kSmallCols && k * m_stride(m, k) <= kSmallFloats;
+}
 
 // Numeric factorisation on the GPU (factor.cu): everything the device needs
 // beyond the symbolic structure of CholFactor.  Each supernode s has a dense
@@ -102,7 +122,7 @@ struct CholFactor {
     double flops = 0.0;
     // per supernode
     std::vector<int> sk, sm;         // pivot count k_s, row count m_s
-    std::vector<int64_t> moff;       // offset of M_s in mval (column major m x k)
+    std::vector<int64_t> moff;       // offset of M_s in mval (column major m x k, columns m_stride apart)
     std::vector<int> roff;           // offset of the row list in rows
     std::vector<int> rows;           // row lists (vertex ids; first k = pivots)
     std::vector<float> mval;         // FP32 M_s blocks, column major

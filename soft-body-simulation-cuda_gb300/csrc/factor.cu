@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(256) k_fm(FDev d, const int2* __restrict__ ite
     const double* F = d.pool + d.foff[s];
     double* X = d.pool + d.foff[s] + (int64_t)m * m;
     float* M = d.mval + d.moff[s];
+    const int64_t ld = m_stride(m, k);
     __shared__ double Xs[kNB][kNB + 1];
     __shared__ double Xq[kNB][kNB + 1];
     __shared__ double Lq[kNB][kNB + 1];
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(256) k_fm(FDev d, const int2* __restrict__ ite
             if (col < k && row < m) {
                 const double v = Xs[tr][tc + 8 * u];
                 X[(int64_t)col * m + row] = v;
-                M[(int64_t)col * m + row] = (float)v;
+                M[col * ld + row] = (float)v;
             }
         }
     }

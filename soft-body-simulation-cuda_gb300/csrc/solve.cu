@@ -40,6 +40,7 @@ __device__ __forceinline__ void fwd_warp_item(const CholArgs& a, const int* w, f
     const bool valid = row < m;
     const int cend = !valid ? c0 : (row < k ? min(c1, row + 1) : c1);
     const float* Mr = a.mval + moff + row;
+    const int ld = m_stride(m, k);
     const int vid = valid ? __ldg(&rows[row]) : 0;
     float ax = 0.f, ay = 0.f, az = 0.f;
     for (int cb = c0; cb < c1; cb += 32) {
@@ -50,7 +51,7 @@ __device__ __forceinline__ void fwd_warp_item(const CholArgs& a, const int* w, f
         for (int c = cb; c < cb + nc; c += 8) {
             float mv[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) mv[q] = (c + q < cend) ? __ldg(Mr + (size_t)(c + q) * m) : 0.f;
+            for (int q = 0; q < 8; ++q) mv[q] = (c + q < cend) ? __ldg(Mr + (size_t)(c + q) * ld) : 0.f;
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 if (c + q < cb + nc) {
@@ -79,7 +80,7 @@ __device__ __forceinline__ void bwd_warp_item(const CholArgs& a, const int* w, f
     const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
     const int roff = h0.z, m = h0.w, k = h1.x, c = h1.y;
     const int* rows = a.rows + roff;
-    const float* Mc = a.mval + moff + (size_t)c * m;
+    const float* Mc = a.mval + moff + (size_t)c * m_stride(m, k);
     float ax = 0.f, ay = 0.f, az = 0.f;
 #pragma unroll 4
     for (int i = c + lane; i < m; i += 32) {
@@ -105,83 +106,134 @@ __device__ __forceinline__ void bwd_warp_item(const CholArgs& a, const int* w, f
 }
 
 // ---- per-level launches: one per level and direction.  A launch's CTAs
-// (kLevelThreads threads) take, by index, first the level's block items, then
-// its small supernodes (one warp each), then its tiny ones (kTinyLanes lanes
-// each), then -- in the solve's first backward launch, when asked -- the
-// resets of the next iteration's vectors.  Each CTA reads its descriptors,
-// row ids and factor entries into registers before the grid dependency wait,
-// so that a level's factor bytes are under way while the level before drains;
-// after the wait come one gather from L2, the products, one reduction and the
-// stores.  What bounds a narrow level is that chain of latencies, about 3 us
-// with the launch, so a level is one launch and nothing is staged by another.
+// (kLevelThreads threads) take, by index, first the level's block items (a
+// 128 x 32 tile of M_s, 32 rows a warp), then its small supernodes (one warp
+// each), then its tiny ones (kTinyLanes lanes each), then -- in the solve's
+// first backward launch, when asked -- the resets of the next iteration's
+// vectors.
+//
+// What bounds a narrow level is the chain launch -> descriptor -> factor
+// entries -> gather -> products -> scatter, each a trip to L2 or HBM; what
+// bounds a wide one is how many bytes its resident CTAs have on the way and
+// how many shared-memory accesses they queue.  So a tile's entries are copied
+// 16 bytes a lane, asynchronously, before the grid dependency wait: 16 KB a
+// CTA that hold no registers, 11 CTAs on an SM.  A lane copies and uses 4 rows
+// of 8 columns: forward it needs one staged right-hand side for 12 products,
+// backward its 4 rows' z once for all 96.  After the wait come one gather, the
+// products, a few exchanges and the scatter.  A warp uses only its own part of
+// the shared memory until the backward tile's last sum.
+// Holding the tile in registers instead (8 and 7 CTAs) is 4 to 8 % slower on
+// the 40^3 cube and on a batch of 128 bodies; one row or column a lane takes
+// twice the shared-memory accesses and sums chains of 32.
+__device__ __forceinline__ void cp_async16(void* dst, const float* src, bool live) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Block item {moff, roff, m, k, r0, c0, c1}: the tile rows r0 .. r0 + 128,
-// pivot columns c0 .. c1 (at most 32) of M_s; both directions use the same
-// items.
-struct BlockItem {
-    const float* M;   // M_s, column major
+struct Supernode {
+    const float* M;   // M_s, column major, columns ld apart
     const int* rows;
-    int m, k, r0, c0, c1;
+    int m, k, ld;
 };
 
-__device__ __forceinline__ BlockItem block_item(const CholArgs& a, const int* list, int item) {
-    const int4* w = reinterpret_cast<const int4*>(list + (size_t)kItemInts * item);
-    const int4 h0 = __ldg(w), h1 = __ldg(w + 1);
+__device__ __forceinline__ Supernode supernode(const CholArgs& a, const int4 h0, int k) {
     const int64_t moff = (int64_t)(uint32_t)h0.x | ((int64_t)h0.y << 32);
-    return BlockItem{a.mval + moff, a.rows + h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    return Supernode{a.mval + moff, a.rows + h0.z, h0.w, k, m_stride(h0.w, k)};
 }
 
-// Forward block, static part: thread t owns row r0 + t, its (at most 32)
-// entries of the tile in registers.  A warp's loads of one column are
-// contiguous.
-struct FwdBlockPre {
-    float mv[kTileCols];
-    int vid, sv, ncols, row, k, m;
-    bool first;   // the tile holds the first pivot columns
+// Block item {moff, roff, m, k, r0, c0, c1}: warp w takes the rows
+// r0 + 32 w .. + 32 of the tile; lane l holds the rows rw + 4 (l & 7) .. + 4
+// of the columns c0 + 4 q + (l >> 3), q < 8 (zero past the last row or
+// column), the vertex of row rw + l and that of pivot column c0 + l.
+constexpr int kLaneCols = kTileCols / 4;
+struct TilePre {
+    int vid, cvid;    // -1: none
+    int row, k, m;
+    bool first;       // the tile holds the first pivot columns
 };
 
-__device__ __forceinline__ void fwd_block_load(const CholArgs& a, int item, FwdBlockPre& p) {
-    const BlockItem b = block_item(a, a.blocks, item);
-    const int row = b.r0 + threadIdx.x;
-    const bool active = row < b.m && row >= b.c0;  // rows above the tile's columns have nothing in it
-    const int cend = !active ? b.c0 : (row < b.k ? min(b.c1, row + 1) : b.c1);
-    const float* Mr = b.M + row;
+__device__ __forceinline__ void tile_load(const CholArgs& a, int item, float4* tile, TilePre& p) {
+    const int4* w = reinterpret_cast<const int4*>(a.blocks + (size_t)kItemInts * item);
+    const int4 h0 = __ldg(w), h1 = __ldg(w + 1);
+    const Supernode s = supernode(a, h0, h1.x);
+    const int r0 = h1.y, c0 = h1.z, c1 = h1.w;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rw = r0 + 32 * warp, i = rw + 4 * (lane & 7), cl = c0 + (lane >> 3);
+    // rows above the first column hold zeros, and so does the padding of a column
+    const int cend = i < s.m && i + 3 >= c0 ? c1 : c0;
+    const float* col = s.M + (size_t)cl * s.ld + i;
+    float4* t = tile + 32 * kLaneCols * warp + lane;
 #pragma unroll
-    for (int q = 0; q < kTileCols; ++q) p.mv[q] = (b.c0 + q < cend) ? __ldg(Mr + (size_t)(b.c0 + q) * b.m) : 0.f;
-    p.vid = active ? __ldg(&b.rows[row]) : -1;
-    p.ncols = b.c1 - b.c0;
-    p.sv = (int)threadIdx.x < p.ncols ? __ldg(&b.rows[b.c0 + threadIdx.x]) : 0;
-    p.row = row;
-    p.k = b.k;
-    p.m = b.m;
-    p.first = b.c0 == 0;
+    for (int q = 0; q < kLaneCols; ++q) {
+        const bool live = cl + 4 * q < cend;
+        cp_async16(t + 32 * q, live ? col + (size_t)(4 * q) * s.ld : a.mval, live);
+    }
+    p.row = rw + lane;
+    p.k = s.k;
+    p.m = s.m;
+    p.first = c0 == 0;
+    p.vid = p.row < s.m && p.row >= c0 ? __ldg(&s.rows[p.row]) : -1;
+    p.cvid = c0 + lane < c1 ? __ldg(&s.rows[c0 + lane]) : -1;
 }
 
-// Vector part: the pivot right-hand sides staged in shared memory, then the
-// row's sum into y (pivot rows; stored where no other tile adds to it) or out
-// of r (ancestor rows, pivots of later levels).  The backward pass adds the
-// partial sums of a supernode with more rows than a tile into x, which is
-// cleared here.
-__device__ __forceinline__ void fwd_block_run(const CholArgs& a, const FwdBlockPre& p, float4* rs) {
-    if (threadIdx.x < kTileCols)
-        rs[threadIdx.x] = (int)threadIdx.x < p.ncols ? __ldcg(&a.r[p.sv]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    if (p.vid < 0) return;
-    float ax = 0.f, ay = 0.f, az = 0.f;
+// Halving exchange between the lanes that differ in bit `off`: each keeps
+// half of its 2 n values (the upper half where the bit is set) and adds the
+// partner's.
+template <int n>
+__device__ __forceinline__ void halve(float3 (&v)[2 * n], int lane, int off) {
+    const bool up = lane & off;
 #pragma unroll
-    for (int q = 0; q < kTileCols; ++q) {
-        const float4 v = rs[q];
-        ax = fmaf(p.mv[q], v.x, ax);
-        ay = fmaf(p.mv[q], v.y, ay);
-        az = fmaf(p.mv[q], v.z, az);
+    for (int j = 0; j < n; ++j) {
+        const float3 give = up ? v[j] : v[j + n], keep = up ? v[j + n] : v[j];
+        v[j] = make_float3(keep.x + __shfl_xor_sync(0xffffffffu, give.x, off),
+                           keep.y + __shfl_xor_sync(0xffffffffu, give.y, off),
+                           keep.z + __shfl_xor_sync(0xffffffffu, give.z, off));
     }
-    if (p.row >= p.k) {
-        atomicAdd(&a.r[p.vid], make_float4(-ax, -ay, -az, 0.f));
+}
+
+__device__ __forceinline__ void fma3(float3& s, float m, const float4& v) {
+    s.x = fmaf(m, v.x, s.x);
+    s.y = fmaf(m, v.y, s.y);
+    s.z = fmaf(m, v.z, s.z);
+}
+
+// Forward: each lane's four row sums over its eight columns, exchanged so
+// that lane l ends with the row 4 (l & 7) + 2 (l >> 3 & 1) + (l >> 4); the sum
+// goes into y (pivot rows; stored where no other tile adds to it) or out of r
+// (ancestor rows, pivots of later levels).  The backward pass adds the partial
+// sums of a supernode with more rows than a tile into x, which is cleared
+// here.
+__device__ __forceinline__ void fwd_tile_run(const CholArgs& a, const TilePre& p, const float4* tile, float4* vec) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* rs = vec + 32 * warp;
+    rs[lane] = p.cvid >= 0 ? __ldcg(&a.r[p.cvid]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int mine = 4 * (lane & 7) + 2 * (lane >> 3 & 1) + (lane >> 4);
+    const int vid = __shfl_sync(0xffffffffu, p.vid, mine), row = p.row - lane + mine;
+    cp_async_wait();
+    __syncwarp();
+    const float4* t4 = tile + 32 * kLaneCols * warp + lane;
+    float3 s[4] = {};
+#pragma unroll
+    for (int q = 0; q < kLaneCols; ++q) {
+        const float4 v = rs[4 * q + (lane >> 3)], m = t4[32 * q];
+        fma3(s[0], m.x, v);
+        fma3(s[1], m.y, v);
+        fma3(s[2], m.z, v);
+        fma3(s[3], m.w, v);
+    }
+    halve<2>(s, lane, 8);
+    float3 t[2] = {s[0], s[1]};
+    halve<1>(t, lane, 16);
+    if (vid < 0) return;
+    if (row >= p.k) {
+        atomicAdd(&a.r[vid], make_float4(-t[0].x, -t[0].y, -t[0].z, 0.f));
         return;
     }
-    if (p.row < kTileCols) a.y[p.vid] = make_float4(ax, ay, az, 0.f);
-    else atomicAdd(&a.y[p.vid], make_float4(ax, ay, az, 0.f));
-    if (p.first && p.m > kTileRows) a.x[p.vid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 sum = make_float4(t[0].x, t[0].y, t[0].z, 0.f);
+    if (row < kTileCols) a.y[vid] = sum;
+    else atomicAdd(&a.y[vid], sum);
+    if (p.first && p.m > kTileRows) a.x[vid] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // z of a row: y at a pivot, -x at an ancestor.
@@ -191,202 +243,115 @@ __device__ __forceinline__ float4 z_of(const CholArgs& a, bool pivot, int vid) {
     return make_float4(-v.x, -v.y, -v.z, 0.f);
 }
 
-// Sums of 8 columns x 3 coordinates over the 32 lanes of a warp: three
-// exchanges that halve the columns a lane holds, then two plain ones.  Lane l
-// ends with the sums of column (l >> 2).
-__device__ __forceinline__ float3 reduce_cols8(float (&v)[8][3], int lane) {
-    float w[4][3], u[2][3], t[3];
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float keep = b4 ? v[j + 4][d] : v[j][d], give = b4 ? v[j][d] : v[j + 4][d];
-            w[j][d] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-        }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float keep = b3 ? w[j + 2][d] : w[j][d], give = b3 ? w[j][d] : w[j + 2][d];
-            u[j][d] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-        }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const float keep = b2 ? u[1][d] : u[0][d], give = b2 ? u[0][d] : u[1][d];
-        t[d] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-        t[d] += __shfl_xor_sync(0xffffffffu, t[d], 2);
-        t[d] += __shfl_xor_sync(0xffffffffu, t[d], 1);
-    }
-    return make_float3(t[0], t[1], t[2]);
-}
-
-// Backward block, static part: warp w owns the tile's columns c0 + 8 w ..,
-// lane l its rows r0 + l, + 32, ..: 4 x 8 entries in registers.
-constexpr int kBwdWarpCols = kTileCols / (kLevelThreads / 32);
-constexpr int kBwdRows = kTileRows / 32;
-static_assert(kBwdWarpCols == 8, "reduce_cols8");
-struct BwdBlockPre {
-    float mv[kBwdRows][kBwdWarpCols];
-    int vid;      // of row r0 + thread, -1 past the last
-    int cv;       // vertex of this lane's result column, -1: none
-    bool pivot, split;
-};
-
-__device__ __forceinline__ void bwd_block_load(const CholArgs& a, int item, BwdBlockPre& p) {
-    const BlockItem b = block_item(a, a.blocks, item);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cw = b.c0 + kBwdWarpCols * warp;
-    const float* Mc = b.M + (size_t)cw * b.m;
-#pragma unroll
-    for (int t = 0; t < kBwdRows; ++t) {
-        const int i = b.r0 + lane + 32 * t;
-#pragma unroll
-        for (int j = 0; j < kBwdWarpCols; ++j)
-            p.mv[t][j] = (i < b.m && cw + j < b.c1 && i >= cw + j) ? __ldg(Mc + (size_t)j * b.m + i) : 0.f;
-    }
-    const int row = b.r0 + threadIdx.x;
-    p.vid = row < b.m ? __ldg(&b.rows[row]) : -1;
-    p.pivot = row < b.k;
-    const int c = cw + (lane >> 2);
-    p.cv = ((lane & 3) == 0 && c < b.c1) ? __ldg(&b.rows[c]) : -1;
-    p.split = b.m > kTileRows;
-}
-
-// Vector part: z of the tile's rows staged in shared memory, the products,
-// the warp's reduction; sums stored, or added where the supernode's rows take
+// Backward: each lane's eight column sums over its four rows, exchanged so
+// that one lane holds the warp's sum of a column, then one warp adds the four
+// warps' sums, which are stored, or added where the supernode's rows take
 // several tiles.
-__device__ __forceinline__ void bwd_block_run(const CholArgs& a, const BwdBlockPre& p, float4* zs) {
-    zs[threadIdx.x] = p.vid >= 0 ? z_of(a, p.pivot, p.vid) : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    float acc[kBwdWarpCols][3];
+__device__ __forceinline__ void bwd_tile_run(const CholArgs& a, const TilePre& p, const float4* tile, float4* vec) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* zs = vec + 32 * warp;
+    zs[lane] = p.vid >= 0 ? z_of(a, p.row < p.k, p.vid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    cp_async_wait();
+    __syncwarp();
+    const int r = 4 * (lane & 7);
+    const float4 z0 = zs[r], z1 = zs[r + 1], z2 = zs[r + 2], z3 = zs[r + 3];
+    const float4* t4 = tile + 32 * kLaneCols * warp + lane;
+    float3 s[8];
 #pragma unroll
-    for (int j = 0; j < kBwdWarpCols; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.f;
-#pragma unroll
-    for (int t = 0; t < kBwdRows; ++t) {
-        const float4 z = zs[lane + 32 * t];
-#pragma unroll
-        for (int j = 0; j < kBwdWarpCols; ++j) {
-            acc[j][0] = fmaf(p.mv[t][j], z.x, acc[j][0]);
-            acc[j][1] = fmaf(p.mv[t][j], z.y, acc[j][1]);
-            acc[j][2] = fmaf(p.mv[t][j], z.z, acc[j][2]);
-        }
+    for (int q = 0; q < kLaneCols; ++q) {
+        const float4 m = t4[32 * q];
+        s[q] = make_float3(m.x * z0.x, m.x * z0.y, m.x * z0.z);
+        fma3(s[q], m.y, z1);
+        fma3(s[q], m.z, z2);
+        fma3(s[q], m.w, z3);
     }
-    const float3 s = reduce_cols8(acc, lane);
-    if (p.cv < 0) return;
-    if (p.split) atomicAdd(&a.x[p.cv], make_float4(s.x, s.y, s.z, 0.f));
-    else a.x[p.cv] = make_float4(s.x, s.y, s.z, 0.f);
+    halve<4>(s, lane, 4);
+    float3 u[4] = {s[0], s[1], s[2], s[3]};
+    halve<2>(u, lane, 2);
+    float3 t[2] = {u[0], u[1]};
+    halve<1>(t, lane, 1);
+    __syncwarp();  // every lane has read its z
+    // the lane kept q = l & 7 of its columns 4 q + (l >> 3)
+    zs[4 * (lane & 7) + (lane >> 3)] = make_float4(t[0].x, t[0].y, t[0].z, 0.f);
+    __syncthreads();
+    if (warp != 0 || p.cvid < 0) return;
+    static_assert(kLevelThreads == 128, "four partial sums");
+    const float4 q0 = vec[lane], q1 = vec[32 + lane], q2 = vec[64 + lane], q3 = vec[96 + lane];
+    const float4 sum = make_float4((q0.x + q1.x) + (q2.x + q3.x), (q0.y + q1.y) + (q2.y + q3.y),
+                                   (q0.z + q1.z) + (q2.z + q3.z), 0.f);
+    if (p.m > kTileRows) atomicAdd(&a.x[p.cvid], sum);
+    else a.x[p.cvid] = sum;
 }
 
-// Small supernodes {moff, roff, m, k} (m < kBlockMinRows = 64 rows, at most
-// kSmallCols pivots): one warp, lane l owns rows l and l + 32.  Forward: the
-// first kSmallPre columns before the wait, the rest after it.
-constexpr int kSmallPre = 16;
+// One column's sum over its first 4 n rows in shared memory (16-byte aligned)
+// against z, four rows a load, each row of the four in a chain of its own.
+__device__ __forceinline__ float3 column_sum(const float* col, const float4* z, int n) {
+    float3 s[4] = {};
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) {
+        const float4 mq = *reinterpret_cast<const float4*>(col + 4 * q);
+        fma3(s[0], mq.x, z[4 * q]);
+        fma3(s[1], mq.y, z[4 * q + 1]);
+        fma3(s[2], mq.z, z[4 * q + 2]);
+        fma3(s[3], mq.w, z[4 * q + 3]);
+    }
+    return make_float3((s[0].x + s[1].x) + (s[2].x + s[3].x), (s[0].y + s[1].y) + (s[2].y + s[3].y),
+                       (s[0].z + s[1].z) + (s[2].z + s[3].z));
+}
+
+// Small supernodes {moff, roff, m, k} (is_small): one warp copies the whole
+// block; forward lane = rows l and l + 32, backward lane = column.
 struct SmallPre {
-    float mv[2][kSmallPre];
-    const float* M;
-    int m, k, vid[2];
+    int m, k, ld, vid[2];
 };
 
-__device__ __forceinline__ void small_load(const CholArgs& a, int item, bool live, int lane, SmallPre& p) {
-    p.m = p.k = 0;
-    p.M = a.mval;
-    p.vid[0] = p.vid[1] = -1;
-    if (live) {
-        const BlockItem b = block_item(a, a.small, item);
-        p.M = b.M;
-        p.m = b.m;
-        p.k = b.k;
+__device__ __forceinline__ void small_load(const CholArgs& a, int item, float* blk, int lane, SmallPre& p) {
+    const int4* w = reinterpret_cast<const int4*>(a.small + (size_t)kItemInts * item);
+    const int4 h0 = __ldg(w);
+    const Supernode s = supernode(a, h0, __ldg(a.small + (size_t)kItemInts * item + 4));
+    for (int e = 4 * lane; e < s.k * s.ld; e += 128) cp_async16(blk + e, s.M + e, true);
+    p.m = s.m;
+    p.k = s.k;
+    p.ld = s.ld;
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (lane + 32 * h < p.m) p.vid[h] = __ldg(&b.rows[lane + 32 * h]);
-    }
-#pragma unroll
-    for (int c = 0; c < kSmallPre; ++c)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = lane + 32 * h;
-            p.mv[h][c] = (c < p.k && row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
-        }
+    for (int h = 0; h < 2; ++h) p.vid[h] = lane + 32 * h < s.m ? __ldg(&s.rows[lane + 32 * h]) : -1;
 }
 
-__device__ __forceinline__ void fwd_small_run(const CholArgs& a, const SmallPre& p, int lane, float4* stage) {
-    stage[lane] = lane < p.k ? __ldcg(&a.r[p.vid[0]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+__device__ __forceinline__ void fwd_small_run(const CholArgs& a, const SmallPre& p, const float* blk, float4* rs,
+                                              int lane) {
+    rs[lane] = lane < p.k ? __ldcg(&a.r[p.vid[0]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    cp_async_wait();
     __syncwarp();
-    float s[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-#pragma unroll
-    for (int c = 0; c < kSmallPre; ++c) {
-        const float4 v = stage[c];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            s[h][0] = fmaf(p.mv[h][c], v.x, s[h][0]);
-            s[h][1] = fmaf(p.mv[h][c], v.y, s[h][1]);
-            s[h][2] = fmaf(p.mv[h][c], v.z, s[h][2]);
-        }
-    }
-#pragma unroll 4
-    for (int c = kSmallPre; c < p.k; ++c) {
-        const float4 v = stage[c];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = lane + 32 * h;
-            const float mv = (row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
-            s[h][0] = fmaf(mv, v.x, s[h][0]);
-            s[h][1] = fmaf(mv, v.y, s[h][1]);
-            s[h][2] = fmaf(mv, v.z, s[h][2]);
-        }
-    }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if (p.vid[h] < 0) continue;
-        if (lane + 32 * h < p.k) a.y[p.vid[h]] = make_float4(s[h][0], s[h][1], s[h][2], 0.f);
-        else atomicAdd(&a.r[p.vid[h]], make_float4(-s[h][0], -s[h][1], -s[h][2], 0.f));
+        const int row = lane + 32 * h;
+        float sx = 0.f, sy = 0.f, sz = 0.f;
+        const float* t = blk + row;
+#pragma unroll 4
+        for (int c = 0; c < p.k; ++c) {
+            const float mv = t[c * p.ld];
+            const float4 v = rs[c];
+            sx = fmaf(mv, v.x, sx);
+            sy = fmaf(mv, v.y, sy);
+            sz = fmaf(mv, v.z, sz);
+        }
+        if (row < p.k) a.y[p.vid[h]] = make_float4(sx, sy, sz, 0.f);
+        else atomicAdd(&a.r[p.vid[h]], make_float4(-sx, -sy, -sz, 0.f));
     }
 }
 
-// Backward: z of the warp's rows in registers, 8 columns at a time.
-__device__ __forceinline__ void bwd_small_run(const CholArgs& a, const SmallPre& p, int lane) {
-    float4 z[2];
+__device__ __forceinline__ void bwd_small_run(const CholArgs& a, const SmallPre& p, float* blk, int lane) {
+    float4* zs = reinterpret_cast<float4*>(blk + kSmallFloats);
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-        z[h] = p.vid[h] >= 0 ? z_of(a, lane + 32 * h < p.k, p.vid[h]) : make_float4(0.f, 0.f, 0.f, 0.f);
-    auto columns = [&](int c0, const float (&mv)[2][8]) {
-        float acc[8][3];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            acc[j][0] = fmaf(mv[0][j], z[0].x, mv[1][j] * z[1].x);
-            acc[j][1] = fmaf(mv[0][j], z[0].y, mv[1][j] * z[1].y);
-            acc[j][2] = fmaf(mv[0][j], z[0].z, mv[1][j] * z[1].z);
-        }
-        const float3 s = reduce_cols8(acc, lane);
-        const int c = c0 + (lane >> 2);  // pivots are the first rows: vertex in lane c
-        const int vid = __shfl_sync(0xffffffffu, p.vid[0], c & 31);
-        if ((lane & 3) == 0 && c < p.k) a.x[vid] = make_float4(s.x, s.y, s.z, 0.f);
-    };
-    static_assert(kSmallPre % 8 == 0 && kSmallCols <= 32, "column groups");
-#pragma unroll
-    for (int g = 0; g < kSmallPre / 8; ++g) {
-        if (8 * g >= p.k) break;
-        float mv[2][8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            mv[0][j] = p.mv[0][8 * g + j];
-            mv[1][j] = p.mv[1][8 * g + j];
-        }
-        columns(8 * g, mv);
-    }
-    for (int c0 = kSmallPre; c0 < p.k; c0 += 8) {
-        float mv[2][8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int row = lane + 32 * h, c = c0 + j;
-                mv[h][j] = (c < p.k && row < p.m && row >= c) ? __ldg(p.M + (size_t)c * p.m + row) : 0.f;
-            }
-        columns(c0, mv);
-    }
+        zs[lane + 32 * h] =
+            p.vid[h] >= 0 ? z_of(a, lane + 32 * h < p.k, p.vid[h]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    cp_async_wait();
+    __syncwarp();
+    if (lane >= p.k) return;
+    const float3 s = column_sum(blk + lane * p.ld, zs, (p.m + 3) / 4);
+    a.x[p.vid[0]] = make_float4(s.x, s.y, s.z, 0.f);
 }
 
 // Tiny supernodes {moff, roff, m, 1} (one pivot, at most kTinyRows rows --
@@ -462,27 +427,35 @@ constexpr int kTinyPerCta = kLevelThreads / kTinyLanes;
 __host__ __device__ inline int small_ctas(int n) { return (n + kLevelWarps - 1) / kLevelWarps; }
 __host__ __device__ inline int tiny_ctas(int n) { return (n + kTinyPerCta - 1) / kTinyPerCta; }
 
-__global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_fwd_level(CholArgs a, LevelRange v) {
-    __shared__ float4 rs[kLevelThreads];
+__global__ void __launch_bounds__(kLevelThreads, kFwdBlocks) k_chol_fwd_level(CholArgs a, LevelRange v) {
+    extern __shared__ float4 tile[];  // a tile, or kWarpFloats a warp
+    float* blocks = reinterpret_cast<float*>(tile);
+    __shared__ float4 vec[kLevelWarps * 32];
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int u = blockIdx.x;
     if (u < v.nb) {
-        FwdBlockPre p;
-        fwd_block_load(a, v.b0 + u, p);
+        TilePre p;
+        tile_load(a, v.b0 + u, tile, p);
         pdl_wait();
-        if (a.done && *a.done) return;
-        fwd_block_run(a, p, rs);
+        if (a.done && *a.done) {
+            cp_async_wait();
+            return;
+        }
+        fwd_tile_run(a, p, tile, vec);
         return;
     }
     u -= v.nb;
     if (u < small_ctas(v.ns)) {
         const int it = u * kLevelWarps + warp;
-        SmallPre p;
-        small_load(a, v.s0 + it, it < v.ns, lane, p);
+        SmallPre p{};
+        if (it < v.ns) small_load(a, v.s0 + it, blocks + kWarpFloats * warp, lane, p);
         pdl_wait();
-        if (a.done && *a.done) return;
-        if (it < v.ns) fwd_small_run(a, p, lane, rs + 32 * warp);
+        if (a.done && *a.done) {
+            cp_async_wait();
+            return;
+        }
+        if (it < v.ns) fwd_small_run(a, p, blocks + kWarpFloats * warp, vec + 32 * warp, lane);
         return;
     }
     u -= small_ctas(v.ns);
@@ -494,27 +467,35 @@ __global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_fwd_lev
     fwd_tiny_run(a, p, j);
 }
 
-__global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_bwd_level(CholArgs a, LevelRange v, ResetArgs q) {
-    __shared__ float4 zs[kLevelThreads];
+__global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(CholArgs a, LevelRange v, ResetArgs q) {
+    extern __shared__ float4 tile[];  // a tile, or kWarpFloats a warp
+    float* blocks = reinterpret_cast<float*>(tile);
+    __shared__ float4 vec[kLevelWarps * 32];
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int u = blockIdx.x;
     if (u < v.nb) {
-        BwdBlockPre p;
-        bwd_block_load(a, v.b0 + u, p);
+        TilePre p;
+        tile_load(a, v.b0 + u, tile, p);
         pdl_wait();
-        if (a.done && *a.done) return;
-        bwd_block_run(a, p, zs);
+        if (a.done && *a.done) {
+            cp_async_wait();
+            return;
+        }
+        bwd_tile_run(a, p, tile, vec);
         return;
     }
     u -= v.nb;
     if (u < small_ctas(v.ns)) {
         const int it = u * kLevelWarps + warp;
-        SmallPre p;
-        small_load(a, v.s0 + it, it < v.ns, lane, p);
+        SmallPre p{};
+        if (it < v.ns) small_load(a, v.s0 + it, blocks + kWarpFloats * warp, lane, p);
         pdl_wait();
-        if (a.done && *a.done) return;
-        if (it < v.ns) bwd_small_run(a, p, lane);
+        if (a.done && *a.done) {
+            cp_async_wait();
+            return;
+        }
+        if (it < v.ns) bwd_small_run(a, p, blocks + kWarpFloats * warp, lane);
         return;
     }
     u -= small_ctas(v.ns);
@@ -542,6 +523,9 @@ __global__ void __launch_bounds__(kLevelThreads, kLevelMinBlocks) k_chol_bwd_lev
 void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s,
                               const ResetArgs& reset) {
     const int nl = (int)levels.size();
+    auto smem = [](const LevelRange& r) {
+        return sizeof(float) * (r.ns > 0 ? kLevelWarps * kWarpFloats : r.nb > 0 ? kTileRows * kTileCols : 0);
+    };
     auto range = [&](int L) {
         const SolveLevel& v = levels[L];
         return LevelRange{v.blk_begin, v.blk_end - v.blk_begin, v.sml_begin, v.sml_end - v.sml_begin, v.tiny_begin,
@@ -550,14 +534,15 @@ void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& 
     for (int L = 0; L < nl; ++L) {
         const LevelRange r = range(L);
         const int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
-        if (grid > 0) launch_pdl(k_chol_fwd_level, grid, kLevelThreads, 0, s, a, r);
+        if (grid > 0) launch_pdl(k_chol_fwd_level, grid, kLevelThreads, smem(r), s, a, r);
     }
     bool first = reset.y_next != nullptr;
     for (int L = nl - 1; L >= 0; --L) {
         const LevelRange r = range(L);
         int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
         if (first) grid += (reset.nv + kLevelThreads - 1) / kLevelThreads;
-        if (grid > 0) launch_pdl(k_chol_bwd_level, grid, kLevelThreads, 0, s, a, r, first ? reset : ResetArgs{});
+        if (grid > 0)
+            launch_pdl(k_chol_bwd_level, grid, kLevelThreads, smem(r), s, a, r, first ? reset : ResetArgs{});
         first = false;
     }
 }
@@ -608,7 +593,9 @@ __device__ __forceinline__ bool grid_sync(GridSync* g, unsigned& gen, unsigned e
 
 __global__ void __launch_bounds__(kLevelThreads) k_chol_solve_persistent(CholArgs a, const SolveLevel* __restrict__ lv,
                                                                          int nl, GridSync* bar, long long spin) {
-    __shared__ float4 rs[kLevelThreads];
+    __shared__ float4 tile[kLevelWarps * kWarpFloats / 4];
+    float* blocks = reinterpret_cast<float*>(tile);
+    __shared__ float4 vec[kLevelWarps * 32];
     if (a.done && *a.done) return;  // set before this launch: the same for every CTA
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned expect = gridDim.x;
@@ -619,24 +606,19 @@ __global__ void __launch_bounds__(kLevelThreads) k_chol_solve_persistent(CholArg
         const int nb = v.blk_end - v.blk_begin, ns = v.sml_end - v.sml_begin, nt = v.tiny_end - v.tiny_begin;
         const int nsu = small_ctas(ns), ntu = tiny_ctas(nt);
         for (int u = blockIdx.x; u < nb + nsu + ntu; u += gridDim.x) {
-            __syncthreads();  // rs of the previous unit is read
+            __syncthreads();  // the previous unit's shared memory is read
             if (u < nb) {
-                if (fwd) {
-                    FwdBlockPre p;
-                    fwd_block_load(a, v.blk_begin + u, p);
-                    fwd_block_run(a, p, rs);
-                } else {
-                    BwdBlockPre p;
-                    bwd_block_load(a, v.blk_begin + u, p);
-                    bwd_block_run(a, p, rs);
-                }
+                TilePre p;
+                tile_load(a, v.blk_begin + u, tile, p);
+                if (fwd) fwd_tile_run(a, p, tile, vec);
+                else bwd_tile_run(a, p, tile, vec);
             } else if (u < nb + nsu) {
                 const int it = (u - nb) * kLevelWarps + warp;
-                SmallPre p;
-                small_load(a, v.sml_begin + it, it < ns, lane, p);
                 if (it < ns) {
-                    if (fwd) fwd_small_run(a, p, lane, rs + 32 * warp);
-                    else bwd_small_run(a, p, lane);
+                    SmallPre p;
+                    small_load(a, v.sml_begin + it, blocks + kWarpFloats * warp, lane, p);
+                    if (fwd) fwd_small_run(a, p, blocks + kWarpFloats * warp, vec + 32 * warp, lane);
+                    else bwd_small_run(a, p, blocks + kWarpFloats * warp, lane);
                 }
             } else {
                 const int it = (u - nb - nsu) * kTinyPerCta + (int)threadIdx.x / kTinyLanes,

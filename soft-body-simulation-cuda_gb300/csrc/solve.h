@@ -46,8 +46,8 @@ struct ResetArgs {
 };
 
 constexpr int kLevelThreads = kTileRows;  // per-level kernels: one thread a tile row
-// Resident CTAs per SM the per-level kernels' registers are allocated for.
-constexpr int kLevelMinBlocks = 8;
+// Resident CTAs per SM that the per-level kernels' registers are allocated for.
+constexpr int kFwdBlocks = 11, kBwdBlocks = 10;
 constexpr int kTinyLanes = 8;             // lanes of a tiny supernode: most have 7 rows
 
 // Grid-wide barrier of the persistent solve (device memory): arrivals and
