@@ -13,11 +13,9 @@
 //   k_fk     entries of K in the pivot columns of each front
 //   k_fea    extend-add: the children's Schur complements into the front
 //   per panel of 32 pivot columns:
-//     k_fdiag  Cholesky of the 32 x 32 diagonal block (one warp per front)
-//     k_fpanel the panel rows below it: L_i = A_i L_jj^-T
-//     k_ftrail trailing update of the lower triangle, 32 x 32 tiles
-//   k_fm     M_s = [I ; L_os] L_ss^-1, rows independent, by column blocks
-//            from the right; FP64 in the pool, FP32 into mval
+//     k_panel  the diagonal block's factor and inverse, the panel's rows of L
+//              and of M_s
+//     k_trail  trailing update of the front's lower triangle and of M_s
 // A non-positive pivot is recorded in a status word; the host raises
 // PDGB_ERR_NOT_SPD after the last level.
 #include <cuda_runtime.h>
@@ -27,12 +25,13 @@
 
 #include "cholesky.h"
 #include "engine.h"
+#include "pdl.cuh"
 
 namespace pdgb {
 namespace {
 
 constexpr int kNB = 32;           // panel width and tile size
-constexpr int kRowChunk = 256;    // panel rows per CTA
+constexpr int kFillCtas = 304;    // two CTAs an SM: launches with fewer are split further
 constexpr int kZeroChunk = 1 << 16;
 
 struct FDev {
@@ -107,184 +106,248 @@ __global__ void __launch_bounds__(256) k_fea(FDev d, const int* __restrict__ lis
     }
 }
 
-// Cholesky of the diagonal block [j0, j0 + nb) of each front with more than
-// j0 pivots: one warp per front, lane = row, the block in shared memory.
-__global__ void __launch_bounds__(32) k_fdiag(FDev d, const int* __restrict__ list, int j0) {
-    const int s = list[blockIdx.x];
-    const int k = d.sk[s], m = d.sm[s];
-    if (j0 >= k) return;
-    const int nb = min(kNB, k - j0);
-    double* F = d.pool + d.foff[s] + (int64_t)j0 * m + j0;  // F[c m + r] = A[j0 + r][j0 + c]
-    __shared__ double D[kNB][kNB + 1];
-    const int lane = threadIdx.x;
-    for (int c = 0; c < kNB; ++c) D[lane][c] = (lane < nb && c <= lane) ? F[(int64_t)c * m + lane] : 0.0;
-    __syncwarp();
-    bool bad = false;
-    for (int j = 0; j < nb; ++j) {
-        double l = D[j][j];
-        if (!(l > 0.0) || !isfinite(l)) {
-            bad = true;
-            l = 1.0;
-        } else {
-            l = sqrt(l);
-        }
-        __syncwarp();
-        if (lane == j) D[j][j] = l;
-        if (lane > j && lane < nb) D[lane][j] /= l;
-        __syncwarp();
-        if (lane > j && lane < nb) {
-            const double a = D[lane][j];
-            for (int c = j + 1; c <= lane; ++c) D[lane][c] = fma(-a, D[c][j], D[lane][c]);
-        }
-        __syncwarp();
+// ------------------------------------------------------------ panels
+// One panel of kNB pivot columns of every front of a level, two launches:
+//
+//   k_panel  each CTA factors the panel's diagonal block A_JJ = L_JJ L_JJ^T
+//            and inverts it, W = L_JJ^-1, in shared memory (the same few
+//            thousand multiply-adds in every CTA, instead of a launch that
+//            all the others wait for), then takes its share of
+//              L[i, J] = A[i, J] W^T          rows i below the panel
+//              X[J, c] = W X[J, c]            columns c left of the panel
+//   k_trail  rows i below the panel, 32-row tiles:
+//              A[i, c] -= L[i, J] L[c, J]^T   columns c past the panel, c <= i
+//              X[i, c] -= L[i, J] X[J, c]     columns c up to the panel's last
+//
+// X, the m x k block after the front, starts as [I ; 0] (the identity is
+// implicit: X[J, J] = W) and ends as [L_ss^-1 ; -L_os L_ss^-1]: M_s comes out
+// of the same elimination, with the whole GPU on every panel, and its rows go
+// to mval as they become final.
+//
+// FP64 runs at two multiply-adds a clock and SM here, so a 32-cubed tile takes
+// 16 k clocks (8 us) and a chain of small steps on one warp a multiple of
+// that: what counts is to spread each panel's work over the SMs.  A tile's
+// columns are therefore split over 2 or 4 CTAs where a launch has few tiles.
+constexpr int kPanelThreads = 256;
+
+// A launch's fronts: front i has the CTAs from fronts[i].first to the next
+// one's; hint[b] is the front of CTA 64 b, the last hint the last front.
+struct FrontRef {
+    int s, first;
+};
+constexpr int kHintStep = 64;
+
+__device__ __forceinline__ int find_front(const FrontRef* f, const int* hint, int block) {
+    int lo = hint[block / kHintStep];
+    int hi = hint[block / kHintStep + 1];
+    while (lo < hi) {  // the last front that begins at or before the block
+        const int mid = (lo + hi + 1) >> 1;
+        if (f[mid].first <= block) lo = mid;
+        else hi = mid - 1;
     }
-    if (bad && lane == 0) atomicCAS(d.status, 0, s + 1);
-    if (lane < nb)
-        for (int c = 0; c <= lane; ++c) F[(int64_t)c * m + lane] = D[lane][c];
+    return lo;
 }
 
-// Panel rows below the diagonal block: row i of L over columns
-// [j0, j0 + nb) solves x L_jj^T = A[i, j0 : j0 + nb]; items {s, first row}.
-__global__ void __launch_bounds__(kRowChunk) k_fpanel(FDev d, const int2* __restrict__ items, int j0) {
-    const int2 it = items[blockIdx.x];
-    const int s = it.x;
+// 1 / sqrt(d) from the single precision value y: with e = 1 - d y^2 (about
+// 2^-22) it is y (1 - e)^(-1/2) = y (1 + e / 2 + 3 e^2 / 8 + O(e^3)), the
+// rest below the rounding of double.  Outside the range of float the
+// library's function.
+__device__ __forceinline__ double inv_sqrt(double d) {
+    if (!(d > 1e-30 && d < 1e30)) return rsqrt(d);
+    const double y = (double)rsqrtf((float)d);
+    const double e = fma(-d * y, y, 1.0);
+    return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// Lower triangle of the nb x nb block D -> its Cholesky factor, W -> the
+// factor's inverse (both lower, row-major in shared memory).  Step j scales
+// column j of D and row j of W, then takes them out of the rows below: row i
+// has i + 1 entries to update, i - j of D and j + 1 of W.
+__device__ __forceinline__ void factor_block(double (*D)[kNB + 1], double (*W)[kNB + 1], int nb, bool& bad) {
+    const int tid = threadIdx.x;
+    const int row = tid >> 3, part = tid & 7;  // 8 threads a row
+    static_assert(kPanelThreads == 8 * kNB, "8 threads a row");
+    for (int e = tid; e < kNB * kNB; e += kPanelThreads) W[e / kNB][e % kNB] = e / kNB == e % kNB ? 1.0 : 0.0;
+    __syncthreads();
+    for (int j = 0; j < nb; ++j) {
+        if (tid < kNB) {
+            double d = D[j][j];
+            if (!(d > 0.0) || !isfinite(d)) {
+                bad = true;
+                d = 1.0;
+            }
+            const double inv = inv_sqrt(d);
+            __syncwarp();
+            if (tid == j) D[j][j] = d * inv;
+            else if (tid > j && tid < nb) D[tid][j] *= inv;
+            if (tid <= j) W[j][tid] *= inv;
+        }
+        __syncthreads();
+        if (row > j && row < nb) {
+            const double l = D[row][j];
+            for (int c = part; c <= row; c += 8) {
+                if (c > j) D[row][c] = fma(-l, D[c][j], D[row][c]);
+                else W[row][c] = fma(-l, W[j][c], W[row][c]);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kPanelThreads) k_panel(FDev d, const FrontRef* __restrict__ fronts,
+                                                         const int* __restrict__ hint, int j0, int chunk) {
+    __shared__ double D[kNB][kNB + 1], W[kNB][kNB + 1], T[kNB][kNB + 1];
+    pdl_trigger();
+    const int fi = find_front(fronts, hint, blockIdx.x);
+    const int s = fronts[fi].s, part = blockIdx.x - fronts[fi].first;
     const int k = d.sk[s], m = d.sm[s];
-    const int nb = min(kNB, k - j0);
+    const int nb = min(kNB, k - j0), j1 = j0 + nb;
+    const int64_t ld = m_stride(m, k);
     double* F = d.pool + d.foff[s];
-    __shared__ double D[kNB][kNB + 1];
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    double* X = F + (int64_t)m * m;
+    float* M = d.mval + d.moff[s];
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
         const int r = e % kNB, c = e / kNB;
         D[r][c] = (r < nb && c <= r) ? F[(int64_t)(j0 + c) * m + j0 + r] : 0.0;
     }
     __syncthreads();
-    const int i = it.y + threadIdx.x;
-    if (i >= m) return;
-    double x[kNB];
+    bool bad = false;
+    factor_block(D, W, nb, bad);
+    const int nrow = max(1, (m - j1 + chunk - 1) / chunk);
+    if (part == 0) {
+        if (bad) atomicCAS(d.status, 0, s + 1);
+        for (int e = threadIdx.x; e < nb * kNB; e += kPanelThreads) {
+            const int r = e % kNB, c = e / kNB;
+            if (r >= nb || c > r) continue;
+            X[(int64_t)(j0 + c) * m + j0 + r] = W[r][c];
+            M[(int64_t)(j0 + c) * ld + j0 + r] = (float)W[r][c];
+        }
+    }
+    if (part < nrow) {  // (nothing reads L_JJ any more: the diagonal block of F stays as it is)
+        for (int r0 = j1 + part * chunk; r0 < min(m, j1 + (part + 1) * chunk); r0 += kNB) {
+            __syncthreads();
+            for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
+                const int r = e % kNB, q = e / kNB;
+                T[r][q] = (q < nb && r0 + r < m) ? F[(int64_t)(j0 + q) * m + r0 + r] : 0.0;
+            }
+            __syncthreads();
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int q = 0; q < nb; ++q) {
+                const double t = T[lane][q];
 #pragma unroll
-    for (int j = 0; j < kNB; ++j) {
-        if (j < nb) {
-            double v = F[(int64_t)(j0 + j) * m + i];
+                for (int u = 0; u < 4; ++u) acc[u] = fma(t, W[warp + 8 * u][q], acc[u]);  // zero for q > j
+            }
 #pragma unroll
-            for (int q = 0; q < j; ++q) v = fma(-x[q], D[j][q], v);
-            x[j] = v / D[j][j];
-            F[(int64_t)(j0 + j) * m + i] = x[j];
+            for (int u = 0; u < 4; ++u) {
+                const int j = warp + 8 * u;
+                if (j < nb && r0 + lane < m) F[(int64_t)(j0 + j) * m + r0 + lane] = acc[u];
+            }
+        }
+        return;
+    }
+    // X[J, c] = W X[J, c]: column block of the left part
+    const int c0 = (part - nrow) * chunk;
+    for (int cb = c0; cb < min(j0, c0 + chunk); cb += kNB) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
+            const int r = e % kNB, c = e / kNB;
+            T[r][c] = (r < nb && cb + c < j0) ? X[(int64_t)(cb + c) * m + j0 + r] : 0.0;
+        }
+        __syncthreads();
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int q = 0; q < nb; ++q) {
+            const double w = W[lane][q];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[u] = fma(w, T[q][warp + 8 * u], acc[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = cb + warp + 8 * u;
+            if (c < j0 && lane < nb) {
+                X[(int64_t)c * m + j0 + lane] = acc[u];
+                M[(int64_t)c * ld + j0 + lane] = (float)acc[u];
+            }
         }
     }
 }
 
-// Trailing update of the panel over the lower triangle past it:
-// A[r][c] -= sum_q L[r][j0 + q] L[c][j0 + q] for r >= c >= j0 + nb, one
-// 32 x 32 tile per CTA; items {s, tile}, tile t = ti (ti + 1) / 2 + tj.
-__global__ void __launch_bounds__(256) k_ftrail(FDev d, const int2* __restrict__ items, int j0) {
-    const int2 it = items[blockIdx.x];
-    const int s = it.x;
+// Tiles of a panel's trailing update: 32 rows from j1 + 32 ti, and kCols
+// columns of A (the tile column tj <= ti) or of X.
+template <int kCols>
+__global__ void __launch_bounds__(kPanelThreads) k_trail(FDev d, const FrontRef* __restrict__ fronts,
+                                                         const int* __restrict__ hint, int j0) {
+    __shared__ double Lr[kNB][kNB + 1], Lc[kCols][kNB + 1];
+    pdl_trigger();
+    constexpr int kSplit = kNB / kCols;
+    constexpr int kPer = kCols / 8;  // outputs a thread: 8 warps
+    const int fi = find_front(fronts, hint, blockIdx.x);
+    const int s = fronts[fi].s;
+    int t = blockIdx.x - fronts[fi].first;
     const int k = d.sk[s], m = d.sm[s];
-    const int nb = min(kNB, k - j0);
-    const int j1 = j0 + nb;
-    int ti = (int)((sqrt(8.0 * (double)it.y + 1.0) - 1.0) * 0.5);
-    while ((ti + 1) * (ti + 2) / 2 <= it.y) ++ti;
-    while (ti * (ti + 1) / 2 > it.y) --ti;
-    const int tj = it.y - ti * (ti + 1) / 2;
-    const int r0 = j1 + kNB * ti, c0 = j1 + kNB * tj;
+    const int nb = min(kNB, k - j0), j1 = j0 + nb;
+    const int sub = t % kSplit;
+    t /= kSplit;
+    const int T = (m - j1 + kNB - 1) / kNB;
+    const int ta = T * (T + 1) / 2;
+    const bool in_x = t >= ta;
+    int ti, tj;
+    if (in_x) {
+        const int nc = (j1 + kNB - 1) / kNB;
+        ti = (t - ta) / nc;
+        tj = (t - ta) % nc;
+    } else {
+        ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+        while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+        while (ti * (ti + 1) / 2 > t) --ti;
+        tj = t - ti * (ti + 1) / 2;
+    }
+    const int r0 = j1 + kNB * ti, c0 = (in_x ? 0 : j1) + kNB * tj + kCols * sub;
+    const int cend = in_x ? j1 : m;
     double* F = d.pool + d.foff[s];
-    __shared__ double Lr[kNB][kNB + 1], Lc[kNB][kNB + 1];
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    double* X = F + (int64_t)m * m;
+    pdl_wait();
+    for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
         const int r = e % kNB, q = e / kNB;
-        const bool okq = q < nb;
-        Lr[r][q] = (okq && r0 + r < m) ? F[(int64_t)(j0 + q) * m + r0 + r] : 0.0;
-        Lc[r][q] = (okq && c0 + r < m) ? F[(int64_t)(j0 + q) * m + c0 + r] : 0.0;
+        Lr[r][q] = (q < nb && r0 + r < m) ? F[(int64_t)(j0 + q) * m + r0 + r] : 0.0;
+    }
+    if (in_x) {
+        for (int e = threadIdx.x; e < kCols * kNB; e += kPanelThreads) {
+            const int q = e % kNB, c = e / kNB;
+            Lc[c][q] = (q < nb && c0 + c < cend) ? X[(int64_t)(c0 + c) * m + j0 + q] : 0.0;
+        }
+    } else {
+        for (int e = threadIdx.x; e < kCols * kNB; e += kPanelThreads) {
+            const int c = e % kCols, q = e / kCols;
+            Lc[c][q] = (q < nb && c0 + c < cend) ? F[(int64_t)(j0 + q) * m + c0 + c] : 0.0;
+        }
     }
     __syncthreads();
-    const int r = threadIdx.x & 31, cb = threadIdx.x >> 5;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = 0; q < nb; ++q) {
-        const double a = Lr[r][q];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = r0 + lane;
+    double* out = in_x ? X : F;
+    double acc[kPer];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = fma(a, Lc[cb + 8 * u][q], acc[u]);
+    for (int u = 0; u < kPer; ++u) {
+        const int col = c0 + warp + 8 * u;
+        acc[u] = row < m && col < cend && (in_x || col <= row) ? out[(int64_t)col * m + row] : 0.0;
     }
-    const int gr = r0 + r;
-    if (gr >= m) return;
+#pragma unroll 8
+    for (int q = 0; q < kNB; ++q) {
+        const double a = -Lr[lane][q];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int gc = c0 + cb + 8 * u;
-        if (gc < m && gc <= gr) F[(int64_t)gc * m + gr] -= acc[u];
+        for (int u = 0; u < kPer; ++u) acc[u] = fma(a, Lc[warp + 8 * u][q], acc[u]);
     }
-}
-
-// M_s = B L_ss^-1 with B = [I_k ; L_os] (m x k): each row x of M_s solves
-// x L_ss = b, by blocks of 32 columns from the right,
-//   X[:, J] = (B[:, J] - X[:, J+1:] L[J+1:, J]) L_JJ^-1,
-// for the 32 rows {s, r0} of the item.  X is kept in FP64 in the block
-// after the front (zeroed with it) and written to mval in FP32.  Rows below
-// k are rows of L_ss^-1, which vanish right of the diagonal: those blocks
-// are skipped.
-__global__ void __launch_bounds__(256) k_fm(FDev d, const int2* __restrict__ items) {
-    const int2 it = items[blockIdx.x];
-    const int s = it.x, r0 = it.y;
-    const int k = d.sk[s], m = d.sm[s];
-    const double* F = d.pool + d.foff[s];
-    double* X = d.pool + d.foff[s] + (int64_t)m * m;
-    float* M = d.mval + d.moff[s];
+    if (row >= m) return;
     const int64_t ld = m_stride(m, k);
-    __shared__ double Xs[kNB][kNB + 1];
-    __shared__ double Xq[kNB][kNB + 1];
-    __shared__ double Lq[kNB][kNB + 1];
-    const int nbk = (k + kNB - 1) / kNB;
-    // last column that can be nonzero in these rows
-    const int cmax = r0 + kNB <= k ? r0 + kNB - 1 : k - 1;
-    const int jtop = cmax / kNB;
-    const int tr = threadIdx.x & 31, tc = threadIdx.x >> 5;
-    const int row = r0 + tr;
-    for (int J = min(nbk - 1, jtop); J >= 0; --J) {
-        const int c0 = J * kNB, cn = min(kNB, k - c0);
-        double acc[4];
+    float* M = d.mval + d.moff[s];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int col = c0 + tc + 8 * u;
-            double b = 0.0;
-            if (col < k && row < m) b = row < k ? (row == col ? 1.0 : 0.0) : F[(int64_t)col * m + row];
-            acc[u] = b;
-        }
-        for (int Q = J + 1; Q <= min(nbk - 1, jtop); ++Q) {
-            const int q0 = Q * kNB, qn = min(kNB, k - q0);
-            __syncthreads();
-            for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-                const int rr = e % kNB, cc = e / kNB;
-                Xq[rr][cc] = (r0 + rr < m && cc < qn) ? X[(int64_t)(q0 + cc) * m + r0 + rr] : 0.0;
-                Lq[rr][cc] = (rr < qn && cc < cn) ? F[(int64_t)(c0 + cc) * m + q0 + rr] : 0.0;  // L[q0 + rr][c0 + cc]
-            }
-            __syncthreads();
-            for (int q = 0; q < qn; ++q) {
-                const double xv = Xq[tr][q];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) acc[u] = fma(-xv, Lq[q][tc + 8 * u], acc[u]);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u) Xs[tr][tc + 8 * u] = acc[u];
-        for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-            const int rr = e % kNB, cc = e / kNB;
-            Lq[rr][cc] = (rr < cn && cc <= rr) ? F[(int64_t)(c0 + cc) * m + c0 + rr] : 0.0;  // L_JJ
-        }
-        __syncthreads();
-        if (threadIdx.x < kNB) {
-            for (int j = cn - 1; j >= 0; --j) {
-                double v = Xs[tr][j];
-                for (int q = j + 1; q < cn; ++q) v = fma(-Xs[tr][q], Lq[q][j], v);
-                Xs[tr][j] = v / Lq[j][j];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int col = c0 + tc + 8 * u;
-            if (col < k && row < m) {
-                const double v = Xs[tr][tc + 8 * u];
-                X[(int64_t)col * m + row] = v;
-                M[col * ld + row] = (float)v;
-            }
-        }
+    for (int u = 0; u < kPer; ++u) {
+        const int col = c0 + warp + 8 * u;
+        if (col >= cend || (!in_x && col > row)) continue;
+        out[(int64_t)col * m + row] = acc[u];
+        if (in_x && j1 == k) M[col * ld + row] = (float)-acc[u];  // the last panel: rows past the pivots are final
     }
 }
 
@@ -303,15 +366,38 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
     const int nl = (int)P.lvl_ptr.size() - 1;
     // ---- launch lists, built on the host and uploaded at once
     struct Launch {
-        int kind;        // 0 level start (zero / K / extend-add), 1 panel, 2 M_s
+        int kind;        // 0 level start (zero / K / extend-add), 1 panel, 2 trailing update
         int level;
         int j0;
-        size_t i0, n0;   // panel rows items, or M_s items
-        size_t i1, n1;   // trailing tiles
+        size_t front0, hint0;
+        int ctas;
+        int size;        // panel: rows or columns a CTA; trailing update: columns a CTA
         int ychunks, ycols;
     };
     std::vector<Launch> plan;
-    std::vector<int2> items;
+    std::vector<FrontRef> fronts;
+    std::vector<int> hints;
+    // a launch over the fronts of a level with more than j0 pivots, count(k, m)
+    // CTAs each
+    auto launch = [&](int kind, int L, int j0, int size, auto&& count) {
+        Launch l{kind, L, j0, fronts.size(), hints.size(), 0, size, 0, 0};
+        int nf = 0;
+        for (int q = P.lvl_ptr[L]; q < P.lvl_ptr[L + 1]; ++q) {
+            const int sn = P.lvl_sn[q];
+            if (f.sk[sn] <= j0) continue;
+            const int64_t c = count(f.sk[sn], f.sm[sn]);
+            if (c == 0) continue;
+            if (l.ctas + c > INT32_MAX) throw Error{PDGB_ERR_UNSUPPORTED, "factorisation: too many tiles in one launch"};
+            for (; (int64_t)hints.size() - (int64_t)l.hint0 < (l.ctas + c + kHintStep - 1) / kHintStep;) hints.push_back(nf);
+            fronts.push_back(FrontRef{sn, l.ctas});
+            l.ctas += (int)c;
+            ++nf;
+        }
+        if (nf == 0) return;
+        hints.push_back(nf - 1);
+        plan.push_back(l);
+    };
+    auto blocks = [](int n, int size) { return (int64_t)((n + size - 1) / size); };
     for (int L = 0; L < nl; ++L) {
         const int a = P.lvl_ptr[L], b = P.lvl_ptr[L + 1];
         int64_t max_tot = 0;
@@ -322,42 +408,40 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
             max_m = std::max(max_m, f.sm[sn]);
             max_k = std::max(max_k, f.sk[sn]);
         }
-        Launch st{0, L, 0, 0, 0, 0, 0, (int)((max_tot + kZeroChunk - 1) / kZeroChunk), (max_m + kNB - 1) / kNB};
-        plan.push_back(st);
+        plan.push_back(Launch{0, L, 0, 0, 0, 0, 0, (int)((max_tot + kZeroChunk - 1) / kZeroChunk), (max_m + kNB - 1) / kNB});
         for (int j0 = 0; j0 < max_k; j0 += kNB) {
-            Launch pl{1, L, j0, items.size(), 0, 0, 0, 0, 0};
-            for (int q = a; q < b; ++q) {
-                const int sn = P.lvl_sn[q], k = f.sk[sn], m = f.sm[sn];
-                if (k <= j0) continue;
+            auto panel_ctas = [&](int size) {
+                return [=](int k, int m) {
+                    const int j1 = j0 + std::min(kNB, k - j0);
+                    return std::max<int64_t>(1, blocks(m - j1, size)) + blocks(j0, size);
+                };
+            };
+            auto tiles = [&](int k, int m) {
                 const int j1 = j0 + std::min(kNB, k - j0);
-                for (int r = j1; r < m; r += kRowChunk) items.push_back(make_int2(sn, r));
-            }
-            pl.n0 = items.size() - pl.i0;
-            pl.i1 = items.size();
+                const int64_t T = blocks(m - j1, kNB);
+                return T * (T + 1) / 2 + T * blocks(j1, kNB);
+            };
+            int64_t np = 0, nt = 0;
             for (int q = a; q < b; ++q) {
-                const int sn = P.lvl_sn[q], k = f.sk[sn], m = f.sm[sn];
-                if (k <= j0) continue;
-                const int j1 = j0 + std::min(kNB, k - j0);
-                if (m <= j1) continue;
-                const int64_t T = (m - j1 + kNB - 1) / kNB;
-                for (int64_t t = 0; t < T * (T + 1) / 2; ++t) items.push_back(make_int2(sn, (int)t));
+                const int sn = P.lvl_sn[q];
+                if (f.sk[sn] <= j0) continue;
+                np += panel_ctas(kNB)(f.sk[sn], f.sm[sn]);
+                nt += tiles(f.sk[sn], f.sm[sn]);
             }
-            pl.n1 = items.size() - pl.i1;
-            plan.push_back(pl);
+            // every panel CTA factors the diagonal block anew: a few rows each
+            // while the SMs are not full, more of them past that
+            const int size = np <= kFillCtas ? kNB : 4 * kNB;
+            launch(1, L, j0, size, panel_ctas(size));
+            const int cols = nt * 4 <= kFillCtas ? kNB / 4 : nt * 2 <= kFillCtas ? kNB / 2 : kNB;
+            launch(2, L, j0, cols, [&](int k, int m) { return tiles(k, m) * (kNB / cols); });
         }
-        Launch mm{2, L, 0, items.size(), 0, 0, 0, 0, 0};
-        for (int q = a; q < b; ++q) {
-            const int sn = P.lvl_sn[q];
-            for (int r = 0; r < f.sm[sn]; r += kNB) items.push_back(make_int2(sn, r));
-        }
-        mm.n0 = items.size() - mm.i0;
-        plan.push_back(mm);
     }
     // ---- device data
     DBuf<double> pool, kval;
     DBuf<int64_t> foff, moff;
     DBuf<int> sk, sm, cptr, child, rptr, rel, kptr, kpos, lvl, status;
-    DBuf<int2> ditems;
+    DBuf<FrontRef> dfronts;
+    DBuf<int> dhints;
     pool.alloc((size_t)std::max<int64_t>(P.pool, 1));
     put(foff, P.foff, s);
     put(moff, std::vector<int64_t>(f.moff.begin(), f.moff.begin() + ns), s);
@@ -371,7 +455,8 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
     put(kpos, P.kpos, s);
     put(kval, P.kval, s);
     put(lvl, P.lvl_sn, s);
-    put(ditems, items, s);
+    put(dfronts, fronts, s);
+    put(dhints, hints, s);
     status.alloc(1);
     PDGB_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int), s));
     PDGB_CUDA_TRY(cudaMemsetAsync(mval, 0, (size_t)f.mval_size * sizeof(float), s));
@@ -389,12 +474,13 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
             k_fz<<<dim3(nf, l.ychunks), 256, 0, s>>>(d, list);
             k_fk<<<nf, 256, 0, s>>>(d, list);
             k_fea<<<dim3(nf, l.ycols), 256, 0, s>>>(d, list);
-        } else if (l.kind == 1) {
-            k_fdiag<<<nf, 32, 0, s>>>(d, list, l.j0);
-            if (l.n0) k_fpanel<<<(unsigned)l.n0, kRowChunk, 0, s>>>(d, ditems.p + l.i0, l.j0);
-            if (l.n1) k_ftrail<<<(unsigned)l.n1, 256, 0, s>>>(d, ditems.p + l.i1, l.j0);
         } else {
-            if (l.n0) k_fm<<<(unsigned)l.n0, 256, 0, s>>>(d, ditems.p + l.i0);
+            const FrontRef* fr = dfronts.p + l.front0;
+            const int* hint = dhints.p + l.hint0;
+            if (l.kind == 1) launch_pdl(k_panel, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0, l.size);
+            else if (l.size == kNB) launch_pdl(k_trail<kNB>, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0);
+            else if (l.size == kNB / 2) launch_pdl(k_trail<kNB / 2>, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0);
+            else launch_pdl(k_trail<kNB / 4>, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0);
         }
         err = cudaGetLastError();
     }
