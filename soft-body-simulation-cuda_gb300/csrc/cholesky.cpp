@@ -47,24 +47,31 @@ SparseSym assemble_system(int nv, int nt, const uint32_t* tets4, const double* d
                 cx[fill[id[a]]++] = s;
             }
     }
+    // each row's distinct columns summed in place, then only those sorted (a
+    // vertex has 20 to 30 corners, so 80 to 120 entries in 7 to 27 columns)
     SparseSym K;
     K.n = nv;
     K.p.assign(nv + 1, 0);
-    K.i.reserve(cnt[nv] / 2);
-    K.x.reserve(cnt[nv] / 2);
-    std::vector<std::pair<int, double>> row;
+    K.i.reserve(cnt[nv] / 4);
+    K.x.reserve(cnt[nv] / 4);
+    std::vector<double> sum(nv);
+    std::vector<int> seen(nv, -1), cols;
     for (int v = 0; v < nv; ++v) {
-        row.clear();
-        for (int64_t e = cnt[v]; e < cnt[v + 1]; ++e) row.push_back({ci[e], cx[e]});
-        std::sort(row.begin(), row.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-        int last = -1;
-        for (auto& e : row) {
-            if (e.first == last) K.x.back() += e.second;
-            else {
-                K.i.push_back(e.first);
-                K.x.push_back(e.second);
-                last = e.first;
+        cols.clear();
+        for (int64_t e = cnt[v]; e < cnt[v + 1]; ++e) {
+            const int c = ci[e];
+            if (seen[c] != v) {
+                seen[c] = v;
+                sum[c] = cx[e];
+                cols.push_back(c);
+            } else {
+                sum[c] += cx[e];
             }
+        }
+        std::sort(cols.begin(), cols.end());
+        for (int c : cols) {
+            K.i.push_back(c);
+            K.x.push_back(sum[c]);
         }
         K.p[v + 1] = (int64_t)K.i.size();
     }

@@ -450,7 +450,7 @@ void worker_loop(pdgb_server* S) {
         }
         bool ok = true;
         try {
-            const MeshKey key = mesh_key(*r);
+            const MeshKey key = S->cache_cap > 0 ? mesh_key(*r) : MeshKey{0, 0};  // used by the cache only
             if (S->cache_cap > 0) {
                 std::lock_guard<std::mutex> ck(S->cache_mu);
                 auto it = S->cache.find(key.a);
