@@ -63,6 +63,28 @@ __device__ __forceinline__ float len(F3 a) { return sqrtf(dot(a, a)); }
 __device__ __forceinline__ F3 unit(F3 a) { return scl(1.0f / len(a), a); }
 __device__ __forceinline__ float triple(F3 u, F3 v, F3 w) { return dot(u, cross(v, w)); }
 
+// The query's thresholds are double literals in the reference.  FP64 compares
+// in the Newton loop took most of the narrow phase (a conversion and a compare
+// per iteration at two lanes a clock and SM), so they are decided in float:
+// for a float f and a double threshold, f < 1e-6 holds exactly when
+// f <= 1e-6f, the largest float below 1e-6, and so on.
+constexpr float kBelow6 = 1e-6f;            // f < 1e-6   <=>  f <= kBelow6
+constexpr float kUpTo3 = 0.00099999993f;    // f >= -1e-3 <=>  f >= -kUpTo3
+constexpr float kBelow12 = 1e-12f;          // f < -1e-12 <=>  f < -kBelow12
+static_assert((double)kBelow6 < 1e-6 && (double)kBelow6 * (1.0 + 1.2e-7) > 1e-6, "largest float below 1e-6");
+static_assert((double)kUpTo3 <= 1e-3 && (double)kUpTo3 * (1.0 + 1.2e-7) > 1e-3, "largest float up to 1e-3");
+static_assert((double)kBelow12 < 1e-12 && (double)kBelow12 * (1.0 + 1.2e-7) > 1e-12, "largest float below 1e-12");
+
+// a > 1e-12 b in double (a, b >= 0): decided in float where the two differ by
+// more than float's rounding, in double where they do not or could underflow.
+__device__ __forceinline__ bool above_scaled(float a, float b) {
+    if (b > 1e-20f && b < 1e30f) {
+        if (a > 1.00001e-12f * b) return true;
+        if (a < 0.99999e-12f * b) return false;
+    }
+    return a > 1e-12 * b;
+}
+
 // Real roots of a x^2 + b x + c in the numerically stable form; 0 with the
 // vertex -b / 2a in x[0] when the discriminant is negative.
 __device__ int quad_roots(float a, float b, float c, float* x) {
@@ -74,8 +96,8 @@ __device__ int quad_roots(float a, float b, float c, float* x) {
     const float sgn = (b > 0) ? 1.0f : (b < 0 ? -1.0f : 0.0f);
     const float q = -(b + sgn * sqrtf(d)) / 2;
     int n = 0;
-    if (fabsf(a) > 1e-12 * fabsf(q)) x[n++] = q / a;
-    if (fabsf(q) > 1e-12 * fabsf(c)) x[n++] = c / q;
+    if (above_scaled(fabsf(a), fabsf(q))) x[n++] = q / a;
+    if (above_scaled(fabsf(q), fabsf(c))) x[n++] = c / q;
     if (n == 2 && x[0] > x[1]) {
         const float t = x[0];
         x[0] = x[1];
@@ -92,12 +114,17 @@ __device__ float cubic_newton(float a, float b, float c, float d, float x0, int 
         const float ddy0 = 2 * b + x0 * (6 * a);
         if (ddy0 != 0) x0 += dir * sqrtf(fabsf(2 * y0 / ddy0));
     }
+    float before = __int_as_float(0x7fffffff);  // the iterate before x0 (NaN: none)
     for (int it = 0; it < 100; ++it) {
         const float y = d + x0 * (c + x0 * (b + x0 * a));
         const float dy = c + x0 * (2 * b + x0 * 3 * a);
         if (dy == 0) return x0;
         const float x1 = x0 - y / dy;
-        if (fabsf(x0 - x1) < 1e-6) return x0;
+        if (fabsf(x0 - x1) <= kBelow6) return x0;
+        // far roots end up swapping between two neighbouring floats more than
+        // 1e-6 apart: the hundredth iterate is known then
+        if (x1 == before) return (99 - it) % 2 == 0 ? x1 : x0;
+        before = x0;
         x0 = x1;
     }
     return x0;
@@ -128,7 +155,7 @@ __device__ int cubic_roots(float a, float b, float c, float d, float* x) {
 // the barycentric weights (w0 = 1, w1..3 = minus the face coordinates).
 __device__ float face_distance(F3 p, F3 y0, F3 y1, F3 y2, F3& n, float w[4]) {
     n = cross(unit(sub(y1, y0)), unit(sub(y2, y0)));
-    if (dot(n, n) < 1e-6) return FLT_MAX;
+    if (dot(n, n) <= kBelow6) return FLT_MAX;
     n = unit(n);
     const float h = dot(sub(p, y0), n);
     const float b0 = triple(sub(y1, p), sub(y2, p), n), b1 = triple(sub(y2, p), sub(y0, p), n),
@@ -145,7 +172,7 @@ __device__ float face_distance(F3 p, F3 y0, F3 y1, F3 y2, F3& n, float w[4]) {
 // common normal and the weights (w0, w1 on the first, -w2, -w3 on the second).
 __device__ float edge_distance(F3 x0, F3 x1, F3 y0, F3 y1, F3& n, float w[4]) {
     n = cross(unit(sub(x1, x0)), unit(sub(y1, y0)));
-    if (dot(n, n) < 1e-6) return FLT_MAX;
+    if (dot(n, n) <= kBelow6) return FLT_MAX;
     n = unit(n);
     const float h = dot(sub(x0, y0), n);
     const float a0 = triple(sub(y1, x1), sub(y0, x1), n), a1 = triple(sub(y0, x0), sub(y1, x0), n);
@@ -155,6 +182,16 @@ __device__ float edge_distance(F3 x0, F3 x1, F3 y0, F3 y1, F3& n, float w[4]) {
     w[2] = -b0 / (b0 + b1);
     w[3] = -b1 / (b0 + b1);
     return h;
+}
+
+// a < 1e-12 l0 l1 l2 in double: decided in float where it is clear.
+__device__ __forceinline__ bool coplanar(float a, float l0, float l1, float l2) {
+    const float p = l0 * l1 * l2;
+    if (p > 1e-20f && p < 1e30f) {
+        if (a < 0.99999e-12f * p) return true;
+        if (a > 1.00001e-12f * p) return false;
+    }
+    return a < 1e-12 * l0 * l1 * l2;
 }
 
 // Earliest contact time in [0, 1] of a point-face (face: point q0, face
@@ -170,11 +207,11 @@ __device__ float narrow_test(bool face, const F3 x[4], const F3 v[4], F3& n) {
     const float a2 = triple(x01, v02, v03) + triple(v01, x02, v03) + triple(v01, v02, x03);
     const float a3 = triple(v01, v02, v03);
     n = {0.f, 0.f, 0.f};
-    if (fabsf(a0) < 1e-12 * len(x01) * len(x02) * len(x03)) return 1.0f;  // coplanar at t = 0
+    if (coplanar(fabsf(a0), len(x01), len(x02), len(x03))) return 1.0f;  // coplanar at t = 0
     float t[3];
     const int nr = cubic_roots(a3, a2, a1, a0, t);
     for (int i = 0; i < nr; ++i) {
-        if (t[i] < -1e-12 || t[i] > 1) continue;
+        if (t[i] < -kBelow12 || t[i] > 1) continue;
         F3 xt[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) xt[k] = add(x[k], scl(t[i], v[k]));
@@ -183,14 +220,14 @@ __device__ float narrow_test(bool face, const F3 x[4], const F3 v[4], F3& n) {
         bool inside;
         if (face) {
             d = face_distance(xt[0], xt[1], xt[2], xt[3], n, w);
-            inside = fminf(-w[1], fminf(-w[2], -w[3])) >= -1e-3;
+            inside = fminf(-w[1], fminf(-w[2], -w[3])) >= -kUpTo3;
         } else {
             d = edge_distance(xt[0], xt[1], xt[2], xt[3], n, w);
-            inside = fminf(w[0], fminf(w[1], fminf(-w[2], -w[3]))) >= -1e-3;
+            inside = fminf(w[0], fminf(w[1], fminf(-w[2], -w[3]))) >= -kUpTo3;
         }
         const F3 rel = add(add(scl(w[1], v[1]), scl(w[2], v[2])), scl(w[3], v[3]));
         if (dot(n, rel) > 0) n = scl(-1.0f, n);
-        if (fabsf(d) < 1e-6 && inside) return t[i];
+        if (fabsf(d) <= kBelow6 && inside) return t[i];
     }
     return 1.0f;
 }
@@ -371,8 +408,11 @@ __global__ void k_refit(Dev d) {
     if (j >= n) return;
     const int t = d.order_sorted[j];
     int node = n - 1 + j;
-    d.node_lo[node] = d.tri_lo[t];
-    d.node_hi[node] = d.tri_hi[t];
+    // w lanes: the least and the greatest body below the node
+    float4 lo = d.tri_lo[t], hi = d.tri_hi[t];
+    lo.w = hi.w = __uint_as_float(d.tri[t].w);
+    d.node_lo[node] = lo;
+    d.node_hi[node] = hi;
     if (n == 1) return;
     for (int guard = 0; guard < n; ++guard) {
         node = d.parent[node];
@@ -381,8 +421,12 @@ __global__ void k_refit(Dev d) {
         const int2 c = d.child[node];
         const float4 al = __ldcg(&d.node_lo[c.x]), ah = __ldcg(&d.node_hi[c.x]);
         const float4 bl = __ldcg(&d.node_lo[c.y]), bh = __ldcg(&d.node_hi[c.y]);
-        d.node_lo[node] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f);
-        d.node_hi[node] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f);
+        const uint32_t body0 = min(__float_as_uint(al.w), __float_as_uint(bl.w)),
+                       body1 = max(__float_as_uint(ah.w), __float_as_uint(bh.w));
+        d.node_lo[node] =
+            make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __uint_as_float(body0));
+        d.node_hi[node] =
+            make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), __uint_as_float(body1));
         if (node == 0) return;
     }
 }
@@ -392,6 +436,10 @@ __device__ __forceinline__ bool share_vertex(uint4 a, uint4 b) {
            a.z == b.y || a.z == b.z;
 }
 
+// Subtrees that hold triangles of the thread's own body only are skipped: a
+// triangle overlaps its neighbours on the same surface first of all, and a
+// pair of one body is never a candidate.  A visit is a chain of three loads
+// (children, boxes, triangle), so what counts is how many nodes are visited.
 __global__ void k_traverse(Dev d) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = d.ntris;
@@ -409,7 +457,9 @@ __global__ void k_traverse(Dev d) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int ch = kids[k];
-            if (!overlap(lo, hi, d.node_lo[ch], d.node_hi[ch])) continue;
+            const float4 clo = d.node_lo[ch], chi = d.node_hi[ch];
+            if (__float_as_uint(clo.w) == ta.w && __float_as_uint(chi.w) == ta.w) continue;
+            if (!overlap(lo, hi, clo, chi)) continue;
             if (ch >= n - 1) {
                 const int B = d.order_sorted[ch - (n - 1)];
                 if (B <= A) continue;  // each unordered pair once
