@@ -108,7 +108,6 @@ __device__ __forceinline__ void add_run(const float4* __restrict__ slot, int k, 
 // deterministic.
 template <bool kJacobiForm, int kRotation>
 __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4* slot, float4* pos) {
-    pdl_trigger();
     const int vb = a.tile_vptr[tile];
     const int np = a.tile_vptr[tile + 1] - vb;
     const int t0 = a.tile_tet_ptr[tile], t1 = a.tile_tet_ptr[tile + 1];
@@ -135,6 +134,7 @@ __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4*
     // the tile's layout and first geometry are in flight; positions, b and
     // the early-exit flag come from earlier kernels of the step
     pdl_wait();
+    pdl_trigger();
     if (a.done && *a.done) return;
     // the first patch vertex of each thread keeps its id and slot run in
     // registers for the reduction phase
@@ -343,8 +343,8 @@ __global__ void __launch_bounds__(kLocalThreads, PDGB_LOCAL_MIN_BLOCKS) k_local_
         if ((int)(blockIdx.x + gridDim.x) < ntiles) next = tile_bounds(a, blockIdx.x + gridDim.x);
     }
     __syncthreads();
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     if (a.done && *a.done) {
         // the first copies may still be landing in shared memory
         mbar_wait_bounded(&bar[0], 0, kPipeWaitNs);

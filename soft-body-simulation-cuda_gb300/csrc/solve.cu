@@ -19,7 +19,7 @@
 namespace pdgb {
 
 // The per-level kernels are launched with programmatic dependent launch
-// (pdl.cuh): each triggers its dependents at entry and, before its wait,
+// (pdl.cuh): each, before its wait,
 // reads only its item descriptors, factor blocks and row ids -- never r, y,
 // x, z or the early-exit flag, which earlier kernels write.
 
@@ -431,13 +431,13 @@ __global__ void __launch_bounds__(kLevelThreads, kFwdBlocks) k_chol_fwd_level(Ch
     extern __shared__ float4 tile[];  // a tile, or kWarpFloats a warp
     float* blocks = reinterpret_cast<float*>(tile);
     __shared__ float4 vec[kLevelWarps * 32];
-    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int u = blockIdx.x;
     if (u < v.nb) {
         TilePre p;
         tile_load(a, v.b0 + u, tile, p);
         pdl_wait();
+        pdl_trigger();
         if (a.done && *a.done) {
             cp_async_wait();
             return;
@@ -451,6 +451,7 @@ __global__ void __launch_bounds__(kLevelThreads, kFwdBlocks) k_chol_fwd_level(Ch
         SmallPre p{};
         if (it < v.ns) small_load(a, v.s0 + it, blocks + kWarpFloats * warp, lane, p);
         pdl_wait();
+        pdl_trigger();
         if (a.done && *a.done) {
             cp_async_wait();
             return;
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(kLevelThreads, kFwdBlocks) k_chol_fwd_level(Ch
     TinyPre p;
     tiny_load(a, v.t0 + it, it < v.nt, j, p);
     pdl_wait();
+    pdl_trigger();
     if (a.done && *a.done) return;
     fwd_tiny_run(a, p, j);
 }
@@ -471,13 +473,13 @@ __global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(Ch
     extern __shared__ float4 tile[];  // a tile, or kWarpFloats a warp
     float* blocks = reinterpret_cast<float*>(tile);
     __shared__ float4 vec[kLevelWarps * 32];
-    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int u = blockIdx.x;
     if (u < v.nb) {
         TilePre p;
         tile_load(a, v.b0 + u, tile, p);
         pdl_wait();
+        pdl_trigger();
         if (a.done && *a.done) {
             cp_async_wait();
             return;
@@ -491,6 +493,7 @@ __global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(Ch
         SmallPre p{};
         if (it < v.ns) small_load(a, v.s0 + it, blocks + kWarpFloats * warp, lane, p);
         pdl_wait();
+        pdl_trigger();
         if (a.done && *a.done) {
             cp_async_wait();
             return;
@@ -504,6 +507,7 @@ __global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(Ch
         TinyPre p;
         tiny_load(a, v.t0 + it, it < v.nt, j, p);
         pdl_wait();
+        pdl_trigger();
         if (a.done && *a.done) return;
         bwd_tiny_run(a, p, j);
         return;
@@ -515,6 +519,7 @@ __global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(Ch
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < q.nv && q.b) b = __ldg(&q.coef[i]).z != 0.f ? __ldg(&q.pin_rhs[i]) : __ldg(&q.base[i]);
     pdl_wait();
+    pdl_trigger();
     if ((a.done && *a.done) || i >= q.nv) return;
     q.y_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (q.b) q.b[i] = b;
@@ -992,36 +997,60 @@ __global__ void __launch_bounds__(256) k_chol_finish(CholVertexArgs a) {
     a.y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// ---- iterative refinement
+// ---- iterative refinement.  The three kernels are links of the same chain of
+// dependent launches as the levels (pdl.cuh).
 __global__ void __launch_bounds__(256) k_copy_rhs(int nv, const float4* __restrict__ b, float4* bsave,
                                                   const int* done) {
+    pdl_wait();
+    pdl_trigger();
     if (done && *done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < nv) bsave[i] = b[i];
 }
 
-// One warp per row: r = bsave - K x0 accumulated in double over the row's
-// nonzeros (lanes stride the row, then a warp reduction).
-__global__ void __launch_bounds__(256) k_refine_residual(RefineArgs a) {
-    if (a.done && *a.done) return;
-    const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= a.nv) return;
-    double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int e = __ldg(&a.rowptr[row]) + lane; e < __ldg(&a.rowptr[row + 1]); e += 32) {
-        const double kv = __ldg(&a.val[e]);
-        const float4 xv = a.x0[__ldg(&a.colind[e])];
-        sx = fma(kv, (double)xv.x, sx);
-        sy = fma(kv, (double)xv.y, sy);
-        sz = fma(kv, (double)xv.z, sz);
-    }
+// r = bsave - K x0 accumulated in double over the row's nonzeros (7 to 27 on
+// a tet mesh), kRowLanes lanes a row.  FP64 runs at two lanes a clock and SM
+// whether they hold a value or not: with a warp a row, most of its adds were
+// of the reduction and of idle lanes (12.5 us on 5,760 rows).  Row bounds,
+// indices and values are read before the wait.
+constexpr int kRowLanes = 4;
+constexpr int kRowPre = 4;  // entries a lane holds before the wait
+__global__ void __launch_bounds__(128) k_refine_residual(RefineArgs a) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = t / kRowLanes, lane = t % kRowLanes;
+    const bool live = row < a.nv;
+    const int e0 = live ? __ldg(&a.rowptr[row]) + lane : 0, e1 = live ? __ldg(&a.rowptr[row + 1]) : 0;
+    double kv[kRowPre];
+    int ci[kRowPre];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int q = 0; q < kRowPre; ++q) {
+        const int e = e0 + kRowLanes * q;
+        kv[q] = e < e1 ? __ldg(&a.val[e]) : 0.0;
+        ci[q] = e < e1 ? __ldg(&a.colind[e]) : -1;
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (a.done && *a.done) return;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    auto add = [&](double k, const float4& x) {
+        sx = fma(k, (double)x.x, sx);
+        sy = fma(k, (double)x.y, sy);
+        sz = fma(k, (double)x.z, sz);
+    };
+    float4 xv[kRowPre];
+#pragma unroll
+    for (int q = 0; q < kRowPre; ++q) xv[q] = ci[q] >= 0 ? __ldcg(&a.x0[ci[q]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < kRowPre; ++q)
+        if (ci[q] >= 0) add(kv[q], xv[q]);
+    for (int e = e0 + kRowLanes * kRowPre; e < e1; e += kRowLanes) add(__ldg(&a.val[e]), __ldcg(&a.x0[__ldg(&a.colind[e])]));
+#pragma unroll
+    for (int off = kRowLanes / 2; off > 0; off >>= 1) {
         sx += __shfl_xor_sync(0xffffffffu, sx, off);
         sy += __shfl_xor_sync(0xffffffffu, sy, off);
         sz += __shfl_xor_sync(0xffffffffu, sz, off);
     }
-    if (lane == 0) {
+    if (live && lane == 0) {
         const float4 b = a.bsave[row];
         a.b[row] = make_float4((float)((double)b.x - sx), (float)((double)b.y - sy), (float)((double)b.z - sz), 0.f);
         a.y[row] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1029,6 +1058,8 @@ __global__ void __launch_bounds__(256) k_refine_residual(RefineArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_refine_update(RefineArgs a) {
+    pdl_wait();
+    pdl_trigger();
     if (a.done && *a.done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nv) return;
@@ -1037,13 +1068,14 @@ __global__ void __launch_bounds__(256) k_refine_update(RefineArgs a) {
 }
 
 void launch_copy_rhs(int nv, const float4* b, float4* bsave, const int* done, cudaStream_t s) {
-    if (nv > 0) k_copy_rhs<<<(nv + 255) / 256, 256, 0, s>>>(nv, b, bsave, done);
+    if (nv > 0) launch_pdl(k_copy_rhs, (nv + 255) / 256, 256, 0, s, nv, b, bsave, done);
 }
 void launch_refine_residual(const RefineArgs& a, cudaStream_t s) {
-    if (a.nv > 0) k_refine_residual<<<(a.nv + 7) / 8, 256, 0, s>>>(a);
+    constexpr int kRows = 128 / kRowLanes;
+    if (a.nv > 0) launch_pdl(k_refine_residual, (a.nv + kRows - 1) / kRows, 128, 0, s, a);
 }
 void launch_refine_update(const RefineArgs& a, cudaStream_t s) {
-    if (a.nv > 0) k_refine_update<<<(a.nv + 255) / 256, 256, 0, s>>>(a);
+    if (a.nv > 0) launch_pdl(k_refine_update, (a.nv + 255) / 256, 256, 0, s, a);
 }
 
 void launch_chol_vertex(const CholVertexArgs& a, cudaStream_t s) {
