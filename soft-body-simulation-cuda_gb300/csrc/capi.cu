@@ -128,6 +128,13 @@ namespace {
 // factor as one dense supernode.
 constexpr int kDenseTuneMaxVerts = 4096;
 
+// Most tets per tile of a new engine.  512 (two a thread) has the least halo and
+// wins where it fills the SMs; below that more, smaller tiles do.  One Jacobi
+// iteration with 128 / 256 / 512: 5,000 tets 4.3 / 4.6 / 5.1 us, 13,720 tets
+// 4.3 / 4.5 / 5.1 us, 24,035 tets 4.7 / 4.6 / 5.3 us, 71,675 tets 5.6 / 5.7 /
+// 6.4 us, 163,840 tets 10.3 / 8.3 / 8.1 us, 320,000 tets 15.9 / 12.1 / 10.7 us.
+int default_tile_tets(int nt) { return nt <= 20000 ? kTileTets / 4 : nt <= 110000 ? kTileTets / 2 : kTileTets; }
+
 // Factors up to this many stored entries use the single-CTA solve.
 constexpr size_t kCtaSolveMaxEntries = 1u << 15;
 
@@ -187,6 +194,10 @@ LocalArgs local_args(pdgb_engine* e, const int* done) {
     a.done = done;
     a.pipe_grid = e->local_kernel == PDGB_LOCAL_PIPELINED ? e->pipe_grid : 0;
     a.timeout = &e->st.p->local_timeout;
+    // The geometry is read once an iteration, the vertex vectors several times
+    // over: past L2 it is the geometry that has to make room (79 x 61 x 83 cells,
+    // 2.0 M tets: a Jacobi step 963 -> 878 us; 64^3, which fits, 598 -> 592 us).
+    a.geo_evict_first = 1;
     return a;
 }
 
@@ -270,18 +281,22 @@ void record_jacobi_step(pdgb_engine* e) {
     const int n = e->prm.num_iterations;
     launch_begin(begin_args(e), s);
     const std::vector<float> omega = chebyshev_omegas(n, e->prm.rho);
-    const LocalArgs la = local_args(e, nullptr);
+    LocalArgs la = local_args(e, nullptr);
     VertexArgs va{e->nv, e->sn.p, e->prev.p, e->b.p, e->base.p, e->coef.p, e->pin_rhs.p, e->x.p, e->v.p, 1.f,
                   1.0f / e->prm.dt};
     va.sc = scene_args(e);
     for (int i = 0; i < n; ++i) {
+        la.sn = va.sn;
         record_local(e, la, true, i);
         int mode = 0;
-        if (i >= 11) mode |= kReadPrev;                // omega != 1 from iteration 11 on
-        if (i >= 10 && i + 1 < n) mode |= kWritePrev;  // prev is read from iteration 11 on
+        if (i >= 11) mode |= kReadPrev;  // omega != 1 from iteration 11 on
         if (i + 1 == n) mode |= kFinal;
         va.omega = omega[i];
+        // from iteration 10 on the iterate is the next one's prev: the two
+        // buffers take turns
+        va.out = i >= 10 ? va.prev : va.sn;
         launch_jacobi_vertex(va, mode, s);
+        if (i >= 10) std::swap(va.sn, va.prev);
     }
 }
 
@@ -612,7 +627,7 @@ int create_impl(const pdgb_mesh_desc* mesh, const pdgb_params* params, void* str
         }
         build_layout(e->nv, e->nt, e->X0.data(), e->tets.data(), e->mass.data(), e->mu.data(),
                      e->has_dbc ? e->dbc.data() : nullptr, e->prm, e->L, e->nbodies,
-                     e->nbodies > 1 ? e->body_vstart.data() : nullptr);
+                     e->nbodies > 1 ? e->body_vstart.data() : nullptr, default_tile_tets(e->nt));
         upload_mesh(e);
         // initial state X (and V) from the descriptor
         std::vector<float> Vh;

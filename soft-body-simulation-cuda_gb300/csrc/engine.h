@@ -148,6 +148,7 @@ struct LocalArgs {
     // waits for a bulk copy runs out.
     int pipe_grid;
     int* timeout;
+    int geo_evict_first;  // the tets' geometry is the first to leave L2
 };
 
 // Vertex-kernel mode flags.
@@ -198,6 +199,7 @@ struct VertexArgs {
     float omega;
     float dt_inv;
     SceneArgs sc;
+    float4* out;  // single engines: where the new iterate goes (sn, or the buffer of the one before)
 };
 
 struct BeginArgs {

@@ -106,8 +106,33 @@ __device__ __forceinline__ void add_run(const float4* __restrict__ slot, int k, 
 // to b with one float4 atomic (pinned vertices are skipped: their RHS is the
 // pin term).  No shared-memory atomics; within a tile the sums are
 // deterministic.
+__device__ __forceinline__ uint64_t l2_policy(bool evict_first) {
+    uint64_t p, q;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(q));
+    return evict_first ? p : q;
+}
+__device__ __forceinline__ float4 ld_hint(const float4* a, uint64_t policy) {
+    float4 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(a), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ float2 ld_hint(const float2* a, uint64_t policy) {
+    float2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(a), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_hint(const uint2* a, uint64_t policy) {
+    uint2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(a), "l"(policy));
+    return v;
+}
+
 template <bool kJacobiForm, int kRotation>
 __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4* slot, float4* pos) {
+    const uint64_t policy = l2_policy(a.geo_evict_first != 0);
     const int vb = a.tile_vptr[tile];
     const int np = a.tile_vptr[tile + 1] - vb;
     const int t0 = a.tile_tet_ptr[tile], t1 = a.tile_tet_ptr[tile + 1];
@@ -126,10 +151,10 @@ __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4*
     {
         const int lt = threadIdx.x;
         const int t = t0 + (lt < ntile ? lt : 0);
-        GA[0] = __ldg(geo0 + t);
-        GB[0] = __ldg(geo0 + ntp + t);
-        GC[0] = __ldg(geo2 + t);
-        S[0] = __ldg(reinterpret_cast<const uint2*>(a.inc_ent) + t);
+        GA[0] = ld_hint(geo0 + t, policy);
+        GB[0] = ld_hint(geo0 + ntp + t, policy);
+        GC[0] = ld_hint(geo2 + t, policy);
+        S[0] = ld_hint(reinterpret_cast<const uint2*>(a.inc_ent) + t, policy);
     }
     // the tile's layout and first geometry are in flight; positions, b and
     // the early-exit flag come from earlier kernels of the step
@@ -156,10 +181,10 @@ __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4*
     for (int j = 1; j < kPer; ++j) {
         const int lt = threadIdx.x + j * kLocalThreads;
         const int t = t0 + (lt < ntile ? lt : 0);
-        GA[j] = __ldg(geo0 + t);
-        GB[j] = __ldg(geo0 + ntp + t);
-        GC[j] = __ldg(geo2 + t);
-        S[j] = __ldg(reinterpret_cast<const uint2*>(a.inc_ent) + t);
+        GA[j] = ld_hint(geo0 + t, policy);
+        GB[j] = ld_hint(geo0 + ntp + t, policy);
+        GC[j] = ld_hint(geo2 + t, policy);
+        S[j] = ld_hint(reinterpret_cast<const uint2*>(a.inc_ent) + t, policy);
     }
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
@@ -504,10 +529,10 @@ void launch_local(const LocalArgs& a, int ntiles, int max_patch, bool jacobi_for
     }
     const size_t sm = (size_t)max_patch * sizeof(float4);
     if (rotation == PDGB_ROTATION_SVD) {
-        if (jacobi_form) k_local<true, PDGB_ROTATION_SVD><<<ntiles, kLocalThreads, sm, s>>>(a);
+        if (jacobi_form) launch_pdl(k_local<true, PDGB_ROTATION_SVD>, ntiles, kLocalThreads, sm, s, a);
         else launch_pdl(k_local<false, PDGB_ROTATION_SVD>, ntiles, kLocalThreads, sm, s, a);
     } else {
-        if (jacobi_form) k_local<true, PDGB_ROTATION_QUAT><<<ntiles, kLocalThreads, sm, s>>>(a);
+        if (jacobi_form) launch_pdl(k_local<true, PDGB_ROTATION_QUAT>, ntiles, kLocalThreads, sm, s, a);
         else launch_pdl(k_local<false, PDGB_ROTATION_QUAT>, ntiles, kLocalThreads, sm, s, a);
     }
 }
@@ -515,15 +540,34 @@ void launch_local(const LocalArgs& a, int ntiles, int max_patch, bool jacobi_for
 // ------------------------------------------------------- vertex kernels
 // (relax09: the 0.9 under-relaxation of pdUtil.cu:221, relax.cuh)
 
-template <int kMode>
-__device__ __forceinline__ void jacobi_vertex(const VertexArgs& a, int i, float omega) {
-    const float4 s = a.sn[i];
-    const float4 cf = __ldg(&a.coef[i]);
+// The update of vertex i.  kSwap (single engines): the new iterate goes to
+// a.out, the buffer of the iterate before (which it may read as prev), so that
+// sn itself is the next iteration's prev and nothing is copied; otherwise in
+// place, with prev kept by a copy (kWritePrev).  Everything but b was written
+// before the local step that precedes this kernel began, so with kWait it is
+// read before the grid dependency wait.
+template <int kMode, bool kSwap, bool kWait>
+__device__ __forceinline__ void jacobi_vertex(const VertexArgs& a, int i, bool live, float omega) {
+    float4 s = {}, cf = {}, bb = {}, p = {}, base = {};
+    float w = 0.f;
+    if (live) {
+        s = a.sn[i];
+        cf = __ldg(&a.coef[i]);
+        if (cf.z != 0.f) bb = __ldg(&a.pin_rhs[i]);
+        if (kMode & kReadPrev) p = a.prev[i];
+        if (!(kMode & kFinal)) base = a.base[i];
+        w = drag_weight(a.sc, i);
+    }
+    if (kWait) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    if (!live) return;
+    if (cf.z == 0.f) bb = a.b[i];
     const float cm = cf.x, md = cf.y;
-    const float4 bb = (cf.z != 0.f) ? __ldg(&a.pin_rhs[i]) : a.b[i];
     const float den = cm + md;
     float4 nx;
-    if (drag_weight(a.sc, i) > 0.f) {
+    if (w > 0.f) {
         nx = s;  // dragged vertices keep the current iterate (getErrorKern, pdUtil.cu:200-205)
     } else {
         nx.x = (bb.x - cm * s.x) / den + s.x;
@@ -535,24 +579,23 @@ __device__ __forceinline__ void jacobi_vertex(const VertexArgs& a, int i, float 
     nx.z = relax09(nx.z, s.z);
     nx.w = 0.f;
     if (kMode & kReadPrev) {
-        const float4 p = a.prev[i];
         nx.x = (nx.x - p.x) * omega + p.x;
         nx.y = (nx.y - p.y) * omega + p.y;
         nx.z = (nx.z - p.z) * omega + p.z;
     }
-    if (kMode & kWritePrev) a.prev[i] = s;
+    if (!kSwap && (kMode & kWritePrev)) a.prev[i] = s;
     if (kMode & kFinal) {
         finish_vertex(a.sc, i, nx, a.dt_inv, a.x, a.v);
     } else {
-        a.sn[i] = nx;
-        a.b[i] = __ldg(&a.base[i]);
+        (kSwap ? a.out : a.sn)[i] = nx;
+        a.b[i] = base;
     }
 }
 
 template <int kMode>
 __global__ void __launch_bounds__(256) k_jacobi_vertex(VertexArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.nv) jacobi_vertex<kMode>(a, i, a.omega);
+    jacobi_vertex<kMode, true, true>(a, i, i < a.nv, a.omega);
 }
 
 // Multi-request form: CTA i updates 256 vertices of request list[i].x
@@ -565,7 +608,7 @@ __global__ void __launch_bounds__(256) k_jacobi_vertex_multi(const VertexArgs* _
     const int2 w = list[blockIdx.x];
     const VertexArgs& a = req[w.x];
     const int i = w.y + threadIdx.x;
-    if (i < a.nv) jacobi_vertex<kMode>(a, i, omega);
+    jacobi_vertex<kMode, false, false>(a, i, i < a.nv, omega);
 }
 
 void launch_jacobi_vertex_multi(const VertexArgs* req, const int2* list, const int* count, int grid, int mode,
@@ -586,15 +629,11 @@ void launch_jacobi_vertex_multi(const VertexArgs* req, const int2* list, const i
 void launch_jacobi_vertex(const VertexArgs& a, int mode, cudaStream_t s) {
     const int blocks = (a.nv + 255) / 256;
     if (blocks == 0) return;
-    switch (mode & 7) {
-        case 0: k_jacobi_vertex<0><<<blocks, 256, 0, s>>>(a); break;
-        case 1: k_jacobi_vertex<1><<<blocks, 256, 0, s>>>(a); break;
-        case 2: k_jacobi_vertex<2><<<blocks, 256, 0, s>>>(a); break;
-        case 3: k_jacobi_vertex<3><<<blocks, 256, 0, s>>>(a); break;
-        case 4: k_jacobi_vertex<4><<<blocks, 256, 0, s>>>(a); break;
-        case 5: k_jacobi_vertex<5><<<blocks, 256, 0, s>>>(a); break;
-        case 6: k_jacobi_vertex<6><<<blocks, 256, 0, s>>>(a); break;
-        default: k_jacobi_vertex<7><<<blocks, 256, 0, s>>>(a); break;
+    switch (mode & (kReadPrev | kFinal)) {
+        case 0: launch_pdl(k_jacobi_vertex<0>, blocks, 256, 0, s, a); break;
+        case kReadPrev: launch_pdl(k_jacobi_vertex<kReadPrev>, blocks, 256, 0, s, a); break;
+        case kFinal: launch_pdl(k_jacobi_vertex<kFinal>, blocks, 256, 0, s, a); break;
+        default: launch_pdl(k_jacobi_vertex<kReadPrev | kFinal>, blocks, 256, 0, s, a); break;
     }
 }
 
