@@ -365,10 +365,9 @@ int pdgb_get_local_kernel(pdgb_engine* e, int* kind);
  * one cooperative launch over the GPU, the levels of LEVELS separated by a
  * grid-wide barrier whose waits are bounded (a wait that runs out sets a
  * status word: pdgb_last_step_status then returns PDGB_ERR_TIMEOUT).  AUTO
- * picks by size: LEVELS from 2^15 stored factor entries up, below that
- * CLUSTER for a single system and CTA for a batch; pdgb_autotune times CTA,
- * CLUSTER, LEVELS and PERSISTENT.  Takes
- * effect at the next prepare; pdgb_get_solve_mode returns the schedule in
+ * picks LEVELS, the fastest at every size measured; pdgb_autotune times CTA,
+ * CLUSTER, LEVELS and PERSISTENT.  Takes effect at the
+ * next prepare; pdgb_get_solve_mode returns the schedule in
  * use (AUTO before the first prepare or on the Jacobi path). */
 #define PDGB_SOLVE_AUTO 0
 #define PDGB_SOLVE_CTA 1

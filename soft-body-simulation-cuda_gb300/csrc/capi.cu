@@ -135,9 +135,6 @@ constexpr int kDenseTuneMaxVerts = 4096;
 // 6.4 us, 163,840 tets 10.3 / 8.3 / 8.1 us, 320,000 tets 15.9 / 12.1 / 10.7 us.
 int default_tile_tets(int nt) { return nt <= 20000 ? kTileTets / 4 : nt <= 110000 ? kTileTets / 2 : kTileTets; }
 
-// Factors up to this many stored entries use the single-CTA solve.
-constexpr size_t kCtaSolveMaxEntries = 1u << 15;
-
 template <class F> int guarded(F&& f) {
     try {
         f();
@@ -439,21 +436,15 @@ void upload_mesh(pdgb_engine* e) {
 // the kernels use (M/h^2 incl. the pin weight) and the double geometry.
 SparseSym engine_system(const HostLayout& L) { return layout_system(L); }
 
-// Solve schedule: the requested one, or by size.  The per-level launches
-// (programmatic dependent launch, factor blocks loaded before each wait)
-// are fastest from a single 10^3 body up (48 K stored entries: 59 us per
-// solve against 68 us for one cluster; 512 bodies: 0.82 ms against 2.4 ms
-// for one CTA per body); below 2^15 stored entries the chain of launches
-// dominates and one cluster (a single body) or one CTA per body (a batch)
-// walks the whole tree instead.
+// Solve schedule: the requested one, or the per-level launches, which are the
+// fastest at every size: one iteration of a 2^3 body 5.6 us against 11.1 us for
+// one cluster and 12.1 us for one CTA, of 64 such bodies 6.2 against 18.4 and
+// 13.8 us, of a 10^3 body 9.9 against 40 and 114 us.
 int choose_solve_mode(const pdgb_engine* e) {
-    const bool small = (size_t)e->chol.mval_size <= kCtaSolveMaxEntries;
     const int m = e->solve_req;
     if (m == PDGB_SOLVE_DSM && !e->dsm.ok)
         throw Error{PDGB_ERR_UNSUPPORTED, "the factor does not fit the shared memory of one cluster (DSM solve)"};
-    if (m != PDGB_SOLVE_AUTO) return m;
-    if (!small) return PDGB_SOLVE_LEVELS;
-    return e->nbodies > 1 ? PDGB_SOLVE_CTA : PDGB_SOLVE_CLUSTER;
+    return m == PDGB_SOLVE_AUTO ? PDGB_SOLVE_LEVELS : m;
 }
 
 void prepare_cholesky(pdgb_engine* e) {
