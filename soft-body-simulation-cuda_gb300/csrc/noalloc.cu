@@ -26,11 +26,15 @@
 //     (cudaGetSymbolAddress) once for that device.  The address is kept for
 //     the life of the process, so a cudaDeviceReset between calls is not
 //     supported;
-//   - every call waits for its stream (after the mesh check and before it
-//     returns), so no call can be captured into a CUDA graph;
+//   - every call waits for its stream before it returns, so no call can be
+//     captured into a CUDA graph;
 //   - the mesh is checked on the device (tet indices, rest volumes, weights)
 //     before any step: a bad mesh returns PDGB_ERR_BAD_MESH with X and V
 //     untouched.
+//
+// All steps of a call are one cooperative launch: the iterations of a small
+// body are a few microseconds of work each, less than two launches of one
+// (a call of two 20-iteration steps on 5,400 tets took 81 of them).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -51,7 +55,7 @@ constexpr int kNaMaxDevices = 64;
 //   tet part   : per tet 10 floats (DmInv row-major, V0 * mu)       [kNaMaxTets]
 //   vertex part: float4 sn, prev, b, base, coef {M/h^2, diag, pin, m} [kNaMaxVerts]
 //                float  diag accumulator                            [kNaMaxVerts]
-//   flags      : int bad-mesh flag (256 bytes reserved)
+//   flags      : NaFlags (256 bytes reserved)
 // 5.2 MB + 2.6 MB + 0.1 MB = about 8 MB in total.
 constexpr size_t kNaTetBytes = (size_t)kNaMaxTets * 10 * sizeof(float);
 constexpr size_t kNaVecBytes = (size_t)kNaMaxVerts * sizeof(float4);
@@ -59,6 +63,15 @@ constexpr size_t kNaDiagBytes = (size_t)kNaMaxVerts * sizeof(float);
 constexpr size_t kNaScratchBytes = kNaTetBytes + 5 * kNaVecBytes + kNaDiagBytes + 256;
 
 static __device__ __align__(256) unsigned char g_na_scratch[kNaScratchBytes];
+
+// Cleared by each call with the diagonal before them.
+struct NaFlags {
+    int bad;                // set when a tet has an out-of-range index, no float-representable
+                            // DmInv (zero or nearly zero rest volume) or a negative or
+                            // non-finite weight
+    int timeout;            // a barrier wait ran out
+    unsigned arrived;       // CTAs that have arrived at the grid barriers so far
+};
 
 struct NaScratch {
     float* geo;     // [10][kNaMaxTets] SoA
@@ -68,9 +81,7 @@ struct NaScratch {
     float4* base;
     float4* coef;
     float* diag;
-    int* bad;       // set when a tet has an out-of-range index, no float-representable
-                    // DmInv (zero or nearly zero rest volume) or a negative or
-                    // non-finite weight
+    NaFlags* flags;
 };
 
 NaScratch carve(unsigned char* base) {
@@ -83,7 +94,7 @@ NaScratch carve(unsigned char* base) {
     s.base = reinterpret_cast<float4*>(p + 3 * kNaVecBytes);
     s.coef = reinterpret_cast<float4*>(p + 4 * kNaVecBytes);
     s.diag = reinterpret_cast<float*>(p + 5 * kNaVecBytes);
-    s.bad = reinterpret_cast<int*>(p + 5 * kNaVecBytes + kNaDiagBytes);
+    s.flags = reinterpret_cast<NaFlags*>(p + 5 * kNaVecBytes + kNaDiagBytes);
     return s;
 }
 
@@ -95,7 +106,7 @@ __global__ void na_tets(int nv, int nt, const uint32_t* __restrict__ tets, const
     if (t >= nt) return;
     const uint32_t i0 = tets[4 * t], i1 = tets[4 * t + 1], i2 = tets[4 * t + 2], i3 = tets[4 * t + 3];
     if (i0 >= (uint32_t)nv || i1 >= (uint32_t)nv || i2 >= (uint32_t)nv || i3 >= (uint32_t)nv) {
-        atomicExch(s.bad, 1);
+        atomicExch(&s.flags->bad, 1);
         return;
     }
     double D[3][3];
@@ -106,26 +117,27 @@ __global__ void na_tets(int nv, int nt, const uint32_t* __restrict__ tets, const
                        D[0][2] * (D[1][0] * D[2][1] - D[1][1] * D[2][0]);
     const float w = mu[t];
     if (!(det != 0.0) || !isfinite(det) || !(w >= 0.f) || !isfinite(w)) {
-        atomicExch(s.bad, 1);
+        atomicExch(&s.flags->bad, 1);
         return;
     }
+    const double rdet = 1.0 / det;  // FP64 divides are slow here: one, not nine
     double inv[9];
-    inv[0] = (D[1][1] * D[2][2] - D[1][2] * D[2][1]) / det;
-    inv[1] = (D[0][2] * D[2][1] - D[0][1] * D[2][2]) / det;
-    inv[2] = (D[0][1] * D[1][2] - D[0][2] * D[1][1]) / det;
-    inv[3] = (D[1][2] * D[2][0] - D[1][0] * D[2][2]) / det;
-    inv[4] = (D[0][0] * D[2][2] - D[0][2] * D[2][0]) / det;
-    inv[5] = (D[0][2] * D[1][0] - D[0][0] * D[1][2]) / det;
-    inv[6] = (D[1][0] * D[2][1] - D[1][1] * D[2][0]) / det;
-    inv[7] = (D[0][1] * D[2][0] - D[0][0] * D[2][1]) / det;
-    inv[8] = (D[0][0] * D[1][1] - D[0][1] * D[1][0]) / det;
+    inv[0] = (D[1][1] * D[2][2] - D[1][2] * D[2][1]) * rdet;
+    inv[1] = (D[0][2] * D[2][1] - D[0][1] * D[2][2]) * rdet;
+    inv[2] = (D[0][1] * D[1][2] - D[0][2] * D[1][1]) * rdet;
+    inv[3] = (D[1][2] * D[2][0] - D[1][0] * D[2][2]) * rdet;
+    inv[4] = (D[0][0] * D[2][2] - D[0][2] * D[2][0]) * rdet;
+    inv[5] = (D[0][2] * D[1][0] - D[0][0] * D[1][2]) * rdet;
+    inv[6] = (D[1][0] * D[2][1] - D[1][1] * D[2][0]) * rdet;
+    inv[7] = (D[0][1] * D[2][0] - D[0][0] * D[2][1]) * rdet;
+    inv[8] = (D[0][0] * D[1][1] - D[0][1] * D[1][0]) * rdet;
     const double coef = fabs(det) / 6.0 * (double)w;
     // a nearly flat tet has a finite double inverse that overflows float:
     // rejected like a flat one (the layout of pdgb_create does the same)
     bool finite = isfinite((float)coef);
     for (int k = 0; k < 9; ++k) finite = finite && isfinite((float)inv[k]);
     if (!finite) {
-        atomicExch(s.bad, 1);
+        atomicExch(&s.flags->bad, 1);
         return;
     }
     for (int k = 0; k < 9; ++k) s.geo[(size_t)k * kNaMaxTets + t] = (float)inv[k];
@@ -146,99 +158,217 @@ __global__ void na_tets(int nv, int nt, const uint32_t* __restrict__ tets, const
     }
 }
 
-__global__ void na_clear(int nv, NaScratch s) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nv) s.diag[i] = 0.f;
+// Grid barrier of a cooperative launch: the n-th barrier is passed once
+// n gridDim.x CTAs have arrived.  A wait is bounded (some seconds); past it
+// the timeout word ends every CTA at its next barrier.
+constexpr unsigned kNaSpins = 1u << 22;
+__device__ __forceinline__ bool na_barrier(NaFlags* f, unsigned& target) {
+    __shared__ int ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        // released with the CTA's writes and atomics before the barrier above,
+        // acquired before those after the one below
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&f->arrived) : "memory");
+        bool there = false;
+        for (unsigned n = 0; n < kNaSpins && !there; ++n) {
+            unsigned seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&f->arrived) : "memory");
+            there = (int)(seen - target) >= 0;  // the count may wrap
+            if (n % 1024 == 1023 && *reinterpret_cast<volatile int*>(&f->timeout)) break;
+        }
+        if (!there) atomicExch(&f->timeout, 1);
+        ok = there;
+    }
+    __syncthreads();
+    return ok;
 }
 
-__global__ void na_vertex_coef(int nv, const float* __restrict__ mass, const float* __restrict__ dbc, float dt,
-                               float pw, NaScratch s) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const float pin = dbc ? dbc[i] : 0.f;
-    const float mdt2 = (mass[i] + pin * pw) / (dt * dt);
-    s.coef[i] = make_float4(mdt2, s.diag[i], pin > 0.f ? 1.f : 0.f, mass[i]);
+struct NaTet {
+    uint32_t id[4];
+    float D[9], c;
+};
+__device__ __forceinline__ NaTet na_tet(const uint32_t* tets, const NaScratch& s, int t) {
+    const uint4 q = make_uint4(tets[4 * t], tets[4 * t + 1], tets[4 * t + 2], tets[4 * t + 3]);
+    NaTet r{{q.x, q.y, q.z, q.w}, {}, s.geo[(size_t)9 * kNaMaxTets + t]};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) r.D[k] = s.geo[(size_t)k * kNaMaxTets + t];
+    return r;
 }
 
-// s = x + h v + f / (M/h^2); base = b = (M/h^2) s.
-__global__ void na_begin(int nv, const float* __restrict__ X, const float* __restrict__ V, float dt, float g,
-                         NaScratch s) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const float4 cf = s.coef[i];
-    const float dt2_m_1 = 1.0f / cf.x;
-    const float fy = -g * cf.w;
-    const float4 sn = make_float4(X[3 * i] + dt * V[3 * i], X[3 * i + 1] + dt * V[3 * i + 1] + dt2_m_1 * fy,
-                                  X[3 * i + 2] + dt * V[3 * i + 2], 0.f);
-    s.sn[i] = sn;
-    const float4 bs = make_float4(cf.x * sn.x, cf.x * sn.y, cf.x * sn.z, 0.f);
-    s.base[i] = bs;
-    s.b[i] = bs;
-}
-
-// Local step, one thread per tet, residual form c (R - F) B, float4 atomics
-// into the scratch b (pinned vertices ignore b).
-__global__ void na_local(int nv, int nt, const uint32_t* __restrict__ tets, NaScratch s) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt || *s.bad) return;
-    const uint32_t i0 = tets[4 * t], i1 = tets[4 * t + 1], i2 = tets[4 * t + 2], i3 = tets[4 * t + 3];
-    if (i0 >= (uint32_t)nv || i1 >= (uint32_t)nv || i2 >= (uint32_t)nv || i3 >= (uint32_t)nv) return;
-    float D[9];
-    for (int k = 0; k < 9; ++k) D[k] = s.geo[(size_t)k * kNaMaxTets + t];
-    const float c = s.geo[(size_t)9 * kNaMaxTets + t];
-    const float4 p0 = s.sn[i0], p1 = s.sn[i1], p2 = s.sn[i2], p3 = s.sn[i3];
+// Local step of one tet, residual form c (R - F) B, float4 atomics into the
+// scratch b (pinned vertices ignore b).
+__device__ __forceinline__ void na_local(const NaTet& q, const NaScratch& s) {
+    const float* D = q.D;
+    const float4 p0 = __ldcg(&s.sn[q.id[0]]), p1 = __ldcg(&s.sn[q.id[1]]), p2 = __ldcg(&s.sn[q.id[2]]),
+                 p3 = __ldcg(&s.sn[q.id[3]]);
     const float e[3][3] = {{p1.x - p0.x, p2.x - p0.x, p3.x - p0.x},
                            {p1.y - p0.y, p2.y - p0.y, p3.y - p0.y},
                            {p1.z - p0.z, p2.z - p0.z, p3.z - p0.z}};
     float F[9];
+#pragma unroll
     for (int r = 0; r < 3; ++r)
+#pragma unroll
         for (int cc = 0; cc < 3; ++cc) F[3 * r + cc] = e[r][0] * D[cc] + e[r][1] * D[3 + cc] + e[r][2] * D[6 + cc];
     float R[9];
     closest_rotation_horn(F, R);
+#pragma unroll
     for (int k = 0; k < 9; ++k) R[k] -= F[k];
     float M[9];
+#pragma unroll
     for (int r = 0; r < 3; ++r)
+#pragma unroll
         for (int cc = 0; cc < 3; ++cc)
-            M[3 * r + cc] = c * (R[3 * r] * D[3 * cc] + R[3 * r + 1] * D[3 * cc + 1] + R[3 * r + 2] * D[3 * cc + 2]);
-    atomicAdd(&s.b[i0], make_float4(-(M[0] + M[1] + M[2]), -(M[3] + M[4] + M[5]), -(M[6] + M[7] + M[8]), 0.f));
-    atomicAdd(&s.b[i1], make_float4(M[0], M[3], M[6], 0.f));
-    atomicAdd(&s.b[i2], make_float4(M[1], M[4], M[7], 0.f));
-    atomicAdd(&s.b[i3], make_float4(M[2], M[5], M[8], 0.f));
+            M[3 * r + cc] = q.c * (R[3 * r] * D[3 * cc] + R[3 * r + 1] * D[3 * cc + 1] + R[3 * r + 2] * D[3 * cc + 2]);
+    atomicAdd(&s.b[q.id[0]], make_float4(-(M[0] + M[1] + M[2]), -(M[3] + M[4] + M[5]), -(M[6] + M[7] + M[8]), 0.f));
+    atomicAdd(&s.b[q.id[1]], make_float4(M[0], M[3], M[6], 0.f));
+    atomicAdd(&s.b[q.id[2]], make_float4(M[1], M[4], M[7], 0.f));
+    atomicAdd(&s.b[q.id[3]], make_float4(M[2], M[5], M[8], 0.f));
+}
+
+struct NaParams {
+    float dt, dt_inv, gravity, pw, wpin, rho;
+    int iters, steps;
+};
+
+// One vertex: its mass terms, pin right-hand side, state and iterates.
+struct NaVertex {
+    float cm, md, m;
+    bool pinned;
+    float3 pin, x, v, sn, prev, base;
+};
+
+__device__ __forceinline__ float3 na_load3(const float* a, int i) { return make_float3(a[3 * i], a[3 * i + 1], a[3 * i + 2]); }
+__device__ __forceinline__ void na_store3(float* a, int i, float3 v) {
+    a[3 * i] = v.x;
+    a[3 * i + 1] = v.y;
+    a[3 * i + 2] = v.z;
+}
+__device__ __forceinline__ float4 na_f4(float3 v) { return make_float4(v.x, v.y, v.z, 0.f); }
+
+__device__ __forceinline__ NaVertex na_vertex(const float* X0, const float* mass, const float* dbc, const float* X,
+                                              const float* V, const NaParams& p, const NaScratch& s, int i) {
+    NaVertex q{};
+    const float pin = dbc ? dbc[i] : 0.f;
+    q.m = mass[i];
+    q.cm = (q.m + pin * p.pw) / (p.dt * p.dt);
+    q.md = s.diag[i];
+    q.pinned = pin > 0.f;
+    const float3 x0 = na_load3(X0, i);
+    q.pin = make_float3(x0.x * p.wpin, x0.y * p.wpin, x0.z * p.wpin);
+    q.x = na_load3(X, i);
+    q.v = na_load3(V, i);
+    return q;
+}
+
+// s = x + h v + f / (M/h^2); base = b = (M/h^2) s.
+__device__ __forceinline__ void na_begin(NaVertex& q, const NaParams& p, const NaScratch& s, int i) {
+    const float dt2_m_1 = 1.0f / q.cm;
+    const float fy = -p.gravity * q.m;
+    q.sn = make_float3(q.x.x + p.dt * q.v.x, q.x.y + p.dt * q.v.y + dt2_m_1 * fy, q.x.z + p.dt * q.v.z);
+    q.base = make_float3(q.cm * q.sn.x, q.cm * q.sn.y, q.cm * q.sn.z);
+    s.sn[i] = na_f4(q.sn);
+    s.b[i] = na_f4(q.base);
 }
 
 // Jacobi update + 0.9 relaxation + Chebyshev blend (pdUtil.cu:195-226) with
-// the pin RHS x0 * w / h^2 (pdUtil.cu:147-166); the last iteration writes
-// V and X (pdUtil.cu:180-193).
-__global__ void na_vertex(int nv, const float* __restrict__ X0, float wpin, float omega, int read_prev,
-                          int write_prev, int final_iter, float dt_inv, float* X, float* V, NaScratch s) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const float4 sn = s.sn[i];
-    const float4 cf = s.coef[i];
-    float4 bb;
-    if (cf.z != 0.f) bb = make_float4(X0[3 * i] * wpin, X0[3 * i + 1] * wpin, X0[3 * i + 2] * wpin, 0.f);
-    else bb = s.b[i];
-    const float den = cf.x + cf.y;
-    float n[3];
-    const float sv[3] = {sn.x, sn.y, sn.z}, bv[3] = {bb.x, bb.y, bb.z};
-    for (int d = 0; d < 3; ++d) n[d] = relax09((bv[d] - cf.x * sv[d]) / den + sv[d], sv[d]);
-    if (read_prev) {
-        const float4 p = s.prev[i];
-        n[0] = (n[0] - p.x) * omega + p.x;
-        n[1] = (n[1] - p.y) * omega + p.y;
-        n[2] = (n[2] - p.z) * omega + p.z;
-    }
-    if (write_prev) s.prev[i] = sn;
-    if (final_iter) {
-        for (int d = 0; d < 3; ++d) {
-            V[3 * i + d] = (n[d] - X[3 * i + d]) * dt_inv;
-            X[3 * i + d] = n[d];
-        }
+// the pin RHS x0 * w / h^2 (pdUtil.cu:147-166); the last iteration makes V and
+// X (pdUtil.cu:180-193).
+__device__ __forceinline__ void na_update(NaVertex& q, float omega, int iter, const NaParams& p, const NaScratch& s,
+                                          int i) {
+    const float4 b4 = __ldcg(&s.b[i]);
+    const float3 bb = q.pinned ? q.pin : make_float3(b4.x, b4.y, b4.z);
+    const float den = q.cm + q.md;
+    float3 n = make_float3(relax09((bb.x - q.cm * q.sn.x) / den + q.sn.x, q.sn.x),
+                           relax09((bb.y - q.cm * q.sn.y) / den + q.sn.y, q.sn.y),
+                           relax09((bb.z - q.cm * q.sn.z) / den + q.sn.z, q.sn.z));
+    if (iter >= 11)
+        n = make_float3((n.x - q.prev.x) * omega + q.prev.x, (n.y - q.prev.y) * omega + q.prev.y,
+                        (n.z - q.prev.z) * omega + q.prev.z);
+    q.prev = q.sn;
+    if (iter + 1 == p.iters) {
+        q.v = make_float3((n.x - q.x.x) * p.dt_inv, (n.y - q.x.y) * p.dt_inv, (n.z - q.x.z) * p.dt_inv);
+        q.x = n;
     } else {
-        s.sn[i] = make_float4(n[0], n[1], n[2], 0.f);
-        s.b[i] = s.base[i];
+        q.sn = n;
+        s.sn[i] = na_f4(n);
+        s.b[i] = na_f4(q.base);
     }
 }
+
+__device__ __forceinline__ float na_omega(float omega, int iter, float rho) {
+    return iter <= 10 ? 1.f : iter == 11 ? 2 / (2 - rho * rho) : 4 / (4 - rho * rho * omega);
+}
+
+// Every step of the call.  A thread owns one tet, whose geometry stays in its
+// registers, and one vertex, whose state and iterates do: what goes through L2
+// is the iterate (published, gathered by the tets) and the sums b.  With fewer
+// threads than tets or vertices (kOwn false) they are walked in strides, the
+// vertex data in the scratch and X, V.
+template <bool kOwn, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
+    na_run(int nv, int nt, const uint32_t* __restrict__ tets, const float* __restrict__ X0,
+           const float* __restrict__ mass, const float* __restrict__ dbc, NaParams p, float* X, float* V, NaScratch s,
+           unsigned target) {
+    if (s.flags->bad || s.flags->timeout) return;  // set before this launch: the same for every CTA
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+    if (kOwn) {
+        NaTet tet{};
+        NaVertex q{};
+        if (g < nt) tet = na_tet(tets, s, g);
+        if (g < nv) q = na_vertex(X0, mass, dbc, X, V, p, s, g);
+        for (int step = 0; step < p.steps; ++step) {
+            if (g < nv) na_begin(q, p, s, g);
+            float omega = 1.f;
+            for (int i = 0; i < p.iters; ++i) {
+                if (!na_barrier(s.flags, target)) return;
+                if (g < nt) na_local(tet, s);
+                omega = na_omega(omega, i, p.rho);
+                if (!na_barrier(s.flags, target)) return;
+                if (g < nv) na_update(q, omega, i, p, s, g);
+            }
+        }
+        if (g < nv) {
+            na_store3(X, g, q.x);
+            na_store3(V, g, q.v);
+        }
+        return;
+    }
+    for (int step = 0; !kOwn && step < p.steps; ++step) {
+        for (int i = g; i < nv; i += all) {
+            NaVertex q = na_vertex(X0, mass, dbc, X, V, p, s, i);
+            na_begin(q, p, s, i);
+            s.base[i] = na_f4(q.base);
+            s.prev[i] = na_f4(q.sn);
+        }
+        float omega = 1.f;
+        for (int it = 0; it < p.iters; ++it) {
+            if (!na_barrier(s.flags, target)) return;
+            for (int t = g; t < nt; t += all) na_local(na_tet(tets, s, t), s);
+            omega = na_omega(omega, it, p.rho);
+            if (!na_barrier(s.flags, target)) return;
+            for (int i = g; i < nv; i += all) {
+                NaVertex q = na_vertex(X0, mass, dbc, X, V, p, s, i);
+                const float4 sn = s.sn[i], pr = s.prev[i], ba = s.base[i];
+                q.sn = make_float3(sn.x, sn.y, sn.z);
+                q.prev = make_float3(pr.x, pr.y, pr.z);
+                q.base = make_float3(ba.x, ba.y, ba.z);
+                na_update(q, omega, it, p, s, i);
+                s.prev[i] = na_f4(q.prev);
+                if (it + 1 == p.iters) {
+                    na_store3(X, i, q.x);
+                    na_store3(V, i, q.v);
+                }
+            }
+        }
+    }
+}
+
+// Threads per CTA: as few CTAs as hold a tet and a vertex a thread (a barrier
+// costs by the CTA: 22 x 256 threads pass it in 1.3 us), as many as the SMs
+// once 256 threads each are not enough.
+constexpr int kNaLaunchIters = 8192;  // iterations of one launch, a fraction of a second at the most
+int na_threads(int n, int sms) { return n <= 256 * sms ? 256 : n <= 512 * sms ? 512 : 1024; }
 
 std::mutex g_na_mutex;
 unsigned char* g_na_ptr[kNaMaxDevices] = {};
@@ -270,34 +400,44 @@ extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_param
     const NaScratch s = carve(base);
     cudaStream_t st = (cudaStream_t)stream;
     const int nv = mesh->num_verts, nt = mesh->num_tets;
-    const int vb = (nv + 255) / 256, tb = (nt + 255) / 256;
-    if (cudaMemsetAsync(s.bad, 0, sizeof(int), st) != cudaSuccess) return PDGB_ERR_CUDA;
-    na_clear<<<vb, 256, 0, st>>>(nv, s);
-    na_tets<<<tb, 256, 0, st>>>(nv, nt, mesh->tets, mesh->X0, mesh->mu, s);
-    na_vertex_coef<<<vb, 256, 0, st>>>(nv, mesh->mass, mesh->dbc, p->dt, p->positional_weight, s);
-    // The mesh check is read back before the first step, so that a bad mesh
-    // leaves the caller's X and V untouched.
-    int hbad = 0;
+    if (cudaMemsetAsync(s.diag, 0, kNaDiagBytes + sizeof(NaFlags), st) != cudaSuccess) return PDGB_ERR_CUDA;
+    na_tets<<<(nt + 255) / 256, 256, 0, st>>>(nv, nt, mesh->tets, mesh->X0, mesh->mu, s);
     if (cudaGetLastError() != cudaSuccess) return PDGB_ERR_CUDA;
-    if (cudaMemcpyAsync(&hbad, s.bad, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PDGB_ERR_CUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return PDGB_ERR_CUDA;
-    if (hbad) return PDGB_ERR_BAD_MESH;
-    const float dt_inv = 1.0f / p->dt;
-    const float wpin = p->positional_weight * (dt_inv * dt_inv);
-    const int n = p->num_iterations;
-    for (int k = 0; k < nsteps; ++k) {
-        na_begin<<<vb, 256, 0, st>>>(nv, X, V, p->dt, p->gravity, s);
-        float omega = 1.f;
-        for (int i = 0; i < n; ++i) {
-            if (i <= 10) omega = 1;
-            else if (i == 11) omega = 2 / (2 - p->rho * p->rho);
-            else omega = 4 / (4 - p->rho * p->rho * omega);
-            na_local<<<tb, 256, 0, st>>>(nv, nt, mesh->tets, s);
-            na_vertex<<<vb, 256, 0, st>>>(nv, mesh->X0, wpin, omega, i >= 11, i >= 10 && i + 1 < n, i + 1 == n,
-                                          dt_inv, X, V, s);
+    if (nsteps > 0) {
+        int sms = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PDGB_ERR_CUDA;
+        const int n = nv > nt ? nv : nt, threads = na_threads(n, sms);
+        const int want = (n + threads - 1) / threads, grid = want < sms ? want : sms;
+        const bool own = (long long)grid * threads >= n;
+        const auto kernel = threads == 256 ? (own ? na_run<true, 256> : na_run<false, 256>)
+                            : threads == 512 ? (own ? na_run<true, 512> : na_run<false, 512>)
+                                             : (own ? na_run<true, 1024> : na_run<false, 1024>);
+        const float dt_inv = 1.0f / p->dt;
+        NaParams np{p->dt, dt_inv, p->gravity, p->positional_weight, p->positional_weight * (dt_inv * dt_inv),
+                    p->rho, p->num_iterations, 0};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const int most = p->num_iterations >= kNaLaunchIters ? 1 : kNaLaunchIters / p->num_iterations;
+        unsigned arrived = 0;
+        for (int done = 0; done < nsteps; done += np.steps) {
+            np.steps = nsteps - done < most ? nsteps - done : most;
+            if (cudaLaunchKernelEx(&cfg, kernel, nv, nt, mesh->tets, mesh->X0, mesh->mass, mesh->dbc, np, X, V, s,
+                                   arrived) != cudaSuccess)
+                return PDGB_ERR_CUDA;
+            arrived += 2u * (unsigned)np.iters * (unsigned)np.steps * (unsigned)grid;
         }
     }
-    if (cudaGetLastError() != cudaSuccess) return PDGB_ERR_CUDA;
+    NaFlags flags{};
+    if (cudaMemcpyAsync(&flags, s.flags, sizeof(flags), cudaMemcpyDeviceToHost, st) != cudaSuccess) return PDGB_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return PDGB_ERR_CUDA;
+    if (flags.bad) return PDGB_ERR_BAD_MESH;
+    if (flags.timeout) return PDGB_ERR_TIMEOUT;
     return PDGB_OK;
 }
