@@ -148,55 +148,119 @@ __device__ __forceinline__ int find_front(const FrontRef* f, const int* hint, in
     return lo;
 }
 
-// 1 / sqrt(d) from the single precision value y: with e = 1 - d y^2 (about
-// 2^-22) it is y (1 - e)^(-1/2) = y (1 + e / 2 + 3 e^2 / 8 + O(e^3)), the
-// rest below the rounding of double.  Outside the range of float the
-// library's function.
-__device__ __forceinline__ double inv_sqrt(double d) {
-    if (!(d > 1e-30 && d < 1e30)) return rsqrt(d);
-    const double y = (double)rsqrtf((float)d);
-    const double e = fma(-d * y, y, 1.0);
-    return fma(y, e * fma(0.375, e, 0.5), y);
+// Lower triangle of the nb x nb block D -> its Cholesky factor, W -> the
+// factor's inverse (both lower, row-major in shared memory).  The pivots are a
+// chain of 32 reciprocal square roots, each some eight dependent FP64
+// operations of 64 clocks or more; everything else is kept out of it.  Eight
+// columns at a time, warp 0 (lane = row) factors the columns in registers while
+// the other warps bring W up to date with the eight before:
+//   rows J of W   W[J, c] = L_JJ^-1 W[J, c]
+//   rows below    W[r, c] -= L[r, J] W[J, c]
+// then all warps take the columns out of the rest of D.  One column a step with
+// two barriers, all warps on each, took 50 us a block; this takes 22.
+constexpr int kSub = 8;
+
+struct PanelShared {
+    double D[kNB][kNB + 1], W[kNB][kNB + 1], T[kNB][kNB + 1];
+    double inv[kNB];  // 1 / L_jj
+};
+
+// Warp 0: columns c0 .. c0 + 8 of D.  With y the single precision value of
+// 1 / sqrt(d) and e = 1 - d y^2 (about 2^-22), 1 / sqrt(d) is y (1 - e)^(-1/2) =
+// y (1 + e / 2 + 3 e^2 / 8 + O(e^3)), the rest below the rounding of double.
+// Outside the range of float the library's function.
+__device__ __forceinline__ void factor_columns(PanelShared& S, int c0, int nb, bool& bad) {
+    const int lane = threadIdx.x;
+    double a[kSub];
+#pragma unroll
+    for (int c = 0; c < kSub; ++c) a[c] = S.D[lane][c0 + c];
+#pragma unroll
+    for (int c = 0; c < kSub; ++c) {
+        if (c0 + c >= nb) break;
+        double d = __shfl_sync(0xffffffffu, a[c], c0 + c);
+        if (!(d > 0.0) || !isfinite(d)) {
+            bad = true;
+            d = 1.0;
+            if (lane == c0 + c) a[c] = 1.0;
+        }
+        double inv;
+        if (d > 1e-30 && d < 1e30) {
+            const double y = (double)rsqrtf((float)d);
+            const double e = fma(-d * y, y, 1.0);
+            const double ay = a[c] * y;
+            const double q = e * fma(0.375, e, 0.5);
+            a[c] = fma(ay, q, ay);
+            inv = fma(y, q, y);
+        } else {
+            inv = rsqrt(d);
+            a[c] *= inv;
+        }
+        if (lane == 0) S.inv[c0 + c] = inv;
+#pragma unroll
+        for (int k = c + 1; k < kSub; ++k) a[k] = fma(-a[c], __shfl_sync(0xffffffffu, a[c], c0 + k), a[k]);
+    }
+#pragma unroll
+    for (int c = 0; c < kSub; ++c)
+        if (lane >= c0 + c) S.D[lane][c0 + c] = a[c];
 }
 
-// Lower triangle of the nb x nb block D -> its Cholesky factor, W -> the
-// factor's inverse (both lower, row-major in shared memory).  Step j scales
-// column j of D and row j of W, then takes them out of the rows below: row i
-// has i + 1 entries to update, i - j of D and j + 1 of W.
-__device__ __forceinline__ void factor_block(double (*D)[kNB + 1], double (*W)[kNB + 1], int nb, bool& bad) {
-    const int tid = threadIdx.x;
-    const int row = tid >> 3, part = tid & 7;  // 8 threads a row
-    static_assert(kPanelThreads == 8 * kNB, "8 threads a row");
-    for (int e = tid; e < kNB * kNB; e += kPanelThreads) W[e / kNB][e % kNB] = e / kNB == e % kNB ? 1.0 : 0.0;
-    __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-        if (tid < kNB) {
-            double d = D[j][j];
-            if (!(d > 0.0) || !isfinite(d)) {
-                bad = true;
-                d = 1.0;
-            }
-            const double inv = inv_sqrt(d);
-            __syncwarp();
-            if (tid == j) D[j][j] = d * inv;
-            else if (tid > j && tid < nb) D[tid][j] *= inv;
-            if (tid <= j) W[j][tid] *= inv;
+// Warps 1 .. 7: W after the columns c0 .. c0 + 8 of L.
+__device__ __forceinline__ void update_inverse(PanelShared& S, int c0, int nb) {
+    const int t = threadIdx.x - 32;
+    const int n = min(nb, c0 + kSub);  // rows of W that end here, and its columns so far
+    if (t < n) {
+        double w[kSub];
+#pragma unroll
+        for (int i = 0; i < kSub; ++i) {
+            w[i] = 0.0;
+            if (c0 + i >= nb) continue;
+            double v = S.W[c0 + i][t];
+#pragma unroll
+            for (int q = 0; q < i; ++q) v = fma(-S.D[c0 + i][c0 + q], w[q], v);
+            w[i] = t <= c0 + i ? v * S.inv[c0 + i] : 0.0;
+            S.W[c0 + i][t] = w[i];
         }
+    }
+    asm volatile("bar.sync 1, 224;" ::: "memory");
+    const int rows = nb - n;
+    for (int e = t; e < rows * n; e += kPanelThreads - 32) {
+        const int r = n + e / n, c = e % n;
+        double v = S.W[r][c];
+#pragma unroll
+        for (int q = 0; q < kSub; ++q) v = fma(-S.D[r][c0 + q], S.W[c0 + q][c], v);
+        S.W[r][c] = v;
+    }
+}
+
+__device__ __forceinline__ void factor_block(PanelShared& S, int nb, bool& bad) {
+    static_assert(kPanelThreads == 256, "warps 1 to 7 share barrier 1");
+    for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) S.W[e / kNB][e % kNB] = e / kNB == e % kNB ? 1.0 : 0.0;
+    __syncthreads();
+    int c0 = 0;
+    for (; c0 < nb; c0 += kSub) {
+        if (threadIdx.x < 32) factor_columns(S, c0, nb, bad);
+        else if (c0 > 0) update_inverse(S, c0 - kSub, nb);
         __syncthreads();
-        if (row > j && row < nb) {
-            const double l = D[row][j];
-            for (int c = part; c <= row; c += 8) {
-                if (c > j) D[row][c] = fma(-l, D[c][j], D[row][c]);
-                else W[row][c] = fma(-l, W[j][c], W[row][c]);
-            }
+        const int r0 = c0 + kSub, n = nb - r0;
+        for (int e = threadIdx.x; e < n * n; e += kPanelThreads) {
+            const int r = r0 + e / n, c = r0 + e % n;
+            if (c > r) continue;
+            double v = S.D[r][c];
+#pragma unroll
+            for (int q = 0; q < kSub; ++q) v = fma(-S.D[r][c0 + q], S.D[c][c0 + q], v);
+            S.D[r][c] = v;
         }
         __syncthreads();
     }
+    if (threadIdx.x >= 32) update_inverse(S, c0 - kSub, nb);
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(kPanelThreads) k_panel(FDev d, const FrontRef* __restrict__ fronts,
                                                          const int* __restrict__ hint, int j0, int chunk) {
-    __shared__ double D[kNB][kNB + 1], W[kNB][kNB + 1], T[kNB][kNB + 1];
+    __shared__ PanelShared S;
+    auto& W = S.W;
+    auto& T = S.T;
     pdl_trigger();
     const int fi = find_front(fronts, hint, blockIdx.x);
     const int s = fronts[fi].s, part = blockIdx.x - fronts[fi].first;
@@ -210,11 +274,11 @@ __global__ void __launch_bounds__(kPanelThreads) k_panel(FDev d, const FrontRef*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e = threadIdx.x; e < kNB * kNB; e += kPanelThreads) {
         const int r = e % kNB, c = e / kNB;
-        D[r][c] = (r < nb && c <= r) ? F[(int64_t)(j0 + c) * m + j0 + r] : 0.0;
+        S.D[r][c] = (r < nb && c <= r) ? F[(int64_t)(j0 + c) * m + j0 + r] : 0.0;
     }
     __syncthreads();
     bool bad = false;
-    factor_block(D, W, nb, bad);
+    factor_block(S, nb, bad);
     const int nrow = max(1, (m - j1 + chunk - 1) / chunk);
     if (part == 0) {
         if (bad) atomicCAS(d.status, 0, s + 1);
