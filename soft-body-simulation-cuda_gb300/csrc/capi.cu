@@ -292,7 +292,7 @@ void record_jacobi_step(pdgb_engine* e) {
         // from iteration 10 on the iterate is the next one's prev: the two
         // buffers take turns
         va.out = i >= 10 ? va.prev : va.sn;
-        launch_jacobi_vertex(va, mode, s);
+        launch_jacobi_vertex(va, mode, e->L.ntiles <= kOneWaveTiles, s);
         if (i >= 10) std::swap(va.sn, va.prev);
     }
 }

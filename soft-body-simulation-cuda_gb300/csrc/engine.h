@@ -232,6 +232,11 @@ void launch_local_multi(const LocalArgs* req, const int2* list, const int* count
                         bool jacobi_form = true);
 void launch_jacobi_vertex_multi(const VertexArgs* req, const int2* list, const int* count, int grid, int mode,
                                 float omega, cudaStream_t s);
+// Up to one wave of tiles (4 CTAs on each of 152 SMs) the Jacobi step's two
+// kernels both ask for the largest shared memory, so that one starts beside the
+// other (47 x 5 x 61 cells, two steps: 139 -> 126 us); past that the local step
+// gains more from its L1 (64^3: 592 us against 602 us).
+constexpr int kOneWaveTiles = 608;
 void launch_local(const LocalArgs& a, int ntiles, int max_patch, bool jacobi_form, int rotation, cudaStream_t s);
 // Resident CTAs of the pipelined local step for this mesh's largest patch
 // (2 per SM when its shared memory allows), capped at ntiles; 0 when it
@@ -240,7 +245,7 @@ int local_pipe_grid(int ntiles, int max_patch);
 // Check of the bounded bulk-copy wait (pdgb_bulk_wait_check): src holds 64
 // words 0..63; out[0] = timed out, out[1] = data intact.
 void launch_bulk_wait_check(const void* src, int extra, unsigned long long limit_ns, int* out, cudaStream_t s);
-void launch_jacobi_vertex(const VertexArgs& a, int mode, cudaStream_t s);
+void launch_jacobi_vertex(const VertexArgs& a, int mode, bool small, cudaStream_t s);
 void launch_gather_state(int nv, const int* vperm, const float* X, const float* V, float4* x, float4* v,
                          cudaStream_t s);
 void launch_scatter_state(int nv, const int* vperm, const float4* x, const float4* v, float* X, float* V,

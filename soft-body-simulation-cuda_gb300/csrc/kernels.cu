@@ -528,11 +528,12 @@ void launch_local(const LocalArgs& a, int ntiles, int max_patch, bool jacobi_for
         return;
     }
     const size_t sm = (size_t)max_patch * sizeof(float4);
+    const bool small = ntiles <= kOneWaveTiles;
     if (rotation == PDGB_ROTATION_SVD) {
         if (jacobi_form) launch_pdl(k_local<true, PDGB_ROTATION_SVD>, ntiles, kLocalThreads, sm, s, a);
         else launch_pdl(k_local<false, PDGB_ROTATION_SVD>, ntiles, kLocalThreads, sm, s, a);
     } else {
-        if (jacobi_form) launch_pdl(k_local<true, PDGB_ROTATION_QUAT>, ntiles, kLocalThreads, sm, s, a);
+        if (jacobi_form) launch_pdl_carve(k_local<true, PDGB_ROTATION_QUAT>, small, ntiles, kLocalThreads, sm, s, a);
         else launch_pdl(k_local<false, PDGB_ROTATION_QUAT>, ntiles, kLocalThreads, sm, s, a);
     }
 }
@@ -626,14 +627,14 @@ void launch_jacobi_vertex_multi(const VertexArgs* req, const int2* list, const i
     }
 }
 
-void launch_jacobi_vertex(const VertexArgs& a, int mode, cudaStream_t s) {
+void launch_jacobi_vertex(const VertexArgs& a, int mode, bool small, cudaStream_t s) {
     const int blocks = (a.nv + 255) / 256;
     if (blocks == 0) return;
     switch (mode & (kReadPrev | kFinal)) {
-        case 0: launch_pdl(k_jacobi_vertex<0>, blocks, 256, 0, s, a); break;
-        case kReadPrev: launch_pdl(k_jacobi_vertex<kReadPrev>, blocks, 256, 0, s, a); break;
-        case kFinal: launch_pdl(k_jacobi_vertex<kFinal>, blocks, 256, 0, s, a); break;
-        default: launch_pdl(k_jacobi_vertex<kReadPrev | kFinal>, blocks, 256, 0, s, a); break;
+        case 0: launch_pdl_carve(k_jacobi_vertex<0>, small, blocks, 256, 0, s, a); break;
+        case kReadPrev: launch_pdl_carve(k_jacobi_vertex<kReadPrev>, small, blocks, 256, 0, s, a); break;
+        case kFinal: launch_pdl_carve(k_jacobi_vertex<kFinal>, small, blocks, 256, 0, s, a); break;
+        default: launch_pdl_carve(k_jacobi_vertex<kReadPrev | kFinal>, small, blocks, 256, 0, s, a); break;
     }
 }
 

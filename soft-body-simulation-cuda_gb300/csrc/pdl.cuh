@@ -26,19 +26,35 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// An SM changes its split between L1 and shared memory only when it is idle, so
+// a kernel that wants another split than its predecessor cannot start beside
+// it: the kernels of a chain all ask for the largest shared memory.
+template <typename... P> inline void prefer_shared(void (*kernel)(P...)) {
+    PDGB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       cudaSharedmemCarveoutMaxShared));
+}
+
 template <typename... P, typename... A>
-inline void launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+inline void launch_pdl_carve(void (*kernel)(P...), bool most_shared, int grid, int block, size_t smem, cudaStream_t s,
+                             A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = most_shared ? 2 : 1;
     PDGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    launch_pdl_carve(kernel, false, grid, block, smem, s, args...);
 }
 
 }  // namespace pdgb
