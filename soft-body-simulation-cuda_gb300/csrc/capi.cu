@@ -63,6 +63,7 @@ struct pdgb_engine {
     float chol_dt = 0.f, chol_pw = -1.f;
     DBuf<int> ch_fwd, ch_bwd, ch_rows, ch_body_level, ch_body_order, ch_blocks, ch_small, ch_tiny;
     DBuf<float4> y2;  // second y buffer: solves alternate, each clears the other one's
+    DBuf<float4> b2;  // second right-hand side, where the root's product is the whole solve
     DBuf<int4> ch_levels;
     DBuf<SolveLevel> ch_step_lv;  // per-level item ranges on the device (persistent solve)
     // distributed-shared-memory solve of a single body (when it fits)
@@ -311,7 +312,7 @@ void record_chol_step(pdgb_engine* e) {
     // without the convergence test nothing sets the flag: the step's kernels do
     // not wait for a read of it
     const int* done = use_tol ? &st->done : nullptr;
-    const LocalArgs la = local_args(e, done);
+    LocalArgs la = local_args(e, done);
     CholArgs ca{e->ch_fwd.p, e->ch_bwd.p, e->ch_rows.p, e->ch_mval.p, e->ch_levels.p, e->ch_body_level.p,
                 e->ch_body_order.p, e->b.p, e->y.p, e->sn.p, done, e->ch_blocks.p, e->ch_small.p, e->ch_tiny.p};
     CholVertexArgs cv{};
@@ -341,10 +342,21 @@ void record_chol_step(pdgb_engine* e) {
     const bool fused = e->solve_mode == PDGB_SOLVE_LEVELS && !use_tol;
     float4* ybuf[2] = {e->y.p, fused ? e->y2.p : e->y.p};
     int parity = 0;  // y buffer of the next solve; zero when the step begins
+    RootArgs root{};
+    if (e->solve_mode == PDGB_SOLVE_LEVELS && e->chol.root >= 0) {
+        const CholFactor& f = e->chol;
+        const int k = f.sk[f.root];
+        root = RootArgs{e->ch_mval.p + f.root_off, e->ch_rows.p + f.roff[f.root], k, m_stride(k, k)};
+    }
+    // A solve that is one product has no launch after its last read of b: the
+    // next iteration's b is another buffer, and there is no y to clear
+    const bool one = fused && root.k > 0 && e->chol.nlevels == 1;
+    float4* bbuf[2] = {e->b.p, one ? e->b2.p : e->b.p};
     auto solve = [&](float4* x, bool last) {
         CholArgs args = ca;
         args.x = x;
         args.y = ybuf[parity];
+        args.r = la.b;
         if (e->solve_mode == PDGB_SOLVE_CTA) launch_chol_solve_cta(args, e->nbodies, s);
         else if (e->solve_mode == PDGB_SOLVE_CLUSTER) launch_chol_solve_cluster(args, e->nbodies, s);
         else if (e->solve_mode == PDGB_SOLVE_DSM) launch_chol_solve_dsm(args, dsm_args(e), e->dsm.smem_bytes, s);
@@ -353,16 +365,21 @@ void record_chol_step(pdgb_engine* e) {
                                          kPersistSpinLimit, s);
         else {
             ResetArgs reset{};
-            if (fused)
+            if (one) {
+                if (last) reset = ResetArgs{e->nv, nullptr, la.b == bbuf[0] ? bbuf[1] : bbuf[0], e->base.p, e->coef.p, e->pin_rhs.p};
+            } else if (fused) {
                 reset = ResetArgs{e->nv, ybuf[parity ^ 1], last ? e->b.p : nullptr, e->base.p, e->coef.p, e->pin_rhs.p};
-            launch_chol_solve_levels(args, e->chol.step_levels, s, reset);
+            }
+            launch_chol_solve_levels(args, e->chol.step_levels, s, reset, root);
             if (fused) parity ^= 1;
         }
     };
     for (int i = 0; i < n; ++i) {
+        la.b = bbuf[i & 1];
+        ra.b = la.b;
         record_local(e, la, false, i);
-        if (drag_rhs) launch_drag_rhs(e->nv, cv.sc, e->base.p, e->b.p, done, s);
-        if (refine > 0) launch_copy_rhs(e->nv, e->b.p, e->bsave.p, done, s);
+        if (drag_rhs) launch_drag_rhs(e->nv, cv.sc, e->base.p, la.b, done, s);
+        if (refine > 0) launch_copy_rhs(e->nv, la.b, e->bsave.p, done, s);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i], s, cudaEventRecordExternal));
         solve(e->sn.p, refine == 0);
         if (e->timing) PDGB_CUDA_TRY(cudaEventRecordWithFlags(e->solve_events[2 * i + 1], s, cudaEventRecordExternal));
@@ -483,7 +500,9 @@ void prepare_cholesky(pdgb_engine* e) {
     e->pool_bytes = 0;
     if (gpu) {
         // FP64 numeric factorisation on the GPU, straight into the M_s blocks
-        e->ch_mval.alloc((size_t)std::max<int64_t>(f.mval_size, 1));
+        if (e->nbodies == 1) plan_root_inverse(e->chol);
+        if (f.root >= 0) e->b2.alloc(e->nv);
+        e->ch_mval.alloc((size_t)std::max<int64_t>(f.mval_total, 1));
         e->numeric_ms = gpu_factor(f, e->ch_mval.p, s);
         e->pool_bytes = (long long)f.fp.pool * (long long)sizeof(double);
         e->chol.fp = FrontPlan();  // the plan is not needed after the factorisation
@@ -542,7 +561,10 @@ void prepare(pdgb_engine* e) {
     build_vertex_coefficients(e->mass.data(), e->has_dbc ? e->dbc.data() : nullptr, e->prm, e->L);
     e->coef.upload(e->L.coef, e->stream);
     e->pin_rhs.upload(e->L.pin_rhs, e->stream);
-    if (e->prm.solver == PDGB_SOLVER_CHOLESKY) prepare_cholesky(e);
+    if (e->prm.solver == PDGB_SOLVER_CHOLESKY) {
+        configure_chol_kernels();
+        prepare_cholesky(e);
+    }
     PDGB_CUDA_TRY(cudaMemsetAsync(e->y.p, 0, (size_t)e->nv * sizeof(float4), e->stream));
     if (e->y2.p) PDGB_CUDA_TRY(cudaMemsetAsync(e->y2.p, 0, (size_t)e->nv * sizeof(float4), e->stream));
     // resident CTAs of the pipelined local step for the current tile cut
@@ -1574,6 +1596,7 @@ int solve_launches(const pdgb_engine* e) {
     int n = 0;
     for (const SolveLevel& v : e->chol.step_levels)
         n += 2 * (v.blk_end > v.blk_begin || v.sml_end > v.sml_begin || v.tiny_end > v.tiny_begin);
+    if (e->chol.root >= 0) n -= 1;  // the root: one product
     return n;
 }
 }  // namespace

@@ -408,6 +408,7 @@ std::vector<int> postorder(const std::vector<int>& parent) {
 // subtree sizes: the 40^3 grid has 13 levels and 31.2 M entries when each
 // supernode is only merged with the last child before it (at most 2,048 or a
 // quarter added zeros), and 8 levels and 31.4 M, or 5 and 38.9 M, this way.
+// Up to 1,024 vertices the whole tree can be one supernode.
 // Of the grid of (t, r) the cheapest is taken, a level costing level_entries
 // entries and the one-time factorisation kEntriesPerFlop entries per
 // multiply-add (spread over the solves of about a hundred steps).
@@ -424,7 +425,7 @@ std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& 
     std::vector<int> root(nf), best_root(nf), band(n + 1), height(nf);
     std::vector<int64_t> cols(nf);
     double best = -1.0;
-    for (int t : {8, 16, 24, 32, 48, 96, 192})
+    for (int t : {8, 16, 24, 32, 48, 96, 192, 1024})
         for (double r : {2.0, 3.0, 4.0, 6.0, 10.0, 16.0, 32.0}) {
             double top = t;
             for (int c = 0, q = 0; c <= n; ++c) {
@@ -650,7 +651,7 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
     }
     out.moff[ns] = mtot;
     out.roff[ns] = (int)rtot;
-    out.mval_size = mtot;
+    out.mval_size = out.mval_total = mtot;
     out.rows.resize(rtot);
     for (int s = 0; s < ns; ++s)
         for (int q = 0; q < out.sm[s]; ++q) out.rows[out.roff[s] + q] = perm[sstruct[s][q]];
@@ -821,6 +822,23 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
     out.body_order = {0};
     out.step_levels = out.levels;
     if (gpu_numeric && finish_plan) finish_front_plan(out);
+}
+
+void plan_root_inverse(CholFactor& f) {
+    f.root = -1;
+    f.mval_total = f.mval_size;
+    if (!f.fp.on || f.nlevels > kRootLevels) return;
+    int root = -1;
+    for (int s = 0; s < f.nsuper; ++s) {
+        if (f.fp.parent[s] >= 0) continue;
+        if (root >= 0) return;  // several trees
+        root = s;
+    }
+    const int k = f.sk[root];
+    if (k != f.sm[root] || k > kRootCols) return;
+    f.root = root;
+    f.root_off = f.mval_size;  // a multiple of 4, like every block's
+    f.mval_total = f.mval_size + (int64_t)k * m_stride(k, k);
 }
 
 int64_t front_doubles(const CholFactor& f, int s) {
@@ -1039,7 +1057,7 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
         out.K.n = 0;  // per-body systems are not kept
         f = CholFactor();  // release the per-body copy
     }
-    out.mval_size = mbase;
+    out.mval_size = out.mval_total = mbase;
     if (gpu_numeric) {
         out.fp.on = true;
         finish_front_plan(out);

@@ -146,7 +146,26 @@ struct CholFactor {
     SparseSym K;
     int64_t mval_size = 0;           // FP32 entries of the M_s blocks (= mval.size() when factored on the host)
     FrontPlan fp;                    // numeric factorisation left to the GPU (fp.on)
+    // The inverse of the root's block of the factored system, L^-T L^-1 over its
+    // k pivots, stored past the M_s blocks (symmetric, columns
+    // m_stride(k, k) floats apart): -1 where there is none (plan_root_inverse).
+    int root = -1;                   // the root supernode
+    int64_t root_off = 0;            // its inverse's offset in mval
+    int64_t mval_total = 0;          // floats of the M_s blocks and the root's inverse
 };
+
+// Lets the factorisation on the GPU add the root's inverse to a single body's
+// factor (before gpu_factor).  At the root nothing is left between the forward
+// and the backward pass, so one product with the inverse takes the place of
+// two dependent launches, for the same bytes: a square matrix once instead of
+// a triangle twice.  Worth it where a solve is few launches, up to kRootLevels
+// levels, and up to kRootCols pivots: an iteration of the 6^3 grid 9.1 -> 7.7 us,
+// 12^3 10.1 -> 9.4 us, 14^3 (861 pivots) even, and of 19 x 11 x 23 (1,523) 13.2 ->
+// 15.1 us, where every CTA's gather of all right-hand sides costs more than the
+// launch.
+constexpr int kRootLevels = 3;
+constexpr int kRootCols = 1024;
+void plan_root_inverse(CholFactor& f);
 
 // Plan of the distributed-shared-memory solve of a single body: an 8-CTA
 // cluster, each CTA owning a set of supernodes whose M_s blocks and row
@@ -209,7 +228,8 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
 int64_t front_doubles(const CholFactor& f, int s);
 
 // Numeric factorisation of the plan f.fp on the GPU (factor.cu): writes the
-// FP32 M_s blocks (f.mval_size floats, device memory) and returns the device
+// FP32 M_s blocks and the root's inverse if planned (f.mval_total floats,
+// device memory) and returns the device
 // time in ms.  Waits for the stream.  Throws Error(PDGB_ERR_NOT_SPD) when a
 // pivot is not positive.
 double gpu_factor(const CholFactor& f, float* mval, void* stream);

@@ -415,6 +415,44 @@ __global__ void __launch_bounds__(kPanelThreads) k_trail(FDev d, const FrontRef*
     }
 }
 
+// The root's inverse S = L^-T L^-1 from X = L^-1 (k x k, lower, column major):
+// S[i][j] is the product of columns i and j of X from row max(i, j) on, 32 x 32
+// entries a CTA (column blocks bi >= bj), written to both triangles.
+__global__ void __launch_bounds__(256) k_root_inverse(const double* __restrict__ X, int k, float* S, int ld) {
+    __shared__ double A[kNB][kNB + 1], B[kNB][kNB + 1];
+    int bi = (int)((sqrtf(8.0f * (float)blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+    while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
+    while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
+    const int bj = (int)blockIdx.x - bi * (bi + 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int q0 = kNB * bi; q0 < k; q0 += kNB) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < kNB * kNB; e += 256) {
+            const int q = e % kNB, c = e / kNB;
+            const int ci = kNB * bi + c, cj = kNB * bj + c;
+            // zero above the diagonal, where X is not written
+            A[c][q] = q0 + q < k && ci < k && q0 + q >= ci ? X[(int64_t)ci * k + q0 + q] : 0.0;
+            B[c][q] = q0 + q < k && cj < k && q0 + q >= cj ? X[(int64_t)cj * k + q0 + q] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int q = 0; q < kNB; ++q) {
+            const double a = A[lane][q];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[u] = fma(a, B[warp + 8 * u][q], acc[u]);
+        }
+    }
+    const int i = kNB * bi + lane;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int j = kNB * bj + warp + 8 * u;
+        if (i >= k || j >= k) continue;
+        S[(int64_t)j * ld + i] = (float)acc[u];
+        S[(int64_t)i * ld + j] = (float)acc[u];
+    }
+}
+
 template <class T> void put(DBuf<T>& b, const std::vector<T>& h, cudaStream_t s) {
     b.alloc(std::max<size_t>(h.size(), 1));
     if (!h.empty()) PDGB_CUDA_TRY(cudaMemcpyAsync(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
@@ -523,7 +561,7 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
     put(dhints, hints, s);
     status.alloc(1);
     PDGB_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int), s));
-    PDGB_CUDA_TRY(cudaMemsetAsync(mval, 0, (size_t)f.mval_size * sizeof(float), s));
+    PDGB_CUDA_TRY(cudaMemsetAsync(mval, 0, (size_t)f.mval_total * sizeof(float), s));
     FDev d{pool.p, foff.p, sk.p, sm.p, moff.p, mval, cptr.p, child.p, rptr.p, rel.p, kptr.p, kpos.p, kval.p, status.p};
     cudaEvent_t ev[2];
     PDGB_CUDA_TRY(cudaEventCreate(&ev[0]));
@@ -546,6 +584,12 @@ double gpu_factor(const CholFactor& f, float* mval, void* stream) {
             else if (l.size == kNB / 2) launch_pdl(k_trail<kNB / 2>, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0);
             else launch_pdl(k_trail<kNB / 4>, l.ctas, kPanelThreads, 0, s, d, fr, hint, l.j0);
         }
+        err = cudaGetLastError();
+    }
+    if (err == cudaSuccess && f.root >= 0) {
+        const int k = f.sk[f.root], nb = (k + kNB - 1) / kNB;
+        k_root_inverse<<<nb * (nb + 1) / 2, 256, 0, s>>>(pool.p + P.foff[f.root] + (int64_t)k * k, k, mval + f.root_off,
+                                                         m_stride(k, k));
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) err = cudaEventRecord(ev[1], s);

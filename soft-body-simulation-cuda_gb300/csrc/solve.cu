@@ -427,6 +427,18 @@ constexpr int kTinyPerCta = kLevelThreads / kTinyLanes;
 __host__ __device__ inline int small_ctas(int n) { return (n + kLevelWarps - 1) / kLevelWarps; }
 __host__ __device__ inline int tiny_ctas(int n) { return (n + kTinyPerCta - 1) / kTinyPerCta; }
 
+// Resets of vertex i for the next solve (ResetArgs).  The right-hand side it
+// clears is dead: the forward pass is done, or it is another buffer.
+__device__ __forceinline__ void reset_vertex(const CholArgs& a, const ResetArgs& q, int i) {
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < q.nv && q.b) b = __ldg(&q.coef[i]).z != 0.f ? __ldg(&q.pin_rhs[i]) : __ldg(&q.base[i]);
+    pdl_wait();
+    pdl_trigger();
+    if ((a.done && *a.done) || i >= q.nv) return;
+    if (q.y_next) q.y_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q.b) q.b[i] = b;
+}
+
 __global__ void __launch_bounds__(kLevelThreads, kFwdBlocks) k_chol_fwd_level(CholArgs a, LevelRange v) {
     extern __shared__ float4 tile[];  // a tile, or kWarpFloats a warp
     float* blocks = reinterpret_cast<float*>(tile);
@@ -512,21 +524,88 @@ __global__ void __launch_bounds__(kLevelThreads, kBwdBlocks) k_chol_bwd_level(Ch
         bwd_tiny_run(a, p, j);
         return;
     }
-    // resets for the next solve: the right-hand side is dead once the forward
-    // pass is done, and y_next is the buffer this solve does not use
-    u -= tiny_ctas(v.nt);
-    const int i = u * kLevelThreads + threadIdx.x;
-    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < q.nv && q.b) b = __ldg(&q.coef[i]).z != 0.f ? __ldg(&q.pin_rhs[i]) : __ldg(&q.base[i]);
+    reset_vertex(a, q, (u - tiny_ctas(v.nt)) * kLevelThreads + threadIdx.x);
+}
+
+// x = S r over the root's pivots, S its inverse: a CTA takes 8 rows (which are
+// 8 rows of every column, 32 bytes of each) and copies them, 32 k bytes, to
+// shared memory before the grid dependency wait: the whole inverse is on the
+// SMs while the kernel before it still runs.  After the wait come the k
+// right-hand sides, 12 products a column and half, and a tree over the CTA.
+// What bounds it is the gather (k / 256 float4 a thread from L2) and the
+// launch: an iteration of a dense 343-vertex body 6.3 -> 5.1 us against the two
+// passes over the triangle.
+constexpr int kRootThreads = 256;
+constexpr int kRootRows = 8;
+constexpr int kRootWarps = kRootThreads / 32;
+constexpr int kRootGather = (kRootCols + kRootThreads - 1) / kRootThreads;
+size_t root_smem(int k) { return (size_t)k * 3 * sizeof(float4) + kRootWarps * kRootRows * sizeof(float4); }
+
+__global__ void __launch_bounds__(kRootThreads, 2) k_chol_root(CholArgs a, RootArgs q, int tiles, ResetArgs z) {
+    extern __shared__ float4 tile[];  // [k][2], then r [k], then the warps' sums
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if ((int)blockIdx.x >= tiles) {
+        reset_vertex(a, z, ((int)blockIdx.x - tiles) * kRootThreads + t);
+        return;
+    }
+    float4* rs = tile + 2 * q.k;
+    float4* part = rs + q.k;
+    const int row0 = kRootRows * blockIdx.x, half = t & 1;
+    const bool live = row0 + 4 * half < q.k;
+    for (int c = t >> 1; c < q.k; c += kRootThreads / 2)
+        cp_async16(tile + 2 * c + half, live ? q.inv + (size_t)c * q.ld + row0 + 4 * half : q.inv, live);
+    int vid[kRootGather];
+#pragma unroll
+    for (int g = 0; g < kRootGather; ++g) vid[g] = t + kRootThreads * g < q.k ? __ldg(&q.rows[t + kRootThreads * g]) : -1;
+    const int xv = t < kRootRows && row0 + t < q.k ? __ldg(&q.rows[row0 + t]) : -1;
     pdl_wait();
     pdl_trigger();
-    if ((a.done && *a.done) || i >= q.nv) return;
-    q.y_next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (q.b) q.b[i] = b;
+    const bool skip = a.done && *a.done;  // the same for every thread
+    if (!skip) {
+        float4 v[kRootGather];
+#pragma unroll
+        for (int g = 0; g < kRootGather; ++g) v[g] = vid[g] >= 0 ? __ldcg(&a.r[vid[g]]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int g = 0; g < kRootGather; ++g)
+            if (vid[g] >= 0) rs[t + kRootThreads * g] = v[g];
+    }
+    cp_async_wait();
+    if (skip) return;
+    __syncthreads();
+    float3 s[4] = {};
+    for (int c = t >> 1; c < q.k; c += kRootThreads / 2) {
+        const float4 m = tile[2 * c + half], v = rs[c];
+        fma3(s[0], m.x, v);
+        fma3(s[1], m.y, v);
+        fma3(s[2], m.z, v);
+        fma3(s[3], m.w, v);
+    }
+    // lanes of one parity hold the same four rows
+    halve<2>(s, lane, 16);
+    float3 u[2] = {s[0], s[1]};
+    halve<1>(u, lane, 8);
+    float3 w = u[0];
+#pragma unroll
+    for (int off = 4; off > 1; off >>= 1) {
+        w.x += __shfl_xor_sync(0xffffffffu, w.x, off);
+        w.y += __shfl_xor_sync(0xffffffffu, w.y, off);
+        w.z += __shfl_xor_sync(0xffffffffu, w.z, off);
+    }
+    if ((lane & 6) == 0)
+        part[kRootRows * warp + 4 * half + 2 * (lane >> 4) + (lane >> 3 & 1)] = make_float4(w.x, w.y, w.z, 0.f);
+    __syncthreads();
+    if (xv < 0) return;
+    float3 x = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int g = 0; g < kRootWarps; ++g) {
+        const float4 e = part[kRootRows * g + t];
+        x = make_float3(x.x + e.x, x.y + e.y, x.z + e.z);
+    }
+    a.x[xv] = make_float4(x.x, x.y, x.z, 0.f);
 }
 
 void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s,
-                              const ResetArgs& reset) {
+                              const ResetArgs& reset, const RootArgs& root) {
     const int nl = (int)levels.size();
     auto smem = [](const LevelRange& r) {
         return sizeof(float) * (r.ns > 0 ? kLevelWarps * kWarpFloats : r.nb > 0 ? kTileRows * kTileCols : 0);
@@ -536,13 +615,21 @@ void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& 
         return LevelRange{v.blk_begin, v.blk_end - v.blk_begin, v.sml_begin, v.sml_end - v.sml_begin, v.tiny_begin,
                           v.tiny_end - v.tiny_begin};
     };
-    for (int L = 0; L < nl; ++L) {
+    const int top = root.k > 0 ? nl - 1 : nl;  // levels of the two passes: the root, alone on its own, has the product
+    for (int L = 0; L < top; ++L) {
         const LevelRange r = range(L);
         const int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
         if (grid > 0) launch_pdl(k_chol_fwd_level, grid, kLevelThreads, smem(r), s, a, r);
     }
-    bool first = reset.y_next != nullptr;
-    for (int L = nl - 1; L >= 0; --L) {
+    bool first = reset.nv > 0;
+    if (root.k > 0) {
+        // with no level below the root the product does the resets
+        const int tiles = (root.k + kRootRows - 1) / kRootRows;
+        const bool here = first && top == 0;
+        const int grid = tiles + (here ? (reset.nv + kRootThreads - 1) / kRootThreads : 0);
+        launch_pdl(k_chol_root, grid, kRootThreads, root_smem(root.k), s, a, root, tiles, here ? reset : ResetArgs{});
+    }
+    for (int L = top - 1; L >= 0; --L) {
         const LevelRange r = range(L);
         int grid = r.nb + small_ctas(r.ns) + tiny_ctas(r.nt);
         if (first) grid += (reset.nv + kLevelThreads - 1) / kLevelThreads;
@@ -1086,6 +1173,21 @@ void launch_chol_vertex(const CholVertexArgs& a, cudaStream_t s) {
 void launch_chol_finish(const CholVertexArgs& a, cudaStream_t s) {
     const int blocks = (a.nv + 255) / 256;
     if (blocks) k_chol_finish<<<blocks, 256, 0, s>>>(a);
+}
+
+// The kernels between two local steps of a chain all ask for one split of L1 and
+// shared memory (19 x 11 x 23 refined twice, two steps: 930 -> 882 us); the
+// local step gains more from its L1 (10^3: 186 us as it is, 197 with the rest).
+void configure_chol_kernels() {
+    PDGB_CUDA_TRY(cudaFuncSetAttribute(k_chol_root, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)root_smem(kRootCols)));
+    prefer_shared(k_chol_root);
+    prefer_shared(k_chol_fwd_level);
+    prefer_shared(k_chol_bwd_level);
+    prefer_shared(k_copy_rhs);
+    prefer_shared(k_refine_residual);
+    prefer_shared(k_refine_update);
+    prefer_shared(k_chol_vertex);
+    prefer_shared(k_chol_finish);
 }
 
 }  // namespace pdgb

@@ -45,6 +45,15 @@ struct ResetArgs {
     const float4* pin_rhs;
 };
 
+// The product with the root's inverse (CholFactor::root): k = 0, none.
+struct RootArgs {
+    const float* inv;   // k x k, symmetric, columns ld apart
+    const int* rows;    // the root's pivots
+    int k, ld;
+};
+size_t root_smem(int k);
+void configure_chol_kernels();  // shared-memory limits of the step's kernels, on the current device
+
 constexpr int kLevelThreads = kTileRows;  // per-level kernels: one thread a tile row
 // Resident CTAs per SM that the per-level kernels' registers are allocated for.
 constexpr int kFwdBlocks = 11, kBwdBlocks = 10;
@@ -91,7 +100,7 @@ struct CholVertexArgs {
 
 // One launch per level and direction (large systems).
 void launch_chol_solve_levels(const CholArgs& a, const std::vector<SolveLevel>& levels, cudaStream_t s,
-                              const ResetArgs& reset = ResetArgs{});
+                              const ResetArgs& reset = ResetArgs{}, const RootArgs& root = RootArgs{});
 // The whole solve in one persistent cooperative launch over the GPU (all
 // bodies of a batch), levels separated by a bounded grid barrier; levels is
 // the device copy of the per-level item ranges.

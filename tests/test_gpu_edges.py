@@ -54,6 +54,22 @@ def test_sparse_solve_over_forms(dims, iters, tol, refine):
         _against_oracle(e, body, params, 4)
 
 
+# The product with the root's inverse: up to 1,024 pivots, 8 rows a CTA; the
+# whole solve (two right-hand sides in turn) or above one or two levels; odd and
+# even iteration counts, the convergence test, refinement.
+@pytest.mark.parametrize("dims,order,iters,tol,refine", [((1, 1, 1), 2, 1, 0.0, 0), ((1, 4, 6), 2, 2, 0.0, 1),
+                                                         ((16, 9, 5), 2, 3, 0.0, 0), ((15, 7, 7), 2, 4, 0.0, 0),
+                                                         ((18, 8, 5), 2, 3, 0.0, 0), ((6, 6, 6), 0, 3, 1e-4, 2),
+                                                         ((10, 10, 10), 0, 3, 0.0, 2), ((10, 10, 10), 0, 4, 1e-4, 0),
+                                                         ((31, 2, 29), 0, 5, 0.0, 1)])
+def test_root_product_over_forms(dims, order, iters, tol, refine):
+    body = mesh.make_grid_body(*dims, young=1e5, jitter=0.1, seed=13)
+    params = SolverParams(num_iterations=iters, tol=tol, solver=1, refine_steps=refine)
+    with PdSolver(body, params) as e:
+        e.set_ordering(order)
+        _against_oracle(e, body, params, 3)
+
+
 @pytest.mark.parametrize("mode", [N.PDGB_SOLVE_CTA, N.PDGB_SOLVE_CLUSTER, N.PDGB_SOLVE_LEVELS, N.PDGB_SOLVE_PERSISTENT])
 def test_batch_of_uneven_trees(mode):
     """Trees of different heights share the levels' launches."""
