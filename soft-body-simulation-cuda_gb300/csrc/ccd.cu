@@ -1,24 +1,28 @@
 // Continuous collision between bodies on the GPU (see ccd.h).
 //
-// Per detection:
-//   1. swept box of every surface triangle (X -> XTilde) and the scene box;
-//   2. 30-bit Morton code of each box centre, radix sort (CUB);
-//   3. LBVH over the sorted codes (Karras, "Maximizing parallelism in the
-//      construction of BVHs, octrees, and k-d trees", HPG 2012), the code
-//      extended by the sorted position so that keys are unique;
-//   4. bottom-up box refit: every leaf walks to the root, and at each
-//      internal node the second of its two children to arrive (an atomic
-//      arrival count, nobody waits) merges the children's boxes;
-//   5. traversal: each triangle collects the triangles of other bodies
-//      sharing no vertex whose boxes overlap its own (pairs kept once, by
-//      the larger triangle index);
-//   6. narrow phase: per pair and direction 3 point-face and 9 edge-edge
+// The triangles stand in a fixed order, body after body and along each body's
+// Morton curve at rest (build_ccd_surface): 32 in a row are a group, 32 groups
+// a node above them, and so on.  The candidates do not depend on the tree, so
+// a detection only computes its boxes:
+//   1. k_boxes: swept box of every surface triangle (X -> XTilde), of every
+//      group and of every 32 groups (k_boxes_up: what is above);
+//   2. k_groups: a warp a group, 32 boxes a step down the tree: the pairs of
+//      groups whose boxes overlap;
+//   3. k_pairs: a warp a pair of groups: its triangles of different bodies that
+//      share no vertex and whose boxes overlap (pairs kept once);
+//   4. k_narrow: per pair and direction 3 point-face and 9 edge-edge
 //      continuous tests; per vertex (point-face) and per edge (edge-edge)
 //      the earliest contact before t = 1 by a 64-bit atomic minimum of
 //      (contact time bits, face / other edge index);
-//   7. marking: tI = 0.5 and the earliest touching contact's normal for the
-//      vertices of every such contact (the reference's storeTi rule with its
+//   5. k_mark, k_result: tI = 0.5 and the earliest touching contact's normal for
+//      the vertices of every such contact (the reference's storeTi rule with its
 //      write race replaced by the earliest-contact choice).
+// Counts stay on the device; the host reads them once, at the end, and runs the
+// detection again with larger lists when one was too short.
+// What bounds a detection of some thousand triangles is latency: each kernel is
+// a chain of a few loads.  A binary tree over Morton codes sorted anew each time
+// (radix sort, build, refit, a stack a thread) took 240 us for 8 bodies of
+// 6 to 12 cells a side.
 // The reference's candidate set is the same (its BVH traversal is exact);
 // its query and reduction semantics are restated in narrow_test() below
 // (intersections.cu:286-334, narrowphase.cu:8-127).
@@ -28,13 +32,12 @@
 // oracle and the reference's code compiled for the host.
 #include "ccd.h"
 
-#include <cub/device/device_radix_sort.cuh>
-
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
 #include <utility>
 
+#include "pdl.cuh"
 #include "scene.cuh"
 
 namespace pdgb {
@@ -42,8 +45,13 @@ namespace pdgb {
 namespace {
 
 constexpr unsigned long long kNone = ~0ull;
-constexpr int kStack = 64;
 constexpr int kThreads = 256;
+constexpr int kBoxThreads = 1024;  // 32 groups of 32 triangles
+constexpr unsigned int kMostPairs = 1u << 30;
+// CTAs of the kernels that go over a list whose length is on the device: 4 on an
+// SM, the fewest that their registers allow.
+constexpr int kListCtas = 4 * 152;
+constexpr int kMaxLevels = 7;      // 32^7 > 2^31 triangles
 
 inline int blocks_for(long long n) { return (int)((n + kThreads - 1) / kThreads); }
 
@@ -194,52 +202,94 @@ __device__ __forceinline__ bool coplanar(float a, float l0, float l1, float l2) 
     return a < 1e-12 * l0 * l1 * l2;
 }
 
+// Coplanarity cubic a[3] t^3 + .. + a[0] of four points x + t v: their signed
+// volume at t.
+__device__ __forceinline__ void volume_cubic(const F3 x[4], const F3 v[4], float a[4], F3& x01, F3& x02, F3& x03) {
+    x01 = sub(x[1], x[0]), x02 = sub(x[2], x[0]), x03 = sub(x[3], x[0]);
+    const F3 v01 = sub(v[1], v[0]), v02 = sub(v[2], v[0]), v03 = sub(v[3], v[0]);
+    a[0] = triple(x01, x02, x03);
+    a[1] = triple(v01, x02, x03) + triple(x01, v02, x03) + triple(x01, x02, v03);
+    a[2] = triple(x01, v02, v03) + triple(v01, x02, v03) + triple(v01, v02, x03);
+    a[3] = triple(v01, v02, v03);
+}
+
+__device__ __forceinline__ float abs_sum(F3 a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
+__device__ __forceinline__ float abs_max(F3 a) { return fmaxf(fabsf(a.x), fmaxf(fabsf(a.y), fabsf(a.z))); }
+
+// False where narrow_test() returns 1 for certain, without its Newton
+// iterations (nine of ten candidates' queries): coplanar at t = 0, or a volume
+// that stays away from zero.  On [0, 1] the cubic lies between the least and the
+// greatest of its Bernstein coefficients.  A contact has a computed distance of
+// at most 1e-6, and distance times the product of two edges (each at most 2 L,
+// L the largest |x0k| + |v0k|) times the sine of their angle is the volume:
+// 4e-6 L^2 at most.  Rounding moves the volume and the distance's normal by some
+// tens of units in the last place of L^3 and of C L^2 (C the largest
+// coordinate; the normal's error grows with the sine's inverse and cancels it).
+// The line lies at 2e-5 L^2 + 4e-5 L^2 (C + L), 330 units; NaN is kept.
+__device__ __forceinline__ bool may_touch(const F3 x[4], const F3 v[4]) {
+    float a[4];
+    F3 x01, x02, x03;
+    volume_cubic(x, v, a, x01, x02, x03);
+    if (coplanar(fabsf(a[0]), len(x01), len(x02), len(x03))) return false;
+    float L = fmaxf(abs_sum(x01) + abs_sum(sub(v[1], v[0])), abs_sum(x02) + abs_sum(sub(v[2], v[0])));
+    L = fmaxf(L, abs_sum(x03) + abs_sum(sub(v[3], v[0])));
+    float c = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c = fmaxf(c, abs_max(x[k]) + abs_max(v[k]));
+    const float line = L * L * (2e-5f + 4e-5f * (c + L));
+    const float c1 = a[0] + a[1] / 3.0f, c2 = a[0] + (2.0f * a[1] + a[2]) / 3.0f, c3 = a[0] + a[1] + a[2] + a[3];
+    const bool above = a[0] > line && c1 > line && c2 > line && c3 > line;
+    const bool below = a[0] < -line && c1 < -line && c2 < -line && c3 < -line;
+    return !(above || below);
+}
+
+// Distance, normal n (pointing against the relative motion of the face side)
+// and barycentric test of a query's four points at time t.
+__device__ __forceinline__ float contact_at(bool face, const F3 x[4], const F3 v[4], float t, F3& n, bool& inside) {
+    F3 xt[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) xt[k] = add(x[k], scl(t, v[k]));
+    float w[4] = {0.f, 0.f, 0.f, 0.f};
+    float d;
+    if (face) {
+        d = face_distance(xt[0], xt[1], xt[2], xt[3], n, w);
+        inside = fminf(-w[1], fminf(-w[2], -w[3])) >= -kUpTo3;
+    } else {
+        d = edge_distance(xt[0], xt[1], xt[2], xt[3], n, w);
+        inside = fminf(w[0], fminf(w[1], fminf(-w[2], -w[3]))) >= -kUpTo3;
+    }
+    const F3 rel = add(add(scl(w[1], v[1]), scl(w[2], v[2])), scl(w[3], v[3]));
+    if (dot(n, rel) > 0) n = scl(-1.0f, n);
+    return d;
+}
+
 // Earliest contact time in [0, 1] of a point-face (face: point q0, face
 // q1..q3) or edge-edge (q0q1 against q2q3) query, 1 when none; n is the
-// contact normal (pointing against the relative motion of the face side).
-// Contact: the four points coplanar at a root of the cubic, within 1e-6 of
-// each other's plane / line and inside by the barycentric test.
+// contact normal.  Contact: the four points coplanar at a root of the cubic,
+// within 1e-6 of each other's plane / line and inside by the barycentric test.
 __device__ float narrow_test(bool face, const F3 x[4], const F3 v[4], F3& n) {
-    const F3 x01 = sub(x[1], x[0]), x02 = sub(x[2], x[0]), x03 = sub(x[3], x[0]);
-    const F3 v01 = sub(v[1], v[0]), v02 = sub(v[2], v[0]), v03 = sub(v[3], v[0]);
-    const float a0 = triple(x01, x02, x03);
-    const float a1 = triple(v01, x02, x03) + triple(x01, v02, x03) + triple(x01, x02, v03);
-    const float a2 = triple(x01, v02, v03) + triple(v01, x02, v03) + triple(v01, v02, x03);
-    const float a3 = triple(v01, v02, v03);
+    float a[4];
+    F3 x01, x02, x03;
+    volume_cubic(x, v, a, x01, x02, x03);
     n = {0.f, 0.f, 0.f};
-    if (coplanar(fabsf(a0), len(x01), len(x02), len(x03))) return 1.0f;  // coplanar at t = 0
+    if (coplanar(fabsf(a[0]), len(x01), len(x02), len(x03))) return 1.0f;  // coplanar at t = 0
     float t[3];
-    const int nr = cubic_roots(a3, a2, a1, a0, t);
+    const int nr = cubic_roots(a[3], a[2], a[1], a[0], t);
     for (int i = 0; i < nr; ++i) {
         if (t[i] < -kBelow12 || t[i] > 1) continue;
-        F3 xt[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) xt[k] = add(x[k], scl(t[i], v[k]));
-        float w[4] = {0.f, 0.f, 0.f, 0.f};
-        float d;
         bool inside;
-        if (face) {
-            d = face_distance(xt[0], xt[1], xt[2], xt[3], n, w);
-            inside = fminf(-w[1], fminf(-w[2], -w[3])) >= -kUpTo3;
-        } else {
-            d = edge_distance(xt[0], xt[1], xt[2], xt[3], n, w);
-            inside = fminf(w[0], fminf(w[1], fminf(-w[2], -w[3]))) >= -kUpTo3;
-        }
-        const F3 rel = add(add(scl(w[1], v[1]), scl(w[2], v[2])), scl(w[3], v[3]));
-        if (dot(n, rel) > 0) n = scl(-1.0f, n);
+        const float d = contact_at(face, x, v, t[i], n, inside);
         if (fabsf(d) <= kBelow6 && inside) return t[i];
     }
     return 1.0f;
 }
 
-__device__ __forceinline__ float query(bool face, const uint32_t ids[4], const float4* x, const float4* xt, F3& n) {
-    F3 p[4], v[4];
+__device__ __forceinline__ void load_query(const uint32_t ids[4], const float4* x, const float4* xt, F3 p[4], F3 v[4]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         p[k] = f3(x[ids[k]]);
         v[k] = sub(f3(xt[ids[k]]), p[k]);
     }
-    return narrow_test(face, p, v, n);
 }
 
 __device__ __forceinline__ unsigned long long time_key(float t, uint32_t tag) {
@@ -254,14 +304,6 @@ __device__ __forceinline__ int ord(float f) {
 }
 __device__ __forceinline__ float unord(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-__device__ __forceinline__ unsigned int spread10(unsigned int v) {
-    v = (v * 0x00010001u) & 0xFF0000FFu;
-    v = (v * 0x00000101u) & 0x0F00F00Fu;
-    v = (v * 0x00000011u) & 0xC30C30C3u;
-    v = (v * 0x00000005u) & 0x49249249u;
-    return v;
-}
-
 __device__ __forceinline__ bool overlap(float4 alo, float4 ahi, float4 blo, float4 bhi) {
     return !(ahi.x < blo.x || alo.x > bhi.x || ahi.y < blo.y || alo.y > bhi.y || ahi.z < blo.z || alo.z > bhi.z);
 }
@@ -275,21 +317,18 @@ struct Dev {
     const uint4* tri_edges;
     const uint2* edges;
     const int* vcaller;
-    float4* tri_lo;   // [ntris] swept boxes, triangle order
-    float4* tri_hi;
-    float4* node_lo;  // [2 ntris - 1]: internal nodes, then leaves in sorted order
-    float4* node_hi;
-    int* scene;       // [6] ordered min xyz, max xyz
-    unsigned int* code;
-    unsigned int* code_sorted;
-    int* order;
-    int* order_sorted;
-    int2* child;      // [ntris - 1]
-    int* parent;      // [2 ntris - 1]
-    int* visit;       // [ntris - 1]
-    int2* pairs;
-    int* counters;    // [0] pairs found, [1] traversal stack overflow
-    int pair_cap;
+    const uint4* stri;  // [ntris] the triangles in tree order
+    const int* order;   // [ntris] tree position -> triangle
+    // swept boxes: level 0 the triangles in tree order, a node of level l the
+    // 32^l triangles from 32^l j on; w lanes: the least and the greatest body
+    float4* lo;
+    float4* hi;
+    int top;  // first level from 1 on of at most 32 nodes
+    int off[kMaxLevels], cnt[kMaxLevels];
+    int2* groups;  // overlapping pairs of level-1 nodes
+    int2* pairs;   // candidate triangles
+    int group_cap, pair_cap;
+    unsigned int* counters;       // [0] pairs found, [1] group pairs found, [2] marked vertices
     unsigned long long* vf_best;  // [nv]
     unsigned long long* ee_best;  // [nedges]
     unsigned long long* vwin;     // [nv]
@@ -299,135 +338,150 @@ struct Dev {
     float4* nrm;
 };
 
-__global__ void k_init(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 3) {
-        d.scene[i] = ord(FLT_MAX);
-        d.scene[3 + i] = ord(-FLT_MAX);
-    }
-    if (i < 2) d.counters[i] = 0;
-    if (i < d.nv) {
-        d.vf_best[i] = kNone;
-        d.vwin[i] = kNone;
-    }
-    if (i < d.nedges) d.ee_best[i] = kNone;
-    if (i < d.ntris - 1) d.visit[i] = 0;
+struct Box {
+    float4 lo, hi;
+};
+
+__device__ __forceinline__ Box empty_box() {
+    return {make_float4(FLT_MAX, FLT_MAX, FLT_MAX, __uint_as_float(0xffffffffu)),
+            make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, __uint_as_float(0u))};
 }
 
-__global__ void k_boxes(Dev d) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.ntris) return;
-    const uint4 tr = d.tri[t];
-    const uint32_t id[3] = {tr.x, tr.y, tr.z};
-    float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.f), hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f);
+// Least upper box of a warp's boxes (w lanes included), in every lane.
+__device__ __forceinline__ Box warp_box(const Box& b) {
+    constexpr unsigned kAll = 0xffffffffu;
+    Box r;
+    r.lo.x = unord(__reduce_min_sync(kAll, ord(b.lo.x)));
+    r.lo.y = unord(__reduce_min_sync(kAll, ord(b.lo.y)));
+    r.lo.z = unord(__reduce_min_sync(kAll, ord(b.lo.z)));
+    r.lo.w = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(b.lo.w)));
+    r.hi.x = unord(__reduce_max_sync(kAll, ord(b.hi.x)));
+    r.hi.y = unord(__reduce_max_sync(kAll, ord(b.hi.y)));
+    r.hi.z = unord(__reduce_max_sync(kAll, ord(b.hi.z)));
+    r.hi.w = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(b.hi.w)));
+    return r;
+}
+
+// Everything below a and b is of one body.
+__device__ __forceinline__ bool one_body(const Box& a, const Box& b) {
+    const uint32_t body = __float_as_uint(a.lo.w);
+    return __float_as_uint(a.hi.w) == body && __float_as_uint(b.lo.w) == body && __float_as_uint(b.hi.w) == body;
+}
+
+// The boxes of levels 0 to 2 in one pass, a CTA a level-2 node, and the cleared
+// results.
+__global__ void __launch_bounds__(kBoxThreads) k_boxes(Dev d) {
+    __shared__ Box sub_box[32];
+    const int p = blockIdx.x * kBoxThreads + threadIdx.x;
+    if (p < 3) d.counters[p] = 0;
+    if (p < d.nv) {
+        d.vf_best[p] = kNone;
+        d.vwin[p] = kNone;
+    }
+    if (p < d.nedges) d.ee_best[p] = kNone;
+    if (blockIdx.x * kBoxThreads >= d.ntris) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Box b = empty_box();
+    if (p < d.ntris) {
+        const uint4 tr = d.stri[p];
+        const uint32_t id[3] = {tr.x, tr.y, tr.z};
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const float4 p = s ? d.xt[id[k]] : d.x[id[k]];
-            lo.x = fminf(lo.x, p.x);
-            lo.y = fminf(lo.y, p.y);
-            lo.z = fminf(lo.z, p.z);
-            hi.x = fmaxf(hi.x, p.x);
-            hi.y = fmaxf(hi.y, p.y);
-            hi.z = fmaxf(hi.z, p.z);
+            for (int s = 0; s < 2; ++s) {
+                const float4 q = s ? d.xt[id[k]] : d.x[id[k]];
+                b.lo.x = fminf(b.lo.x, q.x);
+                b.lo.y = fminf(b.lo.y, q.y);
+                b.lo.z = fminf(b.lo.z, q.z);
+                b.hi.x = fmaxf(b.hi.x, q.x);
+                b.hi.y = fmaxf(b.hi.y, q.y);
+                b.hi.z = fmaxf(b.hi.z, q.z);
+            }
+        b.lo.w = b.hi.w = __uint_as_float(tr.w);
+        d.lo[p] = b.lo;
+        d.hi[p] = b.hi;
+    }
+    b = warp_box(b);
+    if (lane == 0) {
+        sub_box[warp] = b;
+        if (p < d.ntris) {
+            d.lo[d.off[1] + (p >> 5)] = b.lo;
+            d.hi[d.off[1] + (p >> 5)] = b.hi;
         }
-    d.tri_lo[t] = lo;
-    d.tri_hi[t] = hi;
-    atomicMin(&d.scene[0], ord(lo.x));
-    atomicMin(&d.scene[1], ord(lo.y));
-    atomicMin(&d.scene[2], ord(lo.z));
-    atomicMax(&d.scene[3], ord(hi.x));
-    atomicMax(&d.scene[4], ord(hi.y));
-    atomicMax(&d.scene[5], ord(hi.z));
-}
-
-__global__ void k_morton(Dev d) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.ntris) return;
-    const float lo[3] = {unord(d.scene[0]), unord(d.scene[1]), unord(d.scene[2])};
-    const float hi[3] = {unord(d.scene[3]), unord(d.scene[4]), unord(d.scene[5])};
-    const float4 a = d.tri_lo[t], b = d.tri_hi[t];
-    const float c[3] = {0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z)};
-    unsigned int q[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float ext = hi[k] - lo[k];
-        const float u = ext > 0.f ? (c[k] - lo[k]) / ext : 0.f;
-        q[k] = (unsigned int)fminf(fmaxf(u * 1024.f, 0.f), 1023.f);
     }
-    d.code[t] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
-    d.order[t] = t;
+    if (d.top < 2) return;
+    __syncthreads();
+    if (warp > 0) return;
+    b = warp_box(sub_box[lane]);
+    if (lane == 0) {
+        d.lo[d.off[2] + blockIdx.x] = b.lo;
+        d.hi[d.off[2] + blockIdx.x] = b.hi;
+    }
 }
 
-// Length of the common prefix of the keys (code, position) at sorted
-// positions i and j; -1 outside [0, n).
-__device__ __forceinline__ int prefix(const Dev& d, int i, int j) {
-    if (j < 0 || j >= d.ntris) return -1;
-    const unsigned long long ki = ((unsigned long long)d.code_sorted[i] << 32) | (unsigned int)i;
-    const unsigned long long kj = ((unsigned long long)d.code_sorted[j] << 32) | (unsigned int)j;
-    return __clzll(ki ^ kj);
+// The boxes of a level from 3 on, a warp a node.
+__global__ void __launch_bounds__(kThreads) k_boxes_up(Dev d, int level) {
+    pdl_wait();
+    pdl_trigger();
+    const int j = (blockIdx.x * kThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (j >= d.cnt[level]) return;
+    const int c = 32 * j + lane;
+    Box b = empty_box();
+    if (c < d.cnt[level - 1]) b = {d.lo[d.off[level - 1] + c], d.hi[d.off[level - 1] + c]};
+    b = warp_box(b);
+    if (lane == 0) {
+        d.lo[d.off[level] + j] = b.lo;
+        d.hi[d.off[level] + j] = b.hi;
+    }
 }
 
-// Internal node i of the radix tree over n sorted keys: its key range and
-// split decide the two children (Karras 2012).  Nodes 0 .. n-2 are internal
-// (0 is the root), n-1 .. 2n-2 the leaves in sorted order.
-__global__ void k_build(Dev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = d.ntris;
-    if (i >= n - 1) return;
-    const int dir = (prefix(d, i, i + 1) - prefix(d, i, i - 1)) > 0 ? 1 : -1;
-    const int dmin = prefix(d, i, i - dir);
-    int lmax = 2;
-    while (lmax < 2 * n && prefix(d, i, i + lmax * dir) > dmin) lmax *= 2;  // keys are unique: lmax <= 2n
-    int l = 0;
-    for (int t = lmax / 2; t >= 1; t /= 2)
-        if (prefix(d, i, i + (l + t) * dir) > dmin) l += t;
-    const int j = i + l * dir;
-    const int dnode = prefix(d, i, j);
-    int s = 0;
-    int step = l;
-    do {
-        step = (step + 1) / 2;
-        if (prefix(d, i, i + (s + step) * dir) > dnode) s += step;
-    } while (step > 1);
-    const int split = i + s * dir + (dir < 0 ? -1 : 0);
-    const int lo = i < j ? i : j, hi = i < j ? j : i;
-    const int left = (lo == split) ? (n - 1 + split) : split;
-    const int right = (hi == split + 1) ? (n - 1 + split + 1) : split + 1;
-    d.child[i] = make_int2(left, right);
-    d.parent[left] = i;
-    d.parent[right] = i;
-}
-
-// Leaf boxes, then the bottom-up merge: the second child to arrive at a node
-// computes the node's box and goes on; the first stops.  No thread waits.
-__global__ void k_refit(Dev d) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = d.ntris;
-    if (j >= n) return;
-    const int t = d.order_sorted[j];
-    int node = n - 1 + j;
-    // w lanes: the least and the greatest body below the node
-    float4 lo = d.tri_lo[t], hi = d.tri_hi[t];
-    lo.w = hi.w = __uint_as_float(d.tri[t].w);
-    d.node_lo[node] = lo;
-    d.node_hi[node] = hi;
-    if (n == 1) return;
-    for (int guard = 0; guard < n; ++guard) {
-        node = d.parent[node];
-        __threadfence();
-        if (atomicAdd(&d.visit[node], 1) == 0) return;
-        const int2 c = d.child[node];
-        const float4 al = __ldcg(&d.node_lo[c.x]), ah = __ldcg(&d.node_hi[c.x]);
-        const float4 bl = __ldcg(&d.node_lo[c.y]), bh = __ldcg(&d.node_hi[c.y]);
-        const uint32_t body0 = min(__float_as_uint(al.w), __float_as_uint(bl.w)),
-                       body1 = max(__float_as_uint(ah.w), __float_as_uint(bh.w));
-        d.node_lo[node] =
-            make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __uint_as_float(body0));
-        d.node_hi[node] =
-            make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), __uint_as_float(body1));
-        if (node == 0) return;
+// Pairs of groups (g, h >= g) whose boxes overlap and that are not of one body.
+// A step down the tree tests 32 boxes, so the chain of loads is a few steps long
+// where a binary tree's was some tens, and a poor order of the bodies costs
+// little: a million triangles have 1,024 level-2 nodes, 32 steps.
+__global__ void __launch_bounds__(kThreads) k_groups(Dev d) {
+    __shared__ unsigned int todo[kThreads / 32][kMaxLevels];
+    __shared__ int first[kThreads / 32][kMaxLevels];
+    pdl_wait();
+    pdl_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+    if (g >= d.cnt[1]) return;
+    const Box own = {d.lo[d.off[1] + g], d.hi[d.off[1] + g]};
+    int l = d.top, at = 0;
+    for (;;) {
+        const int c = at + lane;
+        bool hit = false;
+        // the last group below node c: ((c + 1) 32^(l-1)) - 1
+        if (c < d.cnt[l] && ((long long)(c + 1) << (5 * (l - 1))) > g) {
+            const Box b = {d.lo[d.off[l] + c], d.hi[d.off[l] + c]};
+            hit = !one_body(own, b) && overlap(own.lo, own.hi, b.lo, b.hi);
+        }
+        unsigned int m = __ballot_sync(0xffffffffu, hit);
+        if (l == 1) {
+            if (m) {
+                unsigned int slot = 0;
+                if (lane == 0) slot = atomicAdd(&d.counters[1], (unsigned)__popc(m));
+                slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(m & ((1u << lane) - 1));
+                if (hit && slot < (unsigned)d.group_cap) d.groups[slot] = make_int2(g, c);
+            }
+            m = 0;
+        }
+        // the next node to go into: here, or the nearest level above that has one
+        while (m == 0) {
+            if (++l > d.top) return;
+            m = todo[warp][l];
+            at = first[warp][l];
+        }
+        const int bit = __ffs(m) - 1;
+        __syncwarp();
+        if (lane == 0) {
+            todo[warp][l] = m & (m - 1);
+            first[warp][l] = at;
+        }
+        __syncwarp();
+        at = 32 * (at + bit);
+        --l;
     }
 }
 
@@ -436,82 +490,151 @@ __device__ __forceinline__ bool share_vertex(uint4 a, uint4 b) {
            a.z == b.y || a.z == b.z;
 }
 
-// Subtrees that hold triangles of the thread's own body only are skipped: a
-// triangle overlaps its neighbours on the same surface first of all, and a
-// pair of one body is never a candidate.  A visit is a chain of three loads
-// (children, boxes, triangle), so what counts is how many nodes are visited.
-__global__ void k_traverse(Dev d) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = d.ntris;
-    if (j >= n || n < 2) return;
-    const int A = d.order_sorted[j];
-    const uint4 ta = d.tri[A];
-    const float4 lo = d.tri_lo[A], hi = d.tri_hi[A];
-    int stack[kStack];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-        const int node = stack[--sp];
-        const int2 c = d.child[node];
-        const int kids[2] = {c.x, c.y};
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int ch = kids[k];
-            const float4 clo = d.node_lo[ch], chi = d.node_hi[ch];
-            if (__float_as_uint(clo.w) == ta.w && __float_as_uint(chi.w) == ta.w) continue;
-            if (!overlap(lo, hi, clo, chi)) continue;
-            if (ch >= n - 1) {
-                const int B = d.order_sorted[ch - (n - 1)];
-                if (B <= A) continue;  // each unordered pair once
-                const uint4 tb = d.tri[B];
-                if (tb.w == ta.w || share_vertex(ta, tb)) continue;
-                const int slot = atomicAdd(&d.counters[0], 1);
-                if (slot < d.pair_cap) d.pairs[slot] = make_int2(A, B);
-            } else if (sp < kStack) {
-                stack[sp++] = ch;
-            } else {
-                d.counters[1] = 1;  // deeper than the stack: result incomplete, reported
-            }
+__device__ __forceinline__ float4 shfl4(float4 a, int from) {
+    return make_float4(__shfl_sync(0xffffffffu, a.x, from), __shfl_sync(0xffffffffu, a.y, from),
+                       __shfl_sync(0xffffffffu, a.z, from), __shfl_sync(0xffffffffu, a.w, from));
+}
+
+// Candidate triangles of the overlapping groups, a warp a pair of groups: a lane
+// keeps its triangle of the first group, those of the second that reach into the
+// first's box go round, and the hits of all 32 x 32 take one atomic.
+__global__ void __launch_bounds__(kThreads) k_pairs(Dev d) {
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (kThreads / 32);
+    const int ngroups = (int)min(d.counters[1], (unsigned)d.group_cap);
+    for (int i = (blockIdx.x * kThreads + threadIdx.x) >> 5; i < ngroups; i += warps) {
+        const int2 gh = d.groups[i];
+        const int p = 32 * gh.x + lane, q = 32 * gh.y + lane;
+        Box a = empty_box(), b = empty_box();
+        uint4 ta = {}, tb = {};
+        if (p < d.ntris) a = {d.lo[p], d.hi[p]}, ta = d.stri[p];
+        if (q < d.ntris) b = {d.lo[q], d.hi[q]}, tb = d.stri[q];
+        unsigned int m =
+            __ballot_sync(0xffffffffu, overlap(d.lo[d.off[1] + gh.x], d.hi[d.off[1] + gh.x], b.lo, b.hi) && q < d.ntris);
+        unsigned int hits = 0;
+        for (; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            const float4 blo = shfl4(b.lo, k), bhi = shfl4(b.hi, k);
+            const bool over = p < d.ntris && (gh.x != gh.y || lane < k) && ta.w != __float_as_uint(blo.w) &&
+                              overlap(a.lo, a.hi, blo, bhi);
+            if (!__any_sync(0xffffffffu, over)) continue;
+            const uint4 t = make_uint4(__shfl_sync(0xffffffffu, tb.x, k), __shfl_sync(0xffffffffu, tb.y, k),
+                                       __shfl_sync(0xffffffffu, tb.z, k), 0u);
+            if (over && !share_vertex(ta, t)) hits |= 1u << k;
         }
+        if (!__any_sync(0xffffffffu, hits != 0)) continue;
+        const int mine = __popc(hits);
+        int upto = mine;
+#pragma unroll
+        for (int s = 1; s < 32; s *= 2) {
+            const int o = __shfl_up_sync(0xffffffffu, upto, s);
+            if (lane >= s) upto += o;
+        }
+        unsigned int slot = 0;
+        if (lane == 31) slot = atomicAdd(&d.counters[0], (unsigned)upto);
+        slot = __shfl_sync(0xffffffffu, slot, 31) + (unsigned)(upto - mine);
+        const int A = mine ? d.order[p] : 0;
+        for (; hits; hits &= hits - 1, ++slot)
+            if (slot < (unsigned)d.pair_cap) d.pairs[slot] = make_int2(A, d.order[32 * gh.y + __ffs(hits) - 1]);
     }
 }
 
-// One thread per (pair, direction, query): q < 3 point-face, else edge-edge.
-__global__ void k_narrow(Dev d, int npairs) {
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= 24LL * npairs) return;
-    const int pi = (int)(g / 24), r = (int)(g % 24);
-    const int dirn = r / 12, q = r % 12;
-    const int2 pr = d.pairs[pi];
-    const int P = dirn ? pr.y : pr.x, Fc = dirn ? pr.x : pr.y;
-    const uint4 tp = d.tri[P], tf = d.tri[Fc];
-    const uint32_t pv[3] = {tp.x, tp.y, tp.z};
-    F3 nn;
-    if (q < 3) {
-        const uint32_t ids[4] = {pv[q], tf.x, tf.y, tf.z};
-        const float t = query(true, ids, d.x, d.xt, nn);
-        if (t < 1.0f) atomicMin(&d.vf_best[pv[q]], time_key(t, (uint32_t)Fc));
+// Query r < 24 of a candidate pair: 12 a direction, r % 12 < 3 point-face, else
+// edge-edge; ids of its four vertices, where its contact goes and its tag.
+struct Query {
+    uint32_t ids[4];
+    unsigned long long* best;
+    uint32_t tag;
+    bool face;
+};
+__device__ __forceinline__ Query get_query(const Dev& d, long long g) {
+    const int2 pr = d.pairs[g / 24];
+    const int r = (int)(g % 24), q = r % 12;
+    const int P = r >= 12 ? pr.y : pr.x, Fc = r >= 12 ? pr.x : pr.y;
+    Query o;
+    o.face = q < 3;
+    if (o.face) {
+        const uint4 tp = d.tri[P], tf = d.tri[Fc];
+        o.ids[0] = q == 0 ? tp.x : q == 1 ? tp.y : tp.z;
+        o.ids[1] = tf.x, o.ids[2] = tf.y, o.ids[3] = tf.z;
+        o.best = d.vf_best + o.ids[0];
+        o.tag = (uint32_t)Fc;
     } else {
         const uint4 ep = d.tri_edges[P], ef = d.tri_edges[Fc];
-        const uint32_t pe[3] = {ep.x, ep.y, ep.z}, fe[3] = {ef.x, ef.y, ef.z};
-        const uint32_t ea = pe[(q - 3) / 3], eb = fe[(q - 3) % 3];
+        const int i = (q - 3) / 3, j = (q - 3) % 3;
+        const uint32_t ea = i == 0 ? ep.x : i == 1 ? ep.y : ep.z, eb = j == 0 ? ef.x : j == 1 ? ef.y : ef.z;
         const uint2 a = d.edges[ea], b = d.edges[eb];
-        const uint32_t ids[4] = {a.x, a.y, b.x, b.y};
-        const float t = query(false, ids, d.x, d.xt, nn);
-        if (t < 1.0f) atomicMin(&d.ee_best[ea], time_key(t, eb));
+        o.ids[0] = a.x, o.ids[1] = a.y, o.ids[2] = b.x, o.ids[3] = b.y;
+        o.best = d.ee_best + ea;
+        o.tag = eb;
     }
+    return o;
+}
+
+// A CTA takes up to kBatch queries at a time: those that may touch (may_touch())
+// are listed, point-face from the front and edge-edge from the back, and only
+// the listed ones go through the cubic's Newton iterations, 32 of a kind a warp.
+// With a query a thread a warp waited for its slowest lane's iterations.
+constexpr int kBatch = 4 * kThreads;
+__global__ void __launch_bounds__(kThreads) k_narrow(Dev d) {
+    __shared__ unsigned short list[kBatch];
+    __shared__ int found[2];
+    pdl_wait();
+    pdl_trigger();
+    const int t = threadIdx.x;
+    const long long total = 24LL * (long long)min(d.counters[0], (unsigned)d.pair_cap);
+    // as many CTAs as possible take part
+    const long long share = (total + (long long)gridDim.x * kThreads - 1) / ((long long)gridDim.x * kThreads);
+    const int batch = kThreads * (int)min(share, (long long)(kBatch / kThreads));
+    for (long long base = (long long)blockIdx.x * batch; base < total; base += (long long)gridDim.x * batch) {
+        if (t < 2) found[t] = 0;
+        __syncthreads();
+        for (int u = t; u < batch && base + u < total; u += kThreads) {
+            const Query q = get_query(d, base + u);
+            F3 p[4], v[4];
+            load_query(q.ids, d.x, d.xt, p, v);
+            if (!may_touch(p, v)) continue;
+            const int slot = atomicAdd(&found[q.face ? 0 : 1], 1);
+            list[q.face ? slot : kBatch - 1 - slot] = (unsigned short)u;
+        }
+        __syncthreads();
+        const int nf = found[0], ne = found[1], warps_f = (nf + 31) & ~31;
+        for (int i = t; i < warps_f + ne; i += kThreads) {
+            if (i >= nf && i < warps_f) continue;
+            const Query q = get_query(d, base + list[i < nf ? i : kBatch - 1 - (i - warps_f)]);
+            F3 p[4], v[4], n;
+            load_query(q.ids, d.x, d.xt, p, v);
+            const float tc = narrow_test(q.face, p, v, n);
+            if (tc < 1.0f) atomicMin(q.best, time_key(tc, q.tag));
+        }
+        __syncthreads();
+    }
+}
+
+// The normal that narrow_test() gave with the contact time in best: its
+// evaluation at that time, or the whole query where the key clamped the time.
+__device__ __forceinline__ F3 contact_normal(const Dev& d, bool face, const uint32_t ids[4], unsigned long long best) {
+    const float t = __uint_as_float((unsigned int)(best >> 32));
+    F3 p[4], v[4], n;
+    load_query(ids, d.x, d.xt, p, v);
+    bool inside;
+    if (t > 0.f) contact_at(face, p, v, t, n, inside);
+    else narrow_test(face, p, v, n);
+    return n;
 }
 
 // Winning contact per touched vertex: smallest (time, source) key, the
 // source being the caller id of a point-face contact's point or nv + edge.
-__global__ void k_mark(Dev d) {
+__global__ void __launch_bounds__(kThreads) k_mark(Dev d) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < d.nv && d.vf_best[i] != kNone) {
         const unsigned long long best = d.vf_best[i];
         const uint4 tf = d.tri[(uint32_t)(best & 0xffffffffu)];
         const uint32_t ids[4] = {(uint32_t)i, tf.x, tf.y, tf.z};
-        F3 nn;
-        query(true, ids, d.x, d.xt, nn);
+        const F3 nn = contact_normal(d, true, ids, best);
         d.vf_n[i] = make_float4(nn.x, nn.y, nn.z, 0.f);
         const uint32_t src = d.vcaller ? (uint32_t)d.vcaller[i] : (uint32_t)i;
         const unsigned long long key = (best & 0xffffffff00000000ull) | src;
@@ -524,8 +647,7 @@ __global__ void k_mark(Dev d) {
         const unsigned long long best = d.ee_best[i];
         const uint2 a = d.edges[i], b = d.edges[(uint32_t)(best & 0xffffffffu)];
         const uint32_t ids[4] = {a.x, a.y, b.x, b.y};
-        F3 nn;
-        query(false, ids, d.x, d.xt, nn);
+        const F3 nn = contact_normal(d, false, ids, best);
         d.ee_n[i] = make_float4(nn.x, nn.y, nn.z, 0.f);
         const unsigned long long key = (best & 0xffffffff00000000ull) | (uint32_t)(d.nv + i);
         atomicMin(&d.vwin[a.x], key);
@@ -533,20 +655,29 @@ __global__ void k_mark(Dev d) {
     }
 }
 
-// Normals from the winning contacts (each vertex has exactly one writer).
-__global__ void k_normals(Dev d) {
+// tI, and the normals from the winning contacts (each hit vertex has exactly one
+// writer; the others' are cleared).
+__global__ void __launch_bounds__(kThreads) k_result(Dev d) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < d.nv && d.vf_best[i] != kNone) {
-        const unsigned long long best = d.vf_best[i];
-        const uint4 tf = d.tri[(uint32_t)(best & 0xffffffffu)];
-        const uint32_t src = d.vcaller ? (uint32_t)d.vcaller[i] : (uint32_t)i;
-        const unsigned long long key = (best & 0xffffffff00000000ull) | src;
-        const float4 n = d.vf_n[i];
-        const float4 m = make_float4(-n.x, -n.y, -n.z, 0.f);
-        if (d.vwin[i] == key) d.nrm[i] = n;
-        if (d.vwin[tf.x] == key) d.nrm[tf.x] = m;
-        if (d.vwin[tf.y] == key) d.nrm[tf.y] = m;
-        if (d.vwin[tf.z] == key) d.nrm[tf.z] = m;
+    bool hit = false;
+    if (i < d.nv) {
+        hit = d.vwin[i] != kNone;
+        d.tI[i] = hit ? 0.5f : 1.0f;
+        if (!hit) d.nrm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (d.vf_best[i] != kNone) {
+            const unsigned long long best = d.vf_best[i];
+            const uint4 tf = d.tri[(uint32_t)(best & 0xffffffffu)];
+            const uint32_t src = d.vcaller ? (uint32_t)d.vcaller[i] : (uint32_t)i;
+            const unsigned long long key = (best & 0xffffffff00000000ull) | src;
+            const float4 n = d.vf_n[i];
+            const float4 m = make_float4(-n.x, -n.y, -n.z, 0.f);
+            if (d.vwin[i] == key) d.nrm[i] = n;
+            if (d.vwin[tf.x] == key) d.nrm[tf.x] = m;
+            if (d.vwin[tf.y] == key) d.nrm[tf.y] = m;
+            if (d.vwin[tf.z] == key) d.nrm[tf.z] = m;
+        }
     }
     if (i < d.nedges && d.ee_best[i] != kNone) {
         const unsigned long long key = (d.ee_best[i] & 0xffffffff00000000ull) | (uint32_t)(d.nv + i);
@@ -554,15 +685,8 @@ __global__ void k_normals(Dev d) {
         if (d.vwin[a.x] == key) d.nrm[a.x] = d.ee_n[i];
         if (d.vwin[a.y] == key) d.nrm[a.y] = d.ee_n[i];
     }
-}
-
-__global__ void k_finish(Dev d, int* marked) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.nv) return;
-    const bool hit = d.vwin[i] != kNone;
-    d.tI[i] = hit ? 0.5f : 1.0f;
-    if (!hit) d.nrm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (hit) atomicAdd(marked, 1);
+    const unsigned int m = __ballot_sync(0xffffffffu, hit);
+    if ((threadIdx.x & 31) == 0 && m) atomicAdd(&d.counters[2], (unsigned)__popc(m));
 }
 
 // CCDKernel (collisionUtil.cu:50-70): a vertex with tI < 1 keeps X and gets
@@ -594,7 +718,46 @@ __global__ void k_respond(int nv, const float* tI, const float4* nrm, float4* x,
 }  // namespace
 
 // ------------------------------------------------------------ host side
-CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm) {
+namespace {
+// Tree order of the triangles: by body, a body's along the Morton curve of its
+// own box (10 bits an axis) at the positions X.
+void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const float* X, std::vector<int>& order) {
+    std::vector<KeyId> key(ntris), tmp;
+    for (int t = 0; t < ntris; ++t) key[t] = {(uint64_t)(uint32_t)tri_body[t], t};
+    radix_sort(key, tmp);
+    auto centre = [&](int t, int k) {
+        const uint32_t* v = tris + 3 * (size_t)t;
+        return X[3 * (size_t)v[0] + k] + X[3 * (size_t)v[1] + k] + X[3 * (size_t)v[2] + k];
+    };
+    for (int b = 0, end = 0; b < ntris; b = end) {
+        const uint64_t body = key[b].key;
+        float lo[3], hi[3];
+        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = centre(key[b].id, k);
+        for (end = b; end < ntris && key[end].key == body; ++end)
+            for (int k = 0; k < 3; ++k) {
+                const float c = centre(key[end].id, k);
+                lo[k] = std::min(lo[k], c);
+                hi[k] = std::max(hi[k], c);
+            }
+        for (int q = b; q < end; ++q) {
+            uint64_t m = 0;
+            for (int k = 0; k < 3; ++k) {
+                const float ext = hi[k] - lo[k];
+                const float u = ext > 0.f ? (centre(key[q].id, k) - lo[k]) / ext : 0.f;
+                const uint64_t c = u > 0.f ? (uint64_t)std::min(u * 1024.f, 1023.f) : 0;  // NaN: 0
+                for (int bit = 0; bit < 10; ++bit) m |= (c >> bit & 1) << (3 * bit + 2 - k);
+            }
+            key[q].key = body << 30 | m;
+        }
+    }
+    radix_sort(key, tmp);
+    order.resize(ntris);
+    for (int q = 0; q < ntris; ++q) order[q] = key[q].id;
+}
+}  // namespace
+
+CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm,
+                             const float* X) {
     if (nv <= 0 || ntris < 0 || (ntris > 0 && (!tris || !tri_body)))
         throw Error{PDGB_ERR_INVALID_ARGUMENT, "collision surface: bad sizes or null arrays"};
     CcdSurface s;
@@ -634,46 +797,56 @@ CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int*
     }
     s.edges.resize(edges.size());
     for (size_t e = 0; e < edges.size(); ++e) s.edges[e] = make_uint2(iv(edges[e].first), iv(edges[e].second));
+    tree_order(ntris, tris, tri_body, X, s.order);
     return s;
 }
 
 struct CcdContext::Buffers {
-    DBuf<uint4> tri, tri_edges;
+    DBuf<uint4> tri, stri, tri_edges;
     DBuf<uint2> edges;
-    DBuf<float4> tri_lo, tri_hi, node_lo, node_hi, vf_n, ee_n, nrm;
-    DBuf<int> scene, order, order_sorted, parent, visit, counters, marked;
-    DBuf<unsigned int> code, code_sorted;
-    DBuf<int2> child, pairs;
+    DBuf<int> order;
+    DBuf<float4> lo, hi, vf_n, ee_n, nrm;
+    DBuf<unsigned int> counters;
+    DBuf<int2> groups, pairs;
     DBuf<unsigned long long> vf_best, ee_best, vwin;
     DBuf<float> tI;
-    DBuf<unsigned char> sort_tmp;
-    size_t sort_bytes = 0;
-    int pair_cap = 0;
+    int group_cap = 0, pair_cap = 0;
+    int top = 1, off[kMaxLevels] = {}, cnt[kMaxLevels] = {};
     cudaEvent_t ev[2] = {nullptr, nullptr};
+    unsigned int* counts = nullptr;  // pinned copy of the counters
+    ~Buffers() {
+        if (ev[0]) cudaEventDestroy(ev[0]);
+        if (ev[1]) cudaEventDestroy(ev[1]);
+        if (counts) cudaFreeHost(counts);
+    }
 };
 
 CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t stream)
     : b_(new Buffers), nv_(s.nv), ntris_(s.ntris), nedges_(s.nedges), vcaller_(vcaller), stream_(stream) {
     Buffers& b = *b_;
-    const size_t n = (size_t)std::max(ntris_, 1);
     b.tri.upload(s.tri, stream);
     b.tri_edges.upload(s.tri_edges, stream);
     b.edges.upload(s.edges, stream);
-    b.tri_lo.alloc(n);
-    b.tri_hi.alloc(n);
-    b.node_lo.alloc(2 * n);
-    b.node_hi.alloc(2 * n);
-    b.scene.alloc(6);
-    b.code.alloc(n);
-    b.code_sorted.alloc(n);
-    b.order.alloc(n);
-    b.order_sorted.alloc(n);
-    b.child.alloc(n);
-    b.parent.alloc(2 * n);
-    b.visit.alloc(n);
-    b.counters.alloc(2);
-    b.marked.alloc(1);
-    b.pair_cap = (int)std::min<size_t>(std::max<size_t>(16 * n, 4096), 1u << 30);
+    std::vector<uint4> sorted(ntris_);
+    for (int q = 0; q < ntris_; ++q) sorted[q] = s.tri[s.order[q]];
+    b.stri.upload(sorted, stream);
+    b.order.upload(s.order, stream);
+    size_t nodes = 0;
+    for (int l = 0; l < kMaxLevels; ++l) {
+        b.cnt[l] = l == 0 ? ntris_ : (b.cnt[l - 1] + 31) / 32;
+        b.off[l] = (int)nodes;
+        nodes += (size_t)b.cnt[l];
+        if (nodes > 0x7fffffff) throw Error{PDGB_ERR_UNSUPPORTED, "collision surface too large"};
+    }
+    while (b.cnt[b.top] > 32) ++b.top;
+    b.lo.alloc(std::max<size_t>(nodes, 1));
+    b.hi.alloc(std::max<size_t>(nodes, 1));
+    b.counters.alloc(3);
+    PDGB_CUDA_TRY(cudaMallocHost(&b.counts, 3 * sizeof(unsigned int)));
+    const size_t n = (size_t)std::max(ntris_, 1);
+    b.group_cap = std::max(16 * b.cnt[1], 256);
+    b.groups.alloc(b.group_cap);
+    b.pair_cap = (int)std::min<size_t>(std::max<size_t>(16 * n, 4096), kMostPairs);
     b.pairs.alloc(b.pair_cap);
     b.vf_best.alloc(nv_);
     b.vwin.alloc(nv_);
@@ -682,9 +855,6 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     b.ee_n.alloc(std::max(nedges_, 1));
     b.tI.alloc(nv_);
     b.nrm.alloc(nv_);
-    PDGB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, b.sort_bytes, b.code.p, b.code_sorted.p, b.order.p,
-                                                  b.order_sorted.p, (int)n, 0, 30, stream));
-    b.sort_tmp.alloc(std::max<size_t>(b.sort_bytes, 1));
     PDGB_CUDA_TRY(cudaEventCreate(&b.ev[0]));
     PDGB_CUDA_TRY(cudaEventCreate(&b.ev[1]));
     // no contact until the first detection
@@ -694,12 +864,7 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     PDGB_CUDA_TRY(cudaStreamSynchronize(stream));
 }
 
-CcdContext::~CcdContext() {
-    if (b_) {
-        if (b_->ev[0]) cudaEventDestroy(b_->ev[0]);
-        if (b_->ev[1]) cudaEventDestroy(b_->ev[1]);
-    }
-}
+CcdContext::~CcdContext() = default;
 
 const float* CcdContext::tI() const { return b_->tI.p; }
 const float4* CcdContext::normals() const { return b_->nrm.p; }
@@ -718,21 +883,14 @@ void CcdContext::detect(const float4* x, const float4* xt) {
     d.tri_edges = b.tri_edges.p;
     d.edges = b.edges.p;
     d.vcaller = vcaller_;
-    d.tri_lo = b.tri_lo.p;
-    d.tri_hi = b.tri_hi.p;
-    d.node_lo = b.node_lo.p;
-    d.node_hi = b.node_hi.p;
-    d.scene = b.scene.p;
-    d.code = b.code.p;
-    d.code_sorted = b.code_sorted.p;
+    d.stri = b.stri.p;
     d.order = b.order.p;
-    d.order_sorted = b.order_sorted.p;
-    d.child = b.child.p;
-    d.parent = b.parent.p;
-    d.visit = b.visit.p;
-    d.pairs = b.pairs.p;
+    d.lo = b.lo.p;
+    d.hi = b.hi.p;
+    d.top = b.top;
+    std::copy(b.off, b.off + kMaxLevels, d.off);
+    std::copy(b.cnt, b.cnt + kMaxLevels, d.cnt);
     d.counters = b.counters.p;
-    d.pair_cap = b.pair_cap;
     d.vf_best = b.vf_best.p;
     d.ee_best = b.ee_best.p;
     d.vwin = b.vwin.p;
@@ -740,50 +898,45 @@ void CcdContext::detect(const float4* x, const float4* xt) {
     d.ee_n = b.ee_n.p;
     d.tI = b.tI.p;
     d.nrm = b.nrm.p;
-    const long long init_n = std::max<long long>({(long long)nv_, (long long)nedges_, (long long)ntris_, 6});
-    k_init<<<blocks_for(init_n), kThreads, 0, s>>>(d);
-    int npairs = 0;
-    if (ntris_ >= 2) {
-        k_boxes<<<blocks_for(ntris_), kThreads, 0, s>>>(d);
-        k_morton<<<blocks_for(ntris_), kThreads, 0, s>>>(d);
-        size_t bytes = b.sort_bytes;
-        PDGB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(b.sort_tmp.p, bytes, b.code.p, b.code_sorted.p, b.order.p,
-                                                      b.order_sorted.p, ntris_, 0, 30, s));
-        k_build<<<blocks_for(ntris_ - 1), kThreads, 0, s>>>(d);
-        k_refit<<<blocks_for(ntris_), kThreads, 0, s>>>(d);
-        for (int attempt = 0;; ++attempt) {
-            k_traverse<<<blocks_for(ntris_), kThreads, 0, s>>>(d);
-            int cnt[2] = {0, 0};
-            PDGB_CUDA_TRY(cudaMemcpyAsync(cnt, b.counters.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
-            PDGB_CUDA_TRY(cudaStreamSynchronize(s));
-            if (cnt[1]) throw Error{PDGB_ERR_UNSUPPORTED, "collision BVH deeper than the traversal stack"};
-            if (cnt[0] <= b.pair_cap) {
-                npairs = cnt[0];
-                break;
-            }
-            if (attempt > 0 || cnt[0] > (1 << 30)) throw Error{PDGB_ERR_OUT_OF_MEMORY, "too many collision candidates"};
-            b.pair_cap = cnt[0] + cnt[0] / 4;  // grow once to the count found, then rerun
-            b.pairs.alloc(b.pair_cap);
-            d.pairs = b.pairs.p;
-            d.pair_cap = b.pair_cap;
-            stats_.regrows++;
-            PDGB_CUDA_TRY(cudaMemsetAsync(b.counters.p, 0, 2 * sizeof(int), s));
+    const int most = std::max({nv_, nedges_, ntris_, 3});
+    const int outs = blocks_for(std::max(nv_, nedges_));
+    // The lists grow to the counts found and the detection runs again: the count
+    // of pairs is whole once the list of groups is.
+    for (int attempt = 0;; ++attempt) {
+        d.groups = b.groups.p;
+        d.pairs = b.pairs.p;
+        d.group_cap = b.group_cap;
+        d.pair_cap = b.pair_cap;
+        k_boxes<<<(int)(((long long)most + kBoxThreads - 1) / kBoxThreads), kBoxThreads, 0, s>>>(d);
+        if (ntris_ >= 2) {
+            for (int l = 3; l <= b.top; ++l) launch_pdl(k_boxes_up, blocks_for(32LL * b.cnt[l]), kThreads, 0, s, d, l);
+            launch_pdl(k_groups, blocks_for(32LL * b.cnt[1]), kThreads, 0, s, d);
+            launch_pdl(k_pairs, (int)std::min<long long>(blocks_for(32LL * b.group_cap), kListCtas), kThreads, 0, s, d);
+            launch_pdl(k_narrow, (int)std::min<long long>(blocks_for(24LL * b.pair_cap), kListCtas), kThreads, 0, s, d);
         }
-        if (npairs > 0) k_narrow<<<blocks_for(24LL * npairs), kThreads, 0, s>>>(d, npairs);
+        launch_pdl(k_mark, outs, kThreads, 0, s, d);
+        launch_pdl(k_result, outs, kThreads, 0, s, d);
+        PDGB_CUDA_TRY(cudaGetLastError());
+        PDGB_CUDA_TRY(cudaEventRecord(b.ev[1], s));
+        PDGB_CUDA_TRY(cudaMemcpyAsync(b.counts, b.counters.p, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        PDGB_CUDA_TRY(cudaStreamSynchronize(s));
+        const bool groups = b.counts[1] > (unsigned)b.group_cap, pairs = b.counts[0] > (unsigned)b.pair_cap;
+        if (!groups && !pairs) break;
+        if (attempt > 1 || std::max(b.counts[0], b.counts[1]) > kMostPairs)
+            throw Error{PDGB_ERR_OUT_OF_MEMORY, "too many collision candidates"};
+        if (groups) {
+            b.group_cap = (int)(b.counts[1] + b.counts[1] / 4);
+            b.groups.alloc(b.group_cap);
+        } else {
+            b.pair_cap = (int)(b.counts[0] + b.counts[0] / 4);
+            b.pairs.alloc(b.pair_cap);
+            stats_.regrows++;
+        }
     }
-    PDGB_CUDA_TRY(cudaMemsetAsync(b.marked.p, 0, sizeof(int), s));
-    k_mark<<<blocks_for(std::max(nv_, nedges_)), kThreads, 0, s>>>(d);
-    k_normals<<<blocks_for(std::max(nv_, nedges_)), kThreads, 0, s>>>(d);
-    k_finish<<<blocks_for(nv_), kThreads, 0, s>>>(d, b.marked.p);
-    PDGB_CUDA_TRY(cudaGetLastError());
-    PDGB_CUDA_TRY(cudaEventRecord(b.ev[1], s));
-    int marked = 0;
-    PDGB_CUDA_TRY(cudaMemcpyAsync(&marked, b.marked.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PDGB_CUDA_TRY(cudaStreamSynchronize(s));
     float ms = 0.f;
     PDGB_CUDA_TRY(cudaEventElapsedTime(&ms, b.ev[0], b.ev[1]));
-    stats_.pairs = npairs;
-    stats_.marked = marked;
+    stats_.pairs = b.counts[0];
+    stats_.marked = (int)b.counts[2];
     stats_.ms = ms;
 }
 

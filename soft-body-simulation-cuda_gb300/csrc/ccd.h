@@ -24,11 +24,14 @@ struct CcdSurface {
     std::vector<uint4> tri;        // x, y, z: internal vertex ids; w: body
     std::vector<uint4> tri_edges;  // x, y, z: edge ids of the triangle
     std::vector<uint2> edges;      // internal vertex ids (ascending caller id)
+    std::vector<int> order;        // tree position -> triangle
 };
 
 // tris: [3 ntris] caller vertex ids; tri_body: [ntris]; viperm: caller ->
-// internal vertex (null: identity).  Throws Error on bad input.
-CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm);
+// internal vertex (null: identity); X: [3 nv] finite positions, caller order,
+// that the triangles' tree order follows.  Throws Error on bad input.
+CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm,
+                             const float* X);
 
 struct CcdStats {
     long long pairs = 0;        // candidate triangle pairs of the last detection
@@ -48,8 +51,8 @@ public:
     CcdContext& operator=(const CcdContext&) = delete;
 
     // Detection between x (start, internal order) and xt (end): fills tI and
-    // normals (device, internal order).  Waits for the stream (the candidate
-    // count decides the narrow phase's size, as in the reference).
+    // normals (device, internal order).  Waits for the stream once: the
+    // candidate count decides whether the lists were long enough.
     void detect(const float4* x, const float4* xt);
     // CCDKernel + the fixed-body correction of XTilde and v (the reference
     // applies it after the collision response, pdSolver.cu:228-231).

@@ -88,13 +88,8 @@ template <class F> void in_parts(int n, F&& f) {
         if (e) std::rethrow_exception(e);
 }
 
-// Sorts (key, id) pairs by key, equal keys in their present order: least
-// significant byte first, passes whose byte is the same everywhere skipped.
-// Three to four times as fast as a comparison sort from some thousand pairs.
-struct KeyId {
-    uint64_t key;
-    int id;
-};
+}  // namespace
+
 void radix_sort(std::vector<KeyId>& a, std::vector<KeyId>& tmp) {
     const size_t n = a.size();
     if (n < 512) {
@@ -118,8 +113,6 @@ void radix_sort(std::vector<KeyId>& a, std::vector<KeyId>& tmp) {
         a.swap(tmp);
     }
 }
-
-}  // namespace
 
 std::vector<float> chebyshev_omegas(int n, float rho) {
     std::vector<float> w(std::max(n, 0));

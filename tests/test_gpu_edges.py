@@ -181,3 +181,37 @@ def test_collision_query_over_scales(scale, offset):
     assert info["candidate_pairs"] == pairs and info["vertices_hit"] == marked
     assert np.array_equal(tI, tIo)  # the same decisions
     assert np.abs(nrm - nrmo).max() <= 1e-6
+
+
+def _soup(n, bodies, seed, size=0.06, speed=0.08, room=0.5, stretch=1.0):
+    rng = np.random.default_rng(seed)
+    cent = rng.uniform(-room, room, (n, 1, 3))
+    X = cent + rng.uniform(-size, size, (n, 3, 3)) * np.array([stretch, 1.0, 1.0])
+    X = X.reshape(-1, 3).astype(np.float32)
+    XT = (X + rng.uniform(-speed, speed, X.shape)).astype(np.float32)
+    tris = np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    return tris, rng.integers(0, bodies, n).astype(np.int32), X, XT
+
+
+# Groups of 32 triangles and tree levels of 32: one triangle, at and past one
+# group, one and two levels, three; the lists that grow (every box over every
+# other: 561 group pairs past 528, pairs past 16 a triangle); slivers a hundredth
+# as wide as long, far from the origin; hardly moving and fast ones.
+@pytest.mark.parametrize("n,bodies,kw", [(1, 1, {}), (2, 2, {"room": 0.02}), (31, 3, {"room": 0.1}), (32, 2, {"room": 0.1}),
+                                         (33, 2, {"room": 0.1}), (1024, 5, {"room": 0.7}), (1025, 40, {"room": 0.7}),
+                                         (1056, 2, {"room": 0.01, "size": 0.3}), (33000, 300, {"room": 4.0}),
+                                         (600, 4, {"stretch": 100.0, "size": 0.01}),
+                                         (600, 4, {"speed": 1e-4, "room": 0.15}), (600, 4, {"speed": 3.0})])
+def test_collision_tree_and_lists(n, bodies, kw):
+    tris, body, X, XT = _soup(n, bodies, 40 + n % 17, **kw)
+    if kw.get("stretch"):
+        X, XT = X + np.float32(20.0), XT + np.float32(20.0)
+    if n == 1025:  # triangles of different bodies that share vertices
+        tris[1:400:2, 0] = tris[0:400:2, 1][:200]
+    tI, nrm, info = ccd_detect(tris, body, X, XT)
+    tIo, nrmo, (pairs, _, marked) = O.ccd_detect(tris, body, X, XT)
+    assert info["candidate_pairs"] == pairs and info["vertices_hit"] == marked
+    assert np.array_equal(tI, tIo)  # the same float operations decide both
+    assert np.abs(nrm - nrmo).max() <= 1e-6
+    if n == 1056:
+        assert info["regrows"] == 1
