@@ -228,8 +228,8 @@ void clear_nonfinite(pdgb_engine* e) {
 // Collision detection + response after a step (PdSolver::Update,
 // pdSolver.cu:218-231).
 void run_collision(pdgb_engine* e) {
-    e->ccd->detect(e->x.p, e->xt.p);
-    e->ccd->respond(e->x.p, e->xt.p, e->v.p, scene_args(e));
+    const CcdResponse response{e->x.p, e->v.p, scene_args(e)};
+    e->ccd->detect(e->x.p, e->xt.p, &response);
 }
 
 BeginArgs begin_args(pdgb_engine* e) {

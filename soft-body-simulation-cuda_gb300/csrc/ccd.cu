@@ -122,17 +122,26 @@ __device__ float cubic_newton(float a, float b, float c, float d, float x0, int 
         const float ddy0 = 2 * b + x0 * (6 * a);
         if (ddy0 != 0) x0 += dir * sqrtf(fabsf(2 * y0 / ddy0));
     }
-    float before = __int_as_float(0x7fffffff);  // the iterate before x0 (NaN: none)
-    for (int it = 0; it < 100; ++it) {
+    // Far roots and roots of near-planar queries end up going round a few floats
+    // more than 1e-6 apart, mostly two, for the rest of the hundred steps.  A step
+    // depends on the iterate alone, so once one repeats (Brent's cycle finding: the
+    // iterates 2, 4, 8, .. are kept) whole rounds are left out.  8 bodies in
+    // contact, where one query of sixty took 100 or 200 steps and its warp with
+    // it: 62 -> 34 us (31 with the runs dealt out, k_narrow()).
+    float kept = __int_as_float(0x7fffffff);  // NaN: none
+    int kept_at = 0, next = 2, steps = 100;
+    for (int it = 1; it <= steps; ++it) {
         const float y = d + x0 * (c + x0 * (b + x0 * a));
         const float dy = c + x0 * (2 * b + x0 * 3 * a);
         if (dy == 0) return x0;
         const float x1 = x0 - y / dy;
         if (fabsf(x0 - x1) <= kBelow6) return x0;
-        // far roots end up swapping between two neighbouring floats more than
-        // 1e-6 apart: the hundredth iterate is known then
-        if (x1 == before) return (99 - it) % 2 == 0 ? x1 : x0;
-        before = x0;
+        if (x1 == kept) steps = it + (steps - it) % (it - kept_at);
+        if (it == next) {
+            kept = x1;
+            kept_at = it;
+            next *= 2;
+        }
         x0 = x1;
     }
     return x0;
@@ -584,14 +593,17 @@ __global__ void __launch_bounds__(kThreads) k_narrow(Dev d) {
     pdl_trigger();
     const int t = threadIdx.x;
     const long long total = 24LL * (long long)min(d.counters[0], (unsigned)d.pair_cap);
-    // as many CTAs as possible take part
-    const long long share = (total + (long long)gridDim.x * kThreads - 1) / ((long long)gridDim.x * kThreads);
-    const int batch = kThreads * (int)min(share, (long long)(kBatch / kThreads));
-    for (long long base = (long long)blockIdx.x * batch; base < total; base += (long long)gridDim.x * batch) {
+    // runs of 32 queries, dealt out to the CTAs in turn: contact is local, and so
+    // is the work that the sieve leaves
+    const int share = (int)((total + 32LL * gridDim.x - 1) / (32LL * gridDim.x));
+    for (int run = 0; run < share; run += kBatch / 32) {
+        const int batch = 32 * min(share - run, kBatch / 32);
+        auto query_at = [&](int u) { return 32 * ((long long)(run + (u >> 5)) * gridDim.x + blockIdx.x) + (u & 31); };
         if (t < 2) found[t] = 0;
         __syncthreads();
-        for (int u = t; u < batch && base + u < total; u += kThreads) {
-            const Query q = get_query(d, base + u);
+        for (int u = t; u < batch; u += kThreads) {
+            if (query_at(u) >= total) break;
+            const Query q = get_query(d, query_at(u));
             F3 p[4], v[4];
             load_query(q.ids, d.x, d.xt, p, v);
             if (!may_touch(p, v)) continue;
@@ -602,7 +614,7 @@ __global__ void __launch_bounds__(kThreads) k_narrow(Dev d) {
         const int nf = found[0], ne = found[1], warps_f = (nf + 31) & ~31;
         for (int i = t; i < warps_f + ne; i += kThreads) {
             if (i >= nf && i < warps_f) continue;
-            const Query q = get_query(d, base + list[i < nf ? i : kBatch - 1 - (i - warps_f)]);
+            const Query q = get_query(d, query_at(list[i < nf ? i : kBatch - 1 - (i - warps_f)]));
             F3 p[4], v[4], n;
             load_query(q.ids, d.x, d.xt, p, v);
             const float tc = narrow_test(q.face, p, v, n);
@@ -692,10 +704,13 @@ __global__ void __launch_bounds__(kThreads) k_result(Dev d) {
 // CCDKernel (collisionUtil.cu:50-70): a vertex with tI < 1 keeps X and gets
 // v = -(d . n) n with d = XTilde - X; the others move to XTilde.  Then the
 // fixed-body correction of XTilde and v.
-__global__ void k_respond(int nv, const float* tI, const float4* nrm, float4* x, const float4* xt, float4* v,
-                          SceneArgs sc) {
+// Nothing where a list of the detection was too short: it runs again, and the
+// response with it.
+__global__ void __launch_bounds__(kThreads) k_respond(Dev det, int nv, const float* tI, const float4* nrm,
+                                                     float4* x, const float4* xt, float4* v, SceneArgs sc) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
+    if (i >= nv || det.counters[0] > (unsigned)det.pair_cap || det.counters[1] > (unsigned)det.group_cap) return;
     const float4 p = x[i], q = xt[i];
     float4 vel = v[i];
     if (tI[i] < 1.0f) {
@@ -869,7 +884,7 @@ CcdContext::~CcdContext() = default;
 const float* CcdContext::tI() const { return b_->tI.p; }
 const float4* CcdContext::normals() const { return b_->nrm.p; }
 
-void CcdContext::detect(const float4* x, const float4* xt) {
+void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* response) {
     Buffers& b = *b_;
     cudaStream_t s = stream_;
     PDGB_CUDA_TRY(cudaEventRecord(b.ev[0], s));
@@ -918,6 +933,9 @@ void CcdContext::detect(const float4* x, const float4* xt) {
         launch_pdl(k_result, outs, kThreads, 0, s, d);
         PDGB_CUDA_TRY(cudaGetLastError());
         PDGB_CUDA_TRY(cudaEventRecord(b.ev[1], s));
+        if (response)
+            launch_pdl(k_respond, blocks_for(nv_), kThreads, 0, s, d, nv_, b.tI.p, b.nrm.p, response->x, xt, response->v,
+                       response->sc);
         PDGB_CUDA_TRY(cudaMemcpyAsync(b.counts, b.counters.p, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         PDGB_CUDA_TRY(cudaStreamSynchronize(s));
         const bool groups = b.counts[1] > (unsigned)b.group_cap, pairs = b.counts[0] > (unsigned)b.pair_cap;
@@ -938,12 +956,6 @@ void CcdContext::detect(const float4* x, const float4* xt) {
     stats_.pairs = b.counts[0];
     stats_.marked = (int)b.counts[2];
     stats_.ms = ms;
-}
-
-void CcdContext::respond(float4* x, const float4* xt, float4* v, const SceneArgs& sc) {
-    Buffers& b = *b_;
-    k_respond<<<blocks_for(nv_), kThreads, 0, stream_>>>(nv_, b.tI.p, b.nrm.p, x, xt, v, sc);
-    PDGB_CUDA_TRY(cudaGetLastError());
 }
 
 }  // namespace pdgb

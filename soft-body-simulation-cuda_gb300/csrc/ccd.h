@@ -41,6 +41,14 @@ struct CcdStats {
     double ms = 0.0;            // device time of the last detection + response
 };
 
+// CCDKernel + the fixed-body correction of XTilde and v (the reference
+// applies it after the collision response, pdSolver.cu:228-231).
+struct CcdResponse {
+    float4* x;
+    float4* v;
+    SceneArgs sc;
+};
+
 class CcdContext {
 public:
     // vcaller: device array internal -> caller vertex id (null: identity),
@@ -51,12 +59,10 @@ public:
     CcdContext& operator=(const CcdContext&) = delete;
 
     // Detection between x (start, internal order) and xt (end): fills tI and
-    // normals (device, internal order).  Waits for the stream once: the
-    // candidate count decides whether the lists were long enough.
-    void detect(const float4* x, const float4* xt);
-    // CCDKernel + the fixed-body correction of XTilde and v (the reference
-    // applies it after the collision response, pdSolver.cu:228-231).
-    void respond(float4* x, const float4* xt, float4* v, const SceneArgs& sc);
+    // normals (device, internal order), and does the response if there is one to
+    // do.  Waits for the stream once, behind both: the counts decide whether the
+    // lists were long enough.
+    void detect(const float4* x, const float4* xt, const CcdResponse* response = nullptr);
 
     const float* tI() const;
     const float4* normals() const;
