@@ -328,8 +328,9 @@ int pdgb_inspect_layout(const pdgb_mesh_desc* mesh, pdgb_layout_info* info, int*
 int pdgb_set_ordering(pdgb_engine* e, int ordering);
 
 /* Rotation of the local step.  QUAT (default): the closest proper rotation
- * from the dominant eigenvector of Horn's 4x4 quaternion matrix, converged to
- * float precision.  SVD: the reference's scheme -- 4 approximate-Givens
+ * from the largest eigenvalue of Horn's 4x4 quaternion matrix and, where that
+ * does not determine it well (inverted elements), from its eigenvector;
+ * converged to float precision.  SVD: the reference's scheme -- 4 approximate-Givens
  * Jacobi sweeps of a McAdams-style 3x3 SVD, R = U V^T (svd.cuh:7-14,
  * pdUtil.cu:113-122) -- which is not fully converged on stretched elements. */
 #define PDGB_ROTATION_QUAT 0

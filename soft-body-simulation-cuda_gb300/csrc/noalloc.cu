@@ -211,7 +211,7 @@ __device__ __forceinline__ void na_local(const NaTet& q, const NaScratch& s) {
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc) F[3 * r + cc] = e[r][0] * D[cc] + e[r][1] * D[3 + cc] + e[r][2] * D[6 + cc];
     float R[9];
-    closest_rotation_horn(F, R);
+    closest_rotation_quat(F, R);
 #pragma unroll
     for (int k = 0; k < 9; ++k) R[k] -= F[k];
     float M[9];

@@ -215,3 +215,34 @@ def test_collision_tree_and_lists(n, bodies, kw):
     assert np.abs(nrm - nrmo).max() <= 1e-6
     if n == 1056:
         assert info["regrows"] == 1
+
+
+# The closed form and the squarings meet where 2 (s1 + s2)(s1 + s3)(s2 + s3) =
+# |F|^3: strains up to there and past it, flat and inverted elements, scales down
+# to where squares leave float's range.  Both round a result of condition
+# |F| / (s2 + s3), at most 4 here: some ten units of 6e-8 times that.
+@pytest.mark.parametrize("strain", [0.0, 0.01, 0.3, 1.0])
+@pytest.mark.parametrize("scale", [1e-12, 1e-4, 1.0, 1e4, 1e12])
+def test_rotation_over_strains_and_scales(strain, scale):
+    rng = np.random.default_rng(5)
+    n = 4000
+    U, V = (np.linalg.qr(rng.normal(size=(n, 3, 3)))[0] for _ in range(2))
+    U *= np.sign(np.linalg.det(U))[:, None, None]
+    V *= np.sign(np.linalg.det(V))[:, None, None]
+    s = 1.0 + strain * rng.normal(size=(n, 3))
+    s[: n // 8, 2] = 0.0
+    s[n // 8: n // 4, 2] = -0.3
+    F = np.einsum("nij,nj,nkj->nik", U, s, V).astype(np.float32)
+    Fd = F.astype(np.float64)
+    u, sv, vt = np.linalg.svd(Fd)
+    sign = np.sign(np.linalg.det(u @ vt))
+    D = np.ones((n, 3))
+    D[:, 2] = sign
+    R = np.einsum("nij,nj,njk->nik", u, D, vt)
+    well = sv[:, 1] + sign * sv[:, 2] > 0.25 * np.linalg.norm(sv, axis=1)
+    assert well.mean() > 0.5
+    F = np.ascontiguousarray(F * np.float32(scale))
+    out = np.empty_like(F)
+    N.check(N.lib().pdgb_closest_rotations(n, F.ctypes.data, out.ctypes.data, N.PDGB_ROTATION_QUAT), "rotations")
+    err = np.abs(out - R).max(axis=(1, 2))[well]
+    assert err.max() < 4 * 10 * 6e-8 and np.sqrt(np.mean(err ** 2)) < 6e-7
