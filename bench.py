@@ -540,11 +540,15 @@ def run_serving(args, window: float, rate: float = 0.0, solver: str = "", cache:
 
 def launches_per_step(info, params) -> int:
     """Kernels of one step graph: prologue, per iteration local + global
-    (Jacobi: 1 vertex kernel; Cholesky: 2 per solve level + 1 vertex kernel),
-    Cholesky epilogue."""
+    (Jacobi: 1 vertex kernel; Cholesky: the solve, and with refinement a copy of
+    the right-hand side and residual, solve and update each), Cholesky epilogue.
+    The per-level solve does the vertex kernel's resets unless the convergence
+    test is on; the other schedules launch it."""
     if params.solver == 0:
         return 1 + 2 * params.num_iterations
-    return 2 + params.num_iterations * (2 + info["solve_launches"])
+    solve, refine = info["solve_launches"], params.refine_steps
+    vertex = 0 if info["solve_mode"] == 3 and params.tol == 0 else 1
+    return 2 + params.num_iterations * (1 + solve + vertex + (1 + refine * (2 + solve) if refine else 0))
 
 
 # Default timed steps per workload: about 1.5 s of device time, so that the

@@ -202,10 +202,7 @@ __device__ __forceinline__ float sym4_frob2(const float a[10]) {
 }
 
 template <int kTail = 8>
-__device__ __forceinline__ void closest_rotation_horn(const float F[9], float R[9]) {
-    float f2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) f2 = fmaf(F[i], F[i], f2);
+__device__ __forceinline__ void closest_rotation_horn(const float F[9], float f2, float R[9]) {
     f2 = fmaxf(f2, 1e-30f);
     const float c = 0.6f * f2 * rsqrtf(f2);      // shift; precision irrelevant
     const float sc = __fdividef(0.25f, c);       // eigenvalues of A / (4c) <= 1
@@ -250,38 +247,25 @@ __device__ __forceinline__ void closest_rotation_horn(const float F[9], float R[
 }
 
 // Closest proper rotation in closed form from the largest eigenvalue l of N(F)
-// (above), false where it is not well determined.  l = max tr(R^T F) over the
-// rotations, so R = dl/dF, and l is the largest root of N's characteristic
-// quartic p(l) = l^4 - 2 f l^2 - 8 d l + 2 |C|^2 - f^2 with C = F^T F, f = tr C,
-// d = det F.  Differentiating p(l(F), F) = 0:
+// (above).  l = max tr(R^T F) over the rotations, so R = dl/dF, and l is the
+// largest root of N's characteristic quartic
+//   p(l) = l^4 - 2 f l^2 - 8 d l + 2 |C|^2 - f^2
+// with C = F^T F, f = tr C, d = det F.  Differentiating p(l(F), F) = 0:
 //   R = ((l^2 + f) F + 2 l cof F - 2 F C) / (l^3 - f l - 2 d).
 // Newton starts at sqrt(3 f) less its second-order distance from l: two steps up
-// to strains of 20 %, more where the second was not small.  The divisor is
-// 2 (s1 + s2)(s1 + s3)(s2 + s3) in F's signed singular values, 3.08 f^1.5 at a
-// rotation and 1.41 f^1.5 for an element pressed flat.  Down to f^1.5 R's error
-// against double is no larger than that of closest_rotation_horn() (rms 6.4e-8 ..
-// 7.7e-8 against 7.1e-8 .. 7.8e-8 over strains of 0.1 to 150 %); below, and where
-// f^2 could leave float's range, that one is used.  The local step takes 452
-// instructions a tet with it and 512 with the squarings alone, of which a warp
-// does the most of its lanes: 47 x 5 x 61 cells 4.9 -> 4.5 us, 128 uneven bodies
-// 43.7 -> 39.7 us, 64^3, where shared memory bounds it, 28.1 -> 27.9 us.
-__device__ __forceinline__ bool closest_rotation_root(const float F[9], float R[9]) {
-    const float c00 = fmaf(F[0], F[0], fmaf(F[3], F[3], F[6] * F[6]));
-    const float c11 = fmaf(F[1], F[1], fmaf(F[4], F[4], F[7] * F[7]));
-    const float c22 = fmaf(F[2], F[2], fmaf(F[5], F[5], F[8] * F[8]));
+// to strains of 20 %, more where the second was not small.  c, K: C's diagonal
+// and the first row of cof F; root = f^0.5.
+__device__ __forceinline__ void closest_rotation_root(const float F[9], const float c[3], const float K0[3], float f,
+                                                      float inv, float root, float d, float R[9]) {
     const float c01 = fmaf(F[0], F[1], fmaf(F[3], F[4], F[6] * F[7]));
     const float c02 = fmaf(F[0], F[2], fmaf(F[3], F[5], F[6] * F[8]));
     const float c12 = fmaf(F[1], F[2], fmaf(F[4], F[5], F[7] * F[8]));
-    const float f = c00 + c11 + c22;
-    const float K[9] = {fmaf(F[4], F[8], -F[5] * F[7]), fmaf(F[5], F[6], -F[3] * F[8]), fmaf(F[3], F[7], -F[4] * F[6]),
+    const float K[9] = {K0[0], K0[1], K0[2],
                         fmaf(F[2], F[7], -F[1] * F[8]), fmaf(F[0], F[8], -F[2] * F[6]), fmaf(F[1], F[6], -F[0] * F[7]),
                         fmaf(F[1], F[5], -F[2] * F[4]), fmaf(F[2], F[3], -F[0] * F[5]), fmaf(F[0], F[4], -F[1] * F[3])};
-    const float d = fmaf(F[0], K[0], fmaf(F[1], K[1], F[2] * K[2]));
-    const float diag = fmaf(c00, c00, fmaf(c11, c11, c22 * c22));
+    const float diag = fmaf(c[0], c[0], fmaf(c[1], c[1], c[2] * c[2]));
     const float off = fmaf(c01, c01, fmaf(c02, c02, c12 * c12));
     const float p0 = fmaf(2.f, fmaf(2.f, off, diag), -f * f), p1 = -8.f * d;
-    const float inv = rsqrtf(f), root = f * inv;
-    // first guess to third order in the strain
     const float v = fmaf(3.f, fmaf(2.f, off, diag), -f * f) * (inv * inv) * (inv * inv);
     float l = root * fmaf(-0.2165064f, fminf(v, 0.4f), 1.7320508f), step;
     auto newton = [&] {
@@ -294,11 +278,10 @@ __device__ __forceinline__ bool closest_rotation_root(const float F[9], float R[
     for (int it = 0; it < 5 && fabsf(step) > 1e-4f * l; ++it) newton();
     const float l2 = l * l;
     const float den = fmaf(l, l2 - f, -2.f * d);
-    if (!(den > f * root && f > 1e-15f)) return false;  // NaN: false
     float r = __fdividef(1.f, den);
     r = fmaf(r, fmaf(-den, r, 1.f), r);
     // R = r (F B + 2 l K), B = (l^2 + f) I - 2 C
-    const float b00 = fmaf(-2.f, c00, l2 + f), b11 = fmaf(-2.f, c11, l2 + f), b22 = fmaf(-2.f, c22, l2 + f);
+    const float b00 = fmaf(-2.f, c[0], l2 + f), b11 = fmaf(-2.f, c[1], l2 + f), b22 = fmaf(-2.f, c[2], l2 + f);
     const float b01 = -2.f * c01, b02 = -2.f * c02, b12 = -2.f * c12;
 #pragma unroll
     for (int q = 0; q < 9; q += 3) {
@@ -306,11 +289,32 @@ __device__ __forceinline__ bool closest_rotation_root(const float F[9], float R[
         R[q + 1] = r * fmaf(2.f * l, K[q + 1], fmaf(F[q], b01, fmaf(F[q + 1], b11, F[q + 2] * b12)));
         R[q + 2] = r * fmaf(2.f * l, K[q + 2], fmaf(F[q], b02, fmaf(F[q + 1], b12, F[q + 2] * b22)));
     }
-    return true;
 }
 
+// The rotation of a tet: in closed form where all of the warp's elements have
+// det F > 0.06 |F|^3 (0.19 at a rotation; stretched to 3.6 times or pressed to a
+// fifth), else by the squarings, so that a warp never pays for both: with the
+// choice made by the lane, 64^3 on its way from rest through 50 steps, where the
+// iteration diverges and elements invert, took 0.767 ms a step, with the squarings
+// alone 0.722, this way 0.700.
+// There the divisor 2 (s1 + s2)(s1 + s3)(s2 + s3) in F's singular values is at
+// least 1.4 |F|^3 (3.08 at a rotation), and the closed form's error against
+// double is no larger than the squarings' (rms 6.3e-8 .. 7.0e-8 against 7.1e-8 ..
+// 7.7e-8 over strains of 0.1 to 150 %).  Where |F|^4 could leave float's range
+// the squarings run as well.  The local step takes 452 instructions a tet in
+// closed form and 512 with two squarings, and 70 more for each further one:
+// 47 x 5 x 61 cells 4.9 -> 4.5 us, 128 uneven bodies 43.7 -> 39.7 us, 64^3 near rest,
+// where shared memory bounds it, 28.1 -> 27.6 us.
 __device__ __forceinline__ void closest_rotation_quat(const float F[9], float R[9]) {
-    if (!closest_rotation_root(F, R)) closest_rotation_horn(F, R);
+    const float c[3] = {fmaf(F[0], F[0], fmaf(F[3], F[3], F[6] * F[6])), fmaf(F[1], F[1], fmaf(F[4], F[4], F[7] * F[7])),
+                        fmaf(F[2], F[2], fmaf(F[5], F[5], F[8] * F[8]))};
+    const float f = c[0] + c[1] + c[2];
+    const float K[3] = {fmaf(F[4], F[8], -F[5] * F[7]), fmaf(F[5], F[6], -F[3] * F[8]), fmaf(F[3], F[7], -F[4] * F[6])};
+    const float d = fmaf(F[0], K[0], fmaf(F[1], K[1], F[2] * K[2]));
+    const float inv = rsqrtf(f), root = f * inv;
+    const bool well = d > 0.06f * f * root && f > 1e-15f && f < 1e15f;  // NaN: false
+    if (__all_sync(__activemask(), well)) closest_rotation_root(F, c, K, f, inv, root, d, R);
+    else closest_rotation_horn(F, f, R);
 }
 
 }  // namespace pdgb

@@ -217,8 +217,8 @@ def test_collision_tree_and_lists(n, bodies, kw):
         assert info["regrows"] == 1
 
 
-# The closed form and the squarings meet where 2 (s1 + s2)(s1 + s3)(s2 + s3) =
-# |F|^3: strains up to there and past it, flat and inverted elements, scales down
+# The closed form and the squarings meet where det F = 0.06 |F|^3, for a whole
+# warp: strains up to there and past it, flat and inverted elements, scales down
 # to where squares leave float's range.  Both round a result of condition
 # |F| / (s2 + s3), at most 4 here: some ten units of 6e-8 times that.
 @pytest.mark.parametrize("strain", [0.0, 0.01, 0.3, 1.0])
