@@ -515,7 +515,7 @@ int pdgb_download_xtilde(pdgb_engine* e, float* XT, int memory);
  * src/collision/bvh.cu:153-165, broadphase.cu, narrowphase.cu,
  * intersections.cu:286-334; src/simulation/collisionUtil.cu:50-70):
  *   - candidates: surface triangles of different bodies that share no
- *     vertex and whose swept boxes (X -> XTilde) overlap (GPU LBVH);
+ *     vertex and whose swept boxes (X -> XTilde) overlap;
  *   - per pair, both ways: 3 point-face and 9 edge-edge continuous tests
  *     (coplanarity cubic, proximity 1e-6, barycentric slack 1e-3);
  *   - per vertex / per edge the earliest contact; every vertex of such a
@@ -526,8 +526,8 @@ int pdgb_download_xtilde(pdgb_engine* e, float* XT, int memory);
  *     The fixed-body correction of XTilde and V follows (pdSolver.cu:228).
  * Triangles are caller vertex ids (3 per triangle); tri_body gives each
  * triangle's body (NULL: the body of its first vertex, from the engine's
- * body ranges).  Detection waits for the stream once per step (the
- * candidate count sizes the narrow phase, as in the reference). */
+ * body ranges).  Detection waits for the stream once per step: the
+ * counts decide whether its lists were long enough. */
 typedef struct pdgb_collision_info {
     long long candidate_pairs;  /* triangle pairs tested by the last detection */
     int vertices_hit;           /* vertices with tI < 1 after it               */
