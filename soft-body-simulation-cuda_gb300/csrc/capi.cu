@@ -453,6 +453,9 @@ void upload_mesh(pdgb_engine* e) {
 // the kernels use (M/h^2 incl. the pin weight) and the double geometry.
 SparseSym engine_system(const HostLayout& L) { return layout_system(L); }
 
+// A whole factor is on the device (prepare_cholesky).
+bool has_factor(const pdgb_engine* e) { return e->chol_ordering >= 0; }
+
 // Solve schedule: the requested one, or the per-level launches, which are the
 // fastest at every size: one iteration of a 2^3 body 5.6 us against 11.1 us for
 // one cluster and 12.1 us for one CTA, of 64 such bodies 6.2 against 18.4 and
@@ -470,11 +473,14 @@ void prepare_cholesky(pdgb_engine* e) {
     // ... and its vectors and blocks share a cluster's shared memory: there
     // every stored entry counts and a level is only a cluster barrier
     const double level_entries = e->solve_req == PDGB_SOLVE_DSM ? kDsmLevelEntries : kLevelEntries;
-    if (level_entries == e->chol_level_entries && e->chol_ordering == e->ordering && e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight &&
-        e->chol.n == e->nv && e->factor_dev == dev) {
+    if (has_factor(e) && level_entries == e->chol_level_entries && e->chol_ordering == e->ordering &&
+        e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight && e->factor_dev == dev) {
         e->solve_mode = choose_solve_mode(e);
         return;  // the system matrix depends only on the mesh, dt and the pin weight
     }
+    // until everything below is in place there is no factor: what throws on the
+    // way leaves half of this one in the buffers of the one before
+    e->chol_ordering = -1;
     const bool gpu = dev == PDGB_FACTOR_GPU;
     auto t0 = std::chrono::steady_clock::now();
     SparseSym K;
@@ -549,11 +555,11 @@ void prepare_cholesky(pdgb_engine* e) {
             e->dsm_lvl.upload(e->dsm.lvl, s);
         }
     }
-    e->solve_mode = choose_solve_mode(e);
     e->chol_level_entries = level_entries;
     e->chol_ordering = e->ordering;
     e->chol_dt = e->prm.dt;
     e->chol_pw = e->prm.positional_weight;
+    e->solve_mode = choose_solve_mode(e);  // throws where the DSM solve does not fit: the factor stays
 }
 
 void prepare(pdgb_engine* e) {
@@ -1521,7 +1527,7 @@ int pdgb_local_step_bytes(pdgb_engine* e, double* bytes) {
 int pdgb_solve_bytes(pdgb_engine* e, double* bytes) {
     if (!e || !bytes) return PDGB_ERR_INVALID_ARGUMENT;
     *bytes = 0.0;
-    if (e->prm.solver != PDGB_SOLVER_CHOLESKY || e->chol.n != e->nv) return PDGB_OK;
+    if (e->prm.solver != PDGB_SOLVER_CHOLESKY || !has_factor(e)) return PDGB_OK;
     // forward + backward: factor values and row indices (4 B + 4 B per
     // nonzero of the scalar L) and column pointers, plus the 3-column
     // right-hand sides: read b 12 n, write and read y 24 n, write x 12 n
@@ -1604,7 +1610,7 @@ int solve_launches(const pdgb_engine* e) {
 int pdgb_get_factor_info(pdgb_engine* e, pdgb_factor_info* info) {
     if (!e || !info) return PDGB_ERR_INVALID_ARGUMENT;
     std::memset(info, 0, sizeof(*info));
-    if (e->prm.solver != PDGB_SOLVER_CHOLESKY || e->chol.n != e->nv) return PDGB_OK;
+    if (e->prm.solver != PDGB_SOLVER_CHOLESKY || !has_factor(e)) return PDGB_OK;
     const CholFactor& f = e->chol;
     info->nnz_L = f.nnz_L;
     info->m_entries = m_entries(f);
@@ -1636,7 +1642,7 @@ int pdgb_set_factor_device(pdgb_engine* e, int device) {
 int pdgb_get_factor_blocks(pdgb_engine* e, float* out, long long capacity) {
     if (!e || !out || capacity < 0) return PDGB_ERR_INVALID_ARGUMENT;
     return guarded([&] {
-        if (e->prm.solver != PDGB_SOLVER_CHOLESKY || e->chol.n != e->nv || !e->ch_mval.p)
+        if (e->prm.solver != PDGB_SOLVER_CHOLESKY || !has_factor(e))
             throw Error{PDGB_ERR_INVALID_ARGUMENT, "no prepared Cholesky factor"};
         const CholFactor& f = e->chol;
         if (capacity < m_entries(f)) throw Error{PDGB_ERR_INVALID_ARGUMENT, "capacity below the factor's m_entries"};
