@@ -169,7 +169,7 @@ __device__ __forceinline__ void local_tile(const LocalArgs& a, int tile, float4*
     int e0_first = 0, e1_first = 0;
     for (int k = threadIdx.x; k < np; k += kLocalThreads) {
         const uint32_t v = __ldg(&a.tile_verts[vb + k]);
-        const float4 p = __ldg(&a.sn[v & ~kPinnedBit]);
+        const float4 p = a.sn[v & ~kPinnedBit];  // written while this grid was already resident: no non-coherent load
         const int e0 = k ? __ldg(&iend[k - 1]) : 0;
         pos[k] = make_float4(p.x, p.y, p.z, __int_as_float(e0));
         if (k == (int)threadIdx.x) {
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kLocalThreads, PDGB_LOCAL_MIN_BLOCKS) k_local_
         const uint32_t* tvb = tv + pbuf * tvs + (in.z & 3);
         const uint16_t* ieb = ie + pbuf * ies + (in.z & 7);
         for (int k = tid; k < in.w; k += kLocalThreads) {
-            const float4 p = __ldg(&a.sn[tvb[k] & ~kPinnedBit]);
+            const float4 p = a.sn[tvb[k] & ~kPinnedBit];
             pos[k] = make_float4(p.x, p.y, p.z, __int_as_float(k ? (int)ieb[k - 1] : 0));
         }
     };
