@@ -25,6 +25,7 @@
 
 #include "cholesky.h"
 #include "engine.h"
+#include "panel.h"
 #include "pdl.cuh"
 
 namespace pdgb {
@@ -241,9 +242,9 @@ __device__ __forceinline__ void factor_block(PanelShared& S, int nb, bool& bad) 
         if (threadIdx.x < 32) factor_columns(S, c0, nb, bad);
         else if (c0 > 0) update_inverse(S, c0 - kSub, nb);
         __syncthreads();
-        const int r0 = c0 + kSub, n = nb - r0;
-        for (int e = threadIdx.x; e < n * n; e += kPanelThreads) {
-            const int r = r0 + e / n, c = r0 + e % n;
+        const int r0 = c0 + kSub, entries = trailing_entries(nb, r0);
+        for (int e = threadIdx.x; e < entries; e += kPanelThreads) {
+            const auto [r, c] = trailing_entry(nb, r0, e);
             if (c > r) continue;
             double v = S.D[r][c];
 #pragma unroll
