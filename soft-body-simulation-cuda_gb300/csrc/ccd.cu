@@ -822,10 +822,9 @@ struct CcdContext::Buffers {
     DBuf<int> order;
     DBuf<float4> lo, hi, vf_n, ee_n, nrm;
     DBuf<unsigned int> counters;
-    DBuf<int2> groups, pairs;
+    CcdList groups, pairs;
     DBuf<unsigned long long> vf_best, ee_best, vwin;
     DBuf<float> tI;
-    int group_cap = 0, pair_cap = 0;
     int top = 1, off[kMaxLevels] = {}, cnt[kMaxLevels] = {};
     cudaEvent_t ev[2] = {nullptr, nullptr};
     unsigned int* counts = nullptr;  // pinned copy of the counters
@@ -859,10 +858,10 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     b.counters.alloc(3);
     PDGB_CUDA_TRY(cudaMallocHost(&b.counts, 3 * sizeof(unsigned int)));
     const size_t n = (size_t)std::max(ntris_, 1);
-    b.group_cap = std::max(16 * b.cnt[1], 256);
-    b.groups.alloc(b.group_cap);
-    b.pair_cap = (int)std::min<size_t>(std::max<size_t>(16 * n, 4096), kMostPairs);
-    b.pairs.alloc(b.pair_cap);
+    b.groups.least = std::max(16 * b.cnt[1], 256);
+    b.groups.ensure();
+    b.pairs.least = (int)std::min<size_t>(std::max<size_t>(16 * n, 4096), kMostPairs);
+    b.pairs.ensure();
     b.vf_best.alloc(nv_);
     b.vwin.alloc(nv_);
     b.vf_n.alloc(nv_);
@@ -918,16 +917,18 @@ void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* re
     // The lists grow to the counts found and the detection runs again: the count
     // of pairs is whole once the list of groups is.
     for (int attempt = 0;; ++attempt) {
-        d.groups = b.groups.p;
-        d.pairs = b.pairs.p;
-        d.group_cap = b.group_cap;
-        d.pair_cap = b.pair_cap;
+        b.groups.ensure();
+        b.pairs.ensure();
+        d.groups = b.groups.items.p;
+        d.pairs = b.pairs.items.p;
+        d.group_cap = b.groups.cap;
+        d.pair_cap = b.pairs.cap;
         k_boxes<<<(int)(((long long)most + kBoxThreads - 1) / kBoxThreads), kBoxThreads, 0, s>>>(d);
         if (ntris_ >= 2) {
             for (int l = 3; l <= b.top; ++l) launch_pdl(k_boxes_up, blocks_for(32LL * b.cnt[l]), kThreads, 0, s, d, l);
             launch_pdl(k_groups, blocks_for(32LL * b.cnt[1]), kThreads, 0, s, d);
-            launch_pdl(k_pairs, (int)std::min<long long>(blocks_for(32LL * b.group_cap), kListCtas), kThreads, 0, s, d);
-            launch_pdl(k_narrow, (int)std::min<long long>(blocks_for(24LL * b.pair_cap), kListCtas), kThreads, 0, s, d);
+            launch_pdl(k_pairs, (int)std::min<long long>(blocks_for(32LL * b.groups.cap), kListCtas), kThreads, 0, s, d);
+            launch_pdl(k_narrow, (int)std::min<long long>(blocks_for(24LL * b.pairs.cap), kListCtas), kThreads, 0, s, d);
         }
         launch_pdl(k_mark, outs, kThreads, 0, s, d);
         launch_pdl(k_result, outs, kThreads, 0, s, d);
@@ -938,16 +939,14 @@ void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* re
                        response->sc);
         PDGB_CUDA_TRY(cudaMemcpyAsync(b.counts, b.counters.p, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         PDGB_CUDA_TRY(cudaStreamSynchronize(s));
-        const bool groups = b.counts[1] > (unsigned)b.group_cap, pairs = b.counts[0] > (unsigned)b.pair_cap;
+        const bool groups = b.counts[1] > (unsigned)b.groups.cap, pairs = b.counts[0] > (unsigned)b.pairs.cap;
         if (!groups && !pairs) break;
         if (attempt > 1 || std::max(b.counts[0], b.counts[1]) > kMostPairs)
             throw Error{PDGB_ERR_OUT_OF_MEMORY, "too many collision candidates"};
         if (groups) {
-            b.group_cap = (int)(b.counts[1] + b.counts[1] / 4);
-            b.groups.alloc(b.group_cap);
+            b.groups.grow((long long)b.counts[1] + b.counts[1] / 4);
         } else {
-            b.pair_cap = (int)(b.counts[0] + b.counts[0] / 4);
-            b.pairs.alloc(b.pair_cap);
+            b.pairs.grow((long long)b.counts[0] + b.counts[0] / 4);
             stats_.regrows++;
         }
     }

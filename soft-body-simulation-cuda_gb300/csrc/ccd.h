@@ -33,6 +33,23 @@ struct CcdSurface {
 CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm,
                              const float* X);
 
+// A device list that grows, and the capacity its kernels get: never more than it
+// holds, also after an allocation that failed (which leaves no list).
+struct CcdList {
+    DBuf<int2> items;
+    int cap = 0;
+    int least = 1;  // what it starts with
+
+    void grow(long long count) {
+        cap = 0;
+        items.alloc((size_t)count);
+        cap = (int)count;
+    }
+    void ensure() {
+        if (cap == 0) grow(least);
+    }
+};
+
 struct CcdStats {
     long long pairs = 0;        // candidate triangle pairs of the last detection
     long long sources = 0;      // vertices / edges whose earliest contact is before t = 1

@@ -61,6 +61,7 @@ template <class T> struct DBuf {
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
+            cudaGetLastError();  // reported here: not left for the check of a later launch
             throw Error{PDGB_ERR_OUT_OF_MEMORY, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes failed"};
         }
         n = count;

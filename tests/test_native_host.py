@@ -21,3 +21,9 @@ def test_the_panel_update_stays_in_its_block(tmp_path):
     """Block sizes that leave one to seven columns for the last step of eight."""
     r = _run(tmp_path, "panel_indices")
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout
+
+
+def test_a_collision_list_is_never_longer_than_its_memory(tmp_path):
+    """An allocation that fails while the list grows, then once more."""
+    r = _run(tmp_path, "list_growth")
+    assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
