@@ -11,7 +11,6 @@
 #include <cstring>
 #include <exception>
 #include <numeric>
-#include <system_error>
 #include <thread>
 
 #include "engine.h"
@@ -69,6 +68,7 @@ template <class F> void in_parts(int n, F&& f) {
     }
     std::vector<std::exception_ptr> failed(parts);
     std::vector<std::thread> others;
+    others.reserve(parts - 1);
     auto run = [&](int q) {
         try {
             f((int)((int64_t)n * q / parts), (int)((int64_t)n * (q + 1) / parts));
@@ -79,7 +79,7 @@ template <class F> void in_parts(int n, F&& f) {
     int started = 1;
     try {
         for (; started < parts; ++started) others.emplace_back(run, started);
-    } catch (const std::system_error&) {  // no more threads: the rest here
+    } catch (...) {  // no more threads, or no memory for one: the rest here
     }
     run(0);
     for (int q = started; q < parts; ++q) run(q);

@@ -27,3 +27,9 @@ def test_a_collision_list_is_never_longer_than_its_memory(tmp_path):
     """An allocation that fails while the list grows, then once more."""
     r = _run(tmp_path, "list_growth")
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
+
+
+def test_the_layout_survives_every_failed_allocation(tmp_path):
+    """With threads already running, too."""
+    r = _run(tmp_path, "layout_no_memory", "layout.cpp", link=("-L/usr/local/cuda/lib64", "-lcudart"))
+    assert r.returncode == 0 and r.stdout == "ok 1\n", r.stdout + r.stderr
