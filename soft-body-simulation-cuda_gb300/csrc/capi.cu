@@ -59,7 +59,7 @@ struct pdgb_engine {
     // Cholesky factor
     CholFactor chol;
     int chol_ordering = -1;
-    double chol_level_entries = -1.0;
+    SolveKind chol_kind = SolveKind::kSingle;
     float chol_dt = 0.f, chol_pw = -1.f;
     DBuf<int> ch_fwd, ch_bwd, ch_rows, ch_body_level, ch_body_order, ch_blocks, ch_small, ch_tiny;
     DBuf<float4> y2;  // second y buffer: solves alternate, each clears the other one's
@@ -472,8 +472,8 @@ void prepare_cholesky(pdgb_engine* e) {
     const int dev = e->solve_req == PDGB_SOLVE_DSM ? PDGB_FACTOR_HOST : e->factor_req;
     // ... and its vectors and blocks share a cluster's shared memory: there
     // every stored entry counts and a level is only a cluster barrier
-    const double level_entries = e->solve_req == PDGB_SOLVE_DSM ? kDsmLevelEntries : kLevelEntries;
-    if (has_factor(e) && level_entries == e->chol_level_entries && e->chol_ordering == e->ordering &&
+    const SolveCost price = e->solve_req == PDGB_SOLVE_DSM ? SolveCost{SolveKind::kDsm, kDsmLevelEntries} : SolveCost{};
+    if (has_factor(e) && price.kind == e->chol_kind && e->chol_ordering == e->ordering &&
         e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight && e->factor_dev == dev) {
         e->solve_mode = choose_solve_mode(e);
         return;  // the system matrix depends only on the mesh, dt and the pin weight
@@ -498,7 +498,7 @@ void prepare_cholesky(pdgb_engine* e) {
                                e->L.dminv_d.data(), e->L.coef_d.data(), mdt2, e->ordering, xyz.data(), e->chol,
                                gpu);
     } else {
-        cholesky_factor(K, e->ordering, xyz.data(), e->chol, gpu, true, level_entries);
+        cholesky_factor(K, e->ordering, xyz.data(), e->chol, gpu, true, price);
     }
     cudaStream_t s = e->stream;
     const CholFactor& f = e->chol;
@@ -555,7 +555,7 @@ void prepare_cholesky(pdgb_engine* e) {
             e->dsm_lvl.upload(e->dsm.lvl, s);
         }
     }
-    e->chol_level_entries = level_entries;
+    e->chol_kind = price.kind;
     e->chol_ordering = e->ordering;
     e->chol_dt = e->prm.dt;
     e->chol_pw = e->prm.positional_weight;

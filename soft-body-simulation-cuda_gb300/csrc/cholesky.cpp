@@ -426,12 +426,12 @@ double item_entries(int k, int m) {
 // entries and the one-time factorisation kEntriesPerFlop entries per
 // multiply-add (spread over the solves of about a hundred steps).
 std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& fm, const std::vector<int>& fpar,
-                            double level_entries) {
+                            const SolveCost& price) {
     constexpr double kEntriesPerFlop = 3e-4;
     // bodies that share their launches fill the GPU with items; a single body's
     // levels do not (by items 16^3 takes 468 us a step, by entries 455), and for
     // the DSM solve what counts is what fits
-    const bool by_items = level_entries > kDsmLevelEntries && level_entries < kLevelEntries;
+    const bool by_items = price.kind == SolveKind::kShared;
     const int nf = (int)fk.size();
     std::vector<int> sub(fk);  // columns of the subtree
     int n = 0;
@@ -472,7 +472,7 @@ std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& 
                     h = std::max(h, height[s] + 1);
                 }
             }
-            const double cost = level_entries * levels + entries + kEntriesPerFlop * flops;
+            const double cost = price.level_entries * levels + entries + kEntriesPerFlop * flops;
             if (best < 0.0 || cost < best) {
                 best = cost;
                 best_root.swap(root);
@@ -523,7 +523,7 @@ bool partial_cholesky(double* F, int m, int k) {
 }  // namespace
 
 void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFactor& out,
-                     bool gpu_numeric, bool finish_plan, double level_entries) {
+                     bool gpu_numeric, bool finish_plan, const SolveCost& price) {
     const int n = K.n;
     out = CholFactor();
     out.n = n;
@@ -584,7 +584,7 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
             const int up = parent[sfirst[s + 1] - 1];
             if (up >= 0) fpar[s] = col2f[up];
         }
-        const std::vector<int> root = amalgamate(fk, fm, fpar, level_entries);
+        const std::vector<int> root = amalgamate(fk, fm, fpar, price);
         std::vector<int> start(nf + 1, 0);  // first column of the supernode rooted at s (0 columns elsewhere)
         for (int s = 0; s < nf; ++s) start[root[s] + 1] += fk[s];
         std::vector<int> sf;
@@ -987,7 +987,7 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
             std::vector<double> md(mdt2.begin() + v0, mdt2.begin() + v0 + nvb);
             SparseSym Kb = assemble_system(nvb, ntb, lt.data(), dminv + 9 * (size_t)t0, coef + t0, md);
             cholesky_factor(Kb, ordering, xyz ? xyz + 3 * (size_t)v0 : nullptr, fs[b], gpu_numeric, false,
-                            kLevelEntries * factor_size(nvb) / weight);
+                            SolveCost{SolveKind::kShared, kLevelEntries * factor_size(nvb) / weight});
         } catch (const Error& e) {
             failed[b] = e.status;
         } catch (...) {

@@ -202,17 +202,23 @@ void build_dsm_plan(const CholFactor& f, int ctas, int warps_per_cta, size_t max
 // GPU factorisation (factor.cu) instead of computing mval on the host;
 // finish_plan: complete it (finish_front_plan) -- a batch completes the
 // combined plan of its bodies instead.
-// level_entries: what a level of the solve costs, in stored entries, when
-// supernodes are amalgamated.  kLevelEntries is a single body's: about 6 us
-// of dependent launches a level, forward and backward, against 8 bytes an
-// entry at some 5 TB/s.  Bodies that share their launches pay a share:
-// batches by size, requests of a server 1 / kServerBodies.
+// price: how supernodes are amalgamated.  A level of the solve costs
+// level_entries stored entries: kLevelEntries for a single body, about 6 us of
+// dependent launches a level, forward and backward, against 8 bytes an entry at
+// some 5 TB/s.  Bodies that share their launches pay a share, batches by size,
+// requests of a server 1 / kServerBodies, and count items instead of entries,
+// however small the share.  In the DSM solve a level is a cluster barrier and
+// every stored entry takes shared memory.
+enum class SolveKind { kSingle, kShared, kDsm };
 constexpr double kLevelEntries = 3.75e6;
 constexpr double kServerBodies = 16.0;
 constexpr double kDsmLevelEntries = 1e3;
+struct SolveCost {
+    SolveKind kind = SolveKind::kSingle;
+    double level_entries = kLevelEntries;
+};
 void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFactor& out,
-                     bool gpu_numeric = false, bool finish_plan = true,
-                     double level_entries = kLevelEntries);
+                     bool gpu_numeric = false, bool finish_plan = true, const SolveCost& price = SolveCost{});
 
 // Factors the block-diagonal system of independent bodies, one block per
 // body (vertex range vstart[b]..vstart[b+1], tets tstart[b]..tstart[b+1] in

@@ -471,7 +471,7 @@ void worker_loop(pdgb_server* S) {
                     auto f = std::make_shared<CholFactor>();
                     const std::vector<float> xyz = layout_xyz(*L);
                     cholesky_factor(layout_system(*L), PDGB_ORDER_AMD, xyz.data(), *f, true, true,
-                                    kLevelEntries / kServerBodies);
+                                    SolveCost{SolveKind::kShared, kLevelEntries / kServerBodies});
                     f->K = SparseSym();  // no refinement residuals in the server
                     me->f = f;
                 }
