@@ -467,12 +467,19 @@ int choose_solve_mode(const pdgb_engine* e) {
     return m == PDGB_SOLVE_AUTO ? PDGB_SOLVE_LEVELS : m;
 }
 
+// How the requested schedule's factor is amalgamated.
+SolveCost solve_cost(const pdgb_engine* e) {
+    switch (e->solve_req) {
+        case PDGB_SOLVE_CTA: return {SolveKind::kCta, kCtaLevelEntries};
+        case PDGB_SOLVE_DSM: return {SolveKind::kDsm, kDsmLevelEntries};
+        default: return {e->nbodies > 1 ? SolveKind::kShared : SolveKind::kSingle, kLevelEntries};
+    }
+}
+
 void prepare_cholesky(pdgb_engine* e) {
     // the distributed-shared-memory solve stages the factor from host memory
     const int dev = e->solve_req == PDGB_SOLVE_DSM ? PDGB_FACTOR_HOST : e->factor_req;
-    // ... and its vectors and blocks share a cluster's shared memory: there
-    // every stored entry counts and a level is only a cluster barrier
-    const SolveCost price = e->solve_req == PDGB_SOLVE_DSM ? SolveCost{SolveKind::kDsm, kDsmLevelEntries} : SolveCost{};
+    const SolveCost price = solve_cost(e);
     if (has_factor(e) && price.kind == e->chol_kind && e->chol_ordering == e->ordering &&
         e->chol_dt == e->prm.dt && e->chol_pw == e->prm.positional_weight && e->factor_dev == dev) {
         e->solve_mode = choose_solve_mode(e);
@@ -496,7 +503,7 @@ void prepare_cholesky(pdgb_engine* e) {
         for (int i = 0; i < e->nv; ++i) mdt2[i] = (double)e->L.coef[i].x;
         cholesky_factor_bodies(e->nbodies, e->L.body_ivstart, e->L.body_itstart, e->L.tets_int.data(),
                                e->L.dminv_d.data(), e->L.coef_d.data(), mdt2, e->ordering, xyz.data(), e->chol,
-                               gpu);
+                               gpu, price);
     } else {
         cholesky_factor(K, e->ordering, xyz.data(), e->chol, gpu, true, price);
     }
@@ -506,7 +513,7 @@ void prepare_cholesky(pdgb_engine* e) {
     e->pool_bytes = 0;
     if (gpu) {
         // FP64 numeric factorisation on the GPU, straight into the M_s blocks
-        if (e->nbodies == 1) plan_root_inverse(e->chol);
+        if (price.kind == SolveKind::kSingle) plan_root_inverse(e->chol);
         if (f.root >= 0) e->b2.alloc(e->nv);
         e->ch_mval.alloc((size_t)std::max<int64_t>(f.mval_total, 1));
         e->numeric_ms = gpu_factor(f, e->ch_mval.p, s);
@@ -1011,13 +1018,13 @@ int pdgb_autotune(pdgb_engine* e, int steps, pdgb_tune_report* rep) {
                 e->ordering = ord;
                 e->prepared = false;
             }
-            for (int cap : caps)
-                for (int mode : modes) {
+            for (int mode : modes) {  // outside the tiles: the CTA solve has a factor of its own
+                if (mode != e->solve_req) {
+                    e->solve_req = mode;
+                    e->prepared = false;
+                }
+                for (int cap : caps) {
                     set_tile_cap(e, cap);
-                    if (mode != e->solve_req) {
-                        e->solve_req = mode;
-                        e->prepared = false;
-                    }
                     const double t = time_steps(e, steps);
                     copy_state(true);
                     ++tried;
@@ -1028,6 +1035,7 @@ int pdgb_autotune(pdgb_engine* e, int steps, pdgb_tune_report* rep) {
                         best_ord = ord;
                     }
                 }
+            }
         }
         // the pipelined local step at the chosen configuration (and at its
         // natural 512-tet tiles)

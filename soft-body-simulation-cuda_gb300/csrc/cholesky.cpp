@@ -964,7 +964,7 @@ void finish_front_plan(CholFactor& out) {
 void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const std::vector<int>& tstart,
                             const uint32_t* tets4, const double* dminv, const double* coef,
                             const std::vector<double>& mdt2, int ordering, const float* xyz, CholFactor& out,
-                            bool gpu_numeric) {
+                            bool gpu_numeric, const SolveCost& price) {
     std::vector<CholFactor> fs(nbodies);
     std::vector<int> order(nbodies);
     std::iota(order.begin(), order.end(), 0);
@@ -972,8 +972,8 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
         return tstart[a + 1] - tstart[a] > tstart[b + 1] - tstart[b];
     });
     std::vector<int> failed(nbodies, 0);
-    // a level is one chain of launches for all bodies: each pays a share of
-    // it, by its expected factor size
+    // kShared: a level is one chain of launches for all bodies, and each pays a
+    // share of it, by its expected factor size
     double weight = 0.0;
     auto factor_size = [](int nv) { return std::pow((double)nv, 1.58); };
     for (int b = 0; b < nbodies; ++b) weight += factor_size(vstart[b + 1] - vstart[b]);
@@ -986,8 +986,9 @@ void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const s
             for (size_t i = 0; i < lt.size(); ++i) lt[i] = tets4[4 * (size_t)t0 + i] - (uint32_t)v0;
             std::vector<double> md(mdt2.begin() + v0, mdt2.begin() + v0 + nvb);
             SparseSym Kb = assemble_system(nvb, ntb, lt.data(), dminv + 9 * (size_t)t0, coef + t0, md);
-            cholesky_factor(Kb, ordering, xyz ? xyz + 3 * (size_t)v0 : nullptr, fs[b], gpu_numeric, false,
-                            SolveCost{SolveKind::kShared, kLevelEntries * factor_size(nvb) / weight});
+            SolveCost own = price;
+            if (price.kind == SolveKind::kShared) own.level_entries *= factor_size(nvb) / weight;
+            cholesky_factor(Kb, ordering, xyz ? xyz + 3 * (size_t)v0 : nullptr, fs[b], gpu_numeric, false, own);
         } catch (const Error& e) {
             failed[b] = e.status;
         } catch (...) {

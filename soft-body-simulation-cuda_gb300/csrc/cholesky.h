@@ -202,16 +202,24 @@ void build_dsm_plan(const CholFactor& f, int ctas, int warps_per_cta, size_t max
 // GPU factorisation (factor.cu) instead of computing mval on the host;
 // finish_plan: complete it (finish_front_plan) -- a batch completes the
 // combined plan of its bodies instead.
-// price: how supernodes are amalgamated.  A level of the solve costs
-// level_entries stored entries: kLevelEntries for a single body, about 6 us of
-// dependent launches a level, forward and backward, against 8 bytes an entry at
-// some 5 TB/s.  Bodies that share their launches pay a share, batches by size,
-// requests of a server 1 / kServerBodies, and count items instead of entries,
-// however small the share.  In the DSM solve a level is a cluster barrier and
-// every stored entry takes shared memory.
-enum class SolveKind { kSingle, kShared, kDsm };
+// price: how supernodes are amalgamated for a schedule, a level of the solve
+// against stored entries (SolveCost).
+enum class SolveKind {
+    kSingle,  // one body: a launch, a grid's or a cluster's barrier a level
+    kShared,  // bodies that share their launches: they count items instead of
+              // entries, however small their share of a level
+    kCta,     // one CTA a body: a level is a CTA's barrier
+    kDsm,     // one cluster, and every stored entry takes its shared memory
+};
+// Entries that a level costs.  Launches: about 6 us of dependent ones, forward and
+// backward, against 8 bytes an entry at some 5 TB/s.  Batches pay it by size,
+// requests of a server 1 / kServerBodies.  For one CTA a barrier is less and an
+// entry more: ten iterations of a 13^3 body, of a 60 x 6 x 3 one and of 16 of 2^3
+// beside 32 of 10^3 take 1,715, 1,044 and 1,096 us at 1e4 and 2,297, 1,179 and
+// 1,202 with the tree for launches.
 constexpr double kLevelEntries = 3.75e6;
 constexpr double kServerBodies = 16.0;
+constexpr double kCtaLevelEntries = 1e4;
 constexpr double kDsmLevelEntries = 1e3;
 struct SolveCost {
     SolveKind kind = SolveKind::kSingle;
@@ -224,11 +232,11 @@ void cholesky_factor(const SparseSym& K, int ordering, const float* xyz, CholFac
 // body (vertex range vstart[b]..vstart[b+1], tets tstart[b]..tstart[b+1] in
 // the engine's order), in parallel over bodies, and concatenates the
 // factors: rows keep engine vertex ids, work items and levels are grouped
-// per body.
+// per body.  price: a body's, or with kShared what the level costs all of them.
 void cholesky_factor_bodies(int nbodies, const std::vector<int>& vstart, const std::vector<int>& tstart,
                             const uint32_t* tets4, const double* dminv, const double* coef,
                             const std::vector<double>& mdt2, int ordering, const float* xyz, CholFactor& out,
-                            bool gpu_numeric = false);
+                            bool gpu_numeric, const SolveCost& price);
 
 // Doubles of the pool that supernode s takes: its front and its M_s block.
 int64_t front_doubles(const CholFactor& f, int s);

@@ -786,8 +786,13 @@ void launch_grid_sync_check(GridSync* bar, int ctas, int rounds, int missing, lo
 // ---- one body per CTA: warps stride over the items of a level,
 // __syncthreads between levels (global writes of the block become visible
 // to the whole block at the barrier).  Bodies are independent, so CTAs
-// never wait on each other.
-__global__ void __launch_bounds__(kCtaSolveThreads) k_chol_solve_cta(CholArgs a) {
+// never wait on each other.  What bounds a body is the chain of its items: a batch
+// has two bodies an SM (32 registers and a few spilled; 4,096 of 4^3 take 3.7 ms a
+// step of ten iterations, 9.5 with one), a single body all the registers that the
+// eight entries a lane has on the way want (58; with the 46 that the compiler
+// stopped at, 10^3 took 982 us instead of 802).
+template <int kPerSm>
+__global__ void __launch_bounds__(kCtaSolveThreads, kPerSm) k_chol_solve_cta(CholArgs a) {
     __shared__ float4 stage[kCtaSolveThreads / 32][32];
     if (a.done && *a.done) return;
     constexpr int kWarps = kCtaSolveThreads / 32;
@@ -809,7 +814,8 @@ __global__ void __launch_bounds__(kCtaSolveThreads) k_chol_solve_cta(CholArgs a)
 }
 
 void launch_chol_solve_cta(const CholArgs& a, int nbodies, cudaStream_t s) {
-    if (nbodies > 0) k_chol_solve_cta<<<nbodies, kCtaSolveThreads, 0, s>>>(a);
+    if (nbodies == 1) k_chol_solve_cta<1><<<1, kCtaSolveThreads, 0, s>>>(a);
+    else if (nbodies > 1) k_chol_solve_cta<2><<<nbodies, kCtaSolveThreads, 0, s>>>(a);
 }
 
 // ---- one body per thread-block cluster: the cluster's warps stride over
@@ -818,7 +824,11 @@ void launch_chol_solve_cta(const CholArgs& a, int nbodies, cudaStream_t s) {
 // the level's global writes and atomics of every CTA of the cluster visible
 // to all of them.  All CTAs of a cluster run the same level loops, so every
 // thread arrives at every barrier; the hardware co-schedules the cluster.
-__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterSolveThreads)
+// Without a bound on the CTAs an SM the compiler keeps to 40 registers, too few
+// for the eight entries a lane has on the way: with two an SM (58 registers) a
+// 16^3, a 28^3 and a dense 10^3 body take 1,272, 7,265 and 565 us a step instead
+// of 1,645, 9,300 and 726.
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterSolveThreads, 2)
     k_chol_solve_cluster(CholArgs a) {
     __shared__ float4 stage[kClusterSolveThreads / 32][32];
     if (a.done && *a.done) return;  // the flag is fixed for the kernel: uniform over the cluster
