@@ -1394,7 +1394,7 @@ int pdgb_ccd_detect(int num_verts, int num_tris, const uint32_t* tris, const int
         }
         DBuf<float4> d;
         d.upload(h, nullptr);
-        CcdContext ctx(surf, nullptr, nullptr);
+        CcdContext ctx(surf, nullptr, nullptr, true);
         ctx.detect(d.p, d.p + nv);
         std::vector<float4> n(nv);
         PDGB_CUDA_TRY(cudaMemcpyAsync(tI, ctx.tI(), nv * sizeof(float), cudaMemcpyDeviceToHost, nullptr));

@@ -734,35 +734,62 @@ __global__ void __launch_bounds__(kThreads) k_respond(Dev det, int nv, const flo
 
 // ------------------------------------------------------------ host side
 namespace {
-// Tree order of the triangles: by body, a body's along the Morton curve of its
-// own box (10 bits an axis) at the positions X.
+struct Extent {
+    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+
+    void add(const float* c) {
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = std::min(lo[k], c[k]);  // NaN: left out
+            hi[k] = std::max(hi[k], c[k]);
+        }
+    }
+};
+
+// Bits 0 .. 9 of x spread to every third bit.
+uint64_t spread3(uint64_t x) {
+    x = (x | x << 16) & 0x030000FF;
+    x = (x | x << 8) & 0x0300F00F;
+    x = (x | x << 4) & 0x030C30C3;
+    return (x | x << 2) & 0x09249249;
+}
+
+// Tree order of the triangles at the positions X: by body, a body's along the
+// Morton curve of its own box (10 bits an axis).
 void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const float* X, std::vector<int>& order) {
     std::vector<KeyId> key(ntris), tmp;
-    for (int t = 0; t < ntris; ++t) key[t] = {(uint64_t)(uint32_t)tri_body[t], t};
-    radix_sort(key, tmp);
-    auto centre = [&](int t, int k) {
+    std::vector<float> centre(3 * (size_t)ntris);
+    for (int t = 0; t < ntris; ++t) {
         const uint32_t* v = tris + 3 * (size_t)t;
-        return X[3 * (size_t)v[0] + k] + X[3 * (size_t)v[1] + k] + X[3 * (size_t)v[2] + k];
-    };
-    for (int b = 0, end = 0; b < ntris; b = end) {
-        const uint64_t body = key[b].key;
-        float lo[3], hi[3];
-        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = centre(key[b].id, k);
-        for (end = b; end < ntris && key[end].key == body; ++end)
-            for (int k = 0; k < 3; ++k) {
-                const float c = centre(key[end].id, k);
-                lo[k] = std::min(lo[k], c);
-                hi[k] = std::max(hi[k], c);
-            }
-        for (int q = b; q < end; ++q) {
+        float* c = &centre[3 * (size_t)t];
+        for (int k = 0; k < 3; ++k) c[k] = X[3 * (size_t)v[0] + k] + X[3 * (size_t)v[1] + k] + X[3 * (size_t)v[2] + k];
+        key[t] = {(uint64_t)(uint32_t)tri_body[t], t};
+    }
+    radix_sort(key, tmp);
+    std::vector<int> start;  // first triangle of each body
+    std::vector<Extent> box;
+    for (int q = 0; q < ntris; ++q) {
+        if (q == 0 || key[q].key != key[q - 1].key) {
+            start.push_back(q);
+            box.emplace_back();
+        }
+        box.back().add(&centre[3 * (size_t)key[q].id]);
+    }
+    start.push_back(ntris);
+    for (size_t b = 0; b < box.size(); ++b) {
+        const Extent& e = box[b];
+        float scale[3];
+        for (int k = 0; k < 3; ++k) {
+            const float ext = e.hi[k] - e.lo[k];
+            scale[k] = ext > 0.f ? 1024.f / ext : 0.f;
+        }
+        for (int q = start[b]; q < start[b + 1]; ++q) {
+            const float* c = &centre[3 * (size_t)key[q].id];
             uint64_t m = 0;
             for (int k = 0; k < 3; ++k) {
-                const float ext = hi[k] - lo[k];
-                const float u = ext > 0.f ? (centre(key[q].id, k) - lo[k]) / ext : 0.f;
-                const uint64_t c = u > 0.f ? (uint64_t)std::min(u * 1024.f, 1023.f) : 0;  // NaN: 0
-                for (int bit = 0; bit < 10; ++bit) m |= (c >> bit & 1) << (3 * bit + 2 - k);
+                const float u = (c[k] - e.lo[k]) * scale[k];
+                m |= spread3(u > 0.f ? (uint64_t)std::min(u, 1023.f) : 0) << (2 - k);  // NaN: 0
             }
-            key[q].key = body << 30 | m;
+            key[q].key = key[q].key << 30 | m;
         }
     }
     radix_sort(key, tmp);
@@ -779,39 +806,41 @@ CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int*
     s.nv = nv;
     s.ntris = ntris;
     auto iv = [&](uint32_t c) { return viperm ? (uint32_t)viperm[c] : c; };
-    std::vector<std::pair<uint32_t, uint32_t>> edges;  // caller ids, ascending
-    edges.reserve(3 * (size_t)ntris);
+    // edges by caller ids (smaller, larger), in ascending order: the sides of all
+    // triangles sorted, equal ones one edge
+    auto side_key = [&](int t, int k) {  // side 0-1, 0-2 or 1-2
+        const uint32_t a = tris[3 * (size_t)t + (k == 2)], b = tris[3 * (size_t)t + (k == 0 ? 1 : 2)];
+        return (uint64_t)std::min(a, b) << 32 | std::max(a, b);
+    };
+    std::vector<KeyId> side, tmp;
+    side.reserve(3 * (size_t)ntris);
+    s.tri.resize(ntris);
+    s.tri_edges.resize(ntris);
     for (int t = 0; t < ntris; ++t) {
         uint32_t c[3] = {tris[3 * (size_t)t], tris[3 * (size_t)t + 1], tris[3 * (size_t)t + 2]};
         for (uint32_t v : c)
             if (v >= (uint32_t)nv)
                 throw Error{PDGB_ERR_BAD_MESH, "collision triangle " + std::to_string(t) + " references vertex " +
                                                    std::to_string(v) + " >= num_verts"};
-        for (int k = 0; k < 3; ++k) {
-            uint32_t a = c[k], b = c[(k + 1) % 3];
-            if (a > b) std::swap(a, b);
-            edges.push_back({a, b});
-        }
-    }
-    std::sort(edges.begin(), edges.end());
-    edges.erase(std::unique(edges.begin(), edges.end()), edges.end());
-    if (edges.size() + (size_t)nv >= 0xffffffffull || ntris > 0x7fffffff)
-        throw Error{PDGB_ERR_UNSUPPORTED, "collision surface too large"};
-    auto edge_id = [&](uint32_t a, uint32_t b) {
-        if (a > b) std::swap(a, b);
-        return (uint32_t)(std::lower_bound(edges.begin(), edges.end(), std::make_pair(a, b)) - edges.begin());
-    };
-    s.nedges = (int)edges.size();
-    s.tri.resize(ntris);
-    s.tri_edges.resize(ntris);
-    for (int t = 0; t < ntris; ++t) {
-        uint32_t c[3] = {tris[3 * (size_t)t], tris[3 * (size_t)t + 1], tris[3 * (size_t)t + 2]};
-        s.tri_edges[t] = make_uint4(edge_id(c[0], c[1]), edge_id(c[0], c[2]), edge_id(c[1], c[2]), 0u);
+        for (int k = 0; k < 3; ++k) side.push_back({side_key(t, k), t});
         std::sort(c, c + 3);
         s.tri[t] = make_uint4(iv(c[0]), iv(c[1]), iv(c[2]), (uint32_t)tri_body[t]);
+        s.tri_edges[t].w = 0u;
     }
-    s.edges.resize(edges.size());
-    for (size_t e = 0; e < edges.size(); ++e) s.edges[e] = make_uint2(iv(edges[e].first), iv(edges[e].second));
+    radix_sort(side, tmp);
+    for (size_t q = 0; q < side.size(); ++q) {
+        const uint64_t key = side[q].key;
+        if (q == 0 || key != side[q - 1].key)
+            s.edges.push_back(make_uint2(iv((uint32_t)(key >> 32)), iv((uint32_t)(key & 0xffffffffu))));
+        const uint32_t id = (uint32_t)(s.edges.size() - 1);
+        uint4& e = s.tri_edges[side[q].id];
+        if (side_key(side[q].id, 0) == key) e.x = id;
+        if (side_key(side[q].id, 1) == key) e.y = id;
+        if (side_key(side[q].id, 2) == key) e.z = id;
+    }
+    if (s.edges.size() + (size_t)nv >= 0xffffffffull)
+        throw Error{PDGB_ERR_UNSUPPORTED, "collision surface too large"};
+    s.nedges = (int)s.edges.size();
     tree_order(ntris, tris, tri_body, X, s.order);
     return s;
 }
@@ -827,15 +856,17 @@ struct CcdContext::Buffers {
     DBuf<float> tI;
     int top = 1, off[kMaxLevels] = {}, cnt[kMaxLevels] = {};
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    unsigned int* counts = nullptr;  // pinned copy of the counters
+    // copy of the counters; page-locking a buffer takes 150 us, the copy to one that
+    // is not a few
+    unsigned int *counts = nullptr, *pinned = nullptr, pageable[3] = {};
     ~Buffers() {
         if (ev[0]) cudaEventDestroy(ev[0]);
         if (ev[1]) cudaEventDestroy(ev[1]);
-        if (counts) cudaFreeHost(counts);
+        if (pinned) cudaFreeHost(pinned);
     }
 };
 
-CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t stream)
+CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t stream, bool once)
     : b_(new Buffers), nv_(s.nv), ntris_(s.ntris), nedges_(s.nedges), vcaller_(vcaller), stream_(stream) {
     Buffers& b = *b_;
     b.tri.upload(s.tri, stream);
@@ -856,7 +887,8 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     b.lo.alloc(std::max<size_t>(nodes, 1));
     b.hi.alloc(std::max<size_t>(nodes, 1));
     b.counters.alloc(3);
-    PDGB_CUDA_TRY(cudaMallocHost(&b.counts, 3 * sizeof(unsigned int)));
+    if (!once) PDGB_CUDA_TRY(cudaMallocHost(&b.pinned, 3 * sizeof(unsigned int)));
+    b.counts = b.pinned ? b.pinned : b.pageable;
     const size_t n = (size_t)std::max(ntris_, 1);
     b.groups.least = std::max(16 * b.cnt[1], 256);
     b.groups.ensure();

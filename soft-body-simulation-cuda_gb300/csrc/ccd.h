@@ -69,8 +69,8 @@ struct CcdResponse {
 class CcdContext {
 public:
     // vcaller: device array internal -> caller vertex id (null: identity),
-    // kept by the caller for the context's lifetime.
-    CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t stream);
+    // kept by the caller for the context's lifetime.  once: for one detection.
+    CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t stream, bool once = false);
     ~CcdContext();
     CcdContext(const CcdContext&) = delete;
     CcdContext& operator=(const CcdContext&) = delete;
