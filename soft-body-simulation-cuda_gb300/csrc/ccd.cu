@@ -743,6 +743,12 @@ struct Extent {
             hi[k] = std::max(hi[k], c[k]);
         }
     }
+    // Volume with every side at least 1/100 of `side`, so that flat ones count.
+    double volume(double side) const {
+        double v = 1.0;
+        for (int k = 0; k < 3; ++k) v *= std::max((double)hi[k] - lo[k], 0.01 * side);
+        return v;
+    }
 };
 
 // Bits 0 .. 9 of x spread to every third bit.
@@ -753,18 +759,27 @@ uint64_t spread3(uint64_t x) {
     return (x | x << 2) & 0x09249249;
 }
 
-// Tree order of the triangles at the positions X: by body, a body's along the
-// Morton curve of its own box (10 bits an axis).
+// Tree order of the triangles at the positions X (10 bits of a Morton code an
+// axis): by body, a body's along the curve of its own box, which stays as good
+// as it is however the bodies move.  Where they are mixed in space -- their boxes
+// together more than four times the scene's -- a body's neighbours on its curve
+// are far apart, and all triangles follow one curve: 33,000 triangles of 300
+// bodies spread over one box take 650 us a detection by body, 200,000 of 40
+// bodies 1,990 us (MIXED and MIXED this way).
 void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const float* X, std::vector<int>& order) {
     std::vector<KeyId> key(ntris), tmp;
     std::vector<float> centre(3 * (size_t)ntris);
+    Extent scene;
     for (int t = 0; t < ntris; ++t) {
         const uint32_t* v = tris + 3 * (size_t)t;
         float* c = &centre[3 * (size_t)t];
         for (int k = 0; k < 3; ++k) c[k] = X[3 * (size_t)v[0] + k] + X[3 * (size_t)v[1] + k] + X[3 * (size_t)v[2] + k];
+        scene.add(c);
         key[t] = {(uint64_t)(uint32_t)tri_body[t], t};
     }
     radix_sort(key, tmp);
+    double side = 0.0, bodies = 0.0;
+    for (int k = 0; k < 3; ++k) side = std::max(side, (double)scene.hi[k] - scene.lo[k]);
     std::vector<int> start;  // first triangle of each body
     std::vector<Extent> box;
     for (int q = 0; q < ntris; ++q) {
@@ -775,8 +790,10 @@ void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const floa
         box.back().add(&centre[3 * (size_t)key[q].id]);
     }
     start.push_back(ntris);
+    for (const Extent& b : box) bodies += b.volume(side);
+    const bool mixed = bodies > 4.0 * scene.volume(side);  // not finite: false
     for (size_t b = 0; b < box.size(); ++b) {
-        const Extent& e = box[b];
+        const Extent& e = mixed ? scene : box[b];
         float scale[3];
         for (int k = 0; k < 3; ++k) {
             const float ext = e.hi[k] - e.lo[k];
@@ -789,7 +806,7 @@ void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const floa
                 const float u = (c[k] - e.lo[k]) * scale[k];
                 m |= spread3(u > 0.f ? (uint64_t)std::min(u, 1023.f) : 0) << (2 - k);  // NaN: 0
             }
-            key[q].key = key[q].key << 30 | m;
+            key[q].key = mixed ? m : (key[q].key << 30 | m);
         }
     }
     radix_sort(key, tmp);
