@@ -1321,8 +1321,10 @@ int pdgb_set_collision_surface(pdgb_engine* e, const uint32_t* tris, const int* 
                                     e->body_vstart.begin()) - 1;
             }
         }
-        const CcdSurface surf = build_ccd_surface(e->nv, num_tris, tris, body.data(), e->L.viperm.data(), e->X0.data());
+        std::vector<float4> x(e->nv);  // as it is now
+        PDGB_CUDA_TRY(cudaMemcpyAsync(x.data(), e->x.p, x.size() * sizeof(float4), cudaMemcpyDeviceToHost, e->stream));
         PDGB_CUDA_TRY(cudaStreamSynchronize(e->stream));
+        const CcdSurface surf = build_ccd_surface(e->nv, num_tris, tris, body.data(), e->L.viperm.data(), x.data(), false);
         e->ccd.reset(new CcdContext(surf, e->vperm.p, e->stream));
     });
 }
@@ -1386,12 +1388,12 @@ int pdgb_ccd_detect(int num_verts, int num_tris, const uint32_t* tris, const int
         const size_t nv = num_verts;
         for (size_t i = 0; i < 3 * nv; ++i)
             if (!std::isfinite(X[i]) || !std::isfinite(XT[i])) throw Error{PDGB_ERR_NONFINITE, "non-finite position"};
-        const CcdSurface surf = build_ccd_surface(num_verts, num_tris, tris, tri_body, nullptr, X);
         std::vector<float4> h(2 * nv);
         for (size_t i = 0; i < nv; ++i) {
             h[i] = make_float4(X[3 * i], X[3 * i + 1], X[3 * i + 2], 0.f);
             h[nv + i] = make_float4(XT[3 * i], XT[3 * i + 1], XT[3 * i + 2], 0.f);
         }
+        const CcdSurface surf = build_ccd_surface(num_verts, num_tris, tris, tri_body, nullptr, h.data(), true);
         DBuf<float4> d;
         d.upload(h, nullptr);
         CcdContext ctx(surf, nullptr, nullptr, true);

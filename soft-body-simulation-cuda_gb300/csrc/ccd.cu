@@ -52,6 +52,7 @@ constexpr unsigned int kMostPairs = 1u << 30;
 // SM, the fewest that their registers allow.
 constexpr int kListCtas = 4 * 152;
 constexpr int kMaxLevels = 7;      // 32^7 > 2^31 triangles
+constexpr int kCounters = 4;
 
 inline int blocks_for(long long n) { return (int)((n + kThreads - 1) / kThreads); }
 
@@ -337,7 +338,7 @@ struct Dev {
     int2* groups;  // overlapping pairs of level-1 nodes
     int2* pairs;   // candidate triangles
     int group_cap, pair_cap;
-    unsigned int* counters;       // [0] pairs found, [1] group pairs found, [2] marked vertices
+    unsigned int* counters;       // [0] pairs found, [1] group pairs found, [2] marked vertices, [3] steps down the tree
     unsigned long long* vf_best;  // [nv]
     unsigned long long* ee_best;  // [nedges]
     unsigned long long* vwin;     // [nv]
@@ -382,7 +383,7 @@ __device__ __forceinline__ bool one_body(const Box& a, const Box& b) {
 __global__ void __launch_bounds__(kBoxThreads) k_boxes(Dev d) {
     __shared__ Box sub_box[32];
     const int p = blockIdx.x * kBoxThreads + threadIdx.x;
-    if (p < 3) d.counters[p] = 0;
+    if (p < kCounters) d.counters[p] = 0;
     if (p < d.nv) {
         d.vf_best[p] = kNone;
         d.vwin[p] = kNone;
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kThreads) k_groups(Dev d) {
     if (g >= d.cnt[1]) return;
     const Box own = {d.lo[d.off[1] + g], d.hi[d.off[1] + g]};
     int l = d.top, at = 0;
-    for (;;) {
+    for (unsigned int steps = 1;; ++steps) {
         const int c = at + lane;
         bool hit = false;
         // the last group below node c: ((c + 1) 32^(l-1)) - 1
@@ -478,7 +479,10 @@ __global__ void __launch_bounds__(kThreads) k_groups(Dev d) {
         }
         // the next node to go into: here, or the nearest level above that has one
         while (m == 0) {
-            if (++l > d.top) return;
+            if (++l > d.top) {
+                if (lane == 0) atomicAdd(&d.counters[3], steps);
+                return;
+            }
             m = todo[warp][l];
             at = first[warp][l];
         }
@@ -768,7 +772,7 @@ struct Extent {
     }
 };
 
-// Tree order of the triangles at the positions X: body after body along the
+// Tree order of the triangles at the positions x: body after body along the
 // Morton curve of the scene, a body's triangles along that of its own box, which
 // stays as good as it is however the body moves.  (In the order of their numbers,
 // 10,000 scattered bodies of 2^3 cells took 6.8 ms a detection and 40,000 of one
@@ -776,17 +780,22 @@ struct Extent {
 // Where bodies are mixed in space -- their boxes together more than four times the
 // scene's -- a body's neighbours on its curve are far apart, and all triangles
 // follow one curve: 33,000 triangles of 300 bodies spread over one box take 650 us
-// a detection by body and 180 this way, 200,000 of 40 bodies 1,990 and 490.
-void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const float* X, std::vector<int>& order) {
+// a detection by body and 180 this way, 200,000 of 40 bodies 1,990 and 490.  Only
+// for positions that are now: bodies may all have one place when the surface is
+// set and be put into theirs later, and then this order is the worst.
+void tree_order(const std::vector<uint4>& tri, const float4* x, bool now, std::vector<int>& order) {
+    const int ntris = (int)tri.size();
     std::vector<KeyId> key(ntris), tmp;
     std::vector<float> centre(3 * (size_t)ntris);
     Extent scene;
     for (int t = 0; t < ntris; ++t) {
-        const uint32_t* v = tris + 3 * (size_t)t;
+        const float4 p = x[tri[t].x], q = x[tri[t].y], r = x[tri[t].z];
         float* c = &centre[3 * (size_t)t];
-        for (int k = 0; k < 3; ++k) c[k] = X[3 * (size_t)v[0] + k] + X[3 * (size_t)v[1] + k] + X[3 * (size_t)v[2] + k];
+        c[0] = p.x + q.x + r.x;
+        c[1] = p.y + q.y + r.y;
+        c[2] = p.z + q.z + r.z;
         scene.add(c);
-        key[t] = {(uint64_t)(uint32_t)tri_body[t], t};
+        key[t] = {(uint64_t)tri[t].w, t};
     }
     radix_sort(key, tmp);
     double side = 0.0, bodies = 0.0;
@@ -802,7 +811,7 @@ void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const floa
     }
     start.push_back(ntris);
     for (const Extent& b : box) bodies += b.volume(side);
-    const bool mixed = bodies > 4.0 * scene.volume(side);  // not finite: false
+    const bool mixed = now && bodies > 4.0 * scene.volume(side);  // not finite: false
     std::vector<KeyId> along(box.size());  // bodies along the scene's curve
     for (size_t b = 0; b < box.size(); ++b) {
         float mid[3];
@@ -824,7 +833,7 @@ void tree_order(int ntris, const uint32_t* tris, const int* tri_body, const floa
 }  // namespace
 
 CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm,
-                             const float* X) {
+                             const float4* x, bool now) {
     if (nv <= 0 || ntris < 0 || (ntris > 0 && (!tris || !tri_body)))
         throw Error{PDGB_ERR_INVALID_ARGUMENT, "collision surface: bad sizes or null arrays"};
     CcdSurface s;
@@ -866,7 +875,7 @@ CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int*
     if (s.edges.size() + (size_t)nv >= 0xffffffffull)
         throw Error{PDGB_ERR_UNSUPPORTED, "collision surface too large"};
     s.nedges = (int)s.edges.size();
-    tree_order(ntris, tris, tri_body, X, s.order);
+    tree_order(s.tri, x, now, s.order);
     return s;
 }
 
@@ -880,10 +889,15 @@ struct CcdContext::Buffers {
     DBuf<unsigned long long> vf_best, ee_best, vwin;
     DBuf<float> tI;
     int top = 1, off[kMaxLevels] = {}, cnt[kMaxLevels] = {};
+    std::vector<uint4> host_tri;  // for the next order
+    // work of the first detection after the order was made (< 0: not known yet; 0: it
+    // was made for positions that may have changed since), and detections since
+    double base = 0.0;
+    int age = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     // copy of the counters; page-locking a buffer takes 150 us, the copy to one that
     // is not a few
-    unsigned int *counts = nullptr, *pinned = nullptr, pageable[3] = {};
+    unsigned int *counts = nullptr, *pinned = nullptr, pageable[kCounters] = {};
     ~Buffers() {
         if (ev[0]) cudaEventDestroy(ev[0]);
         if (ev[1]) cudaEventDestroy(ev[1]);
@@ -897,10 +911,8 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     b.tri.upload(s.tri, stream);
     b.tri_edges.upload(s.tri_edges, stream);
     b.edges.upload(s.edges, stream);
-    std::vector<uint4> sorted(ntris_);
-    for (int q = 0; q < ntris_; ++q) sorted[q] = s.tri[s.order[q]];
-    b.stri.upload(sorted, stream);
-    b.order.upload(s.order, stream);
+    if (!once) b.host_tri = s.tri;
+    upload_order(s.tri, s.order);
     size_t nodes = 0;
     for (int l = 0; l < kMaxLevels; ++l) {
         b.cnt[l] = l == 0 ? ntris_ : (b.cnt[l - 1] + 31) / 32;
@@ -911,8 +923,8 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
     while (b.cnt[b.top] > 32) ++b.top;
     b.lo.alloc(std::max<size_t>(nodes, 1));
     b.hi.alloc(std::max<size_t>(nodes, 1));
-    b.counters.alloc(3);
-    if (!once) PDGB_CUDA_TRY(cudaMallocHost(&b.pinned, 3 * sizeof(unsigned int)));
+    b.counters.alloc(kCounters);
+    if (!once) PDGB_CUDA_TRY(cudaMallocHost(&b.pinned, kCounters * sizeof(unsigned int)));
     b.counts = b.pinned ? b.pinned : b.pageable;
     const size_t n = (size_t)std::max(ntris_, 1);
     b.groups.least = std::max(16 * b.cnt[1], 256);
@@ -936,6 +948,44 @@ CcdContext::CcdContext(const CcdSurface& s, const int* vcaller, cudaStream_t str
 }
 
 CcdContext::~CcdContext() = default;
+
+void CcdContext::upload_order(const std::vector<uint4>& tri, const std::vector<int>& order) {
+    std::vector<uint4> sorted(ntris_);
+    for (int q = 0; q < ntris_; ++q) sorted[q] = tri[order[q]];
+    b_->stri.upload(sorted, stream_);
+    b_->order.upload(order, stream_);
+    PDGB_CUDA_TRY(cudaStreamSynchronize(stream_));
+}
+
+// The order is as good as the positions that it was made at.  A detection counts
+// what it costs: the steps down the tree and the pairs of groups, some 5 to 60 a
+// group where bodies touch or fly about.  Where it is more, and this is the first
+// detection, or four times what it was when the order was last made, or some time
+// after that, the triangles are ordered anew where they are now.  2,000 bodies of
+// 5^3 cells that all had one place when the surface was set and were then put
+// into theirs took 250 ms a step, 0.75 from the second on this way.
+constexpr double kPoorWork = 64.0;
+constexpr int kOrderAge = 1000;
+
+void CcdContext::keep_order(const float4* x) {
+    Buffers& b = *b_;
+    if (b.host_tri.empty() || b.top < 2) return;  // up to 32 groups are one step
+    const double work = (double)b.counts[3] + 4.0 * b.counts[1];
+    if (b.base < 0.0) b.base = work;  // the first in this order
+    ++b.age;
+    if (work < kPoorWork * b.cnt[1] || (work < 4.0 * b.base && b.age < kOrderAge)) return;
+    try {
+        std::vector<float4> h(nv_);
+        PDGB_CUDA_TRY(cudaMemcpyAsync(h.data(), x, (size_t)nv_ * sizeof(float4), cudaMemcpyDeviceToHost, stream_));
+        PDGB_CUDA_TRY(cudaStreamSynchronize(stream_));
+        std::vector<int> order;
+        tree_order(b.host_tri, h.data(), true, order);
+        upload_order(b.host_tri, order);
+    } catch (const std::bad_alloc&) {  // the present order is as right
+    }
+    b.base = -1.0;
+    b.age = 0;
+}
 
 const float* CcdContext::tI() const { return b_->tI.p; }
 const float4* CcdContext::normals() const { return b_->nrm.p; }
@@ -969,7 +1019,7 @@ void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* re
     d.ee_n = b.ee_n.p;
     d.tI = b.tI.p;
     d.nrm = b.nrm.p;
-    const int most = std::max({nv_, nedges_, ntris_, 3});
+    const int most = std::max({nv_, nedges_, ntris_, kCounters});
     const int outs = blocks_for(std::max(nv_, nedges_));
     // The lists grow to the counts found and the detection runs again: the count
     // of pairs is whole once the list of groups is.
@@ -994,7 +1044,7 @@ void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* re
         if (response)
             launch_pdl(k_respond, blocks_for(nv_), kThreads, 0, s, d, nv_, b.tI.p, b.nrm.p, response->x, xt, response->v,
                        response->sc);
-        PDGB_CUDA_TRY(cudaMemcpyAsync(b.counts, b.counters.p, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+        PDGB_CUDA_TRY(cudaMemcpyAsync(b.counts, b.counters.p, kCounters * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
         PDGB_CUDA_TRY(cudaStreamSynchronize(s));
         const bool groups = b.counts[1] > (unsigned)b.groups.cap, pairs = b.counts[0] > (unsigned)b.pairs.cap;
         if (!groups && !pairs) break;
@@ -1012,6 +1062,7 @@ void CcdContext::detect(const float4* x, const float4* xt, const CcdResponse* re
     stats_.pairs = b.counts[0];
     stats_.marked = (int)b.counts[2];
     stats_.ms = ms;
+    if (ntris_ >= 2) keep_order(x);
 }
 
 }  // namespace pdgb

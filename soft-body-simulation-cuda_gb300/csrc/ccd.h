@@ -28,10 +28,11 @@ struct CcdSurface {
 };
 
 // tris: [3 ntris] caller vertex ids; tri_body: [ntris]; viperm: caller ->
-// internal vertex (null: identity); X: [3 nv] finite positions, caller order,
-// that the triangles' tree order follows.  Throws Error on bad input.
+// internal vertex (null: identity); x: [nv] positions, internal order, that the
+// triangles' tree order follows; now: those of the detection to come.  Throws Error
+// on bad input.
 CcdSurface build_ccd_surface(int nv, int ntris, const uint32_t* tris, const int* tri_body, const int* viperm,
-                             const float* X);
+                             const float4* x, bool now);
 
 // A device list that grows, and the capacity its kernels get: never more than it
 // holds, also after an allocation that failed (which leaves no list).
@@ -87,6 +88,9 @@ public:
     int nv() const { return nv_; }
 
 private:
+    void upload_order(const std::vector<uint4>& tri, const std::vector<int>& order);
+    void keep_order(const float4* x);
+
     struct Buffers;
     std::unique_ptr<Buffers> b_;
     int nv_ = 0, ntris_ = 0, nedges_ = 0;

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from pdgb import ccd_detect
+from pdgb import PdSolver, SolverParams, ccd_detect, mesh, meshio
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,28 @@ def _check(args):
 def test_mixed_and_separate_bodies(n, bodies, room, flat, apart):
     _check(_soup(n, bodies, room, flat, apart))
 
+
+
+def test_bodies_that_leave_the_places_they_were_ordered_at():
+    """150 bodies in one place when the surface is set, then scattered, then thrown:
+    the tree is ordered anew on the way, and every step's candidates and times are
+    the CPU query's."""
+    rng = np.random.default_rng(5)
+    g = mesh.make_grid_body(2, 2, 2, young=1e5, pin=None)
+    n, nv = 150, g.num_verts
+    t = meshio.surface_triangles(g.tets)
+    tris = (t[None] + (np.arange(n) * nv)[:, None, None]).reshape(-1, 3).astype(np.uint32)
+    body = np.repeat(np.arange(n, dtype=np.int32), len(t))
+    X = (g.X[None] + rng.uniform(-3.0, 3.0, (n, 1, 3))).reshape(-1, 3).astype(np.float32)
+    V = np.repeat(rng.normal(size=(n, 3)) * 20.0, nv, 0).astype(np.float32)
+    with PdSolver([g] * n, SolverParams(num_iterations=4, solver=0)) as e:
+        e.set_collision_surface(tris, body)
+        e.enable_collision()
+        e.upload_state(X, V)
+        for _ in range(5):
+            X, _ = e.download_state()
+            e.update(1)
+            tI, _, info = e.collision()
+            tIo, _, (pairs, _, marked) = O.ccd_detect(tris, body, X, e.download_xtilde())
+            assert info["candidate_pairs"] == pairs and info["vertices_hit"] == marked
+            assert np.array_equal(tI, tIo)
