@@ -442,15 +442,19 @@ std::vector<int> amalgamate(const std::vector<int>& fk, const std::vector<int>& 
     std::vector<int> root(nf), best_root(nf), band(n + 1), height(nf);
     std::vector<int64_t> cols(nf);
     double best = -1.0;
-    for (int t : {8, 16, 24, 32, 48, 96, 192, 1024})
+    // least: also no merging at all (t = 0, a band for every size), which is what
+    // stores least where the tree is one long chain
+    const bool least = price.kind == SolveKind::kLeast;
+    for (int t : {0, 8, 16, 24, 32, 48, 96, 192, 1024})
         for (double r : {2.0, 3.0, 4.0, 6.0, 10.0, 16.0, 32.0}) {
+            if (t == 0 && !(least && r == 2.0)) continue;
             double top = t;
             for (int c = 0, q = 0; c <= n; ++c) {
-                while ((double)c > top) {
+                while (t > 0 && (double)c > top) {
                     top *= r;
                     ++q;
                 }
-                band[c] = q;
+                band[c] = t > 0 ? q : c;
             }
             std::fill(cols.begin(), cols.end(), 0);
             std::fill(height.begin(), height.end(), 0);

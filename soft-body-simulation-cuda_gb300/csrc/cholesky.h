@@ -210,6 +210,7 @@ enum class SolveKind {
               // entries, however small their share of a level
     kCta,     // one CTA a body: a level is a CTA's barrier
     kDsm,     // one cluster, and every stored entry takes its shared memory
+    kLeast,   // as few stored entries as there are
 };
 // Entries that a level costs.  Launches: about 6 us of dependent ones, forward and
 // backward, against 8 bytes an entry at some 5 TB/s.  Batches pay it by size,
