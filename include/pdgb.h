@@ -630,9 +630,14 @@ int pdgb_render_surface(pdgb_engine* e, const uint32_t* tris, int num_tris, floa
  *   - The first call on a device looks up the scratch's device address for
  *     that device.  The address is kept until the process exits: a
  *     cudaDeviceReset between calls is not supported.
- *   - The call waits for its stream twice: after the mesh check and before
- *     returning.  So no call can be captured into a CUDA graph: call it on
- *     a stream that is not capturing. */
+ *   - The call waits for its stream once, before returning.  So no call can
+ *     be captured into a CUDA graph: call it on a stream that is not
+ *     capturing.
+ *   - The steps run in one launch whose thread blocks wait for one another,
+ *     each wait for a few seconds at most.  Where one runs out (calls that
+ *     overlap, against the rule above) the call returns PDGB_ERR_TIMEOUT, and
+ *     X and V are lost: some vertices hold a later state than others.  Upload
+ *     them anew; the next call starts from a cleared scratch. */
 typedef struct pdgb_noalloc_mesh {
     int num_verts;
     int num_tets;
@@ -644,6 +649,13 @@ typedef struct pdgb_noalloc_mesh {
 } pdgb_noalloc_mesh;
 int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_params* params, float* X, float* V, int nsteps,
                       void* stream);
+
+/* pdgb_step_noalloc with at most max_ctas thread blocks (0: no such limit), each
+ * wait for `missing` more arrivals than there are blocks (> 0: it can only run
+ * out) and for spin_limit polls: for checking the forms for small GPUs and the
+ * bounded wait. */
+int pdgb_noalloc_check(const pdgb_noalloc_mesh* mesh, const pdgb_params* params, float* X, float* V, int nsteps,
+                       void* stream, int max_ctas, int missing, int spin_limit);
 
 /* The local step's rotation on n row-major 3x3 matrices F (host arrays,
  * 9 floats each): R = the closest proper rotation as the engine computes it

@@ -26,8 +26,8 @@
 //     (cudaGetSymbolAddress) once for that device.  The address is kept for
 //     the life of the process, so a cudaDeviceReset between calls is not
 //     supported;
-//   - every call waits for its stream before it returns, so no call can be
-//     captured into a CUDA graph;
+//   - every call waits for its stream once, before it returns, so no call can
+//     be captured into a CUDA graph;
 //   - the mesh is checked on the device (tet indices, rest volumes, weights)
 //     before any step: a bad mesh returns PDGB_ERR_BAD_MESH with X and V
 //     untouched.
@@ -159,10 +159,14 @@ __global__ void na_tets(int nv, int nt, const uint32_t* __restrict__ tets, const
 }
 
 // Grid barrier of a cooperative launch: the n-th barrier is passed once
-// n gridDim.x CTAs have arrived.  A wait is bounded (some seconds); past it
-// the timeout word ends every CTA at its next barrier.
+// n gridDim.x CTAs have arrived.  A wait is bounded (kNaSpins: some seconds);
+// past it the timeout word ends every CTA at its next barrier.  A check makes it
+// wait for `missing` more arrivals than there are CTAs.
 constexpr unsigned kNaSpins = 1u << 22;
-__device__ __forceinline__ bool na_barrier(NaFlags* f, unsigned& target) {
+struct NaWait {
+    unsigned spins, missing;
+};
+__device__ __forceinline__ bool na_barrier(NaFlags* f, unsigned& target, const NaWait& w) {
     __shared__ int ok;
     __syncthreads();
     target += gridDim.x;
@@ -171,10 +175,10 @@ __device__ __forceinline__ bool na_barrier(NaFlags* f, unsigned& target) {
         // acquired before those after the one below
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&f->arrived) : "memory");
         bool there = false;
-        for (unsigned n = 0; n < kNaSpins && !there; ++n) {
+        for (unsigned n = 0; n < w.spins && !there; ++n) {
             unsigned seen;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&f->arrived) : "memory");
-            there = (int)(seen - target) >= 0;  // the count may wrap
+            there = (int)(seen - target - w.missing) >= 0;  // the count may wrap
             if (n % 1024 == 1023 && *reinterpret_cast<volatile int*>(&f->timeout)) break;
         }
         if (!there) atomicExch(&f->timeout, 1);
@@ -229,6 +233,7 @@ __device__ __forceinline__ void na_local(const NaTet& q, const NaScratch& s) {
 struct NaParams {
     float dt, dt_inv, gravity, pw, wpin, rho;
     int iters, steps;
+    NaWait wait;
 };
 
 // One vertex: its mass terms, pin right-hand side, state and iterates.
@@ -303,8 +308,8 @@ __device__ __forceinline__ float na_omega(float omega, int iter, float rho) {
 // Every step of the call.  A thread owns one tet, whose geometry stays in its
 // registers, and one vertex, whose state and iterates do: what goes through L2
 // is the iterate (published, gathered by the tets) and the sums b.  With fewer
-// threads than tets or vertices (kOwn false) they are walked in strides, the
-// vertex data in the scratch and X, V.
+// threads than tets or vertices (kOwn false: 1,024 a CTA on fewer than 128 SMs)
+// they are walked in strides, the vertex data in the scratch and X, V.
 template <bool kOwn, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1)
     na_run(int nv, int nt, const uint32_t* __restrict__ tets, const float* __restrict__ X0,
@@ -321,10 +326,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (g < nv) na_begin(q, p, s, g);
             float omega = 1.f;
             for (int i = 0; i < p.iters; ++i) {
-                if (!na_barrier(s.flags, target)) return;
+                if (!na_barrier(s.flags, target, p.wait)) return;
                 if (g < nt) na_local(tet, s);
                 omega = na_omega(omega, i, p.rho);
-                if (!na_barrier(s.flags, target)) return;
+                if (!na_barrier(s.flags, target, p.wait)) return;
                 if (g < nv) na_update(q, omega, i, p, s, g);
             }
         }
@@ -343,10 +348,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         float omega = 1.f;
         for (int it = 0; it < p.iters; ++it) {
-            if (!na_barrier(s.flags, target)) return;
+            if (!na_barrier(s.flags, target, p.wait)) return;
             for (int t = g; t < nt; t += all) na_local(na_tet(tets, s, t), s);
             omega = na_omega(omega, it, p.rho);
-            if (!na_barrier(s.flags, target)) return;
+            if (!na_barrier(s.flags, target, p.wait)) return;
             for (int i = g; i < nv; i += all) {
                 NaVertex q = na_vertex(X0, mass, dbc, X, V, p, s, i);
                 const float4 sn = s.sn[i], pr = s.prev[i], ba = s.base[i];
@@ -378,8 +383,10 @@ unsigned char* g_na_ptr[kNaMaxDevices] = {};
 
 using namespace pdgb;
 
-extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_params* p, float* X, float* V,
-                                 int nsteps, void* stream) {
+namespace {
+// max_ctas: most CTAs of the launch (0: as many as the SMs).
+int step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_params* p, float* X, float* V, int nsteps, void* stream,
+                 int max_ctas, NaWait wait) {
     if (!mesh || !p || !X || !V || !mesh->tets || !mesh->X0 || !mesh->mass || !mesh->mu || nsteps < 0)
         return PDGB_ERR_INVALID_ARGUMENT;
     if (mesh->num_verts <= 0 || mesh->num_tets <= 0) return PDGB_ERR_INVALID_ARGUMENT;
@@ -404,17 +411,19 @@ extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_param
     na_tets<<<(nt + 255) / 256, 256, 0, st>>>(nv, nt, mesh->tets, mesh->X0, mesh->mu, s);
     if (cudaGetLastError() != cudaSuccess) return PDGB_ERR_CUDA;
     if (nsteps > 0) {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PDGB_ERR_CUDA;
-        const int n = nv > nt ? nv : nt, threads = na_threads(n, sms);
-        const int want = (n + threads - 1) / threads, grid = want < sms ? want : sms;
-        const bool own = (long long)grid * threads >= n;
-        const auto kernel = threads == 256 ? (own ? na_run<true, 256> : na_run<false, 256>)
-                            : threads == 512 ? (own ? na_run<true, 512> : na_run<false, 512>)
-                                             : (own ? na_run<true, 1024> : na_run<false, 1024>);
+        int most = 0;
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return PDGB_ERR_CUDA;
+        if (max_ctas > 0 && max_ctas < most) most = max_ctas;
+        const int n = nv > nt ? nv : nt, threads = na_threads(n, most);
+        const int want = (n + threads - 1) / threads, grid = want < most ? want : most;
+        const bool own = grid == want;  // else 1,024 threads
+        const auto kernel = !own ? na_run<false, 1024>
+                            : threads == 256 ? na_run<true, 256>
+                            : threads == 512 ? na_run<true, 512>
+                                             : na_run<true, 1024>;
         const float dt_inv = 1.0f / p->dt;
         NaParams np{p->dt, dt_inv, p->gravity, p->positional_weight, p->positional_weight * (dt_inv * dt_inv),
-                    p->rho, p->num_iterations, 0};
+                    p->rho, p->num_iterations, 0, wait};
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)grid);
         cfg.blockDim = dim3((unsigned)threads);
@@ -424,10 +433,10 @@ extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_param
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const int most = p->num_iterations >= kNaLaunchIters ? 1 : kNaLaunchIters / p->num_iterations;
+        const int at_once = p->num_iterations >= kNaLaunchIters ? 1 : kNaLaunchIters / p->num_iterations;
         unsigned arrived = 0;
         for (int done = 0; done < nsteps; done += np.steps) {
-            np.steps = nsteps - done < most ? nsteps - done : most;
+            np.steps = nsteps - done < at_once ? nsteps - done : at_once;
             if (cudaLaunchKernelEx(&cfg, kernel, nv, nt, mesh->tets, mesh->X0, mesh->mass, mesh->dbc, np, X, V, s,
                                    arrived) != cudaSuccess)
                 return PDGB_ERR_CUDA;
@@ -440,4 +449,16 @@ extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_param
     if (flags.bad) return PDGB_ERR_BAD_MESH;
     if (flags.timeout) return PDGB_ERR_TIMEOUT;
     return PDGB_OK;
+}
+}  // namespace
+
+extern "C" int pdgb_step_noalloc(const pdgb_noalloc_mesh* mesh, const pdgb_params* p, float* X, float* V, int nsteps,
+                                 void* stream) {
+    return step_noalloc(mesh, p, X, V, nsteps, stream, 0, NaWait{kNaSpins, 0u});
+}
+
+extern "C" int pdgb_noalloc_check(const pdgb_noalloc_mesh* mesh, const pdgb_params* p, float* X, float* V, int nsteps,
+                                  void* stream, int max_ctas, int missing, int spin_limit) {
+    if (max_ctas < 0 || missing < 0 || spin_limit < 1) return PDGB_ERR_INVALID_ARGUMENT;
+    return step_noalloc(mesh, p, X, V, nsteps, stream, max_ctas, NaWait{(unsigned)spin_limit, (unsigned)missing});
 }

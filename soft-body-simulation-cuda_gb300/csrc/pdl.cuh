@@ -24,7 +24,6 @@ namespace pdgb {
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // An SM changes its split between L1 and shared memory only when it is idle, so
 // a kernel that wants another split than its predecessor cannot start beside

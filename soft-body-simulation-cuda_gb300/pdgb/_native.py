@@ -277,6 +277,8 @@ SIGNATURES = {
     "pdgb_get_local_kernel": (C.c_int, [C.c_void_p, C.c_void_p]),
     "pdgb_host_factor_check": (C.c_int, [C.POINTER(pdgb_mesh_desc), C.POINTER(pdgb_params), C.c_int, C.c_void_p,
                                          C.c_void_p, C.POINTER(pdgb_factor_info)]),
+    "pdgb_noalloc_check": (C.c_int, [C.POINTER(pdgb_noalloc_mesh), C.POINTER(pdgb_params), C.c_void_p, C.c_void_p,
+                                     C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int]),
     "pdgb_step_noalloc": (C.c_int, [C.POINTER(pdgb_noalloc_mesh), C.POINTER(pdgb_params), C.c_void_p, C.c_void_p,
                                     C.c_int, C.c_void_p]),
     "pdgb_server_default_config": (None, [C.POINTER(pdgb_server_config)]),
