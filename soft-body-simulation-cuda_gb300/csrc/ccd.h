@@ -53,10 +53,9 @@ struct CcdList {
 
 struct CcdStats {
     long long pairs = 0;        // candidate triangle pairs of the last detection
-    long long sources = 0;      // vertices / edges whose earliest contact is before t = 1
     int marked = 0;             // vertices with tI < 1
     int regrows = 0;            // candidate buffer enlargements so far
-    double ms = 0.0;            // device time of the last detection + response
+    double ms = 0.0;            // device time of the last detection
 };
 
 // CCDKernel + the fixed-body correction of XTilde and v (the reference
