@@ -353,7 +353,8 @@ int pdgb_set_local_kernel(pdgb_engine* e, int kind);
 int pdgb_get_local_kernel(pdgb_engine* e, int* kind);
 
 /* Schedule of the Cholesky solve.  CTA: one CTA per body walks the body's
- * whole elimination tree (levels separated by block barriers); CLUSTER: one
+ * whole elimination tree (levels separated by block barriers; it has a factor
+ * of its own, with more levels than the other schedules'); CLUSTER: one
  * cluster of 8 CTAs per body (cluster barriers); LEVELS: one launch per
  * level and direction over the whole GPU, level L of every body of a batch
  * in the same launch (levels counted from the leaves); DSM: a single body
@@ -384,16 +385,16 @@ int pdgb_get_solve_mode(pdgb_engine* e, int* mode);
  * changed).  For benchmarking the local step alone.  Waits for the GPU. */
 int pdgb_time_local(pdgb_engine* e, int launches, double* ms_per_launch);
 
-/* Tiles of the local step: at most max_tets tets each (32..512; 0 = 512).
+/* Tiles of the local step: at most max_tets tets each (32..512; 0 = 512).  A
+ * new engine has 128 up to 20,000 tets, 256 up to 110,000 and 512 past that.
  * Smaller tiles give small meshes more CTAs; vertex and tet order are
  * unchanged, so the state carries over.  Takes effect at the next step. */
 int pdgb_set_tile_size(pdgb_engine* e, int max_tets);
 
 /* Autotuner: times `steps` steps (after one warm-up step) of every
  * candidate configuration on the engine's own mesh -- tile sizes 512, 256,
- * 128, 64 and, on the Cholesky path, the solve schedules CTA and CLUSTER
- * (and LEVELS for a single system) -- keeps the fastest and leaves the
- * engine prepared with it.  The simulation state is restored after every
+ * 128, 64 and, on the Cholesky path, the solve schedules CTA, CLUSTER, LEVELS
+ * and PERSISTENT -- keeps the fastest and leaves the engine prepared with it.  The simulation state is restored after every
  * trial, so tuning does not advance the simulation.  Waits for the GPU. */
 typedef struct pdgb_tune_report {
     int tile_tets;       /* chosen most tets per tile                        */
@@ -527,7 +528,10 @@ int pdgb_download_xtilde(pdgb_engine* e, float* XT, int memory);
  * Triangles are caller vertex ids (3 per triangle); tri_body gives each
  * triangle's body (NULL: the body of its first vertex, from the engine's
  * body ranges).  Detection waits for the stream once per step: the
- * counts decide whether its lists were long enough. */
+ * counts decide whether its lists were long enough.  Its tree of boxes is
+ * ordered by the positions at the call of pdgb_set_collision_surface, and anew
+ * (a copy of the positions to the host and a sort) in a step whose detection
+ * found it poor. */
 typedef struct pdgb_collision_info {
     long long candidate_pairs;  /* triangle pairs tested by the last detection */
     int vertices_hit;           /* vertices with tI < 1 after it               */

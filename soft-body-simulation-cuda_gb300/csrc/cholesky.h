@@ -1,11 +1,12 @@
-// Sparse Cholesky of the scalar PD system K (host side).
+// Sparse Cholesky of the scalar PD system K: ordering, symbolic analysis and the
+// host's numeric factorisation.
 //
 // The reference assembles A = K (x) I_3 (3n x 3n) from per-tet triplets
 // (pdUtil.cu:9-54), orders it with cuSOLVER's host AMD and factors it in
 // FP32 with cuSOLVER's low-level sparse Cholesky (cholesky.cu:72-158).  The
-// engine factors the n x n scalar K once, in FP64 on the host (approximate
-// minimum degree ordering, supernodal multifrontal LL^T), and solves the
-// three coordinates together on the GPU.
+// engine orders the n x n scalar K on the host (approximate minimum degree),
+// factors it once in FP64, on the GPU (factor.cu) or on the host (supernodal
+// multifrontal LL^T both), and solves the three coordinates together on the GPU.
 //
 // Solve representation.  For every supernode s with pivot columns C_s
 // (k_s of them) and off-diagonal rows O_s (m_s - k_s), the GPU stores the
@@ -214,7 +215,10 @@ enum class SolveKind {
 };
 // Entries that a level costs.  Launches: about 6 us of dependent ones, forward and
 // backward, against 8 bytes an entry at some 5 TB/s.  Batches pay it by size,
-// requests of a server 1 / kServerBodies.  For one CTA a barrier is less and an
+// requests of a server 1 / kServerBodies (40 uneven requests of 4 to 19 cells take
+// 151, 126 and 112 ms at 4, 16 and 64, 8 of 28^3 323, 307 and 305, one of 28^3 128,
+// 134 and 133, one of 10^3 64, 64 and 73, twelve of 1 k to 100 k tets 72, 70 and 71).
+// For one CTA a barrier is less and an
 // entry more: ten iterations of a 13^3 body, of a 60 x 6 x 3 one and of 16 of 2^3
 // beside 32 of 10^3 take 1,715, 1,044 and 1,096 us at 1e4 and 2,297, 1,179 and
 // 1,202 with the tree for launches.

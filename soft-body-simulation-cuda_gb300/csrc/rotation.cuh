@@ -251,7 +251,9 @@ __device__ __forceinline__ void closest_rotation_horn(const float F[9], float f2
 // largest root of N's characteristic quartic
 //   p(l) = l^4 - 2 f l^2 - 8 d l + 2 |C|^2 - f^2
 // with C = F^T F, f = tr C, d = det F.  Differentiating p(l(F), F) = 0:
-//   R = ((l^2 + f) F + 2 l cof F - 2 F C) / (l^3 - f l - 2 d).
+//   R = ((l^2 + f) F + 2 l cof F - 2 F C) / (l^3 - f l - 2 d),
+// as in Lin, Chitalu and Komura, "Isotropic ARAP Energy Using Cauchy-Green
+// Invariants" (ACM Trans. Graph. 41(6), 2022).
 // Newton starts at sqrt(3 f) less its second-order distance from l: two steps up
 // to strains of 20 %, more where the second was not small.  c, K: C's diagonal
 // and the first row of cof F; root = f^0.5.
