@@ -965,7 +965,7 @@ void CcdContext::upload_order(const std::vector<uint4>& tri, const std::vector<i
 // 5^3 cells that all had one place when the surface was set and were then put
 // into theirs took 250 ms a step, 0.75 from the second on this way.
 constexpr double kPoorWork = 64.0;
-constexpr int kOrderAge = 1000;
+constexpr int kOrderAge = 1000, kOrderRest = 16;
 
 void CcdContext::keep_order(const float4* x) {
     Buffers& b = *b_;
@@ -973,7 +973,10 @@ void CcdContext::keep_order(const float4* x) {
     const double work = (double)b.counts[3] + 4.0 * b.counts[1];
     if (b.base < 0.0) b.base = work;  // the first in this order
     ++b.age;
-    if (work < kPoorWork * b.cnt[1] || (work < 4.0 * b.base && b.age < kOrderAge)) return;
+    if (work < kPoorWork * b.cnt[1]) return;
+    // not every other step where two kinds of steps take turns
+    const bool grown = work >= 4.0 * b.base && (b.base == 0.0 || b.age >= kOrderRest);
+    if (!grown && b.age < kOrderAge) return;
     try {
         std::vector<float4> h(nv_);
         PDGB_CUDA_TRY(cudaMemcpyAsync(h.data(), x, (size_t)nv_ * sizeof(float4), cudaMemcpyDeviceToHost, stream_));
